@@ -7,11 +7,12 @@
 //   w -= alpha_k v_k + beta_{k-1} v_{k-1}      (+ CGS2 against V when nev > 1)
 //   beta_k = ||w||, v_{k+1} = w / beta_k
 // The step index lives in device memory, so one CUDA graph holding `check`
-// steps is replayed for the whole run. Every `check` steps a one-block kernel
-// solves the tridiagonal T_k for its lowest eigenpair(s) on the device
-// (Rayleigh-quotient iteration seeded with the previous Ritz vector and
-// certified by a division-free positive-definiteness test of T - (theta -
-// delta) I; Sturm multisection otherwise) and flags convergence when
+// steps is replayed for the whole run; the sums (alpha, beta) are finished by
+// the last block of the kernel that forms them, so a step is three kernels.
+// Every `check` steps the host solves the tridiagonal T_k for its lowest
+// eigenpair(s) while the next replay runs (Rayleigh-quotient iteration seeded
+// with the previous Ritz vector and certified by a Sturm count; Sturm
+// multisection and inverse iteration otherwise) and ends the cycle when
 // beta_k |s_k| <= tol / 2. The Ritz vector psi = V s is then formed in one
 // pass and its true residual ||H psi - E psi|| recomputed in FP64; the run
 // restarts from psi until that residual meets the tolerance.
@@ -25,6 +26,7 @@
 #include <cstring>
 
 #include "operator_impl.cuh"
+#include "tridiagonal.hpp"
 
 namespace sed {
 namespace {
@@ -33,21 +35,22 @@ constexpr unsigned kMaxNev = 16;
 constexpr unsigned kRedThreads = 1024;
 constexpr unsigned kVecBlocks = 152 * 8;  // grid of the vector kernels
 
+// What the step kernels share in device memory. alpha and beta follow it in
+// the same buffer (state_bytes), so that one copy per chunk of steps shows
+// the host all it needs.
 struct LzHeader {
   uint32_t k;       // newest normalised Krylov vector
-  uint32_t stop;    // 0 running, 1 converged, 2 storage full, 3 breakdown
+  uint32_t stop;    // kRunning, kFull or kBreakdown
   uint32_t m_max;   // stored vectors
-  uint32_t check;   // convergence check period
-  uint32_t nev;
-  uint32_t size;    // order of T at the last solve
+  uint32_t size;    // order of T so far
   uint32_t steps;   // Lanczos steps taken
-  uint32_t have_s;  // previous Ritz vector of T available
-  uint32_t reorth;  // CGS2 against all stored vectors
-  uint32_t fallbacks;
-  double tol_est;
-  double theta[kMaxNev];
-  double est[kMaxNev];
+  uint32_t pad[11];
 };
+static_assert(sizeof(LzHeader) == 64, "alpha starts on a 64-byte boundary");
+
+enum : uint32_t { kRunning = 0, kConverged = 1, kFull = 2, kBreakdown = 3 };
+
+size_t state_bytes(uint32_t m) { return sizeof(LzHeader) + (size_t)m * 16; }
 
 // ------------------------------------------------------------ vector ops --
 
@@ -60,36 +63,62 @@ __device__ __forceinline__ double norm2(X const* p, uint64_t i) {
   return dot_re(v, v);
 }
 
-// Sums n partials into out (mode 0: alpha[k] = s; mode 1: beta[k] = sqrt(s)).
-__global__ void k_reduce(double const* __restrict__ partial, unsigned n, LzHeader* h,
-                         double* __restrict__ arr, int mode) {
-  __shared__ double red[kRedThreads / 32];
-  if (h->stop) return;
-  // eight independent sums per thread keep eight loads in flight (the
-  // partials of a one-row-per-thread SpMV number D / 256); fixed order
+// The sum of the matvec's partials where its grid is too large to finish it
+// (finish_sum): ind.sum[k]. Virtual thread t of 1024 adds partials t, t +
+// 1024, ... in eight running sums; then a butterfly per warp, and the 32
+// warps in order by the last block to finish. One warp per block: on one SM
+// the 61 738 FP64 additions of a 15.8 M-row SpMV take 17 us of its FP64 pipe
+// alone (30 us in all as one block of 1024 threads), on 32 SMs 4 us.
+__global__ void __launch_bounds__(32) k_sum_partials(unsigned n, Indirect ind, double* warp_sum, uint32_t* done) {
+  if (*ind.stop) return;
+  double const* partial = ind.partial;
   double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  unsigned i = threadIdx.x;
-  for (; i + 7 * blockDim.x < n; i += 8 * blockDim.x)
+  unsigned i = blockIdx.x * 32 + threadIdx.x;
+  for (; i + 31 * 1024 < n; i += 32 * 1024) {
+    double v[32];
 #pragma unroll
-    for (unsigned q = 0; q < 8; ++q) a[q] += partial[i + q * blockDim.x];
-  for (; i < n; i += blockDim.x) a[0] += partial[i];
+    for (unsigned q = 0; q < 32; ++q) v[q] = partial[i + q * 1024];
+#pragma unroll
+    for (unsigned q = 0; q < 32; ++q) a[q & 7] += v[q];
+  }
+  for (; i + 7 * 1024 < n; i += 8 * 1024) {
+    double v[8];
+#pragma unroll
+    for (unsigned q = 0; q < 8; ++q) v[q] = partial[i + q * 1024];
+#pragma unroll
+    for (unsigned q = 0; q < 8; ++q) a[q] += v[q];
+  }
+  for (; i < n; i += 1024) a[0] += partial[i];
   double s = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
-  s = block_sum(s, red);
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  uint32_t last = 0;
   if (threadIdx.x == 0) {
-    uint32_t const k = h->k;
-    if (mode == 0) {
-      arr[k] += s;  // alpha[k] (zeroed before the SpMV)
-    } else {
-      arr[k] = sqrt(s);
-    }
+    warp_sum[blockIdx.x] = s;
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  if (!__shfl_sync(0xffffffffu, last, 0)) return;
+  __threadfence();
+  double const mine = __ldcg(warp_sum + threadIdx.x);
+  s = 0.0;
+  for (int w = 0; w < 32; ++w) s += __shfl_sync(0xffffffffu, mine, w);
+  if (threadIdx.x == 0) {
+    *done = 0;
+    ind.sum[*ind.k] = s;
+    if (ind.clear) *ind.clear = 0;
   }
 }
 
-template <class X>
-__global__ void k_zero_alpha(LzHeader const* h, double* alpha, unsigned long long* wmax) {
-  if (h->stop) return;
-  alpha[h->k] = 0.0;
-  if (wmax) *wmax = 0;  // fused fixed-point step: k_update's max |w| starts here
+// One Krylov matvec with alpha_k; ind.partial holds ceil(D / kBlock) + 32
+// doubles.
+template <class Apply>
+int apply_with_alpha(Indirect ind, uint64_t D, cudaStream_t stream, Apply&& apply) {
+  uint64_t const blocks = (D + kBlock - 1) / kBlock;
+  uint32_t* const done = ind.done;
+  if (blocks > kFusedSumBlocks) ind.done = nullptr;
+  if (int st = apply(ind)) return st;
+  if (!ind.done) { k_sum_partials<<<32, 32, 0, stream>>>((unsigned)blocks, ind, ind.partial + blocks, done); note_launches(1); }
+  return LS_SUCCESS;
 }
 
 // Fused fixed-point Lanczos step (FP64, one vector): k_update leaves max |w|
@@ -105,11 +134,12 @@ struct FixStep {
   FixView fv;
 };
 
-// w = w - alpha_k v_k - beta_{k-1} v_{k-1}; partial ||w||^2.
+// w = w - alpha_k v_k - beta_{k-1} v_{k-1}; beta_k = ||w|| (by the last block).
 template <class X>
 __global__ void k_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader const* h,
-                         double const* __restrict__ alpha, double const* __restrict__ beta,
-                         double* __restrict__ partial, unsigned long long* __restrict__ wmax) {
+                         double const* __restrict__ alpha, double* __restrict__ beta,
+                         double* __restrict__ partial, uint32_t* __restrict__ done,
+                         unsigned long long* __restrict__ wmax) {
   using Vt = typename Store<X>::V;
   __shared__ double red[kBlock / 32];
   __shared__ unsigned long long redm[kBlock / 32];
@@ -138,7 +168,6 @@ __global__ void k_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader 
       m = max(m, (unsigned long long)__double_as_longlong(wi) & 0x7FFFFFFFFFFFFFFFull);
   }
   double const tot = block_sum(part, red);
-  if (threadIdx.x == 0) partial[blockIdx.x] = tot;
   if (wmax) {
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) redm[threadIdx.x >> 5] = m;
@@ -148,6 +177,7 @@ __global__ void k_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader 
       atomicMax(wmax, m);
     }
   }
+  finish_sum(tot, partial, done, [&](double s) { beta[k] = sqrt(s); });
 }
 
 // Classical Gram-Schmidt pass against V[0..k]: c_j = <V_j, w> (partials per
@@ -209,10 +239,11 @@ __global__ void k_cgs_reduce(double const* __restrict__ partial, unsigned nb, Lz
   }
 }
 
-// w -= sum_j c_j V_j; partial ||w||^2.
+// w -= sum_j c_j V_j; beta_k = ||w||.
 template <class X>
 __global__ void k_cgs_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader const* h,
-                             double const* __restrict__ coef, double* __restrict__ partial) {
+                             double const* __restrict__ coef, double* __restrict__ beta,
+                             double* __restrict__ partial, uint32_t* __restrict__ done) {
   using Vt = typename Store<X>::V;
   __shared__ double red[kBlock / 32];
   __shared__ double c[2048];
@@ -238,17 +269,39 @@ __global__ void k_cgs_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHea
     part += dot_re(wi, wi);
   }
   double const tot = block_sum(part, red);
-  if (threadIdx.x == 0) partial[blockIdx.x] = tot;
+  finish_sum(tot, partial, done, [&](double t) { beta[k] = sqrt(t); });
 }
 
+// Ends the step: the last block to get here advances k, or stops the run
+// when the storage is full or the Krylov space is exhausted. Every block has
+// read the header before its thread 0 is counted.
+__device__ __forceinline__ void advance_step(LzHeader* h, double b, uint32_t* done) {
+  __syncthreads();
+  if (threadIdx.x != 0 || atomicAdd(done, 1u) != gridDim.x - 1) return;
+  *done = 0;
+  uint32_t const k = h->k;
+  h->size = k + 1;
+  h->steps += 1;
+  if (!(b > 0.0) || !isfinite(b))
+    h->stop = kBreakdown;
+  else if (k + 2 >= h->m_max)
+    h->stop = kFull;
+  else
+    h->k = k + 1;
+}
+
+// v_{k+1} = w / beta_k (and the next matvec's gather copy), then the next step.
 template <class X>
-__global__ void k_scale_next(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader const* h,
-                             double const* __restrict__ beta, FixStep fx) {
+__global__ void k_scale_next(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader* h,
+                             double const* __restrict__ beta, uint32_t* __restrict__ done, FixStep fx) {
   __shared__ double fac[kFixMaxClasses];
   if (h->stop) return;
   uint32_t const k = h->k;
   double const b = beta[k];
-  if (!(b > 0.0)) return;
+  if (!(b > 0.0)) {
+    advance_step(h, b, done);
+    return;
+  }
   double const inv = 1.0 / b;
   X* w = V + (uint64_t)(k + 1) * ld_v;
   if constexpr (std::is_same<X, double>::value) {
@@ -269,6 +322,7 @@ __global__ void k_scale_next(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHea
         w[i] = v;
         fx.u[i] = F == kFixBad ? 0 : fix_round((F1 ? v * p1 : v) * fac[fx.row_class[i]]);
       }
+      advance_step(h, b, done);
       return;
     }
   }
@@ -277,248 +331,7 @@ __global__ void k_scale_next(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHea
     auto v = Store<X>::load(w, i);
     Store<X>::store(w, i, mulv(inv, v));
   }
-}
-
-// ------------------------------------------------------- tridiagonal ----
-// T: diagonal a[0..n), off-diagonal b[0..n-1). All routines run in one thread
-// unless stated otherwise; work arrays hold 5 n doubles.
-
-// True iff T - x I is positive definite (all leading minors > 0), computed
-// without divisions by the three-term recurrence of the minors with exact
-// power-of-two rescaling.
-__device__ bool tri_pos_def(double const* a, double const* b, uint32_t n, double x) {
-  double p0 = 1.0, p1 = a[0] - x;
-  if (!(p1 > 0.0)) return false;
-  for (uint32_t i = 1; i < n; ++i) {
-    double const p2 = (a[i] - x) * p1 - b[i - 1] * b[i - 1] * p0;
-    if (!(p2 > 0.0)) return false;
-    p0 = p1;
-    p1 = p2;
-    if (p1 > 0x1p+400) {
-      p0 *= 0x1p-400;
-      p1 *= 0x1p-400;
-    } else if (p1 < 0x1p-400 && p0 < 0x1p-400) {
-      p0 *= 0x1p+400;
-      p1 *= 0x1p+400;
-    }
-  }
-  return true;
-}
-
-// Number of eigenvalues of T below x (Sturm count of negative pivots).
-__device__ uint32_t tri_count(double const* a, double const* b, uint32_t n, double x) {
-  uint32_t c = 0;
-  double d = a[0] - x;
-  if (d < 0.0) ++c;
-  for (uint32_t i = 1; i < n; ++i) {
-    if (d == 0.0) d = 1e-300;
-    d = (a[i] - x) - b[i - 1] * b[i - 1] / d;
-    if (d < 0.0) ++c;
-  }
-  return c;
-}
-
-// Solves (T - sigma I) z = r in place (r -> z) by Gaussian elimination with
-// partial pivoting on the tridiagonal (the dgttrf/dgtts2 scheme); exactly
-// singular pivots are perturbed.
-__device__ void tri_solve(double const* a, double const* b, uint32_t n, double sigma, double* r,
-                          double* dl, double* d, double* du, double* du2, uint8_t* piv) {
-  for (uint32_t i = 0; i < n; ++i) d[i] = a[i] - sigma;
-  for (uint32_t i = 0; i + 1 < n; ++i) {
-    dl[i] = b[i];
-    du[i] = b[i];
-  }
-  double const tiny = 1e-300;
-  for (uint32_t i = 0; i + 1 < n; ++i) {
-    if (i + 2 < n) du2[i] = 0.0;
-    if (fabs(d[i]) >= fabs(dl[i])) {
-      if (d[i] == 0.0) d[i] = tiny;
-      double const f = dl[i] / d[i];
-      dl[i] = f;
-      d[i + 1] -= f * du[i];
-      piv[i] = 0;
-    } else {
-      double const f = d[i] / dl[i];
-      d[i] = dl[i];
-      dl[i] = f;
-      double const t = du[i];
-      du[i] = d[i + 1];
-      d[i + 1] = t - f * d[i + 1];
-      if (i + 2 < n) {
-        du2[i] = du[i + 1];
-        du[i + 1] = -f * du[i + 1];
-      }
-      piv[i] = 1;
-    }
-  }
-  if (d[n - 1] == 0.0) d[n - 1] = tiny;
-  for (uint32_t i = 0; i + 1 < n; ++i) {
-    if (piv[i]) {
-      double const t = r[i];
-      r[i] = r[i + 1];
-      r[i + 1] = t - dl[i] * r[i];
-    } else {
-      r[i + 1] -= dl[i] * r[i];
-    }
-  }
-  r[n - 1] /= d[n - 1];
-  if (n > 1) r[n - 2] = (r[n - 2] - du[n - 2] * r[n - 1]) / d[n - 2];
-  for (int i = (int)n - 3; i >= 0; --i) r[i] = (r[i] - du[i] * r[i + 1] - du2[i] * r[i + 2]) / d[i];
-}
-
-__device__ double tri_rayleigh(double const* a, double const* b, uint32_t n, double const* s) {
-  double num = 0.0, den = 0.0;
-  for (uint32_t i = 0; i < n; ++i) {
-    double ts = a[i] * s[i];
-    if (i) ts += b[i - 1] * s[i - 1];
-    if (i + 1 < n) ts += b[i] * s[i + 1];
-    num += s[i] * ts;
-    den += s[i] * s[i];
-  }
-  return num / den;
-}
-
-__device__ void normalise(double* s, uint32_t n) {
-  double m = 0.0;
-  for (uint32_t i = 0; i < n; ++i) m += s[i] * s[i];
-  double const inv = 1.0 / sqrt(m);
-  for (uint32_t i = 0; i < n; ++i) s[i] *= inv;
-}
-
-// One block: lowest nev eigenpairs of T_n (n = k + 1) every `check` steps,
-// convergence flags, then k += 1.
-__global__ void k_tridiag(LzHeader* h, double const* __restrict__ alpha,
-                          double const* __restrict__ beta, double* __restrict__ S /* [nev][m_max] */,
-                          double* __restrict__ work) {
-  __shared__ double lohi[2];
-  __shared__ uint32_t sh_flag;
-  __shared__ double bounds[2];
-  if (h->stop) return;
-  uint32_t const k = h->k;
-  uint32_t const n = k + 1;
-  uint32_t const m_max = h->m_max;
-  double const bk = beta[k];
-  bool const full = k + 2 >= m_max;
-  double anorm = 0.0;
-  bool const breakdown = !(bk > 0.0) || !isfinite(bk);
-  bool const do_check = ((n % h->check) == 0) || full || breakdown;
-  if (!do_check) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      h->steps += 1;
-      h->k = k + 1;
-    }
-    return;
-  }
-  uint32_t const nev = min(h->nev, n);
-  double* dl = work;
-  double* d = work + m_max;
-  double* du = work + 2 * m_max;
-  double* du2 = work + 3 * m_max;
-  uint8_t* piv = reinterpret_cast<uint8_t*>(work + 4 * m_max);
-  // Gershgorin bounds.
-  if (threadIdx.x == 0) {
-    double lo = 1e300, hi = -1e300;
-    for (uint32_t i = 0; i < n; ++i) {
-      double r = (i ? fabs(beta[i - 1]) : 0.0) + (i + 1 < n ? fabs(beta[i]) : 0.0);
-      lo = fmin(lo, alpha[i] - r);
-      hi = fmax(hi, alpha[i] + r);
-    }
-    bounds[0] = lo;
-    bounds[1] = hi;
-  }
-  __syncthreads();
-  anorm = fmax(fabs(bounds[0]), fabs(bounds[1]));
-  bool all_ok = true;
-  for (uint32_t j = 0; j < nev; ++j) {
-    double* s = S + (uint64_t)j * m_max;
-    // Fast path (nev == 1): Rayleigh-quotient iteration from the previous
-    // Ritz vector, certified by a positive-definiteness test.
-    if (threadIdx.x == 0) sh_flag = 0;
-    __syncthreads();
-    if (nev == 1 && h->have_s && threadIdx.x == 0) {
-      uint32_t const prev = h->size;
-      for (uint32_t i = prev; i < n; ++i) s[i] = 0.0;
-      normalise(s, n);
-      double sigma = tri_rayleigh(alpha, beta, n, s);
-      for (int it = 0; it < 3; ++it) {
-        tri_solve(alpha, beta, n, sigma, s, dl, d, du, du2, piv);
-        normalise(s, n);
-        double const ns = tri_rayleigh(alpha, beta, n, s);
-        bool const done = fabs(ns - sigma) <= 1e-15 * fmax(1.0, fabs(ns));
-        sigma = ns;
-        if (done) break;
-      }
-      double const delta = 1e-12 * fmax(1.0, anorm);
-      if (tri_pos_def(alpha, beta, n, sigma - delta)) {
-        h->theta[0] = sigma;
-        sh_flag = 1;
-      }
-    }
-    __syncthreads();
-    if (!sh_flag) {
-      // Sturm multisection for the j-th eigenvalue, all threads.
-      if (threadIdx.x == 0) {
-        lohi[0] = bounds[0] - 1e-12 * fmax(1.0, anorm);
-        lohi[1] = bounds[1] + 1e-12 * fmax(1.0, anorm);
-      }
-      __syncthreads();
-      for (int round = 0; round < 24; ++round) {
-        double const lo = lohi[0], hi = lohi[1];
-        if (hi - lo <= 2e-16 * fmax(fabs(lo), fabs(hi)) + 1e-300) break;
-        double const x = lo + (hi - lo) * (double)(threadIdx.x + 1) / (double)(blockDim.x + 1);
-        bool const above = tri_count(alpha, beta, n, x) > j;  // x above eigenvalue j
-        unsigned const ballot = __ballot_sync(0xffffffffu, above);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          int const first = ballot ? __ffs(ballot) - 1 : (int)blockDim.x;
-          double const nlo = first == 0 ? lo : lo + (hi - lo) * (double)first / (double)(blockDim.x + 1);
-          double const nhi = first == (int)blockDim.x ? hi : lo + (hi - lo) * (double)(first + 1) / (double)(blockDim.x + 1);
-          lohi[0] = nlo;
-          lohi[1] = nhi;
-        }
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) {
-        double const theta = 0.5 * (lohi[0] + lohi[1]);
-        // Inverse iteration, orthogonalised against lower pairs.
-        for (uint32_t i = 0; i < n; ++i) s[i] = 1.0 + 1e-3 * (double)((i * 7919u + j * 104729u) % 1000u) / 1000.0;
-        for (int it = 0; it < 3; ++it) {
-          for (uint32_t q = 0; q < j; ++q) {
-            double const* sq = S + (uint64_t)q * m_max;
-            double dp = 0.0;
-            for (uint32_t i = 0; i < n; ++i) dp += sq[i] * s[i];
-            for (uint32_t i = 0; i < n; ++i) s[i] -= dp * sq[i];
-          }
-          normalise(s, n);
-          tri_solve(alpha, beta, n, theta, s, dl, d, du, du2, piv);
-          normalise(s, n);
-        }
-        h->theta[j] = tri_rayleigh(alpha, beta, n, s);
-        h->fallbacks += 1;
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      double const est = fabs(bk * s[n - 1]);
-      h->est[j] = breakdown ? 0.0 : est;
-      if (!(h->est[j] <= h->tol_est)) all_ok = false;
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    h->size = n;
-    h->have_s = 1;
-    h->steps += 1;
-    if (breakdown)
-      h->stop = 3;
-    else if (nev == h->nev && all_ok)
-      h->stop = 1;
-    else if (full)
-      h->stop = 2;
-    else
-      h->k = k + 1;
-  }
+  advance_step(h, b, done);
 }
 
 // out_i = sum_{j < n} s_j V_j[i]
@@ -611,10 +424,126 @@ __global__ void k_random(X* __restrict__ x, uint64_t D, uint64_t seed) {
   }
 }
 
+// ----------------------------------------------------------------- cycle --
+// Host side of one Krylov cycle: replays the graph of `check` steps and
+// solves T after each replay until the pairs converge, the device stops or
+// `max_steps` are used up.
+class Cycle {
+ public:
+  cudaGraphExec_t graph = nullptr;
+  LzHeader* hdr = nullptr;   // device: header, alpha[m], beta[m]
+  uint32_t m = 0, check = 1;
+  uint32_t stop = kRunning;  // how the cycle ended (kRunning: out of steps)
+  uint32_t steps = 0;        // steps of the cycle
+
+  Cycle() = default;
+  Cycle(Cycle const&) = delete;
+  Cycle& operator=(Cycle const&) = delete;
+  ~Cycle() {
+    if (graph) cudaGraphExecDestroy(graph);
+    for (cudaEvent_t e : ready_)
+      if (e) cudaEventDestroy(e);
+    if (host_) cudaFreeHost(host_);
+  }
+
+  double* alpha() const { return reinterpret_cast<double*>(hdr + 1); }
+  double* beta() const { return alpha() + m; }
+
+  int init(LzHeader* device_state, uint32_t m_max, uint32_t check_every) {
+    hdr = device_state;
+    m = m_max;
+    check = check_every;
+    SED_TRY_CUDA(cudaMallocHost(&host_, 2 * state_bytes(m)));
+    for (cudaEvent_t& e : ready_) SED_TRY_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return LS_SUCCESS;
+  }
+
+  // Captures `check` steps on `stream`.
+  template <class Step>
+  int capture(cudaStream_t stream, Step&& step) {
+    cudaGraph_t g;
+    SED_TRY_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+    set_capturing(true);
+    int st = LS_SUCCESS;
+    for (uint32_t i = 0; i < check && st == LS_SUCCESS; ++i) st = step();
+    set_capturing(false);
+    cudaError_t e = cudaStreamEndCapture(stream, &g);
+    if (st) {
+      if (e == cudaSuccess) cudaGraphDestroy(g);
+      return st;
+    }
+    SED_TRY_CUDA(e);
+    cudaGraphGetNodes(g, nullptr, &nodes_);
+    e = cudaGraphInstantiate(&graph, g, 0);
+    cudaGraphDestroy(g);
+    SED_TRY_CUDA(e);
+    return LS_SUCCESS;
+  }
+
+  // Resets the header: the cycle starts from v_k0 (alpha and beta below k0
+  // are the caller's). The copy leaves host_[0], which no replay uses yet.
+  int start(cudaStream_t stream, uint32_t k0) {
+    LzHeader h{};
+    h.k = k0;
+    h.m_max = m;
+    h.size = k0;
+    std::memcpy(host_, &h, sizeof(h));
+    SED_TRY_CUDA(cudaMemcpyAsync(hdr, host_, sizeof(h), cudaMemcpyHostToDevice, stream));
+    SED_TRY_CUDA(cudaStreamSynchronize(stream));
+    return LS_SUCCESS;
+  }
+
+  // The next replay is queued before the host looks at the last one, so the
+  // device does not wait for the host's solve, as long as the estimates are
+  // more than 1000 times the tolerance: four steps gain less than that, so
+  // the replay in flight when the cycle ends (its steps are not counted) is
+  // at most the rare one.
+  template <class Progress>
+  int run(cudaStream_t stream, Tridiagonal& T, double tol_est, uint64_t max_steps, Progress&& progress) {
+    T.restart();
+    stop = kRunning;
+    steps = 0;
+    bool far = false;
+    uint64_t launched = 0, seen = 0;
+    while (true) {
+      while (launched < seen + (far ? 2 : 1) && (launched == 0 || launched * check < max_steps)) {
+        SED_TRY_CUDA(cudaGraphLaunch(graph, stream));
+        note_launches(nodes_);
+        SED_TRY_CUDA(cudaMemcpyAsync(slot(launched), hdr, state_bytes(m), cudaMemcpyDeviceToHost, stream));
+        SED_TRY_CUDA(cudaEventRecord(ready_[launched & 1], stream));
+        ++launched;
+      }
+      if (seen == launched) return LS_SUCCESS;  // out of steps
+      SED_TRY_CUDA(cudaEventSynchronize(ready_[seen & 1]));
+      LzHeader const& h = *reinterpret_cast<LzHeader const*>(slot(seen));
+      double const* a = reinterpret_cast<double const*>(slot(seen) + sizeof(LzHeader));
+      ++seen;
+      steps = h.steps;
+      bool const halted = h.stop != kRunning;
+      uint32_t const n = halted ? h.size : h.size - h.size % check;
+      bool const done = n > 0 && T.solve(a, a + m, n, h.stop == kBreakdown, tol_est);
+      progress(steps);
+      if (halted || done) {
+        stop = h.stop == kBreakdown ? (uint32_t)kBreakdown : done ? (uint32_t)kConverged : (uint32_t)kFull;
+        steps -= h.size - n;  // steps past the solved order
+        return LS_SUCCESS;
+      }
+      far = n > 0;
+      if (far) far = *std::max_element(T.est.begin(), T.est.end()) > 1e3 * tol_est;
+    }
+  }
+
+ private:
+  char* host_ = nullptr;  // two copies of the state, pinned
+  cudaEvent_t ready_[2] = {nullptr, nullptr};
+  size_t nodes_ = 0;
+  char* slot(uint64_t i) const { return host_ + (i & 1) * state_bytes(m); }
+};
+
 // ------------------------------------------------------------- driver ----
 
 struct Workspace {
-  DeviceBuffer V, header, alpha, beta, s, work, partial, cgs_partial, coef, ritz, y, scratch;
+  DeviceBuffer V, state, s, partial, done, cgs_partial, coef, ritz, y, scratch;
 };
 
 int elem_bytes(int dtype) { return dtype == 0 ? 4 : dtype == 1 ? 8 : dtype == 2 ? 8 : 16; }
@@ -642,51 +571,40 @@ struct Solver {
   cudaStream_t stream;
   Workspace ws;
   uint32_t m_max = 0;
-  unsigned spmv_blocks = 0;
   unsigned vblocks = 0;
-  cudaGraphExec_t graph = nullptr;
-  size_t graph_kernels = 0;
-  LzHeader* hh = nullptr;  // pinned host mirror
+  bool reorth = false;
+  Cycle cycle;
   FixStep fx{};            // fused fixed-point step (FP64, one vector, stream form)
 
   Solver(OperatorData& o, int dt, cudaStream_t s) : op(o), dtype(dt), D(o.basis->D), stream(s) {}
   ~Solver() {
-    if (graph) cudaGraphExecDestroy(graph);
-    if (hh) cudaFreeHost(hh);
+    cudaStreamSynchronize(stream);  // a replay may be in flight on an early exit
     krylov_give(ws.V);
   }
 
   X* V() const { return ws.V.as<X>(); }
-  LzHeader* hdr() const { return ws.header.as<LzHeader>(); }
+  LzHeader* hdr() const { return cycle.hdr; }
 
-  int init(uint32_t m, uint32_t nev, uint32_t check, double tol_est, bool reorth) {
+  int init(uint32_t m, uint32_t check, bool reorthogonalise) {
     m_max = m;
+    reorth = reorthogonalise;
     int dev = op.basis->device;
     vblocks = grid_size(D, dev, 8);
     if (int st = krylov_take((size_t)m_max * D * sizeof(X), ws.V)) return st;
-    if (int st = ws.header.allocate(sizeof(LzHeader))) return st;
-    if (int st = ws.alpha.allocate((size_t)m_max * 8)) return st;
-    if (int st = ws.beta.allocate((size_t)m_max * 8)) return st;
-    if (int st = ws.s.allocate((size_t)kMaxNev * m_max * 8)) return st;
-    if (int st = ws.work.allocate((size_t)5 * m_max * 8 + 64)) return st;
-    uint64_t const nb = std::max<uint64_t>((D + kBlock - 1) / kBlock + 64, vblocks);
+    if (int st = ws.state.allocate(state_bytes(m_max))) return st;
+    if (int st = ws.s.allocate((size_t)m_max * 8)) return st;
+    uint64_t const nb = std::max<uint64_t>((D + kBlock - 1) / kBlock, vblocks) + 32;
     if (int st = ws.partial.allocate(nb * 16)) return st;
+    if (int st = ws.done.allocate(16)) return st;
     if (reorth) {
       if (int st = ws.cgs_partial.allocate((size_t)m_max * vblocks * 8)) return st;
       if (int st = ws.coef.allocate((size_t)m_max * 8)) return st;
     }
     if (int st = ws.ritz.allocate(D * sizeof(X))) return st;
     if (int st = ws.y.allocate(D * sizeof(X))) return st;
-    SED_TRY_CUDA(cudaMallocHost(&hh, sizeof(LzHeader)));
-    std::memset(hh, 0, sizeof(LzHeader));
-    hh->m_max = m_max;
-    hh->check = check;
-    hh->nev = nev;
-    hh->tol_est = tol_est;
-    hh->reorth = reorth ? 1u : 0u;
-    SED_TRY_CUDA(cudaMemcpyAsync(hdr(), hh, sizeof(LzHeader), cudaMemcpyHostToDevice, stream));
-    SED_TRY_CUDA(cudaMemsetAsync(ws.alpha.ptr, 0, (size_t)m_max * 8, stream));
-    SED_TRY_CUDA(cudaMemsetAsync(ws.beta.ptr, 0, (size_t)m_max * 8, stream));
+    if (int st = cycle.init(ws.state.as<LzHeader>(), m_max, check)) return st;
+    SED_TRY_CUDA(cudaMemsetAsync(ws.state.ptr, 0, state_bytes(m_max), stream));
+    SED_TRY_CUDA(cudaMemsetAsync(ws.done.ptr, 0, 16, stream));
     FixSlots fs;
     if (std::is_same<X, double>::value && !reorth && fix_slots(op, &fs))
       fx = FixStep{true, fs.max_bits, fs.F, fs.u, fs.row_class, fs.view};
@@ -708,66 +626,37 @@ struct Solver {
   // One Lanczos step (all kernels read k from the header).
   int enqueue_step() {
     LzHeader* h = hdr();
-    { k_zero_alpha<X><<<1, 1, 0, stream>>>(h, ws.alpha.as<double>(), fx.on ? fx.wmax : nullptr); note_launches(1); }
+    double *alpha = cycle.alpha(), *beta = cycle.beta(), *partial = ws.partial.template as<double>();
+    uint32_t* done = ws.done.template as<uint32_t>();
     Indirect ind;
     ind.k = &h->k;
     ind.stop = &h->stop;
     ind.ld = D;
-    ind.partial = ws.partial.as<double>();
+    ind.partial = partial;
+    ind.done = done;
+    ind.sum = alpha;
+    ind.clear = fx.on ? fx.wmax : nullptr;  // k_update's max |w| starts at zero
     ind.prescaled = fx.on;
-    if (int st = operator_apply_krylov(op, dtype, V(), ind, stream, &spmv_blocks)) return st;
-    { k_reduce<<<1, kRedThreads, 0, stream>>>(ws.partial.as<double>(), spmv_blocks, h, ws.alpha.as<double>(), 0); note_launches(1); }
-    { k_update<X><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, ws.alpha.as<double>(), ws.beta.as<double>(),
-                                                ws.partial.as<double>(), fx.on ? fx.wmax : nullptr); note_launches(1); }
-    if (hh->reorth) {
+    if (int st = apply_with_alpha(ind, D, stream, [&](Indirect i) { return operator_apply_krylov(op, dtype, V(), i, stream); }))
+      return st;
+    { k_update<X><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, alpha, beta, partial, done, fx.on ? fx.wmax : nullptr); note_launches(1); }
+    if (reorth) {
       for (int pass = 0; pass < 2; ++pass) {
         dim3 grid(vblocks, (m_max + 15) / 16);
-        { k_cgs_dots<X><<<grid, kBlock, 0, stream>>>(V(), D, D, h, ws.cgs_partial.as<double>()); note_launches(1); }
-        { k_cgs_reduce<<<1, kRedThreads, 0, stream>>>(ws.cgs_partial.as<double>(), vblocks, h,
-                                                    ws.coef.as<double>(), ws.alpha.as<double>()); note_launches(1); }
-        { k_cgs_update<X><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, ws.coef.as<double>(),
-                                                        ws.partial.as<double>()); note_launches(1); }
+        { k_cgs_dots<X><<<grid, kBlock, 0, stream>>>(V(), D, D, h, ws.cgs_partial.template as<double>()); note_launches(1); }
+        { k_cgs_reduce<<<1, kRedThreads, 0, stream>>>(ws.cgs_partial.template as<double>(), vblocks, h,
+                                                    ws.coef.template as<double>(), alpha); note_launches(1); }
+        { k_cgs_update<X><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, ws.coef.template as<double>(), beta, partial,
+                                                        done); note_launches(1); }
       }
     }
-    { k_reduce<<<1, kRedThreads, 0, stream>>>(ws.partial.as<double>(), vblocks, h, ws.beta.as<double>(), 1); note_launches(1); }
-    { k_scale_next<X><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, ws.beta.as<double>(), fx); note_launches(1); }
-    { k_tridiag<<<1, 32, 0, stream>>>(h, ws.alpha.as<double>(), ws.beta.as<double>(), ws.s.as<double>(),
-                                    ws.work.as<double>()); note_launches(1); }
+    { k_scale_next<X><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, beta, done, fx); note_launches(1); }
     SED_TRY_CUDA(cudaGetLastError());
     return LS_SUCCESS;
   }
 
-  int capture(uint32_t steps) {
-    cudaGraph_t g;
-    SED_TRY_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    set_capturing(true);
-    int st = LS_SUCCESS;
-    for (uint32_t i = 0; i < steps && st == LS_SUCCESS; ++i) st = enqueue_step();
-    set_capturing(false);
-    cudaError_t e = cudaStreamEndCapture(stream, &g);
-    if (st) {
-      if (e == cudaSuccess) cudaGraphDestroy(g);
-      return st;
-    }
-    SED_TRY_CUDA(e);
-    size_t n_nodes = 0;
-    cudaGraphGetNodes(g, nullptr, &n_nodes);
-    graph_kernels = n_nodes;
-    e = cudaGraphInstantiate(&graph, g, 0);
-    cudaGraphDestroy(g);
-    SED_TRY_CUDA(e);
-    return LS_SUCCESS;
-  }
-
-  int read_header() {
-    SED_TRY_CUDA(cudaMemcpyAsync(hh, hdr(), sizeof(LzHeader), cudaMemcpyDeviceToHost, stream));
-    SED_TRY_CUDA(cudaStreamSynchronize(stream));
-    return LS_SUCCESS;
-  }
-
-  int write_header() {
-    SED_TRY_CUDA(cudaMemcpyAsync(hdr(), hh, sizeof(LzHeader), cudaMemcpyHostToDevice, stream));
-    return LS_SUCCESS;
+  int capture() {
+    return cycle.capture(stream, [&] { return enqueue_step(); });
   }
 
   // Writes x (device, type X) to dst (host or device) as `out_dtype`.
@@ -834,8 +723,8 @@ struct Solver {
 // FP32 Lanczos steps: vectors and their updates in FP32, reductions per warp
 // in FP32 and per block in FP64.
 __global__ void k_update32(float* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader const* h,
-                           double const* __restrict__ alpha, double const* __restrict__ beta,
-                           double* __restrict__ partial) {
+                           double const* __restrict__ alpha, double* __restrict__ beta,
+                           double* __restrict__ partial, uint32_t* __restrict__ done) {
   __shared__ double red[kBlock / 32];
   if (h->stop) return;
   uint32_t const k = h->k;
@@ -853,20 +742,24 @@ __global__ void k_update32(float* __restrict__ V, uint64_t ld_v, uint64_t D, LzH
   }
   for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
   double const tot = block_sum((threadIdx.x & 31) == 0 ? (double)part : 0.0, red);
-  if (threadIdx.x == 0) partial[blockIdx.x] = tot;
+  finish_sum(tot, partial, done, [&](double s) { beta[k] = sqrt(s); });
 }
 
-__global__ void k_scale_next32(float* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader const* h,
-                               double const* __restrict__ beta) {
+__global__ void k_scale_next32(float* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader* h,
+                               double const* __restrict__ beta, uint32_t* __restrict__ done) {
   if (h->stop) return;
   uint32_t const k = h->k;
   double const b = beta[k];
-  if (!(b > 0.0)) return;
+  if (!(b > 0.0)) {
+    advance_step(h, b, done);
+    return;
+  }
   float const inv = (float)(1.0 / b);
   float* w = V + (uint64_t)(k + 1) * ld_v;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D;
        i += (uint64_t)gridDim.x * blockDim.x)
     w[i] *= inv;
+  advance_step(h, b, done);
 }
 
 // out = s_0 psi + sum_{j=1}^{n-1} s_j V_j, accumulated in FP64.
@@ -936,7 +829,7 @@ int solve(OperatorData& op, int out_dtype, sed_eigh_options const& o, double* ev
   uint32_t const m = auto_basis(D, sizeof(X), nev, o.max_basis);
   uint32_t const check = m < 64 ? 1u : 4u;
   Solver<X> S(op, dtype, stream);
-  if (int st = S.init(m, nev, check, 0.5 * tol, reorth)) return st;
+  if (int st = S.init(m, check, reorth)) return st;
   // Start vector.
   if (o.start == SED_START_GIVEN && o.start_vectors) {
     size_t const es = sizeof(X);
@@ -946,36 +839,30 @@ int solve(OperatorData& op, int out_dtype, sed_eigh_options const& o, double* ev
     SED_TRY_CUDA(cudaGetLastError());
   }
   if (int st = S.normalise_vec(S.V(), nullptr)) return st;
-  if (int st = S.capture(check)) return st;
-  if (int st = S.prescale()) return st;
+  if (int st = S.capture()) return st;
   uint64_t steps = 0, matvecs = 0, restarts = 0;
   std::vector<double> E(nev, 0.0), R(nev, 1e300);
   bool converged = false;
-  std::vector<double> theta_h(nev), est_h(nev);
+  Tridiagonal T(nev);
   while (!converged) {
-    SED_TRY_CUDA(cudaGraphLaunch(S.graph, stream));
-    note_launches(S.graph_kernels);
-    if (int st = S.read_header()) return st;
-    if (o.progress) {
-      for (uint32_t j = 0; j < nev; ++j) {
-        theta_h[j] = S.hh->theta[j];
-        est_h[j] = S.hh->est[j];
-      }
-      o.progress(o.progress_user, steps + S.hh->steps, theta_h.data(), est_h.data(), nev);
-    }
-    uint32_t const stop = S.hh->stop;
-    if (!stop) {
-      if (steps + S.hh->steps >= max_iter) break;
-      continue;
-    }
-    steps += S.hh->steps;
-    matvecs += S.hh->steps;
-    uint32_t const n = S.hh->size;
+    if (int st = S.cycle.start(stream, 0)) return st;
+    if (int st = S.prescale()) return st;  // the start's and the residual matvecs used the workspace
+    uint64_t const before = steps;
+    if (int st = S.cycle.run(stream, T, 0.5 * tol, max_iter - std::min(steps, max_iter), [&](uint32_t taken) {
+          if (o.progress) o.progress(o.progress_user, before + taken, T.theta.data(), T.est.data(), nev);
+        }))
+      return st;
+    uint32_t const stop = S.cycle.stop;
+    if (stop == kRunning) break;  // out of steps
+    steps += S.cycle.steps;
+    matvecs += S.cycle.steps;
+    uint32_t const n = T.size();
     // Ritz vectors and their true residuals.
     bool all_ok = true;
     for (uint32_t j = 0; j < nev; ++j) {
-      { k_ritz<X, X><<<S.vblocks, kBlock, 0, stream>>>(S.V(), D, D, S.ws.s.template as<double>() + (uint64_t)j * m,
-                                                     n, S.ws.ritz.template as<X>()); note_launches(1); }
+      SED_TRY_CUDA(cudaMemcpyAsync(S.ws.s.ptr, T.vector(j).data(), n * 8, cudaMemcpyHostToDevice, stream));
+      { k_ritz<X, X><<<S.vblocks, kBlock, 0, stream>>>(S.V(), D, D, S.ws.s.template as<double>(), n,
+                                                     S.ws.ritz.template as<X>()); note_launches(1); }
       SED_TRY_CUDA(cudaGetLastError());
       if (int st = S.normalise_vec(S.ws.ritz.template as<X>(), nullptr)) return st;
       double e = 0.0, r = 0.0;
@@ -988,8 +875,8 @@ int solve(OperatorData& op, int out_dtype, sed_eigh_options const& o, double* ev
         if (int st = S.store(S.ws.ritz.template as<X>(), out_dtype, static_cast<char*>(evecs) +
                              (size_t)j * ldv * elem_bytes(out_dtype))) return st;
     }
-    if (all_ok || stop == 3 || steps >= max_iter) {
-      converged = all_ok || stop == 3;
+    if (all_ok || stop == kBreakdown || steps >= max_iter) {
+      converged = all_ok || stop == kBreakdown;
       break;
     }
     // Restart from the (sum of the) Ritz vectors.
@@ -997,28 +884,15 @@ int solve(OperatorData& op, int out_dtype, sed_eigh_options const& o, double* ev
     if (nev == 1) {
       SED_TRY_CUDA(cudaMemcpyAsync(S.V(), S.ws.ritz.ptr, D * sizeof(X), cudaMemcpyDeviceToDevice, stream));
     } else {
-      { k_ritz<X, X><<<S.vblocks, kBlock, 0, stream>>>(S.V(), D, D, S.ws.s.template as<double>(), n, S.ws.ritz.template as<X>()); note_launches(1); }
-      // sum of all nev Ritz directions
-      std::vector<double> ones(n, 0.0);
-      std::vector<double> sh((size_t)nev * m);
-      SED_TRY_CUDA(cudaMemcpy(sh.data(), S.ws.s.ptr, sh.size() * 8, cudaMemcpyDeviceToHost));
+      std::vector<double> all(n, 0.0);  // sum of all nev Ritz directions
       for (uint32_t j = 0; j < nev; ++j)
-        for (uint32_t i = 0; i < n; ++i) ones[i] += sh[(size_t)j * m + i];
-      SED_TRY_CUDA(cudaMemcpy(S.ws.work.ptr, ones.data(), n * 8, cudaMemcpyHostToDevice));
-      { k_ritz<X, X><<<S.vblocks, kBlock, 0, stream>>>(S.V(), D, D, S.ws.work.template as<double>(), n,
+        for (uint32_t i = 0; i < n; ++i) all[i] += T.vector(j)[i];
+      SED_TRY_CUDA(cudaMemcpyAsync(S.ws.s.ptr, all.data(), n * 8, cudaMemcpyHostToDevice, stream));
+      { k_ritz<X, X><<<S.vblocks, kBlock, 0, stream>>>(S.V(), D, D, S.ws.s.template as<double>(), n,
                                                      S.ws.ritz.template as<X>()); note_launches(1); }
       SED_TRY_CUDA(cudaMemcpyAsync(S.V(), S.ws.ritz.ptr, D * sizeof(X), cudaMemcpyDeviceToDevice, stream));
     }
     if (int st = S.normalise_vec(S.V(), nullptr)) return st;
-    uint32_t const keep_nev = S.hh->nev;
-    std::memset(S.hh, 0, sizeof(LzHeader));
-    S.hh->m_max = m;
-    S.hh->check = check;
-    S.hh->nev = keep_nev;
-    S.hh->tol_est = 0.5 * tol;
-    S.hh->reorth = reorth ? 1u : 0u;
-    if (int st = S.write_header()) return st;
-    if (int st = S.prescale()) return st;  // the residual matvecs used the workspace
   }
   SED_TRY_CUDA(cudaStreamSynchronize(stream));
   for (uint32_t j = 0; j < nev; ++j) {
@@ -1065,28 +939,29 @@ int solve_mixed(OperatorData& op, int out_dtype, sed_eigh_options const& o, doub
   uint32_t const m = std::max<uint32_t>(3, auto_basis(D, 4, 1, o.max_basis ? o.max_basis : 300));
   uint32_t const check = m < 64 ? 1u : 4u;
   unsigned const vb = grid_size(D, op.basis->device, 8);
-  DeviceBuffer psi, y, V, hdr_b, alpha, beta, sbuf, work, partial;
+  DeviceBuffer psi, y, V, state, sbuf, partial, done_b;
   if (int st = psi.allocate(D * 8)) return st;
   if (int st = y.allocate(D * 8)) return st;
   struct KrylovGuard {
     DeviceBuffer& b;
-    ~KrylovGuard() { krylov_give(b); }
-  } krylov_guard{V};
+    cudaStream_t s;
+    ~KrylovGuard() {
+      cudaStreamSynchronize(s);  // a replay may be in flight on an early exit
+      krylov_give(b);
+    }
+  } krylov_guard{V, stream};
   if (int st = krylov_take((size_t)m * D * 4, V)) return st;
-  if (int st = hdr_b.allocate(sizeof(LzHeader))) return st;
-  if (int st = alpha.allocate((size_t)m * 8)) return st;
-  if (int st = beta.allocate((size_t)m * 8)) return st;
-  if (int st = sbuf.allocate((size_t)kMaxNev * m * 8)) return st;
-  if (int st = work.allocate((size_t)5 * m * 8 + 64)) return st;
-  uint64_t const nb = std::max<uint64_t>((D + kBlock - 1) / kBlock + 64, vb);
+  if (int st = state.allocate(state_bytes(m))) return st;
+  if (int st = sbuf.allocate((size_t)m * 8)) return st;
+  uint64_t const nb = std::max<uint64_t>((D + kBlock - 1) / kBlock, vb) + 32;
   if (int st = partial.allocate(nb * 16)) return st;
-  LzHeader* hh = nullptr;
-  SED_TRY_CUDA(cudaMallocHost(&hh, sizeof(LzHeader)));
-  struct HostGuard {
-    LzHeader* p;
-    ~HostGuard() { cudaFreeHost(p); }
-  } host_guard{hh};
-  LzHeader* h = hdr_b.as<LzHeader>();
+  if (int st = done_b.allocate(16)) return st;
+  SED_TRY_CUDA(cudaMemsetAsync(done_b.ptr, 0, 16, stream));
+  Cycle cycle;
+  if (int st = cycle.init(state.as<LzHeader>(), m, check)) return st;
+  Tridiagonal T(1);
+  uint32_t* done = done_b.as<uint32_t>();
+  LzHeader* h = cycle.hdr;
   float* Vf = V.as<float>();
   // FP64 start vector
   if (o.start == SED_START_GIVEN && o.start_vectors)
@@ -1111,47 +986,23 @@ int solve_mixed(OperatorData& op, int out_dtype, sed_eigh_options const& o, doub
   if (int st = sum2(0, 0.0, nn, dummy)) return st;
   { k_scale<double><<<vb, kBlock, 0, stream>>>(psi.as<double>(), D, 1.0 / std::sqrt(nn)); note_launches(1); }
   // graph of `check` FP32 steps
-  cudaGraphExec_t graph = nullptr;
-  size_t graph_kernels = 0;
-  {
-    cudaGraph_t g;
-    SED_TRY_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    set_capturing(true);
-    int st = LS_SUCCESS;
-    unsigned spmv_blocks = 0;
-    for (uint32_t i = 0; i < check && st == LS_SUCCESS; ++i) {
-      k_zero_alpha<float><<<1, 1, 0, stream>>>(h, alpha.as<double>(), nullptr);
-      Indirect ind;
-      ind.k = &h->k;
-      ind.stop = &h->stop;
-      ind.ld = D;
-      ind.partial = partial.as<double>();
-      st = operator_apply_krylov32(op, Vf, ind, stream, &spmv_blocks);
-      if (st) break;
-      k_reduce<<<1, kRedThreads, 0, stream>>>(partial.as<double>(), spmv_blocks, h, alpha.as<double>(), 0);
-      k_update32<<<vb, kBlock, 0, stream>>>(Vf, D, D, h, alpha.as<double>(), beta.as<double>(), partial.as<double>());
-      k_reduce<<<1, kRedThreads, 0, stream>>>(partial.as<double>(), vb, h, beta.as<double>(), 1);
-      k_scale_next32<<<vb, kBlock, 0, stream>>>(Vf, D, D, h, beta.as<double>());
-      k_tridiag<<<1, 32, 0, stream>>>(h, alpha.as<double>(), beta.as<double>(), sbuf.as<double>(), work.as<double>());
-    }
-    set_capturing(false);
-    cudaError_t e = cudaStreamEndCapture(stream, &g);
-    if (st) {
-      if (e == cudaSuccess) cudaGraphDestroy(g);
-      return st;
-    }
-    SED_TRY_CUDA(e);
-    cudaGraphGetNodes(g, nullptr, &graph_kernels);
-    e = cudaGraphInstantiate(&graph, g, 0);
-    cudaGraphDestroy(g);
-    SED_TRY_CUDA(e);
-  }
-  struct GraphGuard {
-    cudaGraphExec_t g;
-    ~GraphGuard() {
-      if (g) cudaGraphExecDestroy(g);
-    }
-  } graph_guard{graph};
+  double *alpha = cycle.alpha(), *beta = cycle.beta();
+  if (int st = cycle.capture(stream, [&]() -> int {
+        Indirect ind;
+        ind.k = &h->k;
+        ind.stop = &h->stop;
+        ind.ld = D;
+        ind.partial = partial.as<double>();
+        ind.done = done;
+        ind.sum = alpha;
+        if (int st = apply_with_alpha(ind, D, stream, [&](Indirect i) { return operator_apply_krylov32(op, Vf, i, stream); }))
+          return st;
+        k_update32<<<vb, kBlock, 0, stream>>>(Vf, D, D, h, alpha, beta, partial.as<double>(), done);
+        k_scale_next32<<<vb, kBlock, 0, stream>>>(Vf, D, D, h, beta, done);
+        SED_TRY_CUDA(cudaGetLastError());
+        return LS_SUCCESS;
+      }))
+    return st;
   uint64_t steps32 = 0, matvecs = 0, cycles = 0;
   double E = 0.0, R = 1e300;
   bool converged = false;
@@ -1174,29 +1025,18 @@ int solve_mixed(OperatorData& op, int out_dtype, sed_eigh_options const& o, doub
     // FP32 cycle from v0 = psi, v1 = r / ||r||
     double const rn = R * std::sqrt(pp);
     { k_start_cycle<<<vb, kBlock, 0, stream>>>(psi.as<double>(), y.as<double>(), D, E, 1.0 / rn, Vf, Vf + D); note_launches(1); }
-    std::memset(hh, 0, sizeof(LzHeader));
-    hh->k = 1;
-    hh->m_max = m;
-    hh->check = check;
-    hh->nev = 1;
-    hh->tol_est = std::max(0.5 * tol, 2e-6 * rn);
-    SED_TRY_CUDA(cudaMemcpyAsync(h, hh, sizeof(LzHeader), cudaMemcpyHostToDevice, stream));
     double const a0 = E, b0 = rn;
-    SED_TRY_CUDA(cudaMemcpyAsync(alpha.ptr, &a0, 8, cudaMemcpyHostToDevice, stream));
-    SED_TRY_CUDA(cudaMemcpyAsync(beta.ptr, &b0, 8, cudaMemcpyHostToDevice, stream));
-    SED_TRY_CUDA(cudaStreamSynchronize(stream));
-    while (true) {
-      SED_TRY_CUDA(cudaGraphLaunch(graph, stream));
-      note_launches(graph_kernels);
-      SED_TRY_CUDA(cudaMemcpyAsync(hh, h, sizeof(LzHeader), cudaMemcpyDeviceToHost, stream));
-      SED_TRY_CUDA(cudaStreamSynchronize(stream));
-      if (hh->stop) break;
-      if (steps32 + hh->steps >= max_iter) break;
-    }
-    steps32 += hh->steps;
+    SED_TRY_CUDA(cudaMemcpyAsync(alpha, &a0, 8, cudaMemcpyHostToDevice, stream));
+    SED_TRY_CUDA(cudaMemcpyAsync(beta, &b0, 8, cudaMemcpyHostToDevice, stream));
+    if (int st = cycle.start(stream, 1)) return st;
+    if (int st = cycle.run(stream, T, std::max(0.5 * tol, 2e-6 * rn), max_iter - std::min<uint64_t>(steps32, max_iter),
+                           [](uint32_t) {}))
+      return st;
+    steps32 += cycle.steps;
     ++cycles;
-    uint32_t const n = hh->size ? hh->size : 1;
-    if (!hh->stop) break;  // out of steps
+    if (cycle.stop == kRunning) break;  // out of steps
+    uint32_t const n = T.size();
+    SED_TRY_CUDA(cudaMemcpyAsync(sbuf.ptr, T.vector(0).data(), n * 8, cudaMemcpyHostToDevice, stream));
     { k_ritz_mixed<<<vb, kBlock, 0, stream>>>(psi.as<double>(), Vf, D, D, sbuf.as<double>(), n, y.as<double>()); note_launches(1); }
     SED_TRY_CUDA(cudaMemcpyAsync(psi.ptr, y.ptr, D * 8, cudaMemcpyDeviceToDevice, stream));
     double pn = 0, d2 = 0;

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kRecWarps * 32, kRecBlocks)
 
 // Streamed SpMV over SELL-32 slices. RealOp selects the real table/diagonal.
 // With an Indirect (Krylov) view, x = base + k ld and y = base + (k+1) ld
-// with k read from device memory, and each block writes sum_i Re(x_i* y_i).
+// with k read from device memory, and sum_i Re(x_i* y_i) goes to ind.sum[k].
 template <class X, bool RealOp, bool Packed>
 __global__ void __launch_bounds__(kBlock) k_spmv(StreamView S, uint64_t D, X const* __restrict__ x,
                                                  X* __restrict__ y, Indirect ind) {
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv(StreamView S, uint64_t D, X con
   }
   if (ind.partial) {
     double const tot = block_sum(part, red);
-    if (threadIdx.x == 0) ind.partial[blockIdx.x] = tot;
+    finish_apply(tot, ind);
   }
 }
 
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kBlock)
   }
   if (ind.partial) {
     double const tot = block_sum(part, red);
-    if (threadIdx.x == 0) ind.partial[blockIdx.x] = tot;
+    finish_apply(tot, ind);
   }
 }
 
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix(StreamView S, FixView fv, u
   }
   if (ind.partial) {
     double const tot = block_sum_fixed(part, red);
-    if (threadIdx.x == 0) ind.partial[blockIdx.x] = tot;
+    finish_apply(tot, ind);
   }
 }
 
@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(kBlock)
   }
   if (ind.partial) {
     double const tot = block_sum_fixed(part, red);
-    if (threadIdx.x == 0) ind.partial[blockIdx.x] = tot;
+    finish_apply(tot, ind);
   }
 }
 
@@ -1799,7 +1799,7 @@ __global__ void __launch_bounds__(kBlock)
   if (ind.partial) {
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
     double const tot = block_sum((threadIdx.x & 31) == 0 ? (double)part : 0.0, red);
-    if (threadIdx.x == 0) ind.partial[blockIdx.x] = tot;
+    finish_apply(tot, ind);
   }
 }
 
@@ -1921,11 +1921,10 @@ __global__ void __launch_bounds__(kBlock) k_spmv32_fix(StreamView S, FixView fv,
     for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = (double)part;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double tot = 0.0;
+    double tot = 0.0;
+    if (threadIdx.x == 0)
       for (unsigned w = 0; w < kBlock / 32; ++w) tot += red[w];
-      ind.partial[blockIdx.x] = tot;
-    }
+    finish_apply(tot, ind);
   }
 }
 
@@ -1970,12 +1969,11 @@ void launch_spmv32_fix(OperatorData& op, StreamView const& S, float const* x, fl
   note_launches(1);
 }
 
-int launch32(OperatorData& op, float const* x, float* y, Indirect ind, cudaStream_t stream, unsigned* blocks) {
+int launch32(OperatorData& op, float const* x, float* y, Indirect ind, cudaStream_t stream) {
   StreamForm const& sf = op.stream;
   if (!sf.diag_f.ptr) return fail(LS_CACHE_NOT_BUILT, "FP32 companions are not prepared");
   StreamView const S = stream_view(op);
   unsigned const grid = (unsigned)((sf.n_slices * 32 + kBlock - 1) / kBlock);
-  if (blocks) *blocks = grid;
   OperatorTables const& tb = *op.tables;
   if (tb.fix_ok && op.fix_u32.ptr) {
     uint64_t const D = op.basis->D;
@@ -2005,20 +2003,16 @@ int launch32(OperatorData& op, float const* x, float* y, Indirect ind, cudaStrea
 }
 }  // namespace
 
-int operator_apply_krylov32(OperatorData& op, float* base, Indirect ind, cudaStream_t stream, unsigned* blocks) {
-  return launch32(op, base, base, ind, stream, blocks);
+int operator_apply_krylov32(OperatorData& op, float* base, Indirect ind, cudaStream_t stream) {
+  return launch32(op, base, base, ind, stream);
 }
 
 int operator_apply32(OperatorData& op, float const* x, float* y, cudaStream_t stream) {
-  return launch32(op, x, y, Indirect{}, stream, nullptr);
+  return launch32(op, x, y, Indirect{}, stream);
 }
 
-int operator_apply_krylov(OperatorData& op, int dtype, void* base, Indirect ind, cudaStream_t stream,
-                          unsigned* blocks) {
+int operator_apply_krylov(OperatorData& op, int dtype, void* base, Indirect ind, cudaStream_t stream) {
   bool const use_stream = op.stream.ready && op.form != SED_FORM_ON_THE_FLY;
-  uint64_t const D = op.basis->D;
-  *blocks = use_stream ? (unsigned)((op.stream.n_slices * 32 + kBlock - 1) / kBlock)
-                       : (unsigned)((D + kBlock - 1) / kBlock);
   switch (dtype) {
     case 1: return launch_apply<double>(op, (double const*)base, (double*)base, stream, use_stream, ind);
     case 3: return launch_apply<double2>(op, (double2 const*)base, (double2*)base, stream, use_stream, ind);

@@ -288,14 +288,11 @@ bool fix_slots(OperatorData& op, FixSlots* out);
 int fix_prescale(OperatorData& op, double const* base, Indirect ind, cudaStream_t stream);
 // FP32 streamed SpMV in Krylov-indirect mode (x = base + k ld, y = base +
 // (k+1) ld); FP32 arithmetic, per-block partial sums of x_i y_i in FP64.
-int operator_apply_krylov32(OperatorData& op, float* base, Indirect ind, cudaStream_t stream,
-                            unsigned* blocks);
+int operator_apply_krylov32(OperatorData& op, float* base, Indirect ind, cudaStream_t stream);
 // The same SpMV on explicit FP32 vectors.
 int operator_apply32(OperatorData& op, float const* x, float* y, cudaStream_t stream);
-// Krylov-indirect apply (see Indirect); `blocks` receives the grid size, i.e.
-// the number of partial sums written.
-int operator_apply_krylov(OperatorData& op, int dtype, void* base, Indirect ind, cudaStream_t stream,
-                          unsigned* blocks);
+// Krylov-indirect apply (see Indirect), on at most ceil(D / kBlock) blocks.
+int operator_apply_krylov(OperatorData& op, int dtype, void* base, Indirect ind, cudaStream_t stream);
 int operator_ensure_ready(OperatorData& op);
 
 // V[:, 0..kk) <- V[:, 0..m) Y on the tensor cores (rotate_tc.cu): V FP64,

@@ -106,11 +106,75 @@ struct Indirect {
   uint32_t const* k = nullptr;
   uint32_t const* stop = nullptr;
   uint64_t ld = 0;
-  double* partial = nullptr;
+  double* partial = nullptr;    // per-block sums of Re(x_i* y_i) (see finish_sum)
+  uint32_t* done = nullptr;     // finish_sum's counters
+  double* sum = nullptr;        // the last block writes the total to sum[*k]
+  unsigned long long* clear = nullptr;  // and zeroes this word (may be null)
   // fixed-point matvec: u and F of x were written by the step that produced
   // x (Lanczos' scale kernel), so the matvec skips its own pre-pass
   bool prescaled = false;
 };
+
+// Grid-wide sum of one double per block (`tot`, valid in thread 0) inside the
+// kernel that produces it: the last block to finish adds the partials and its
+// thread 0 calls f(total). The additions have the order of k_sum_partials
+// (each thread stands in for four of its 1024), so the total depends neither
+// on which block comes last nor on the path. A kernel of its own for the sum
+// took 6.4 us per reduction on a ring of 24 sites, this tail about 1.5 us.
+// Each block pays a fence for it: worth it up to kFusedSumBlocks blocks (the
+// fences of 61 738 blocks cost a 15.8 M-row SpMV 25 us, more than the
+// kernel). `partial` holds gridDim.x <= kFusedSumBlocks doubles, *done is
+// zero and left zero; blockDim.x = kBlock. Every thread of the grid calls it.
+constexpr unsigned kFusedSumBlocks = 2048;
+
+template <class F>
+__device__ __forceinline__ void finish_sum(double tot, double* partial, uint32_t* done, F&& f) {
+  __shared__ double warp_sum[32];
+  __shared__ bool last;
+  uint32_t const n = gridDim.x;
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = tot;
+    __threadfence();
+    last = atomicAdd(done, 1u) == n - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  static_assert(kBlock * 4 == 1024 && kFusedSumBlocks == 2048, "four stand-ins, two partials each");
+  double a[4], b[4];
+#pragma unroll
+  for (uint32_t v = 0; v < 4; ++v) {
+    uint32_t const i = threadIdx.x + v * kBlock;
+    a[v] = i < n ? __ldcg(partial + i) : 0.0;
+    b[v] = i + 1024 < n ? __ldcg(partial + i + 1024) : 0.0;
+  }
+#pragma unroll
+  for (uint32_t v = 0; v < 4; ++v) {
+    if (v * kBlock >= n) break;  // sums of nothing
+    double s = n > 1024 ? a[v] + b[v] : a[v];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) warp_sum[(threadIdx.x >> 5) + 8 * v] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (uint32_t w = 0; w < min(32u, (n + 31) / 32); ++w) s += warp_sum[w];
+    *done = 0;
+    f(s);
+  }
+}
+
+// The matvec's own use of it: alpha_k = sum_i Re(x_i* y_i).
+__device__ __forceinline__ void finish_apply(double tot, Indirect const& ind) {
+  if (!ind.done) {  // too many blocks: k_sum_partials follows
+    if (threadIdx.x == 0) ind.partial[blockIdx.x] = tot;
+    return;
+  }
+  finish_sum(tot, ind.partial, ind.done, [&](double s) {
+    ind.sum[*ind.k] = s;
+    if (ind.clear) *ind.clear = 0;
+  });
+}
 
 inline unsigned grid_size(uint64_t work, int device, unsigned per_sm = 16, unsigned block = kBlock) {
   int sms = 152;

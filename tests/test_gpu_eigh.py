@@ -142,3 +142,17 @@ def test_thick_restart_lowest_three(sed, oracle):
     assert np.all(res.residuals <= RES_TOL)
     for k in range(3):
         check_pair(oop, res.eigenvalues[k], res.eigenvectors[:, k])
+
+
+@pytest.mark.parametrize("n", [12, 16, 24, 28, 32])
+def test_ring_energies_over_the_reduction_grids(sed, n):
+    """Ground states whose matvec grids finish their sums in one block, in
+    fewer than 1024, between 1024 and 2048, and through the separate
+    reduction kernel (D / 256 = 1, 2, 114, 1412, 18 363). Rings of 4 k sites:
+    of 4 k + 2 the ground state has momentum pi."""
+    from _bethe import heisenberg_ring_e0
+    from spined.model import build_model
+    b = build_model(lattices.heisenberg_chain(n))
+    res = sed.eigh(b.hamiltonian, seed=n)
+    assert res.residuals[0] <= RES_TOL
+    assert res.eigenvalues[0] == pytest.approx(heisenberg_ring_e0(n), rel=EV_RTOL)
