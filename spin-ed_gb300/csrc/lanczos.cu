@@ -32,8 +32,6 @@ namespace sed {
 namespace {
 
 constexpr unsigned kMaxNev = 16;
-constexpr unsigned kRedThreads = 1024;
-constexpr unsigned kVecBlocks = 152 * 8;  // grid of the vector kernels
 
 // What the step kernels share in device memory. alpha and beta follow it in
 // the same buffer (state_bytes), so that one copy per chunk of steps shows
@@ -121,7 +119,7 @@ int apply_with_alpha(Indirect ind, uint64_t D, cudaStream_t stream, Apply&& appl
   return LS_SUCCESS;
 }
 
-// Fused fixed-point Lanczos step (FP64, one vector): k_update leaves max |w|
+// Fused fixed-point Lanczos step (FP64): the last kernel that changes w leaves max |w|
 // (bit pattern) in *wmax and k_scale_next writes, next to v_{k+1} = w /
 // beta_k, the next matvec's gather copy u = round(sqrt(S) v_{k+1} 2^F) and
 // F, so that matvec skips its own pre-pass. `on` is false otherwise.
@@ -134,8 +132,20 @@ struct FixStep {
   FixView fv;
 };
 
-// w = w - alpha_k v_k - beta_{k-1} v_{k-1}; beta_k = ||w|| (by the last block).
-template <class X>
+// *out = max(*out, the block's largest m); red holds one word per warp.
+__device__ __forceinline__ void block_max_to(unsigned long long m, unsigned long long* red, unsigned long long* out) {
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (unsigned q = 1; q < kBlock / 32; ++q) m = max(m, red[q]);
+    atomicMax(out, m);
+  }
+}
+
+// w = w - alpha_k v_k - beta_{k-1} v_{k-1}; with Norm also beta_k = ||w|| (by
+// the last block) and max |w| (otherwise the Gram-Schmidt passes follow).
+template <class X, bool Norm>
 __global__ void k_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader const* h,
                          double const* __restrict__ alpha, double* __restrict__ beta,
                          double* __restrict__ partial, uint32_t* __restrict__ done,
@@ -163,51 +173,67 @@ __global__ void k_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader 
       wi.im = fma(-a, vi.im, fma(-b, vpi.im, wi.im));
     }
     Store<X>::store(w, i, wi);
+    if constexpr (!Norm) continue;
     part += dot_re(wi, wi);
     if constexpr (std::is_same<Vt, double>::value)
       m = max(m, (unsigned long long)__double_as_longlong(wi) & 0x7FFFFFFFFFFFFFFFull);
   }
+  if constexpr (!Norm) return;
   double const tot = block_sum(part, red);
-  if (wmax) {
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) redm[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (unsigned q = 1; q < kBlock / 32; ++q) m = max(m, redm[q]);
-      atomicMax(wmax, m);
-    }
-  }
+  if (wmax) block_max_to(m, redm, wmax);
   finish_sum(tot, partial, done, [&](double s) { beta[k] = sqrt(s); });
 }
 
 // Classical Gram-Schmidt pass against V[0..k]: c_j = <V_j, w> (partials per
-// block and vector, 16 vectors per blockIdx.y). The vector count NJ of the
-// block's group is a template parameter of the loop body, chosen on the
-// device from k: a predicated-off FP64 FMA still takes its issue slot on
-// GB300's slow FP64 pipe, so the body never pads to 16.
+// block and vector, 16 vectors per blockIdx.y). FP64 issue bounds it (1.75
+// lanes per clock and SM): one FMA per element, and one addition per element
+// to add a block's 256 products where each thread has about one row (D near
+// 304 000). The 16 sums of a warp are transposed while they are added (8 + 4
+// + 2 + 1 + 1 additions per lane instead of 16 x 5; each pair of lanes adds
+// the same two numbers as a butterfly of one sum, so the bits are the same):
+// 251 -> 103 us per pass over 56 vectors of 361 270 rows on average. The
+// vector count NJ of the block's group is a template parameter of the loop
+// body, chosen on the device from k: a predicated-off FP64 FMA still takes
+// its issue slot, so the body never pads to 16.
 template <int NJ, class X>
 __device__ __forceinline__ void cgs_dots_body(X const* __restrict__ V, uint64_t ld_v, uint64_t D, X const* w,
-                                              uint32_t j0, double* red, double* __restrict__ partial) {
-  double acc[NJ];
+                                              uint32_t j0, double (*red)[16], double* __restrict__ partial) {
+  double acc[16];
 #pragma unroll
-  for (int j = 0; j < NJ; ++j) acc[j] = 0.0;
+  for (int j = 0; j < 16; ++j) acc[j] = 0.0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D;
        i += (uint64_t)gridDim.x * blockDim.x) {
     auto const wi = Store<X>::load(w, i);
 #pragma unroll
     for (int j = 0; j < NJ; ++j) acc[j] += dot_re(Store<X>::load(V + (uint64_t)(j0 + j) * ld_v, i), wi);
   }
+  // after the step with offset o a lane holds the sums j whose bit o / 2 is
+  // set as its own lane bit o is
+  uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    double const t = block_sum(acc[j], red);
-    if (threadIdx.x == 0) partial[(uint64_t)(j0 + j) * gridDim.x + blockIdx.x] = t;
+  for (int o = 16; o >= 2; o >>= 1) {
+    bool const up = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (j >= o / 2) break;
+      double const give = up ? acc[j] : acc[j + o / 2], keep = up ? acc[j + o / 2] : acc[j];
+      acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+  if (!(lane & 1)) red[warp][lane >> 1] = acc[0];
+  __syncthreads();
+  if (threadIdx.x < NJ) {
+    double t = 0.0;
+    for (int q = 0; q < (int)kBlock / 32; ++q) t += red[q][threadIdx.x];
+    partial[(uint64_t)(j0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
   }
 }
 
 template <class X>
 __global__ void k_cgs_dots(X const* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader const* h,
                            double* __restrict__ partial /* [m_max][gridDim.x] */) {
-  __shared__ double red[kBlock / 32];
+  __shared__ double red[kBlock / 32][16];
   if (h->stop) return;
   uint32_t const k = h->k;
   uint32_t const j0 = blockIdx.y * 16;
@@ -223,29 +249,33 @@ __global__ void k_cgs_dots(X const* __restrict__ V, uint64_t ld_v, uint64_t D, L
   }
 }
 
-__global__ void k_cgs_reduce(double const* __restrict__ partial, unsigned nb, LzHeader const* h,
-                             double* __restrict__ coef, double* __restrict__ alpha) {
-  __shared__ double red[kRedThreads / 32];
-  if (h->stop) return;
-  uint32_t const k = h->k;
-  for (uint32_t j = 0; j <= k; ++j) {
-    double s = 0.0;
-    for (unsigned i = threadIdx.x; i < nb; i += blockDim.x) s += partial[(uint64_t)j * nb + i];
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) {
-      coef[j] = s;
-      if (j == k) alpha[k] += s;  // the projection on v_k corrects alpha_k
-    }
+// c_j = the sum of vector j's partials, one block per vector (as one block
+// for all of them: 190 us at 56 vectors on average; 5 us so).
+__global__ void __launch_bounds__(1024) k_cgs_reduce(double const* __restrict__ partial, unsigned nb,
+                                                     LzHeader const* h, double* __restrict__ coef,
+                                                     double* __restrict__ alpha) {
+  __shared__ double red[1024 / 32];
+  uint32_t const k = h->k, j = blockIdx.x;
+  if (h->stop || j > k) return;
+  double s = 0.0;
+  for (unsigned i = threadIdx.x; i < nb; i += blockDim.x) s += partial[(uint64_t)j * nb + i];
+  s = block_sum(s, red);
+  if (threadIdx.x == 0) {
+    coef[j] = s;
+    if (j == k) alpha[k] += s;  // the projection on v_k corrects alpha_k
   }
 }
 
-// w -= sum_j c_j V_j; beta_k = ||w||.
-template <class X>
-__global__ void k_cgs_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader const* h,
+// w -= sum_j c_j V_j; on the last pass also beta_k = ||w|| and (wmax not
+// null) max |w|.
+template <class X, bool Last>
+__global__ void __launch_bounds__(kBlock) k_cgs_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHeader const* h,
                              double const* __restrict__ coef, double* __restrict__ beta,
-                             double* __restrict__ partial, uint32_t* __restrict__ done) {
+                             double* __restrict__ partial, uint32_t* __restrict__ done,
+                             unsigned long long* __restrict__ wmax) {
   using Vt = typename Store<X>::V;
   __shared__ double red[kBlock / 32];
+  __shared__ unsigned long long redm[kBlock / 32];
   __shared__ double c[2048];
   if (h->stop) return;
   uint32_t const k = h->k;
@@ -253,9 +283,11 @@ __global__ void k_cgs_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHea
   __syncthreads();
   X* w = V + (uint64_t)(k + 1) * ld_v;
   double part = 0.0;
+  unsigned long long m = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D;
        i += (uint64_t)gridDim.x * blockDim.x) {
     Vt wi = Store<X>::load(w, i);
+#pragma unroll 8
     for (uint32_t j = 0; j <= k; ++j) {
       Vt const vj = Store<X>::load(V + (uint64_t)j * ld_v, i);
       if constexpr (std::is_same<Vt, double>::value) {
@@ -266,10 +298,17 @@ __global__ void k_cgs_update(X* __restrict__ V, uint64_t ld_v, uint64_t D, LzHea
       }
     }
     Store<X>::store(w, i, wi);
-    part += dot_re(wi, wi);
+    if constexpr (Last) {
+      part += dot_re(wi, wi);
+      if constexpr (std::is_same<Vt, double>::value)
+        m = max(m, (unsigned long long)__double_as_longlong(wi) & 0x7FFFFFFFFFFFFFFFull);
+    }
   }
-  double const tot = block_sum(part, red);
-  finish_sum(tot, partial, done, [&](double t) { beta[k] = sqrt(t); });
+  if constexpr (Last) {
+    double const tot = block_sum(part, red);
+    if (wmax) block_max_to(m, redm, wmax);
+    finish_sum(tot, partial, done, [&](double t) { beta[k] = sqrt(t); });
+  }
 }
 
 // Ends the step: the last block to get here advances k, or stops the run
@@ -574,7 +613,7 @@ struct Solver {
   unsigned vblocks = 0;
   bool reorth = false;
   Cycle cycle;
-  FixStep fx{};            // fused fixed-point step (FP64, one vector, stream form)
+  FixStep fx{};            // fused fixed-point step (FP64, stream form)
 
   Solver(OperatorData& o, int dt, cudaStream_t s) : op(o), dtype(dt), D(o.basis->D), stream(s) {}
   ~Solver() {
@@ -606,7 +645,7 @@ struct Solver {
     SED_TRY_CUDA(cudaMemsetAsync(ws.state.ptr, 0, state_bytes(m_max), stream));
     SED_TRY_CUDA(cudaMemsetAsync(ws.done.ptr, 0, 16, stream));
     FixSlots fs;
-    if (std::is_same<X, double>::value && !reorth && fix_slots(op, &fs))
+    if (std::is_same<X, double>::value && fix_slots(op, &fs))
       fx = FixStep{true, fs.max_bits, fs.F, fs.u, fs.row_class, fs.view};
     return LS_SUCCESS;
   }
@@ -635,19 +674,23 @@ struct Solver {
     ind.partial = partial;
     ind.done = done;
     ind.sum = alpha;
-    ind.clear = fx.on ? fx.wmax : nullptr;  // k_update's max |w| starts at zero
+    ind.clear = fx.on ? fx.wmax : nullptr;  // the step's max |w| starts at zero
     ind.prescaled = fx.on;
     if (int st = apply_with_alpha(ind, D, stream, [&](Indirect i) { return operator_apply_krylov(op, dtype, V(), i, stream); }))
       return st;
-    { k_update<X><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, alpha, beta, partial, done, fx.on ? fx.wmax : nullptr); note_launches(1); }
-    if (reorth) {
+    unsigned long long* const wmax = fx.on ? fx.wmax : nullptr;
+    if (!reorth) {
+      { k_update<X, true><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, alpha, beta, partial, done, wmax); note_launches(1); }
+    } else {
+      double *cp = ws.cgs_partial.template as<double>(), *coef = ws.coef.template as<double>();
+      { k_update<X, false><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, alpha, beta, partial, done, nullptr); note_launches(1); }
       for (int pass = 0; pass < 2; ++pass) {
         dim3 grid(vblocks, (m_max + 15) / 16);
-        { k_cgs_dots<X><<<grid, kBlock, 0, stream>>>(V(), D, D, h, ws.cgs_partial.template as<double>()); note_launches(1); }
-        { k_cgs_reduce<<<1, kRedThreads, 0, stream>>>(ws.cgs_partial.template as<double>(), vblocks, h,
-                                                    ws.coef.template as<double>(), alpha); note_launches(1); }
-        { k_cgs_update<X><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, ws.coef.template as<double>(), beta, partial,
-                                                        done); note_launches(1); }
+        { k_cgs_dots<X><<<grid, kBlock, 0, stream>>>(V(), D, D, h, cp); note_launches(1); }
+        { k_cgs_reduce<<<m_max, 1024, 0, stream>>>(cp, vblocks, h, coef, alpha); note_launches(1); }
+        if (pass == 0) { k_cgs_update<X, false><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, coef, beta, partial, done, nullptr); }
+        else { k_cgs_update<X, true><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, coef, beta, partial, done, wmax); }
+        note_launches(1);
       }
     }
     { k_scale_next<X><<<vblocks, kBlock, 0, stream>>>(V(), D, D, h, beta, done, fx); note_launches(1); }
