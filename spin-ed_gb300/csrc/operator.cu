@@ -343,12 +343,11 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert(double const* __restrict
                                                         uint32_t const* __restrict__ weights, CodeView C, FixView fv,
                                                         unsigned long long const* __restrict__ max_bits,
                                                         int64_t* __restrict__ F_out, int64_t* __restrict__ u,
-                                                        uint64_t ldu, Indirect ind) {
+                                                        Indirect ind) {
   __shared__ double fac[kFixMaxClasses];
   if (ind.stop && *ind.stop) return;
   if (ind.k) x += (uint64_t)*ind.k * ind.ld;
   x += (uint64_t)blockIdx.y * ldx;
-  u += (uint64_t)blockIdx.y * ldu;
   int64_t const F = fix_exponent(max_bits[blockIdx.y], fv.bound);
   if (blockIdx.x == 0 && threadIdx.x == 0) F_out[blockIdx.y] = F;
   // x 2^F sqrt(S) as (x 2^F1) (sqrt(S) 2^F2): F1 = 0 unless 2^F is not a
@@ -359,6 +358,7 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert(double const* __restrict
   double const p2 = F == kFixBad ? 0.0 : fix_pow2(F - F1);
   for (uint32_t c = threadIdx.x; c < fv.n_div; c += blockDim.x) fac[c] = fv.sqrt_s[c] * p2;
   __syncthreads();
+  if (blockIdx.x == 0 && threadIdx.x == 0) u[D] = 0;  // the zero row (fix_row_sums)
   if (F1 == 0) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (uint64_t)gridDim.x * blockDim.x) {
       uint32_t const cls = row_class ? (uint32_t)row_class[i] : divisor_class(weights[i], C);
@@ -370,53 +370,6 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert(double const* __restrict
       u[i] = fix_round((x[i] * p1) * fac[cls]);
     }
   }
-}
-
-// Adds +-g to the accumulator of value index t >> 1 (sign t & 1).
-template <int NV>
-__device__ __forceinline__ void fix_add(int64_t (&acc)[NV], uint32_t t, int64_t g) {
-  int64_t const v = (t & 1u) ? -g : g;
-  if constexpr (NV == 1) {
-    acc[0] += v;
-  } else {
-    uint32_t const q = t >> 1;
-#pragma unroll
-    for (int k = 0; k < NV; ++k)
-      if (q == (uint32_t)k) acc[k] += v;
-  }
-}
-
-// The row factors g[cls NV + v] = (c_v / sqrt(S_cls)) 2^-min(F, 1000), one
-// table per block in shared memory (one rounding of c_v / sqrt(S), then an
-// exact power of two). F above 1000 only occurs for vectors whose largest
-// entry is below about 1e-290; the rest of the scaling is then applied by
-// fix_row after the sum, so that g stays a normal number. Every thread of
-// the block calls it; the caller synchronises.
-template <int NV>
-__device__ __forceinline__ void fix_row_factors(FixView const& fv, double const* __restrict__ inv_sqrt_s, int64_t F,
-                                                double* g) {
-  int64_t const Fa = F > 1000 ? 1000 : F;
-  for (uint32_t t = threadIdx.x; t < fv.n_div * NV; t += blockDim.x)
-    g[t] = F == kFixBad ? 0.0 : fix_ldexp(__dmul_rn(inv_sqrt_s[t / NV], fv.c[t % NV]), -Fa);
-}
-
-// The row's epilogue, shared by every fixed-point kernel so that all of them
-// round identically: y_i = d_i x_i + sum_v g[cls][v] acc_v (times
-// 2^-(F - 1000) when F > 1000), with g from fix_row_factors (g points at the
-// row's class).
-template <int NV>
-__device__ __forceinline__ double fix_row(int64_t const (&acc)[NV], double const* g, int64_t F, double dg, double xi) {
-  if (F == kFixBad) return __longlong_as_double(0x7FF8000000000000ll);  // NaN in x gives NaN out
-  if (F > 1000) {
-    double o = 0.0;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) o = __fma_rn(g[k], __ll2double_rn(acc[k]), o);
-    return __fma_rn(o, fix_pow2(1000 - F), __dmul_rn(dg, xi));
-  }
-  double s = __dmul_rn(dg, xi);
-#pragma unroll
-  for (int k = 0; k < NV; ++k) s = __fma_rn(g[k], __ll2double_rn(acc[k]), s);
-  return s;
 }
 
 // Sum of one double per thread over the block, in a fixed order, through
@@ -433,16 +386,15 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* buf) {
   return s;
 }
 
-// Streamed SpMV over SELL-32 slices in fixed point (real operators). Four
-// entries per step: their loads, then their gathers, are issued back to back
-// (a padding slot gathers nothing and adds zero). Indirect (Krylov) mode as
-// in k_spmv.
-template <bool Packed, int NV>
+// Streamed SpMV over SELL-32 slices in fixed point (real operators), eight
+// elements in flight per row (fix_row_sums). Indirect (Krylov) mode as in
+// k_spmv.
+template <bool Packed, int NV, bool Signed>
 __global__ void __launch_bounds__(kBlock) k_spmv_fix(StreamView S, FixView fv, uint64_t D,
                                                      double const* __restrict__ x, int64_t const* __restrict__ u,
                                                      int64_t const* __restrict__ F_in, double* __restrict__ y,
                                                      Indirect ind) {
-  extern __shared__ double fix_smem[];  // g[n_div NV], then code8[n_codes]
+  extern __shared__ double fix_smem[];  // g[n_div NV], then the code bytes
   __shared__ double red[kBlock];
   if (ind.stop && *ind.stop) return;  // uniform across the grid
   if (ind.k) {
@@ -453,7 +405,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix(StreamView S, FixView fv, u
   int64_t const F = F_in[0];
   double* g = fix_smem;
   uint8_t* code8 = reinterpret_cast<uint8_t*>(fix_smem + fv.n_div * NV);
-  for (uint32_t c = threadIdx.x; c < fv.n_codes; c += blockDim.x) code8[c] = fv.code[c];
+  if constexpr (Signed) fix_stage_codes(fv, code8);
   fix_row_factors<NV>(fv, S.inv_sqrt_s, F, g);
   __syncthreads();
   uint64_t const i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -463,43 +415,15 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix(StreamView S, FixView fv, u
     uint32_t const lane = threadIdx.x & 31;
     uint64_t const base = S.slice_ptr[s];
     uint32_t const width = (uint32_t)((S.slice_ptr[s + 1] - base) >> 5);
-    uint32_t const col_mask = Packed ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
-    int64_t acc[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = 0;
     uint32_t const* ent = S.entries + base + lane;
-    constexpr uint32_t U = 8;
-    uint32_t e = 0;
-    for (; e + U <= width; e += U) {
-      uint32_t v[U];
-#pragma unroll
-      for (uint32_t q = 0; q < U; ++q) v[q] = __ldcs(ent + (uint64_t)(e + q) * 32);
-      int64_t g[U];
-      uint32_t t[U];
-#pragma unroll
-      for (uint32_t q = 0; q < U; ++q) {
-        g[q] = 0;
-        t[q] = 0;
-        if (v[q] != kNull) {
-          uint32_t const code =
-              Packed ? (v[q] >> S.col_bits) : (uint32_t)__ldcs(S.codes + base + lane + (uint64_t)(e + q) * 32);
-          g[q] = u[v[q] & col_mask];
-          t[q] = code8[code];
-        }
-      }
-#pragma unroll
-      for (uint32_t q = 0; q < U; ++q) fix_add<NV>(acc, t[q], g[q]);
-    }
-    for (; e < width; ++e) {
-      uint32_t const v = __ldcs(ent + (uint64_t)e * 32);
-      if (v != kNull) {
-        uint32_t const code = Packed ? (v >> S.col_bits) : (uint32_t)__ldcs(S.codes + base + lane + (uint64_t)e * 32);
-        fix_add<NV>(acc, code8[code], u[v & col_mask]);
-      }
-    }
+    int64_t acc[1][NV];
+    fix_row_sums<Packed, NV, Signed, 1, 8>(
+        S, fv, code8, S.codes + base + lane, width, (uint32_t)D, acc,
+        [&](uint32_t e) { return __ldcs(ent + (uint64_t)e * 32); }, [&](uint32_t col, int64_t* v) { v[0] = u[col]; },
+        int64_t{});
     if (i < D) {
       double const xi = __ldcs(x + i);
-      double const yi = fix_row<NV>(acc, g + (uint32_t)__ldcs(S.row_class + i) * NV, F,
+      double const yi = fix_row<NV>(acc[0], g + (uint32_t)__ldcs(S.row_class + i) * NV, F,
                                     __ldcs(static_cast<double const*>(S.diag) + i), xi);
       __stcs(y + i, yi);
       part = xi * yi;
@@ -508,52 +432,6 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix(StreamView S, FixView fv, u
   if (ind.partial) {
     double const tot = block_sum_fixed(part, red);
     finish_apply(tot, ind);
-  }
-}
-
-// Block form in fixed point: K columns, u column c at u + c * D, F_in[c].
-template <bool Packed, int NV, int K>
-__global__ void __launch_bounds__(kBlock) k_spmv_block_fix(StreamView S, FixView fv, uint64_t D,
-                                                           double const* __restrict__ x, uint64_t ldx,
-                                                           int64_t const* __restrict__ u,
-                                                           int64_t const* __restrict__ F_in, double* __restrict__ y,
-                                                           uint64_t ldy) {
-  extern __shared__ double fix_smem[];  // g[K][n_div NV], then code8[n_codes]
-  uint8_t* code8 = reinterpret_cast<uint8_t*>(fix_smem + K * fv.n_div * NV);
-  for (uint32_t c = threadIdx.x; c < fv.n_codes; c += blockDim.x) code8[c] = fv.code[c];
-#pragma unroll
-  for (int c = 0; c < K; ++c) fix_row_factors<NV>(fv, S.inv_sqrt_s, F_in[c], fix_smem + c * fv.n_div * NV);
-  __syncthreads();
-  uint64_t const i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  uint64_t const s = i >> 5;
-  if ((s << 5) >= D) return;
-  uint32_t const lane = threadIdx.x & 31;
-  uint64_t const base = S.slice_ptr[s];
-  uint32_t const width = (uint32_t)((S.slice_ptr[s + 1] - base) >> 5);
-  uint32_t const col_mask = Packed ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
-  int64_t acc[K][NV];
-#pragma unroll
-  for (int c = 0; c < K; ++c)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) acc[c][k] = 0;
-  uint32_t const* ent = S.entries + base + lane;
-  for (uint32_t e = 0; e < width; ++e) {
-    uint32_t const v = __ldcs(ent + (uint64_t)e * 32);
-    if (v != kNull) {
-      uint32_t const col = v & col_mask;
-      uint32_t const code = Packed ? (v >> S.col_bits) : (uint32_t)__ldcs(S.codes + base + lane + (uint64_t)e * 32);
-      uint32_t const t = code8[code];
-#pragma unroll
-      for (int c = 0; c < K; ++c) fix_add<NV>(acc[c], t, u[(uint64_t)c * D + col]);
-    }
-  }
-  if (i < D) {
-    uint32_t const cls = S.row_class[i];
-    double const dg = static_cast<double const*>(S.diag)[i];
-#pragma unroll
-    for (int c = 0; c < K; ++c)
-      y[(uint64_t)c * ldy + i] =
-          fix_row<NV>(acc[c], fix_smem + (c * fv.n_div + cls) * NV, F_in[c], dg, x[(uint64_t)c * ldx + i]);
   }
 }
 
@@ -1009,6 +887,9 @@ int build_tables(OperatorData& op) {
     t->fix.bound = (double)std::max<uint64_t>(1, op.row_bound) * sq[n_div - 1] * (1.0 + 1e-9);
     t->fix.sqrt_s_max = sq[n_div - 1] * (1.0 + 1e-9);
     for (uint32_t v = 0; v < kFixMaxValues; ++v) t->fix.c[v] = v < n_val ? op.off_values[2 * v] : 0.0;
+    bool const one = std::all_of(b.group.phase.begin(), b.group.phase.end(), [](uint32_t ph) { return ph == 0; });
+    t->fix.one_sign = one && b.inv >= 0 ? 1u : 0u;
+    t->fix.second = n_ph * n_div;
     t->fix_nv = n_val <= 1 ? 1u : (n_val <= 2 ? 2u : 4u);
     t->fix_ok = true;
   }
@@ -1192,7 +1073,8 @@ int operator_record_stream(OperatorData& op, cudaStream_t stream) {
   uint64_t const D = b.D;
   uint64_t const n_slices = (D + 31) / 32;
   unsigned col_bits = 1;
-  while (col_bits < 32 && ((uint64_t)1 << col_bits) < std::max<uint64_t>(D, 2)) ++col_bits;
+  // 2^col_bits > D: the column of a padding slot (all bits set) is not a row
+  while (col_bits < 32 && ((uint64_t)1 << col_bits) <= std::max<uint64_t>(D, 1)) ++col_bits;
   if (D >= ((uint64_t)1 << 32) - 1)
     return fail(LS_OUT_OF_MEMORY, "stream form supports fewer than 2^32 - 1 representatives");
   unsigned code_bits = 0;
@@ -1390,9 +1272,17 @@ int operator_record_stream(OperatorData& op, cudaStream_t stream) {
 int fix_reserve(OperatorData& op, uint32_t cols) {
   if (!op.tables || !op.tables->fix_ok || op.fix_cols >= cols) return LS_SUCCESS;
   uint64_t const D = std::max<uint64_t>(1, op.basis->D);
-  if (int st = op.fix_u.allocate(D * cols * 8)) return st;
-  if (int st = op.fix_slots.allocate((size_t)cols * 16)) return st;
   if (!op.fix_event) SED_TRY_CUDA(cudaEventCreateWithFlags(&op.fix_event, cudaEventDisableTiming));
+  DeviceBuffer slots;
+  if (int st = slots.allocate((size_t)cols * 16)) return st;
+  uint32_t const had = op.fix_cols;
+  op.fix_cols = 0;
+  if (int st = op.fix_u.allocate((D + 1) * cols * 8)) {
+    // the narrower workspace goes back, so that narrower passes still run
+    if (had && op.fix_u.allocate((D + 1) * had * 8) == LS_SUCCESS) op.fix_cols = had;
+    return st;
+  }
+  op.fix_slots = std::move(slots);
   op.fix_cols = cols;
   return LS_SUCCESS;
 }
@@ -1404,15 +1294,15 @@ int fix_wait(OperatorData& op) {
 
 namespace {
 
-template <int NV>
 void launch_spmv_fix(OperatorData& op, StreamView const& S, double const* x, int64_t const* u, int64_t const* F,
                      double* y, cudaStream_t stream, Indirect ind) {
   StreamForm const& sf = op.stream;
   OperatorTables const& tb = *op.tables;
   unsigned const grid = (unsigned)((sf.n_slices * 32 + kBlock - 1) / kBlock);
-  size_t const smem = (size_t)tb.fix.n_div * NV * 8 + tb.fix.n_codes;
-  if (sf.packed) k_spmv_fix<true, NV><<<grid, kBlock, smem, stream>>>(S, tb.fix, op.basis->D, x, u, F, y, ind);
-  else k_spmv_fix<false, NV><<<grid, kBlock, smem, stream>>>(S, tb.fix, op.basis->D, x, u, F, y, ind);
+  fix_dispatch(tb, sf.packed, [&](auto packed, auto nv, auto sign) {
+    k_spmv_fix<packed.value, nv.value, sign.value>
+        <<<grid, kBlock, fix_smem_bytes(tb, 1), stream>>>(S, tb.fix, op.basis->D, x, u, F, y, ind);
+  });
   note_launches(1);
 }
 
@@ -1446,16 +1336,12 @@ int launch_apply_fix(OperatorData& op, double const* x, double* y, cudaStream_t 
     unsigned const vg = grid_size(D, b.device, 8);
     k_fix_max<<<vg, kBlock, 0, stream>>>(x, 0, D, mx, ind);
     k_fix_convert<<<vg, kBlock, 0, stream>>>(x, 0, D, use_stream ? op.stream.row_class.as<uint8_t>() : nullptr,
-                                             b.weights.as<uint32_t>(), tb.code, tb.fix, mx, F, u, D, ind);
+                                             b.weights.as<uint32_t>(), tb.code, tb.fix, mx, F, u, ind);
     note_launches(2);
   }
   if (use_stream) {
     StreamView const S = stream_view(op);
-    switch (tb.fix_nv) {
-      case 1: launch_spmv_fix<1>(op, S, x, u, F, y, stream, ind); break;
-      case 2: launch_spmv_fix<2>(op, S, x, u, F, y, stream, ind); break;
-      default: launch_spmv_fix<4>(op, S, x, u, F, y, stream, ind); break;
-    }
+    launch_spmv_fix(op, S, x, u, F, y, stream, ind);
   } else if (b.plan.n_bits > 32) {
     switch (tb.fix_nv) {
       case 1: launch_otf_fix<uint64_t, 1>(op, x, u, F, y, stream, ind); break;
@@ -1499,7 +1385,7 @@ int fix_prescale(OperatorData& op, double const* base, Indirect ind, cudaStream_
   unsigned const vg = grid_size(b.D, b.device, 8);
   k_fix_max<<<vg, kBlock, 0, stream>>>(base, 0, b.D, fs.max_bits, ind);
   k_fix_convert<<<vg, kBlock, 0, stream>>>(base, 0, b.D, fs.row_class, b.weights.as<uint32_t>(), op.tables->code,
-                                           fs.view, fs.max_bits, fs.F, fs.u, b.D, ind);
+                                           fs.view, fs.max_bits, fs.F, fs.u, ind);
   note_launches(2);
   SED_TRY_CUDA(cudaGetLastError());
   return LS_SUCCESS;
@@ -1583,59 +1469,8 @@ void launch_block_k(unsigned K, StreamView const& S, uint64_t D, X const* x, uin
   }
 }
 
-template <int NV, bool Pk>
-void launch_block_fix_k(unsigned K, StreamView const& S, FixView const& fv, uint64_t D, double const* x, uint64_t ldx,
-                        int64_t const* u, int64_t const* F, double* y, uint64_t ldy, unsigned grid, size_t smem,
-                        cudaStream_t stream) {
-  switch (K) {
-    case 16: k_spmv_block_fix<Pk, NV, 16><<<grid, kBlock, smem, stream>>>(S, fv, D, x, ldx, u, F, y, ldy); break;
-    case 8: k_spmv_block_fix<Pk, NV, 8><<<grid, kBlock, smem, stream>>>(S, fv, D, x, ldx, u, F, y, ldy); break;
-    case 4: k_spmv_block_fix<Pk, NV, 4><<<grid, kBlock, smem, stream>>>(S, fv, D, x, ldx, u, F, y, ldy); break;
-    default: k_spmv_block_fix<Pk, NV, 2><<<grid, kBlock, smem, stream>>>(S, fv, D, x, ldx, u, F, y, ldy); break;
-  }
-  note_launches(1);
-}
-
-// K columns in fixed point (the same per-column sums as launch_apply_fix).
-int launch_block_fix(OperatorData& op, unsigned K, double const* x, uint64_t ldx, double* y, uint64_t ldy,
-                     cudaStream_t stream) {
-  if (int st = fix_reserve(op, K)) return st;
-  BasisData& b = *op.basis;
-  OperatorTables const& tb = *op.tables;
-  StreamForm const& sf = op.stream;
-  uint64_t const D = b.D;
-  auto* mx = op.fix_slots.as<unsigned long long>();
-  auto* F = reinterpret_cast<int64_t*>(mx + op.fix_cols);
-  int64_t* u = op.fix_u.as<int64_t>();
-  if (op.fix_event_recorded) SED_TRY_CUDA(cudaStreamWaitEvent(stream, op.fix_event, 0));
-  SED_TRY_CUDA(cudaMemsetAsync(mx, 0, (size_t)K * 8, stream));
-  dim3 const vg(grid_size(D, b.device, 8), K);
-  k_fix_max<<<vg, kBlock, 0, stream>>>(x, ldx, D, mx, Indirect{});
-  k_fix_convert<<<vg, kBlock, 0, stream>>>(x, ldx, D, sf.row_class.as<uint8_t>(), b.weights.as<uint32_t>(), tb.code,
-                                           tb.fix, mx, F, u, D, Indirect{});
-  note_launches(2);
-  StreamView const S = stream_view(op);
-  unsigned const grid = (unsigned)((sf.n_slices * 32 + kBlock - 1) / kBlock);
-  size_t const smem = (size_t)K * tb.fix.n_div * tb.fix_nv * 8 + tb.fix.n_codes;
-  if (smem > 48 * 1024) return fail(LS_SYSTEM_ERROR, "fixed-point block matvec: tables exceed shared memory");
-  switch (tb.fix_nv * 2 + (sf.packed ? 1 : 0)) {
-    case 3: launch_block_fix_k<1, true>(K, S, tb.fix, D, x, ldx, u, F, y, ldy, grid, smem, stream); break;
-    case 2: launch_block_fix_k<1, false>(K, S, tb.fix, D, x, ldx, u, F, y, ldy, grid, smem, stream); break;
-    case 5: launch_block_fix_k<2, true>(K, S, tb.fix, D, x, ldx, u, F, y, ldy, grid, smem, stream); break;
-    case 4: launch_block_fix_k<2, false>(K, S, tb.fix, D, x, ldx, u, F, y, ldy, grid, smem, stream); break;
-    case 9: launch_block_fix_k<4, true>(K, S, tb.fix, D, x, ldx, u, F, y, ldy, grid, smem, stream); break;
-    default: launch_block_fix_k<4, false>(K, S, tb.fix, D, x, ldx, u, F, y, ldy, grid, smem, stream); break;
-  }
-  SED_TRY_CUDA(cudaGetLastError());
-  SED_TRY_CUDA(cudaEventRecord(op.fix_event, stream));
-  op.fix_event_recorded = true;
-  return LS_SUCCESS;
-}
-
 template <class X>
 int launch_block(OperatorData& op, unsigned K, X const* x, uint64_t ldx, X* y, uint64_t ldy, cudaStream_t stream) {
-  if constexpr (std::is_same<X, double>::value)
-    if (op.tables->fix_ok) return launch_block_fix(op, K, x, ldx, y, ldy, stream);
   using V = typename Store<X>::V;
   constexpr bool complex_storage = std::is_same<V, cplx>::value;
   StreamForm const& sf = op.stream;
@@ -1676,18 +1511,13 @@ int operator_apply_device(OperatorData& op, int dtype, uint64_t block, void cons
   }
   size_t const es = (size_t)elem_size(dtype);
   uint64_t c0 = 0;
-  // the fixed-point block kernel keeps K tables of row factors in shared
-  // memory: at most kmax columns per pass fit in 48 KB
-  unsigned kmax = 16;
-  if (dtype == 1 && op.tables->fix_ok) {
-    size_t const per = (size_t)op.tables->fix.n_div * op.tables->fix_nv * 8;
-    size_t const room = 48 * 1024 - op.tables->fix.n_codes;
-    kmax = (unsigned)std::min<size_t>(16, room / per);
-  }
-  if (use_stream && block > 1 && kmax >= 2) {
+  if (fix_cols_apply(op, dtype, block, use_stream, stream))
+    if (int st = fix_cols_blocks(op, dtype, block, static_cast<char const*>(x), ldx, static_cast<char*>(y), ldy, es, stream, &c0))
+      return st;
+  if (use_stream && !(dtype == 1 && op.tables->fix_ok && op.fix_cols >= 1)) {
     // K-column passes over the stream form (K = 16, 8, 4, 2)
     while (block - c0 >= 2) {
-      uint64_t const left = std::min<uint64_t>(block - c0, kmax);
+      uint64_t const left = std::min<uint64_t>(block - c0, 16);
       unsigned const K = left >= 16 ? 16 : left >= 8 ? 8 : left >= 4 ? 4 : 2;
       void const* xc = static_cast<char const*>(x) + c0 * ldx * es;
       void* yc = static_cast<char*>(y) + c0 * ldy * es;
@@ -1841,17 +1671,18 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert32(float const* __restric
   if (blockIdx.x == 0 && threadIdx.x == 0) F_out[0] = F;
   double const p2 = F == kFixBad ? 0.0 : fix_pow2(F);
   for (uint32_t c = threadIdx.x; c < fv.n_div; c += blockDim.x) fac[c] = fv.sqrt_s[c] * p2;
+  if (blockIdx.x == 0 && threadIdx.x == 0) u[D] = 0;  // the zero row (fix_row_sums)
   __syncthreads();
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (uint64_t)gridDim.x * blockDim.x)
     u[i] = F == kFixBad ? 0 : (int32_t)fix_round((double)x[i] * fac[row_class[i]]);
 }
 
-template <bool Packed, int NV>
+template <bool Packed, int NV, bool Signed>
 __global__ void __launch_bounds__(kBlock) k_spmv32_fix(StreamView S, FixView fv, uint64_t D,
                                                        float const* __restrict__ x, int32_t const* __restrict__ u,
                                                        int64_t const* __restrict__ F_in, float* __restrict__ y,
                                                        Indirect ind) {
-  extern __shared__ double fix_smem[];  // g[n_div NV], then code8[n_codes]
+  extern __shared__ double fix_smem[];  // g[n_div NV], then the code bytes
   __shared__ double red[kBlock / 32];
   if (ind.stop && *ind.stop) return;
   if (ind.k) {
@@ -1862,7 +1693,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv32_fix(StreamView S, FixView fv,
   int64_t const F = F_in[0];
   double* g = fix_smem;
   uint8_t* code8 = reinterpret_cast<uint8_t*>(fix_smem + fv.n_div * NV);
-  for (uint32_t c = threadIdx.x; c < fv.n_codes; c += blockDim.x) code8[c] = fv.code[c];
+  if constexpr (Signed) fix_stage_codes(fv, code8);
   fix_row_factors<NV>(fv, S.inv_sqrt_s, F, g);
   __syncthreads();
   uint64_t const i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1872,43 +1703,15 @@ __global__ void __launch_bounds__(kBlock) k_spmv32_fix(StreamView S, FixView fv,
     uint32_t const lane = threadIdx.x & 31;
     uint64_t const base = S.slice_ptr[s];
     uint32_t const width = (uint32_t)((S.slice_ptr[s + 1] - base) >> 5);
-    uint32_t const col_mask = Packed ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
-    int64_t acc[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = 0;
     uint32_t const* ent = S.entries + base + lane;
-    constexpr uint32_t U = 8;
-    uint32_t e = 0;
-    for (; e + U <= width; e += U) {
-      uint32_t v[U];
-#pragma unroll
-      for (uint32_t q = 0; q < U; ++q) v[q] = __ldcs(ent + (uint64_t)(e + q) * 32);
-      int32_t gv[U];
-      uint32_t t[U];
-#pragma unroll
-      for (uint32_t q = 0; q < U; ++q) {
-        gv[q] = 0;
-        t[q] = 0;
-        if (v[q] != kNull) {
-          uint32_t const code =
-              Packed ? (v[q] >> S.col_bits) : (uint32_t)__ldcs(S.codes + base + lane + (uint64_t)(e + q) * 32);
-          gv[q] = u[v[q] & col_mask];
-          t[q] = code8[code];
-        }
-      }
-#pragma unroll
-      for (uint32_t q = 0; q < U; ++q) fix_add<NV>(acc, t[q], (int64_t)gv[q]);
-    }
-    for (; e < width; ++e) {
-      uint32_t const v = __ldcs(ent + (uint64_t)e * 32);
-      if (v != kNull) {
-        uint32_t const code = Packed ? (v >> S.col_bits) : (uint32_t)__ldcs(S.codes + base + lane + (uint64_t)e * 32);
-        fix_add<NV>(acc, code8[code], (int64_t)u[v & col_mask]);
-      }
-    }
+    int64_t acc[1][NV];
+    fix_row_sums<Packed, NV, Signed, 1, 8>(
+        S, fv, code8, S.codes + base + lane, width, (uint32_t)D, acc,
+        [&](uint32_t e) { return __ldcs(ent + (uint64_t)e * 32); }, [&](uint32_t col, int32_t* v) { v[0] = u[col]; },
+        int32_t{});
     if (i < D) {
       float const xf = __ldcs(x + i);
-      double const yi = fix_row<NV>(acc, g + (uint32_t)__ldcs(S.row_class + i) * NV, F,
+      double const yi = fix_row<NV>(acc[0], g + (uint32_t)__ldcs(S.row_class + i) * NV, F,
                                     __ldcs(static_cast<double const*>(S.diag) + i), (double)xf);
       float const yf = (float)yi;
       __stcs(y + i, yf);
@@ -1938,7 +1741,7 @@ int operator_prepare_fp32(OperatorData& op, cudaStream_t stream) {
   OperatorTables const& tb = *op.tables;
   uint64_t const D = op.basis->D;
   if (tb.fix_ok) {
-    if (int st = op.fix_u32.allocate(std::max<uint64_t>(1, D) * 4)) return st;
+    if (int st = op.fix_u32.allocate((D + 1) * 4)) return st;
     if (int st = op.fix_slots32.allocate(16)) return st;
   }
   if (int st = sf.diag_f.allocate(std::max<uint64_t>(1, D) * 4)) return st;
@@ -1953,19 +1756,16 @@ int operator_prepare_fp32(OperatorData& op, cudaStream_t stream) {
 }
 
 namespace {
-template <int NV>
 void launch_spmv32_fix(OperatorData& op, StreamView const& S, float const* x, float* y, Indirect ind,
                        cudaStream_t stream, unsigned grid) {
   OperatorTables const& tb = *op.tables;
   auto* slots = op.fix_slots32.as<unsigned long long>();
   auto* F = reinterpret_cast<int64_t*>(slots + 1);
   int32_t* u = op.fix_u32.as<int32_t>();
-  uint64_t const D = op.basis->D;
-  size_t const smem = (size_t)tb.fix.n_div * NV * 8 + tb.fix.n_codes;
-  if (op.stream.packed)
-    k_spmv32_fix<true, NV><<<grid, kBlock, smem, stream>>>(S, tb.fix, D, x, u, F, y, ind);
-  else
-    k_spmv32_fix<false, NV><<<grid, kBlock, smem, stream>>>(S, tb.fix, D, x, u, F, y, ind);
+  fix_dispatch(tb, op.stream.packed, [&](auto packed, auto nv, auto sign) {
+    k_spmv32_fix<packed.value, nv.value, sign.value>
+        <<<grid, kBlock, fix_smem_bytes(tb, 1), stream>>>(S, tb.fix, op.basis->D, x, u, F, y, ind);
+  });
   note_launches(1);
 }
 
@@ -1984,11 +1784,7 @@ int launch32(OperatorData& op, float const* x, float* y, Indirect ind, cudaStrea
     k_fix_convert32<<<vg, kBlock, 0, stream>>>(x, D, sf.row_class.as<uint8_t>(), tb.fix, slots,
                                                reinterpret_cast<int64_t*>(slots + 1), op.fix_u32.as<int32_t>(), ind);
     note_launches(2);
-    switch (tb.fix_nv) {
-      case 1: launch_spmv32_fix<1>(op, S, x, y, ind, stream, grid); break;
-      case 2: launch_spmv32_fix<2>(op, S, x, y, ind, stream, grid); break;
-      default: launch_spmv32_fix<4>(op, S, x, y, ind, stream, grid); break;
-    }
+    launch_spmv32_fix(op, S, x, y, ind, stream, grid);
     SED_TRY_CUDA(cudaGetLastError());
     return LS_SUCCESS;
   }

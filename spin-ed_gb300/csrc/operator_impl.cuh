@@ -147,6 +147,8 @@ struct FixView {
   double bound;          // (largest row count) x sqrt(largest S), rounded up
   double sqrt_s_max;     // sqrt(largest S), rounded up
   double c[kFixMaxValues];
+  uint32_t one_sign;     // every character of the group is +1
+  uint32_t second;       // codes from here on carry the second value or a later one
 };
 
 // Nearest integer of a finite d with |d| < 2^62 (halves away from zero),
@@ -162,7 +164,7 @@ __device__ __forceinline__ int64_t fix_round(double d) {
   else if (sh >= 64)
     mag = 0;
   else
-    mag = (m + (1ull << (sh - 1))) >> sh;
+    mag = ((m >> (sh - 1)) + 1) >> 1;  // (m + 2^(sh-1)) >> sh
   return (b >> 63) ? -(int64_t)mag : (int64_t)mag;
 }
 
@@ -199,6 +201,130 @@ __device__ __forceinline__ double fix_ldexp(double a, int64_t p) {
   if (p >= -1000 && p <= 1000) return a * fix_pow2(p);
   int64_t const h = p / 2;
   return (a * fix_pow2(h)) * fix_pow2(p - h);
+}
+
+// Adds +-g to the accumulator of value index t >> 1 (sign t & 1).
+template <int NV>
+__device__ __forceinline__ void fix_add(int64_t (&acc)[NV], uint32_t t, int64_t g) {
+  int64_t const v = (t & 1u) ? -g : g;
+  if constexpr (NV == 1) {
+    acc[0] += v;
+  } else {
+    uint32_t const q = t >> 1;
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (q == (uint32_t)k) acc[k] += v;
+  }
+}
+
+// The row factors g[cls NV + v] = (c_v / sqrt(S_cls)) 2^-min(F, 1000), one
+// table per block in shared memory (one rounding of c_v / sqrt(S), then an
+// exact power of two). F above 1000 only occurs for vectors whose largest
+// entry is below about 1e-290; the rest of the scaling is then applied by
+// fix_row after the sum, so that g stays a normal number. Every thread of
+// the block calls it; the caller synchronises.
+template <int NV>
+__device__ __forceinline__ void fix_row_factors(FixView const& fv, double const* __restrict__ inv_sqrt_s, int64_t F,
+                                                double* g) {
+  int64_t const Fa = F > 1000 ? 1000 : F;
+  for (uint32_t t = threadIdx.x; t < fv.n_div * NV; t += blockDim.x)
+    g[t] = F == kFixBad ? 0.0 : fix_ldexp(__dmul_rn(inv_sqrt_s[t / NV], fv.c[t % NV]), -Fa);
+}
+
+// (double)v to nearest (ties to even) with integer instructions: the
+// conversion runs on the FP64 pipe.
+__device__ __forceinline__ double fix_to_double(int64_t v) {
+  uint64_t m = (uint64_t)(v < 0 ? -v : v);  // |v| < 2^62
+  int const z = __clzll((long long)m);
+  m <<= z & 63;
+  uint32_t const rest = (uint32_t)m & 0x7FFu;
+  uint64_t const top = m >> 11;
+  uint64_t b = ((uint64_t)(1085 - z) << 52) + top + ((rest > 0x400u || (rest == 0x400u && (top & 1))) ? 1u : 0u);
+  if (m == 0) b = 0;
+  return __longlong_as_double((long long)(b | (uint64_t)(v < 0) << 63));
+}
+
+// The row's epilogue, shared by every fixed-point kernel so that all of them
+// round identically: y_i = d_i x_i + sum_v g[cls][v] acc_v (times
+// 2^-(F - 1000) when F > 1000), with g from fix_row_factors (g points at the
+// row's class).
+template <int NV>
+__device__ __forceinline__ double fix_row(int64_t const (&acc)[NV], double const* g, int64_t F, double dg, double xi) {
+  if (F == kFixBad) return __longlong_as_double(0x7FF8000000000000ll);  // NaN in x gives NaN out
+  if (F > 1000) {
+    double o = 0.0;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) o = __fma_rn(g[k], fix_to_double(acc[k]), o);
+    return __fma_rn(o, fix_pow2(1000 - F), __dmul_rn(dg, xi));
+  }
+  double s = __dmul_rn(dg, xi);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) s = __fma_rn(g[k], fix_to_double(acc[k]), s);
+  return s;
+}
+
+// The code bytes and the zero byte behind them, by every thread of the block.
+__device__ __forceinline__ void fix_stage_codes(FixView const& fv, uint8_t* code8) {
+  for (uint32_t c = threadIdx.x; c <= fv.n_codes; c += blockDim.x) code8[c] = c < fv.n_codes ? fv.code[c] : 0;
+}
+
+// The integer sums of one row: N gathered columns per element, U elements in
+// flight; gather(col, g) fetches g[0..N). Where the gather copy stays in L2
+// the integer ALU limits it (64 lanes per clock and SM; about 40 instructions
+// per warp and element with the sign and the value looked up), so the loop
+// does without what an operator does not need:
+//  - characters all +1 (!Signed): no sign; one value: no code at all, two: a
+//    comparison of the entry;
+//  - a padding slot reads the zero row `zero_row` that every gather copy has
+//    behind its last row: no branch and no selection.
+// One column, 6x6 torus (585 M elements): 1147 -> 1116 us; 30-site J1-J2 ring
+// (40 M elements) 80 -> 72 us, eight columns of it 515 -> 345 us. Loading the
+// next step's entries before this step's sums gained nothing (72 to 76 us;
+// more copies in flight evict one another).
+template <bool Packed, int NV, bool Signed, int N, uint32_t U, class T, class Entry, class Gather>
+__device__ __forceinline__ void fix_row_sums(StreamView const& S, FixView const& fv, uint8_t const* code8,
+                                             uint16_t const* codes, uint32_t width, uint32_t zero_row,
+                                             int64_t (&acc)[N][NV], Entry&& entry, Gather&& gather, T) {
+  uint32_t const mask = Packed ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
+  uint32_t const second = Packed ? fv.second << S.col_bits : fv.second;
+  constexpr bool kCodes = !Packed && (NV > 1 || Signed);
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) acc[n][k] = 0;
+  auto step = [&](uint32_t e, auto guarded) {
+    uint32_t v[U], c[U];
+    T g[U][N];
+#pragma unroll
+    for (uint32_t p = 0; p < U; ++p) {
+      bool const in = !decltype(guarded)::value || e + p < width;
+      v[p] = in ? entry(e + p) : kNull;
+      if constexpr (kCodes) c[p] = in ? (uint32_t)__ldcs(codes + (uint64_t)(e + p) * 32) : 0u;
+    }
+#pragma unroll
+    for (uint32_t p = 0; p < U; ++p) gather(min(v[p] & mask, zero_row), g[p]);
+#pragma unroll
+    for (uint32_t p = 0; p < U; ++p) {
+      if constexpr (Signed) {
+        uint32_t const t = code8[Packed ? min(v[p] >> S.col_bits, fv.n_codes) : c[p]];
+#pragma unroll
+        for (int n = 0; n < N; ++n) fix_add<NV>(acc[n], t, (int64_t)g[p][n]);
+      } else if constexpr (NV == 1) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) acc[n][0] += g[p][n];
+      } else {
+        bool const later = (Packed ? v[p] : c[p]) >= second;
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          if (later) acc[n][1] += g[p][n];
+          else acc[n][0] += g[p][n];
+        }
+      }
+    }
+  };
+  uint32_t e = 0;
+  for (; e + U <= width; e += U) step(e, std::false_type{});
+  if (e < width) step(e, std::true_type{});
 }
 
 struct OperatorTables {
@@ -286,6 +412,37 @@ bool fix_slots(OperatorData& op, FixSlots* out);
 // The matvec's pre-pass on its own: max |x|, then u and F, for x = base (+ k
 // ld in Krylov mode).
 int fix_prescale(OperatorData& op, double const* base, Indirect ind, cudaStream_t stream);
+// Calls f(packed, nv, signed) with the integral constants of the
+// fixed-point kernel an operator takes. Unsigned variants exist where they
+// save the look-up: one value, or two in packed entries.
+template <class F>
+void fix_dispatch(OperatorTables const& tb, bool packed, F&& f) {
+  using Yes = std::true_type;
+  using No = std::false_type;
+  std::integral_constant<int, 1> n1;
+  std::integral_constant<int, 2> n2;
+  std::integral_constant<int, 4> n4;
+  bool const one = tb.fix.one_sign != 0;
+  if (packed) {
+    switch (tb.fix_nv) {
+      case 1: one ? f(Yes{}, n1, No{}) : f(Yes{}, n1, Yes{}); break;
+      case 2: one ? f(Yes{}, n2, No{}) : f(Yes{}, n2, Yes{}); break;
+      default: f(Yes{}, n4, Yes{}); break;
+    }
+  } else {
+    switch (tb.fix_nv) {
+      case 1: one ? f(No{}, n1, No{}) : f(No{}, n1, Yes{}); break;
+      case 2: f(No{}, n2, Yes{}); break;
+      default: f(No{}, n4, Yes{}); break;
+    }
+  }
+}
+// Shared memory of a fixed-point kernel over K columns: the row factors, then
+// the code bytes and a zero byte for padding slots.
+inline size_t fix_smem_bytes(OperatorTables const& tb, unsigned K) {
+  return (size_t)K * tb.fix.n_div * tb.fix_nv * 8 + tb.fix.n_codes + 1;
+}
+
 // FP32 streamed SpMV in Krylov-indirect mode (x = base + k ld, y = base +
 // (k+1) ld); FP32 arithmetic, per-block partial sums of x_i y_i in FP64.
 int operator_apply_krylov32(OperatorData& op, float* base, Indirect ind, cudaStream_t stream);
@@ -294,6 +451,13 @@ int operator_apply32(OperatorData& op, float const* x, float* y, cudaStream_t st
 // Krylov-indirect apply (see Indirect), on at most ceil(D / kBlock) blocks.
 int operator_apply_krylov(OperatorData& op, int dtype, void* base, Indirect ind, cudaStream_t stream);
 int operator_ensure_ready(OperatorData& op);
+
+// Whether streamed matvecs of this dtype take the integer sums of
+// fix_cols_blocks, and the first `block` columns through it (spmv_cols.cu);
+// *done counts the columns taken.
+bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_stream, cudaStream_t stream);
+int fix_cols_blocks(OperatorData& op, int dtype, uint64_t block, char const* x, uint64_t ldx, char* y, uint64_t ldy,
+                    size_t es, cudaStream_t stream, uint64_t* done);
 
 // V[:, 0..kk) <- V[:, 0..m) Y on the tensor cores (rotate_tc.cu): V FP64,
 // D x m with column stride ld, Y m x kk row-major FP64, both on the device;

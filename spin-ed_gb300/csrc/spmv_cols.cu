@@ -1,0 +1,341 @@
+// spmv_cols.cu — the streamed fixed-point matvec on blocks of columns and on
+// FP32 and complex vectors of real operators (src/SpinED/Internal.hs:411-429;
+// the mathematics is at FixView in operator_impl.cuh).
+//
+// A pass covers K real columns; a complex column is two. The gather copy u
+// holds the K columns of a row next to each other.
+#include "operator_impl.cuh"
+
+namespace sed {
+namespace {
+
+// FP32 and complex
+// vectors of a real operator take the same integer sums as FP64 ones: the
+// FP64 multiply-adds per element of k_spmv (two or four on a pipe of 1.75
+// per clock and SM, after an FP32 load a conversion on the same pipe) bound
+// it at 378 us where this takes 145 (ring of 32 sites, FP32).
+struct Columns {
+  void const* x;
+  void* y;
+  uint64_t ldx, ldy;  // in vector elements
+  uint32_t cols;      // real columns of this pass (the rest of K is padding)
+  bool f32, cx;
+  // offset of entry i of real column q, in reals
+  __device__ __forceinline__ uint64_t at(uint32_t q, uint64_t i, uint64_t ld) const {
+    return cx ? 2 * ((uint64_t)(q >> 1) * ld + i) + (q & 1u) : (uint64_t)q * ld + i;
+  }
+  __device__ __forceinline__ double load(uint32_t q, uint64_t i) const {
+    uint64_t const o = at(q, i, ldx);
+    return f32 ? (double)__ldcs(static_cast<float const*>(x) + o) : __ldcs(static_cast<double const*>(x) + o);
+  }
+  __device__ __forceinline__ void store(uint32_t q, uint64_t i, double v) const {
+    uint64_t const o = at(q, i, ldy);
+    if (f32) __stcs(static_cast<float*>(y) + o, (float)v);
+    else __stcs(static_cast<double*>(y) + o, v);
+  }
+};
+
+// (double)f from the bits: the conversion instruction runs on the FP64 pipe.
+__device__ __forceinline__ double widen(float f) {
+  uint32_t const b = __float_as_uint(f), e = (b >> 23) & 0xFFu;
+  if (e == 0 || e == 0xFF) return (double)f;
+  return __hiloint2double((int)((b & 0x80000000u) | ((e + 896u) << 20) | ((b & 0x7FFFFFu) >> 3)), (int)(b << 29));
+}
+
+// k_fix_max for Columns: blockIdx.y is the vector column.
+__global__ void __launch_bounds__(kBlock) k_fix_max_cols(Columns c, uint64_t D, unsigned long long* __restrict__ max_bits) {
+  __shared__ unsigned long long red[2][kBlock / 32];
+  unsigned long long m[2] = {0, 0};
+  uint64_t const n = c.cx ? 2 * D : D, o = (uint64_t)blockIdx.y * (c.cx ? 2 : 1) * c.ldx;
+  // blockDim and the stride are even: a thread sees one part of a complex column
+  uint64_t const first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+  unsigned long long v = 0;
+  if (c.f32) {
+    float const* p = static_cast<float const*>(c.x) + o;
+    uint32_t w = 0;
+    uint64_t i = first;
+    for (; i + 3 * step < n; i += 4 * step)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) w = max(w, __float_as_uint(p[i + k * step]) & 0x7FFFFFFFu);
+    for (; i < n; i += step) w = max(w, __float_as_uint(p[i]) & 0x7FFFFFFFu);
+    v = (unsigned long long)__double_as_longlong((double)__uint_as_float(w));  // keeps the order, infinities and NaN
+  } else {
+    double const* p = static_cast<double const*>(c.x) + o;
+    uint64_t i = first;
+    for (; i + 3 * step < n; i += 4 * step)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v = max(v, (unsigned long long)__double_as_longlong(p[i + k * step]) & 0x7FFFFFFFFFFFFFFFull);
+    for (; i < n; i += step) v = max(v, (unsigned long long)__double_as_longlong(p[i]) & 0x7FFFFFFFFFFFFFFFull);
+  }
+  m[c.cx ? (threadIdx.x & 1u) : 0u] = v;
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    for (int d = 16; d > 0; d >>= 1) m[p] = max(m[p], __shfl_xor_sync(0xffffffffu, m[p], d));
+    if ((threadIdx.x & 31) == 0) red[p][threadIdx.x >> 5] = m[p];
+  }
+  __syncthreads();
+  if (threadIdx.x < (c.cx ? 2u : 1u)) {
+    unsigned long long t = 0;
+    for (unsigned w = 0; w < kBlock / 32; ++w) t = max(t, red[threadIdx.x][w]);
+    atomicMax(max_bits + blockIdx.y * (c.cx ? 2 : 1) + threadIdx.x, t);
+  }
+}
+
+// k_fix_convert for Columns: u row by row, the K columns of a row next to
+// each other, so that an element's gather is one run of 8 K bytes instead of
+// K sectors. K / 2 lanes share a row, two columns each, so that a warp writes
+// 512 bytes in a row (a lane that wrote a whole row took 59 us for 8 columns
+// of 1.3 M rows); a thread keeps its columns, and what belongs to them, over
+// its rows, since the integer ALU bounds it.
+template <int K>
+__global__ void __launch_bounds__(kBlock) k_fix_convert_cols(Columns c, uint64_t D, uint8_t const* __restrict__ row_class,
+                                                             FixView fv, unsigned long long const* __restrict__ max_bits,
+                                                             int64_t* __restrict__ F_out, int64_t* __restrict__ u) {
+  constexpr uint32_t N = K > 1 ? 2 : 1, L = K / N;  // columns per lane, lanes per row
+  extern __shared__ double fac[];                    // [K][n_div]
+  for (uint32_t t = threadIdx.x; t < K * fv.n_div; t += blockDim.x) {
+    uint32_t const q = t / fv.n_div;
+    double f = 0.0;
+    if (q < c.cols) {
+      int64_t const F = fix_exponent(max_bits[q], fv.bound);
+      int64_t const F1 = (F == kFixBad || (F >= -1000 && F <= 1000)) ? 0 : F / 2;
+      if (F != kFixBad) f = fv.sqrt_s[t % fv.n_div] * fix_pow2(F - F1);
+      if (blockIdx.x == 0 && t % fv.n_div == 0) F_out[q] = F;
+    }
+    fac[t] = f;
+  }
+  // blockDim and the stride are multiples of L: the columns of a thread
+  uint32_t const q0 = (threadIdx.x % L) * N;
+  uint64_t const first = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / L, step = (uint64_t)gridDim.x * blockDim.x / L;
+  uint64_t const es = c.cx ? 2 : 1;
+  bool on[N];        // a column, and not one with a NaN or an infinity
+  double p1[N];      // the first of two factors (F beyond +-1000)
+  bool two = false;
+  uint64_t at[N];
+#pragma unroll
+  for (uint32_t n = 0; n < N; ++n) {
+    uint32_t const q = q0 + n;
+    int64_t const F = q < c.cols ? fix_exponent(max_bits[q], fv.bound) : kFixBad;
+    on[n] = F != kFixBad;
+    int64_t const F1 = (F == kFixBad || (F >= -1000 && F <= 1000)) ? 0 : F / 2;
+    p1[n] = fix_pow2(F1);
+    two = two || F1 != 0;
+    at[n] = c.at(q, 0, c.ldx);
+  }
+  __syncthreads();
+  for (uint64_t i = first; i <= D; i += step) {  // row D is the zero row of fix_row_sums
+    uint32_t const cls = i < D ? row_class[i] : 0u;
+    int64_t v[N];
+#pragma unroll
+    for (uint32_t n = 0; n < N; ++n) {
+      v[n] = 0;
+      if (i < D && on[n]) {
+        uint64_t const o = at[n] + i * es;
+        double xv = c.f32 ? widen(static_cast<float const*>(c.x)[o]) : static_cast<double const*>(c.x)[o];
+        if (two) xv *= p1[n];
+        v[n] = fix_round(xv * fac[(q0 + n) * fv.n_div + cls]);
+      }
+    }
+    if constexpr (N == 1) u[i] = v[0];
+    else reinterpret_cast<longlong2*>(u)[i * L + q0 / 2] = make_longlong2(v[0], v[N - 1]);
+  }
+}
+
+// One row of two adjacent columns as k_spmv sums it (a vector with a NaN or
+// an infinity: only the rows it reaches are affected).
+template <class V>
+__device__ __forceinline__ V general_row(StreamView const& S, Columns const& c, uint32_t const* ent, uint16_t const* codes,
+                                         uint32_t width, uint32_t col_mask, bool packed, uint32_t q) {
+  V acc = zero<V>();
+  for (uint32_t e = 0; e < width; ++e) {
+    uint32_t const v = ent[(uint64_t)e * 32];
+    if (v == kNull) continue;
+    uint32_t const code = packed ? (v >> S.col_bits) : (uint32_t)codes[(uint64_t)e * 32], j = v & col_mask;
+    V const t = load_table<V>(S.table, code, true);
+    if constexpr (std::is_same<V, double>::value) mac(acc, t, c.load(q, j));
+    else mac(acc, t, cplx{c.load(q, j), c.load(q + 1, j)});
+  }
+  return acc;
+}
+
+// Streamed SpMV on K interleaved columns (u row i at u + i K): K / 4 lanes
+// share a row, four columns (one 32-byte sector of u) each, and a slice of 32
+// rows is K / 4 warps. Column by column every element took K sectors, one per
+// column; 16-byte loads by K / 2 lanes took 345 us where 32-byte loads take
+// 319: 8 columns of the 30-site J1-J2 ring (1.3 M rows, 40 M elements), 515
+// at the start. About 246 of these are the 2.6 GB of gathered sectors at the
+// 10.5 TB/s that L2 gives an 83 MB copy, the rest the rows' FP64 epilogues.
+// x, y and the entries pass through L2 once (evict first), so that u stays.
+template <bool Packed, int NV, bool Signed, int K>
+__global__ void __launch_bounds__(kBlock) k_spmv_fix_cols(StreamView S, FixView fv, uint64_t D, Columns c,
+                                                          int64_t const* __restrict__ u,
+                                                          int64_t const* __restrict__ F_in) {
+  constexpr uint32_t N = K < 4 ? K : 4, L = K / N;  // columns per lane, lanes per row
+  extern __shared__ double fix_smem[];                 // g[K][n_div NV], then the code bytes
+  __shared__ bool bad;
+  uint8_t* code8 = reinterpret_cast<uint8_t*>(fix_smem + K * fv.n_div * NV);
+  if constexpr (Signed) fix_stage_codes(fv, code8);
+  for (uint32_t q = 0; q < c.cols; ++q) fix_row_factors<NV>(fv, S.inv_sqrt_s, F_in[q], fix_smem + q * fv.n_div * NV);
+  if (threadIdx.x == 0) {
+    bool b = false;
+    if (c.f32 || c.cx)
+      for (uint32_t q = 0; q < c.cols; ++q) b = b || F_in[q] == kFixBad;
+    bad = b;
+  }
+  __syncthreads();
+  uint64_t const gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  uint64_t const s = gw / L;
+  if ((s << 5) >= D) return;
+  uint32_t const lane = threadIdx.x & 31, row = (uint32_t)(gw % L) * (32 / L) + lane / L, q0 = (lane % L) * N;
+  uint64_t const base = S.slice_ptr[s], i = s * 32 + row;
+  uint32_t const width = (uint32_t)((S.slice_ptr[s + 1] - base) >> 5);
+  uint32_t const col_mask = Packed ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
+  uint32_t const* ent = S.entries + base + row;
+  uint16_t const* codes = S.codes + base + row;
+  if (bad) {
+    if (i >= D || q0 >= c.cols) return;
+    double const f = S.inv_sqrt_s[S.row_class[i]], dg = static_cast<double const*>(S.diag)[i];
+    if (c.cx) {
+      for (uint32_t q = q0; q < q0 + N && q < c.cols; q += 2) {
+        cplx const xi{c.load(q, i), c.load(q + 1, i)};
+        cplx const acc = general_row<cplx>(S, c, ent, codes, width, col_mask, Packed, q);
+        cplx const yi = row_value<cplx>(mulv(cplx{dg, 0.0}, xi), f, acc);
+        c.store(q, i, yi.re);
+        c.store(q + 1, i, yi.im);
+      }
+    } else {
+      for (uint32_t q = q0; q < q0 + N && q < c.cols; ++q)
+        c.store(q, i, row_value<double>(mulv(dg, c.load(q, i)), f,
+                                        general_row<double>(S, c, ent, codes, width, col_mask, Packed, q)));
+    }
+    return;
+  }
+  int64_t acc[N][NV];
+  fix_row_sums<Packed, NV, Signed, (int)N, 8>(
+      S, fv, code8, codes, width, (uint32_t)D, acc,
+      [&](uint32_t e) { return __ldcs(ent + (uint64_t)e * 32); },
+      [&](uint32_t col, int64_t* g) {
+        int64_t const* src = u + (uint64_t)col * K + q0;
+        if constexpr (N == 1) {
+          g[0] = *src;
+        } else if constexpr (N == 2) {
+          longlong2 const v = *reinterpret_cast<longlong2 const*>(src);
+          g[0] = v.x;
+          g[1] = v.y;
+        } else {
+          asm("ld.global.nc.v4.s64 {%0, %1, %2, %3}, [%4];" : "=l"(g[0]), "=l"(g[1]), "=l"(g[2]), "=l"(g[3]) : "l"(src));
+        }
+      },
+      int64_t{});
+  if (i >= D) return;
+  uint32_t const cls = __ldcs(S.row_class + i);
+  double const dg = __ldcs(static_cast<double const*>(S.diag) + i);
+#pragma unroll
+  for (uint32_t n = 0; n < N; ++n)
+    if (q0 + n < c.cols)
+      c.store(q0 + n, i, fix_row<NV>(acc[n], fix_smem + ((q0 + n) * fv.n_div + cls) * NV, F_in[q0 + n], dg, c.load(q0 + n, i)));
+}
+
+
+// A pass of the fixed-point SpMV over c.cols <= K real columns (K = 1, 2, 4,
+// 8, 16; the workspace holds K).
+int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t stream) {
+  BasisData& b = *op.basis;
+  OperatorTables const& tb = *op.tables;
+  StreamForm const& sf = op.stream;
+  uint64_t const D = b.D;
+  auto* mx = op.fix_slots.as<unsigned long long>();
+  auto* F = reinterpret_cast<int64_t*>(mx + op.fix_cols);
+  int64_t* u = op.fix_u.as<int64_t>();
+  if (op.fix_event_recorded) SED_TRY_CUDA(cudaStreamWaitEvent(stream, op.fix_event, 0));
+  SED_TRY_CUDA(cudaMemsetAsync(mx, 0, (size_t)K * 8, stream));
+  unsigned const vg = std::max(1u, grid_size(c.cx ? 2 * D : D, b.device, 8) / (c.cols > 2 ? 4 : 1));
+  uint8_t const* cls = sf.row_class.as<uint8_t>();
+  k_fix_max_cols<<<dim3(vg, c.cx ? c.cols / 2 : c.cols), kBlock, 0, stream>>>(c, D, mx);
+  StreamView const S = stream_view(op);
+  size_t const smem = fix_smem_bytes(tb, K);
+  if (smem > 48 * 1024) return fail(LS_SYSTEM_ERROR, "fixed-point block matvec: tables exceed shared memory");
+  auto pass = [&](auto k_tag) {
+    constexpr int KK = decltype(k_tag)::value;
+    constexpr int LL = KK > 4 ? KK / 4 : 1;
+    uint64_t const warps = sf.n_slices * LL;
+    unsigned const grid = (unsigned)((warps * 32 + kBlock - 1) / kBlock);
+    unsigned const cg = grid_size((D + 1) * (KK > 2 ? KK / 2 : 1), b.device, 8);
+    k_fix_convert_cols<KK><<<cg, kBlock, (size_t)KK * tb.fix.n_div * 8, stream>>>(c, D, cls, tb.fix, mx, F, u);
+    fix_dispatch(tb, sf.packed, [&](auto packed, auto nv, auto sign) {
+      k_spmv_fix_cols<packed.value, nv.value, sign.value, KK><<<grid, kBlock, smem, stream>>>(S, tb.fix, D, c, u, F);
+    });
+  };
+  switch (K) {
+    case 1: pass(std::integral_constant<int, 1>{}); break;
+    case 2: pass(std::integral_constant<int, 2>{}); break;
+    case 4: pass(std::integral_constant<int, 4>{}); break;
+    case 8: pass(std::integral_constant<int, 8>{}); break;
+    default: pass(std::integral_constant<int, 16>{}); break;
+  }
+  note_launches(3);
+  SED_TRY_CUDA(cudaGetLastError());
+  SED_TRY_CUDA(cudaEventRecord(op.fix_event, stream));
+  op.fix_event_recorded = true;
+  return LS_SUCCESS;
+}
+
+}  // namespace
+
+// Whether vectors of this dtype go through launch_fix_cols. FP64 columns
+// always do. The others do from 2^21 element products on: below, the three
+// launches more cost what the sums save (290 000 elements of a complex
+// column: 30 us in the general kernel, 37 here; 77 M FP32 ones: 397 and 180).
+// They do not while the caller's stream is being captured, where the shared
+// workspace could be overwritten between replays (the general kernels use
+// none).
+bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_stream, cudaStream_t stream) {
+  if (!use_stream || !op.tables->fix_ok || op.fix_cols < 1) return false;
+  if (dtype == 1) return true;
+  if (op.stream.n_elements * block * (dtype >= 2 ? 2 : 1) < ((uint64_t)1 << 21)) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return cap == cudaStreamCaptureStatusNone;
+}
+
+// The first `block` columns in passes of fixed width, widest first; *done
+// counts the columns taken. A pass is padded to a power of two (three
+// columns to 4, 5 to 7 to 8, 13 to 15 to 16): an element costs 4 + 8 K bytes
+// of stream and gather, so that one padded pass moves less than two exact
+// ones (7 columns: 68 against 36 + 20 + 12 bytes and three reads of the
+// entries), except at 9 to 12 (8 + 4: 104 against 132). Stops early, with
+// success, where the workspace for even the narrowest pass cannot be had:
+// the caller's general path does the rest.
+int fix_cols_blocks(OperatorData& op, int dtype, uint64_t block, char const* x, uint64_t ldx, char* y, uint64_t ldy,
+                    size_t es, cudaStream_t stream, uint64_t* done) {
+  // a pass keeps K tables of row factors in shared memory: at most kmax
+  // columns fit in 48 KB
+  size_t const table = (size_t)op.tables->fix.n_div * op.tables->fix_nv * 8;
+  unsigned const kmax = (unsigned)std::min<size_t>(16, (48 * 1024 - op.tables->fix.n_codes - 1) / table);
+  bool const cx = dtype >= 2;
+  unsigned const per = cx ? 2 : 1;  // real columns per column
+  while (*done < block) {
+    uint64_t const left = (block - *done) * per;
+    unsigned K = 1;
+    while (K < left && K < 16) K *= 2;
+    if (left >= 9 && left <= 12) K = 8;
+    while (K > per && K > kmax) K /= 2;
+    if (K > kmax) return LS_SUCCESS;
+    while (int st = fix_reserve(op, K)) {
+      if (st != LS_OUT_OF_MEMORY) return st;
+      if (K <= per) return LS_SUCCESS;
+      K /= 2;
+    }
+    if (K == 1 && dtype == 1) return LS_SUCCESS;  // launch_apply_fix
+    unsigned const cols = (unsigned)std::min<uint64_t>(left, K);
+    Columns const c{x + *done * ldx * es, y + *done * ldy * es, ldx, ldy, cols, dtype == 0 || dtype == 2, cx};
+    if (int st = launch_fix_cols(op, K, c, stream)) return st;
+    *done += cols / per;
+  }
+  return LS_SUCCESS;
+}
+
+}  // namespace sed

@@ -267,3 +267,101 @@ def test_fixed_point_matvec_scales_and_specials(sed, oracle, name):
     yw = sed.apply(op, torch.tensor(xw, device="cuda")).cpu().numpy()
     want = oop.matvec(xw).real
     assert np.max(np.abs(yw - want)) <= 1e-13 * np.abs(xw).max() * oop.sparse().__abs__().sum(axis=1).max()
+
+
+# one and two values, characters +1 and +-1 (momentum pi, odd inversion); 0.36 to 0.73 M elements, so that FP32 and
+# complex vectors take the general kernels for the narrow blocks and the integer sums for the wide ones
+COLUMN_MODELS = {
+    "chain24": lattices.heisenberg_chain(24),
+    "chain24_j2": lattices.heisenberg_chain(24, j2=0.3),
+    "chain24_k12": lattices.heisenberg_chain(24, momentum=12, parity=1),
+    "chain22_odd_j2": lattices.heisenberg_chain(22, parity=None, spin_inversion=-1, j2=0.3),
+}
+
+
+@pytest.fixture(scope="module")
+def column_models(sed, oracle):
+    out = {}
+    for name, m in COLUMN_MODELS.items():
+        built, ob, oop = both(sed, oracle, m)
+        built.hamiltonian.prepare(L.SED_FORM_STREAM)
+        out[name] = (built.hamiltonian, len(ob.reps), oop.sparse(), built)
+    return out
+
+
+@pytest.mark.parametrize("block", [1, 2, 3, 4, 5, 7, 8, 9, 13, 16, 19])
+@pytest.mark.parametrize("dtype", ["float32", "float64", "complex64", "complex128"])
+@pytest.mark.parametrize("name", list(COLUMN_MODELS))
+def test_column_passes(sed, column_models, name, dtype, block):
+    """Blocks of every dtype on real operators: passes of 1 to 16 interleaved
+    real columns, padded ones and leftovers among them, against the oracle's
+    matrix. y is rounded once to its type (2^-24 of |y_i| for FP32 parts), x
+    is exact. FP64 columns equal the single-column product bit for bit."""
+    import torch
+    op, D, A, _ = column_models[name]
+    dt = getattr(torch, dtype)
+    gen = torch.Generator(device="cuda").manual_seed(block)
+    x = torch.randn(block, D + 5, dtype=dt, device="cuda", generator=gen).t()[:D]  # stride D + 5
+    x *= torch.logspace(-3, 3, block, device="cuda").to(dt)  # a scale per column
+    y = torch.zeros(block, D + 3, dtype=dt, device="cuda").t()[:D]
+    sed.inplace_apply(op, x, y)
+    eps = 2.0 ** -23 if dtype in ("float32", "complex64") else 1e-13
+    xs, ys = x.cpu().numpy(), y.cpu().numpy()
+    for c in range(block):
+        want = A @ xs[:, c].astype(np.complex128)
+        d = ys[:, c] - (want if np.iscomplexobj(ys) else want.real)
+        assert np.abs(d).max() <= eps * np.abs(want).max()
+        if dtype == "float64":
+            assert torch.equal(y[:, c], sed.apply(op, x[:, c].contiguous()))
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("dtype", ["float32", "complex64", "complex128"])
+def test_non_finite_entries_stay_in_their_rows(sed, oracle, dtype, bad):
+    """FP32 and complex vectors, through the integer sums: a NaN or an
+    infinity reaches the rows that couple to its entry, in its own column, and
+    no others."""
+    import torch
+    built, ob, oop = both(sed, oracle, COLUMN_MODELS["chain24_j2"])
+    op = built.hamiltonian
+    op.prepare(L.SED_FORM_STREAM)
+    D, block, j = len(ob.reps), 5, len(ob.reps) // 3
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(block, D, dtype=getattr(torch, dtype), device="cuda", generator=gen).t()
+    clean = x.cpu().numpy()
+    x[j, 2] = bad
+    y = sed.apply(op, x).cpu().numpy()
+    rows, cols, _ = oop.coo()
+    reached = np.zeros(D, bool)
+    reached[rows[cols == j].astype(np.int64)] = True
+    reached[j] = True
+    for c in range(block):
+        want = oop.matvec(clean[:, c].astype(np.complex128))
+        fine = np.ones(D, bool) if c != 2 else ~reached
+        assert np.array_equal(np.isfinite(y[:, c]), fine)
+        d = y[fine, c] - (want if np.iscomplexobj(y) else want.real)[fine]
+        assert np.abs(d).max() <= 2.0 ** -23 * np.abs(want).max()
+
+
+def test_narrower_passes_when_the_workspace_is_capped(sed, oracle):
+    """A cap on device memory that leaves no room for a wide pass's gather
+    copy: the product runs in narrower passes with the same result."""
+    import torch
+    built, ob, oop = both(sed, oracle, COLUMN_MODELS["chain24"])
+    op, lib = built.hamiltonian, L.load()
+    op.prepare(L.SED_FORM_STREAM)
+    D = len(ob.reps)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.randn(16, D, dtype=torch.float64, device="cuda", generator=gen).t()
+    columns = [sed.apply(op, x[:, c].contiguous()) for c in range(16)]
+    lib.sed_release_workspace()
+    used = lib.sed_device_memory_in_use()
+    try:
+        for room in (0, 2 * 8 * (D + 1), 5 * 8 * (D + 1)):
+            lib.sed_set_device_memory_limit(used + room)
+            y = sed.apply(op, x)
+            assert all(torch.equal(y[:, c], columns[c]) for c in range(16))
+    finally:
+        lib.sed_set_device_memory_limit(0)
+    y = sed.apply(op, x)
+    assert all(torch.equal(y[:, c], columns[c]) for c in range(16))
