@@ -515,61 +515,80 @@ SED_HD Canon<W> canonicalize_img(W x, PlanView const& P, RowTab const& T, Img&& 
   return {best, ph};
 }
 
+// Row-structured plans with line tables: false if some coset image of x has a
+// smaller top row than x, found from the rows and columns of x itself.
+template <class W>
+SED_HD bool lines_may_be_least(W x, PlanView const& P, RowTab const& T) {
+  uint32_t const rm = (uint32_t)P.row_mask;
+  uint32_t const xt = (uint32_t)(x >> ((P.n_rows - 1) * P.row_bits));
+  W v = x;
+#pragma unroll
+  for (uint32_t k = 0; k < SED_MAX_ROWS; ++k) {
+    if (k < P.n_rows) {
+      if (T.lrow[(uint32_t)v & rm] < xt) return false;
+      v >>= P.row_bits;
+    }
+  }
+  if (P.line_cols) {
+#pragma unroll
+    for (uint32_t j = 0; j < SED_MAX_ROWS; ++j) {
+      if (j < P.row_bits) {
+        uint64_t const col = ((((uint64_t)x >> j) & P.col_m) * P.col_k) >> P.col_s;
+        if (T.lcol[(uint32_t)col & rm] < xt) return false;
+      }
+    }
+  }
+  return true;
+}
+
+// Row-structured plans: the stabiliser order of x if no image with x's top
+// row is smaller (x has passed the test of the top rows), else 0.
+template <class W>
+SED_HD uint32_t rows_weight(W x, PlanView const& P, RowTab const& T) {
+  uint32_t S = 0;
+  uint32_t const rm = (uint32_t)P.row_mask;
+  uint32_t const xt = (uint32_t)(x >> ((P.n_rows - 1) * P.row_bits));
+  for (uint32_t c = 0; c < P.n_cosets; ++c) {
+    W const y = coset_apply<W>(x, P, c);
+    for (uint32_t k = 0; k < P.n_rows; ++k) {
+      uint32_t const row = (uint32_t)(y >> (k * P.row_bits)) & rm;
+      for (uint32_t inv = 0; inv <= (P.inv ? 1u : 0u); ++inv) {
+        uint32_t const v = inv ? (row ^ rm) : row;
+        if (T.min[v] != xt) continue;
+        uint32_t set = T.set[v];
+        while (set) {
+          uint32_t const r = (uint32_t)__builtin_ctz_sed(set);
+          set &= set - 1;
+          int const cmp = cand_compare<W>(y, P, k, r, inv ? rm : 0u, x, 1);
+          if (cmp < 0) return 0;
+          if (cmp == 0) {
+            uint32_t const t = k + 1 == P.n_rows ? 0u : k + 1;
+            uint64_t ph = (uint64_t)P.coset_phase[c] + (uint64_t)P.rot_exp[r] * P.rot_phase +
+                          (uint64_t)P.sh_exp[t] * P.shift_phase + (inv ? P.inv_phase : 0u);
+            if (ph % P.L != 0) return 0;
+            ++S;
+          }
+        }
+      }
+    }
+  }
+  return S;
+}
+
 // Stabiliser order of x if x is a representative of the sector, else 0.
 template <class W>
 SED_HD uint32_t representative_weight(W x, PlanView const& P, RowTab const& T) {
   uint32_t S = 0;
   W const mask = (W)P.mask;
   if (P.rows == 1) {
-    uint32_t const rm = (uint32_t)P.row_mask;
-    uint32_t const xt = (uint32_t)(x >> ((P.n_rows - 1) * P.row_bits));
     if (T.lrow) {  // pass A from the lines of x: the image rows of all cosets at once
-      W v = x;
-#pragma unroll
-      for (uint32_t k = 0; k < SED_MAX_ROWS; ++k) {
-        if (k < P.n_rows) {
-          if (T.lrow[(uint32_t)v & rm] < xt) return 0;
-          v >>= P.row_bits;
-        }
-      }
-      if (P.line_cols) {
-#pragma unroll
-        for (uint32_t j = 0; j < SED_MAX_ROWS; ++j) {
-          if (j < P.row_bits) {
-            uint64_t const col = ((((uint64_t)x >> j) & P.col_m) * P.col_k) >> P.col_s;
-            if (T.lcol[(uint32_t)col & rm] < xt) return 0;
-          }
-        }
-      }
+      if (!lines_may_be_least<W>(x, P, T)) return 0;
     } else {
+      uint32_t const xt = (uint32_t)(x >> ((P.n_rows - 1) * P.row_bits));
       for (uint32_t c = 0; c < P.n_cosets; ++c)  // pass A with early rejection
         if (rows_min_top<W>(coset_apply<W>(x, P, c), P, T) < xt) return 0;
     }
-    for (uint32_t c = 0; c < P.n_cosets; ++c) {  // pass B: images whose top row equals x's
-      W const y = coset_apply<W>(x, P, c);
-      for (uint32_t k = 0; k < P.n_rows; ++k) {
-        uint32_t const row = (uint32_t)(y >> (k * P.row_bits)) & rm;
-        for (uint32_t inv = 0; inv <= (P.inv ? 1u : 0u); ++inv) {
-          uint32_t const v = inv ? (row ^ rm) : row;
-          if (T.min[v] != xt) continue;
-          uint32_t set = T.set[v];
-          while (set) {
-            uint32_t const r = (uint32_t)__builtin_ctz_sed(set);
-            set &= set - 1;
-            int const cmp = cand_compare<W>(y, P, k, r, inv ? rm : 0u, x, 1);
-            if (cmp < 0) return 0;
-            if (cmp == 0) {
-              uint32_t const t = k + 1 == P.n_rows ? 0u : k + 1;
-              uint64_t ph = (uint64_t)P.coset_phase[c] + (uint64_t)P.rot_exp[r] * P.rot_phase +
-                            (uint64_t)P.sh_exp[t] * P.shift_phase + (inv ? P.inv_phase : 0u);
-              if (ph % P.L != 0) return 0;
-              ++S;
-            }
-          }
-        }
-      }
-    }
-    return S;
+    return rows_weight<W>(x, P, T);  // pass B: images whose top row equals x's
   }
   if (P.rows == 2) {
     bool reject = false;
