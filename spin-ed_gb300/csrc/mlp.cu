@@ -620,14 +620,75 @@ __global__ void k_to_bf16(float const* __restrict__ p, __nv_bfloat16* __restrict
     pb[q] = __float2bfloat16(p[q]);
 }
 
-// v_r = prior(r) sign(s) exp(a - a_max) / n_r, n_r = sqrt(S_r / |G|)
-__global__ void k_start_from_net(float const* __restrict__ out, uint64_t const* __restrict__ reps,
-                                 uint32_t const* __restrict__ weights, int64_t n, uint64_t sign_mask,
-                                 float a_max, double group_order, double* __restrict__ v) {
+// exp(d) for -600 <= d <= 0 in 64-bit fixed point, rounded once to FP64:
+// table-driven (Tang, ACM TOMS 15, 144 (1989)), exp(d) = 2^-k 2^(i/64)
+// 2^(j/4096) 2^r with k, i, j, r from the bits of d log2(e), r < 2^-12 and
+// 2^r from four terms of its series. Integer instructions only (about 100 on
+// 64 lanes per clock and SM): exp() is some 16 FP64 operations on 1.75. The
+// error before the rounding is below 2^-53 of the value: 2^-53 from cutting d
+// to multiples of 2^-53, the rest 2^-58.
+struct ExpTables {
+  uint64_t sixty_fourths[64], small[64];  // 2^(i / 64) and 2^(j / 4096), 62 fraction bits
+};
+
+ExpTables exp_tables() {
+  ExpTables t;
+  for (int i = 0; i < 64; ++i) {
+    t.sixty_fourths[i] = (uint64_t)std::llroundl(std::ldexp(std::exp2((long double)i / 64.0L), 62));
+    t.small[i] = (uint64_t)std::llroundl(std::ldexp(std::exp2((long double)i / 4096.0L), 62));
+  }
+  return t;
+}
+
+__device__ __forceinline__ double exp_fixed(float d, uint64_t const* t64, uint64_t const* t4096) {
+  uint32_t const b = __float_as_uint(d);
+  int const sh = (int)((b >> 23) & 0xFFu) - 97;  // |d| 2^53 = (24-bit m) 2^sh
+  uint64_t const m = (b & 0x7FFFFFu) | 0x800000u;
+  uint64_t const x53 = sh >= 0 ? m << sh : (sh > -24 ? m >> -sh : 0);
+  uint64_t const log2e = 0xB8AA3B295C17F0BCull;  // 2^63 log2(e)
+  uint64_t const hi = __umul64hi(x53, log2e), lo = x53 * log2e;
+  // |d| log2(e) = (hi >> 52) + frac 2^-64; exp(d) = 2^-(that)
+  uint64_t const frac = hi << 12 | lo >> 52, up = 0 - frac;
+  int const e = -(int)(hi >> 52) - (frac != 0);  // exp(d) = 2^e 2^(up 2^-64)
+  uint64_t const r = up & 0xFFFFFFFFFFFFFull;
+  uint64_t const x = __umul64hi(r, 0xB17217F7D1CF79ABull);  // r ln 2, 64 fraction bits, below 2^52
+  uint64_t const x2 = __umul64hi(x, x);
+  uint32_t const x3 = (uint32_t)__umul64hi(x2, x);  // below 2^27
+  uint32_t const x4 = __umulhi(x3, (uint32_t)(x >> 32));
+  uint64_t const p = x + (x2 >> 1) + x3 / 6 + x4 / 24;
+  uint64_t const t = __umul64hi(t64[up >> 58], t4096[(up >> 52) & 63]);  // 60 fraction bits
+  uint64_t const y = t + __umul64hi(t, p);                               // in [2^60, 2^61)
+  return __longlong_as_double((long long)(((uint64_t)(1022 + e) << 52) + ((y + 0x80) >> 8)));
+}
+
+// v_r = prior(r) sign(s) exp(a - a_max) / n_r, n_r = sqrt(S_r / |G|). FP64
+// issue bounded it with exp, a division and a square root per row (15.8 M
+// rows: 1026 us); the norms of groups up to kNormTable come from a table of
+// the block, exp is exp_fixed: 128 us, of which 84 are the bytes.
+constexpr uint32_t kNormTable = 1024;
+__global__ void __launch_bounds__(256)
+    k_start_from_net(float2 const* out, uint64_t const* __restrict__ reps,
+                     uint32_t const* __restrict__ weights, int64_t n, uint64_t sign_mask, float a_max,
+                     uint32_t group_order, __grid_constant__ const ExpTables tables, double* v /* may be out */) {
+  __shared__ uint64_t t64[64], t4096[64];
+  __shared__ double norm[kNormTable + 1];
+  if (threadIdx.x < 64) {
+    t64[threadIdx.x] = tables.sixty_fourths[threadIdx.x];
+    t4096[threadIdx.x] = tables.small[threadIdx.x];
+  }
+  double const g = (double)group_order;
+  bool const tabled = group_order <= kNormTable;
+  if (tabled)
+    for (uint32_t q = 1 + threadIdx.x; q <= group_order; q += blockDim.x)
+      if (group_order % q == 0) norm[q] = sqrt(g / (double)q);
+  __syncthreads();
   for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < n; b += (int64_t)gridDim.x * blockDim.x) {
-    float const a = out[2 * b], s = out[2 * b + 1];
-    double const amp = exp((double)(a - a_max)) * sqrt(group_order / (double)weights[b]);
-    bool const neg = (s < 0.0f) != (prior_flip(reps[b], sign_mask) != 0.0f);
+    float2 const o = out[b];
+    float const d = o.x - a_max;
+    uint32_t const S = weights[b];
+    double const ex = d <= 0.0f && d >= -600.0f ? exp_fixed(d, t64, t4096) : exp((double)d);
+    double const amp = ex * (tabled ? norm[S] : sqrt(g / (double)S));
+    bool const neg = (o.y < 0.0f) != (prior_flip(reps[b], sign_mask) != 0.0f);
     v[b] = neg ? -amp : amp;
   }
 }
@@ -817,16 +878,17 @@ __device__ __forceinline__ uint64_t tc_state(MlpTcArgs const& p, int64_t tile, i
 // 512 epilogue threads.
 __device__ __forceinline__ void tc_build_x(MlpTcArgs const& p, uint64_t s, uint8_t* X, int t) {
   int const xr = t & 127, part = t >> 7;
+  uint32_t const in = p.n_in >= 64 ? ~0u : (uint32_t)(((1ull << p.n_in) - 1) >> (16 * part)) & 0xFFFFu;
+  uint32_t const bits = (uint32_t)(s >> (16 * part)) & 0xFFFFu;
 #pragma unroll
   for (int cc = 0; cc < 2; ++cc) {
     int const c = 2 * part + cc;
     uint32_t w[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      int const j = 8 * c + 2 * q;
-      uint32_t const lo = j < p.n_in ? (((s >> j) & 1) ? 0x3F80u : 0xBF80u) : 0u;
-      uint32_t const hi = j + 1 < p.n_in ? (((s >> (j + 1)) & 1) ? 0x3F80u : 0xBF80u) : 0u;
-      w[q] = lo | (hi << 16);
+      int const j = 8 * cc + 2 * q;  // BF16 -1, the sign bit cleared where the state's bit is set
+      uint32_t const pair = 0xBF80BF80u ^ ((bits >> j & 1u) << 15) ^ ((bits >> (j + 1) & 1u) << 31);
+      w[q] = pair & (((in >> j & 1u) ? 0xFFFFu : 0u) | ((in >> (j + 1) & 1u) ? 0xFFFF0000u : 0u));
     }
     *reinterpret_cast<uint4*>(X + xr * 128 + ((c ^ (xr & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
   }
@@ -1133,6 +1195,260 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_forward_tc(MlpTcArgs p) {
   }
 }
 
+// Hidden sizes up to 256: the weights (160 KB at 256) stay in shared memory,
+// and TMEM holds two tiles' h1 beside the two accumulator slots, so layer 1
+// of a tile runs between the blocks of layer 2 of the tile before. Rounds r =
+// 0 .. my_tiles take the accumulator uses L1(r) block 0, L2(r - 1) block 0,
+// L1(r) block 1, ...: the epilogue warps always find the next accumulator
+// done, where the one-tile kernel above waited for the chain layer 1, tanh,
+// layer 2 of every tile (5.5 us per tile on an SM, of which 2.0 are the
+// tanh instructions and 1.6 the MMAs) and read 160 KB of weights per tile
+// from L2. The arithmetic and its order are the same. Network 36-256-256-2 on
+// 15.8 M states: 4501 -> 3603 us, bound by the epilogue warps
+// MUFU.
+constexpr int kResMaxHidden = 256;
+size_t tc_resident_smem(int hidden) {
+  return 2 * (size_t)kTcRows * 128 + (size_t)hidden * 128 + (size_t)hidden * hidden * 2 + 4 * (size_t)hidden * 4 +
+         2 * (size_t)4 * kTcRows * 2 * 4 + 1024;
+}
+
+__global__ void __launch_bounds__(kTcThreads, 1) k_mlp_forward_resident(MlpTcArgs p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t weights_in, acc_full[2], acc_empty[2], h1_ready[2][kResMaxHidden / 128], x_ready[2], drain;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  uint8_t* const smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  int const H = p.hidden, NM = 128, blocks = H / NM, ktiles = H / 64;
+  uint8_t* const X = smem;  // two tiles of 128 rows x 128 B
+  uint8_t* const W1 = X + 2 * (size_t)kTcRows * 128;
+  uint8_t* const W2 = W1 + (size_t)H * 128;
+  float* const sb1 = reinterpret_cast<float*>(W2 + (size_t)H * H * 2);
+  float* const sb2 = sb1 + H;
+  float* const sw3 = sb2 + H;        // [2][H]
+  float* const spart = sw3 + 2 * H;  // [2 buffers][4 column slices][128 rows][2]
+  int const t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  int64_t const n_tiles = (p.n + kTcRows - 1) / kTcRows;
+  int const my_tiles = blockIdx.x < n_tiles ? (int)((n_tiles - 1 - blockIdx.x) / gridDim.x + 1) : 0;
+
+  if (t == 0) {
+    tc::mbar_init(&weights_in, 1);
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&acc_full[i], 1);
+      tc::mbar_init(&acc_empty[i], kTcEpiWarps);
+      tc::mbar_init(&x_ready[i], kTcEpiWarps);
+      for (int q = 0; q < kResMaxHidden / 128; ++q) tc::mbar_init(&h1_ready[i][q], kTcEpiWarps);
+    }
+    tc::mbar_init(&drain, 1);
+    abort_flag = 0;
+    tc::fence_mbar_init();
+  }
+  __syncwarp();
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, kTcCols);
+  for (int c = t; c < H; c += kTcThreads) {
+    sb1[c] = __ldg(p.b1 + c);
+    sb2[c] = __ldg(p.b2 + c);
+    sw3[c] = __bfloat162float(p.W3[c]);
+    sw3[H + c] = __bfloat162float(p.W3[H + c]);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  uint32_t const tmem = tmem_slot;
+
+  if (warp == kTcEpiWarps) {
+    // ---- copy warp: both weight images, once
+    if (lane == 0 && my_tiles > 0) {
+      uint32_t const tiles = (uint32_t)(H / 128 + ktiles * blocks);
+      tc::mbar_expect_tx(&weights_in, tiles * kTcTileBytes);
+      for (uint32_t i = 0; i < tiles; ++i) {
+        uint32_t const at = i * kTcTileBytes, in1 = (uint32_t)H * 128;
+        tc::bulk_g2s(W1 + at, at < in1 ? p.w1img + at : p.w2img + (at - in1), kTcTileBytes, &weights_in);
+      }
+      if (!tc::mbar_wait(&weights_in, 0, p.wait_ns)) abort_flag = 1;  // never leave with copies in flight
+    }
+    __syncwarp();
+  } else if (warp == kTcEpiWarps + 1) {
+    // ---- MMA warp (warp-uniform; one elected lane issues and commits)
+    uint32_t const idesc = tc::idesc_bf16_f32(128, (uint32_t)NM);
+    bool ok = my_tiles > 0 && __all_sync(0xffffffffu, tc::mbar_wait(&weights_in, 0, p.wait_ns));
+    tc::fence_after_sync();
+    int64_t u = 0;                   // accumulator use
+    auto slot_free = [&](int64_t uu) {  // the epilogue has drained use uu - 2 of the slot
+      bool const r = uu < 2 || tc::mbar_wait(&acc_empty[uu & 1], (uint32_t)((uu >> 1) - 1) & 1, p.wait_ns);
+      tc::fence_after_sync();
+      return __all_sync(0xffffffffu, r);
+    };
+    for (int r = 0; r <= my_tiles && ok && my_tiles > 0; ++r) {
+      int const b = r & 1;
+      if (r < my_tiles) {
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&x_ready[b], (uint32_t)(r >> 1) & 1, p.wait_ns) && !abort_flag);
+        tc::fence_after_sync();
+      }
+      for (int q = 0; q < blocks && ok; ++q) {
+        if (r < my_tiles) {  // layer 1 of tile r: block q of X W1^T
+          ok = slot_free(u);
+          if (!ok) break;
+          uint32_t const d = tmem + (uint32_t)((u & 1) * NM);
+          uint32_t const at = tc::smem_u32(X + (size_t)b * kTcRows * 128);
+          uint32_t const b0 = tc::smem_u32(W1 + (size_t)q * kTcTileBytes);
+          if (tc::elect_one()) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              tc::mma_bf16(d, tc::desc_sw128(at + 32 * k), tc::desc_sw128(b0 + 32 * k), idesc, k > 0 ? 1u : 0u);
+            tc::mma_commit(&acc_full[u & 1]);
+          }
+          __syncwarp();
+          ++u;
+        }
+        if (r > 0) {  // layer 2 of tile r - 1: block q of h1 W2^T, h1 read from TMEM
+          if (q == 0)
+            for (int h = 0; h < blocks && ok; ++h)
+              ok = __all_sync(0xffffffffu,
+                              tc::mbar_wait(&h1_ready[b ^ 1][h], (uint32_t)((r - 1) >> 1) & 1, p.wait_ns) && !abort_flag);
+          if (ok) ok = slot_free(u);  // also orders the MMAs after the epilogue's TMEM writes
+          if (!ok) break;
+          uint32_t const d = tmem + (uint32_t)((u & 1) * NM), h1 = tmem + kTcH1Col + (uint32_t)((b ^ 1) * (H / 2));
+          uint32_t const b0 = tc::smem_u32(W2 + (size_t)q * kTcTileBytes);
+          if (tc::elect_one()) {
+            for (int kb = 0; kb < ktiles; ++kb)
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                tc::mma_bf16_ts(d, h1 + (uint32_t)(kb * 32 + k * 8),
+                                tc::desc_sw128(b0 + (uint32_t)(kb * blocks * kTcTileBytes) + 32 * k), idesc,
+                                (kb > 0 || k > 0) ? 1u : 0u);
+            tc::mma_commit(&acc_full[u & 1]);
+          }
+          __syncwarp();
+          ++u;
+        }
+      }
+    }
+    // every MMA issued has completed before TMEM is released
+    if (tc::elect_one()) {
+      if (!ok && my_tiles > 0) abort_flag = 1;
+      tc::mma_commit(&drain);
+      if (!tc::mbar_wait(&drain, 0, p.wait_ns)) abort_flag = 1;
+    }
+    __syncwarp();
+  } else {
+    // ---- epilogue warps: warp w reads TMEM lanes 32 (w % 4) .. + 31 (its
+    // rows) and columns 32 (w / 4) .. + 31 of each 128-column block
+    int const quarter = warp & 3, cq = warp >> 2;
+    int const row0 = quarter * 32 + lane;
+    uint32_t const lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+    bool ok = true;
+    int64_t u = 0;
+    auto tile_of = [&](int r) { return (int64_t)blockIdx.x + (int64_t)r * gridDim.x; };
+    auto build_x = [&](int r, uint64_t state) {  // X tile of round r
+      tc_build_x(p, state, X + (size_t)(r & 1) * kTcRows * 128, t);
+      tc::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&x_ready[r & 1]);
+    };
+    for (int r = 0; r < 2 && r < my_tiles; ++r) build_x(r, tc_state(p, tile_of(r), t));
+    float const b3a = __ldg(p.b3), b3s = __ldg(p.b3 + 1);
+    // wait for accumulator use uu and load this warp's 32 columns of it; the
+    // slot is handed back as soon as the load has completed
+    auto load_acc = [&](int64_t uu, float (&v)[32]) {
+      if (ok) ok = tc::mbar_wait(&acc_full[uu & 1], (uint32_t)(uu >> 1) & 1, p.wait_ns) && !abort_flag;
+      tc::fence_after_sync();
+      __syncwarp();
+      if (!ok) return false;
+      tc::tmem_ld32(lane_addr + (uint32_t)((uu & 1) * NM + cq * 32), v);
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&acc_empty[uu & 1]);
+      return true;
+    };
+    // (a, s) of a finished tile: the four column slices' partials plus b3;
+    // run by the first warp of each quarter one round later, off the
+    // epilogue's critical path
+    auto write_out = [&](int r) {
+      float const* const sp = spart + (size_t)(r & 1) * (4 * kTcRows * 2);
+      if (t < kTcRows) {
+        int64_t const row = tile_of(r) * kTcRows + t;
+        int64_t const b = p.n_sites ? row / p.n_sites : row;
+        bool const first = !p.n_sites || row == b * p.n_sites;  // the row that carries b3
+        float sa = first ? b3a : 0.0f, ss = first ? b3s : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          sa += sp[(i * kTcRows + t) * 2];
+          ss += sp[(i * kTcRows + t) * 2 + 1];
+        }
+        if (ok && row < p.n) {
+          if (p.n_sites) {
+            atomicAdd(p.out + 2 * b, sa);
+            atomicAdd(p.out + 2 * b + 1, ss);
+          } else {
+            reinterpret_cast<float2*>(p.out)[row] = make_float2(sa, ss);
+          }
+        }
+      }
+    };
+    // the four warps of a lane quarter share its rows' partials
+    auto quarter_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + quarter) : "memory"); };
+    // After a failed wait a warp skips the remaining work but still passes
+    // every quarter_sync, so that the named barriers never wait for it.
+    for (int r = 0; r <= my_tiles && my_tiles > 0; ++r) {
+      // the states of the tile two rounds on, loaded early
+      uint64_t const s_next = r + 2 < my_tiles ? tc_state(p, tile_of(r + 2), t) : 0;
+      float a = 0.0f, sg = 0.0f;
+      for (int q = 0; q < blocks; ++q) {
+        int const c0 = q * NM + cq * 32;
+        if (r < my_tiles) {  // h1 of tile r = tanh(acc + b1) -> BF16 pairs -> TMEM
+          float v[32];
+          if (!load_acc(u++, v)) break;
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {  // 16-byte broadcast loads of the biases
+            float4 const b = *reinterpret_cast<float4 const*>(sb1 + c0 + 4 * i);
+            pk[2 * i] = tc::pack_bf16x2(tc::tanh_fast(v[4 * i] + b.x), tc::tanh_fast(v[4 * i + 1] + b.y));
+            pk[2 * i + 1] = tc::pack_bf16x2(tc::tanh_fast(v[4 * i + 2] + b.z), tc::tanh_fast(v[4 * i + 3] + b.w));
+          }
+          tc::tmem_st16(lane_addr + kTcH1Col + (uint32_t)((r & 1) * (H / 2) + (c0 >> 1)), pk);
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(&h1_ready[r & 1][q]);
+        }
+        if (r > 0) {  // h2 of tile r - 1 = tanh(acc + b2); partial (a, s) over this warp's columns
+          float v[32];
+          if (!load_acc(u++, v)) break;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {  // 16-byte broadcast loads of b2 and W3
+            float4 const b = *reinterpret_cast<float4 const*>(sb2 + c0 + 4 * i);
+            float4 const wa = *reinterpret_cast<float4 const*>(sw3 + c0 + 4 * i);
+            float4 const ws = *reinterpret_cast<float4 const*>(sw3 + H + c0 + 4 * i);
+            float const h0 = tc::tanh_fast(v[4 * i] + b.x), h1 = tc::tanh_fast(v[4 * i + 1] + b.y);
+            float const h2 = tc::tanh_fast(v[4 * i + 2] + b.z), h3 = tc::tanh_fast(v[4 * i + 3] + b.w);
+            a = fmaf(wa.x, h0, fmaf(wa.y, h1, fmaf(wa.z, h2, fmaf(wa.w, h3, a))));
+            sg = fmaf(ws.x, h0, fmaf(ws.y, h1, fmaf(ws.z, h2, fmaf(ws.w, h3, sg))));
+          }
+        }
+      }
+      // layer 1 of tile r has finished reading its X
+      if (ok && r + 2 < my_tiles) build_x(r + 2, s_next);
+      if (r > 1) write_out(r - 2);  // its partials are complete since the last quarter_sync
+      // two buffers of partials: a buffer is rewritten two rounds later, after
+      // its reader has passed the next quarter_sync
+      if (r > 0) {
+        float* const sp = spart + (size_t)((r - 1) & 1) * (4 * kTcRows * 2);
+        sp[(cq * kTcRows + row0) * 2] = a;
+        sp[(cq * kTcRows + row0) * 2 + 1] = sg;
+      }
+      quarter_sync();
+    }
+    if (my_tiles > 0) write_out(my_tiles - 1);
+    if (!ok) abort_flag = 1;
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (abort_flag && t == 0) atomicExch(p.error, 1);
+  if (warp == 0) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, kTcCols);
+  }
+}
+
 // Weight images for k_mlp_forward_tc from the BF16 parameters: W1 [H][n_in]
 // (zero padded to 64 columns) and W2 [H][H], swizzled as the MMA reads them.
 __global__ void k_mlp_images(__nv_bfloat16 const* __restrict__ W1, __nv_bfloat16 const* __restrict__ W2, int n_in,
@@ -1315,8 +1631,10 @@ int forward_tc(MlpData& d, uint64_t const* states, uint64_t n, float* out) {
     d.img_valid = true;
   }
   if (n == 0) return LS_SUCCESS;
-  size_t const smem = tc_smem_bytes(H);
-  SED_TRY_CUDA(cudaFuncSetAttribute(k_mlp_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  bool const resident = H <= kResMaxHidden;
+  auto* const kernel = resident ? &k_mlp_forward_resident : &k_mlp_forward_tc;
+  size_t const smem = resident ? tc_resident_smem(H) : tc_smem_bytes(H);
+  SED_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   SED_TRY_CUDA(cudaMemsetAsync(d.tc_error.ptr, 0, 4, s));
   uint64_t const rows = d.n_sites ? n * d.n_sites : n;
   if (d.n_sites) SED_TRY_CUDA(cudaMemsetAsync(out, 0, n * 8, s));  // the site rows add into it
@@ -1340,7 +1658,7 @@ int forward_tc(MlpData& d, uint64_t const* states, uint64_t n, float* out) {
   if (d.n_sm == 0) SED_TRY_CUDA(cudaDeviceGetAttribute(&d.n_sm, cudaDevAttrMultiProcessorCount, d.device));
   uint64_t const tiles = (rows + kTcRows - 1) / kTcRows;
   unsigned const grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)d.n_sm);  // persistent: one CTA per SM
-  { k_mlp_forward_tc<<<grid, kTcThreads, smem, s>>>(a); note_launches(1); }
+  { kernel<<<grid, kTcThreads, smem, s>>>(a); note_launches(1); }
   SED_TRY_CUDA(cudaGetLastError());
   int err = 0;
   SED_TRY_CUDA(cudaMemcpyAsync(&err, d.tc_error.ptr, 4, cudaMemcpyDeviceToHost, s));
@@ -1973,37 +2291,36 @@ int sed_mlp_start_vector(sed_mlp* m, ls_spin_basis const* basis, double* out) {
   ScopedDevice dev(d.device);
   if (int st = wait_for_caller({out})) return st;
   uint64_t const D = b.D, chunk = 1u << 18;
-  DeviceBuffer amp, part, vout;
-  if (int st = amp.allocate(D * 8)) return st;  // (a, s) pairs
+  cudaPointerAttributes attr{};
+  bool const dev_out = cudaPointerGetAttributes(&attr, out) == cudaSuccess &&
+                       (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged);
+  (void)cudaGetLastError();
+  // the network's (a, s) pairs take the vector's own place, 8 bytes per row
+  DeviceBuffer part, vout;
+  if (!dev_out)
+    if (int st = vout.allocate(D * 8)) return st;
+  double* const dst = dev_out ? out : vout.as<double>();
+  float* const amp = reinterpret_cast<float*>(dst);
   if (int st = part.allocate(152 * 16 * 4)) return st;
   if (d.n_sites && !fused_shape(d)) {
-    if (int st = forward_patch(d, b.reps.as<uint64_t>(), D, amp.as<float>())) return st;
+    if (int st = forward_patch(d, b.reps.as<uint64_t>(), D, amp)) return st;
   } else if (tc_eligible(d)) {
-    if (int st = forward_tc(d, b.reps.as<uint64_t>(), D, amp.as<float>())) return st;
+    if (int st = forward_tc(d, b.reps.as<uint64_t>(), D, amp)) return st;
   } else {
     for (uint64_t b0 = 0; b0 < D; b0 += chunk) {
       uint64_t const nb = std::min(chunk, D - b0);
       if (int st = forward(d, b.reps.as<uint64_t>() + b0, nb, false)) return st;
-      SED_TRY_CUDA(cudaMemcpyAsync(amp.as<float>() + 2 * b0, d.out.ptr, nb * 8, cudaMemcpyDeviceToDevice, d.stream));
+      SED_TRY_CUDA(cudaMemcpyAsync(amp + 2 * b0, d.out.ptr, nb * 8, cudaMemcpyDeviceToDevice, d.stream));
     }
   }
   unsigned const lb = blocks_for((int64_t)D);
-  { k_max_first<<<lb, 256, 0, d.stream>>>(amp.as<float>(), (int64_t)D, part.as<float>()); note_launches(1); }
+  { k_max_first<<<lb, 256, 0, d.stream>>>(amp, (int64_t)D, part.as<float>()); note_launches(1); }
   std::vector<float> hp(lb);
   SED_TRY_CUDA(cudaMemcpyAsync(hp.data(), part.ptr, lb * 4, cudaMemcpyDeviceToHost, d.stream));
   SED_TRY_CUDA(cudaStreamSynchronize(d.stream));
   float amax = -3.0e38f;
   for (float q : hp) amax = std::max(amax, q);
-  cudaPointerAttributes attr{};
-  bool const dev_out = cudaPointerGetAttributes(&attr, out) == cudaSuccess &&
-                       (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged);
-  (void)cudaGetLastError();
-  double* dst = out;
-  if (!dev_out) {
-    if (int st = vout.allocate(D * 8)) return st;
-    dst = vout.as<double>();
-  }
-  { k_start_from_net<<<lb, 256, 0, d.stream>>>(amp.as<float>(), b.reps.as<uint64_t>(), b.weights.as<uint32_t>(), (int64_t)D, d.sign_mask, amax, (double)b.plan.group_order, dst); note_launches(1); }
+  { k_start_from_net<<<lb, 256, 0, d.stream>>>(reinterpret_cast<float2 const*>(amp), b.reps.as<uint64_t>(), b.weights.as<uint32_t>(), (int64_t)D, d.sign_mask, amax, b.plan.group_order, exp_tables(), dst); note_launches(1); }
   SED_TRY_CUDA(cudaGetLastError());
   if (!dev_out) SED_TRY_CUDA(cudaMemcpyAsync(out, dst, D * 8, cudaMemcpyDeviceToHost, d.stream));
   SED_TRY_CUDA(cudaStreamSynchronize(d.stream));

@@ -298,3 +298,29 @@ def test_patch_network_transfers_between_lattices(sed):
     assert learned.eigenvalues[0] == pytest.approx(rand.eigenvalues[0], rel=1e-10)
     assert learned.residuals[0] <= 1e-8
     assert learned.iterations < rand.iterations, (learned.iterations, rand.iterations)
+
+
+@pytest.mark.parametrize("scale", [0.01, 1.0, 40.0])
+def test_start_vector_amplitudes(sed, scale):
+    """v_r = prior sign exp(a - a_max) / n_r against extended precision, from
+    the network's own outputs: the exponential is rounded once (0.56 ulp), the
+    norm and the product add 2 ulp; amplitudes down to exp(-600) and, below,
+    the library's exp (denormals: absolute)."""
+    from spined.learned import Mlp
+    b = build_model(lattices.heisenberg_chain(16, momentum=0, parity=0, spin_inversion=1))
+    net = Mlp(16, 128, sign_mask=0x5555, seed=3)
+    p = net.get_params()
+    p[-258:-2] *= scale * 10
+    net.set_params(p)
+    reps = sed.basis_get_states(b.basis).copy()
+    out = net.forward(reps)
+    v = net.start_vector(b.basis)
+    a, s = out[:, 0], out[:, 1]
+    d = (a - a.max()).astype(np.float32)
+    want = np.exp(d.astype(np.longdouble)) / b.basis.norms()
+    flip = np.array([bin(int(r) & 0x5555).count("1") & 1 for r in reps], bool)
+    want = np.where((s < 0) != flip, -want, want)
+    err = np.abs(v - want)
+    assert np.all(err <= 3 * 2.0 ** -53 * np.abs(want) + 2.0 ** -1070)
+    if scale == 40.0:
+        assert d.min() < -600
