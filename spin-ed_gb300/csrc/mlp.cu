@@ -304,12 +304,15 @@ __global__ void k_grad_rest(float* __restrict__ g, int n_in, int H, float const*
     if (q >= ob1 && q < oW2) continue;  // b1: k_column_sums
     float t = 0.0f;
     if (q < nW1) {
+#pragma unroll 8
       for (int z = 0; z < s1; ++z) t += w1part[(int64_t)z * nW1 + q];
     } else if (q < ob2) {
       int64_t const e = q - oW2;
+#pragma unroll 8
       for (int z = 0; z < s2; ++z) t += w2part[(int64_t)z * H * H + e];
     } else {
       int const c = q < oW3 ? (int)(q - ob2) : q < ob3 ? H + (int)(q - oW3) : 3 * H + (int)(q - ob3);
+#pragma unroll 16
       for (int b = 0; b < nhb; ++b) t += hpart[(int64_t)b * W + c];
     }
     g[q] = t;
@@ -553,45 +556,54 @@ __global__ void __launch_bounds__(256)
       ts[i] = row_ok ? bts[r] : 0.0f;
       sv[i] = row_ok ? bst[r] : 0;
     }
+    // the rows' sums together: one row after the other, their shuffles and
+    // the loss (FP64 on lane 0) were a serial chain (11.3 -> 10.4 us)
+    float pa[kHeadRows], ps[kHeadRows];
 #pragma unroll
     for (int i = 0; i < kHeadRows; ++i) {
-      int64_t const r = r0 + i;
-      if (r >= n) break;  // warp-uniform
-      float h[kHeadChunks][8];
-      float pa = 0.0f, ps = 0.0f;
+      pa[i] = ps[i] = 0.0f;
 #pragma unroll
       for (int q = 0; q < kHeadChunks; ++q) {
         uint32_t const wv[4] = {u[i][q].x, u[i][q].y, u[i][q].z, u[i][q].w};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          h[q][2 * k] = __uint_as_float(wv[k] << 16);
-          h[q][2 * k + 1] = __uint_as_float(wv[k] & 0xFFFF0000u);
-        }
-#pragma unroll
         for (int j = 0; j < 8; ++j) {
-          pa = fmaf(w0[q][j], h[q][j], pa);
-          ps = fmaf(w1[q][j], h[q][j], ps);
+          float const h = __uint_as_float(j & 1 ? wv[j >> 1] & 0xFFFF0000u : wv[j >> 1] << 16);
+          pa[i] = fmaf(w0[q][j], h, pa[i]);
+          ps[i] = fmaf(w1[q][j], h, ps[i]);
         }
       }
+    }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        pa += __shfl_xor_sync(0xffffffffu, pa, o);
-        ps += __shfl_xor_sync(0xffffffffu, ps, o);
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < kHeadRows; ++i) {
+        pa[i] += __shfl_xor_sync(0xffffffffu, pa[i], o);
+        ps[i] += __shfl_xor_sync(0xffffffffu, ps[i], o);
       }
-      float const a = pa + b30, s = ps + b31;
-      float const da = a - ta[i];
+    float d0[kHeadRows], d1[kHeadRows];
+#pragma unroll
+    for (int i = 0; i < kHeadRows; ++i) {
+      bool const row_ok = r0 + i < n;
+      float const s = ps[i] + b31;
+      float const da = pa[i] + b30 - ta[i];
       float const y = fabsf(ts[i] - prior_flip(sv[i], sign_mask));
       float const pr = 1.0f / (1.0f + expf(-s));
-      float const d0 = 2.0f * da * inv_n, d1 = (pr - y) * inv_n;
+      d0[i] = row_ok ? 2.0f * da * inv_n : 0.0f;
+      d1[i] = row_ok ? (pr - y) * inv_n : 0.0f;
+      if (lane == i && row_ok) l += (double)da * da + (double)(fmaxf(s, 0.0f) - s * y + log1pf(expf(-fabsf(s))));
       if (lane == 0) {
-        l += (double)da * da + (double)(fmaxf(s, 0.0f) - s * y + log1pf(expf(-fabsf(s))));
-        sd0 += d0;
-        sd1 += d1;
+        sd0 += d0[i];
+        sd1 += d1[i];
       }
+    }
+#pragma unroll
+    for (int i = 0; i < kHeadRows; ++i) {
+      if (r0 + i >= n) break;  // warp-uniform
 #pragma unroll
       for (int q = 0; q < kHeadChunks; ++q) {
         int const ch = lane + 32 * q;
         if (ch >= chunks) continue;
+        uint32_t const wv[4] = {u[i][q].x, u[i][q].y, u[i][q].z, u[i][q].w};
         uint32_t pk[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -599,14 +611,15 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             int const j = 2 * k + e;
-            g[e] = (d0 * w0[q][j] + d1 * w1[q][j]) * (1.0f - h[q][j] * h[q][j]);
+            float const h = __uint_as_float(e ? wv[k] & 0xFFFF0000u : wv[k] << 16);
+            g[e] = (d0[i] * w0[q][j] + d1[i] * w1[q][j]) * (1.0f - h * h);
             ab[q][j] += g[e];
-            a0[q][j] = fmaf(d0, h[q][j], a0[q][j]);
-            a1[q][j] = fmaf(d1, h[q][j], a1[q][j]);
+            a0[q][j] = fmaf(d0[i], h, a0[q][j]);
+            a1[q][j] = fmaf(d1[i], h, a1[q][j]);
           }
           pk[k] = tc::pack_bf16x2(g[0], g[1]);
         }
-        reinterpret_cast<uint4*>(g2 + r * H)[ch] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        reinterpret_cast<uint4*>(g2 + (r0 + i) * H)[ch] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
     }
   }
@@ -1205,7 +1218,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_forward_tc(MlpTcArgs p) {
 // tanh instructions and 1.6 the MMAs) and read 160 KB of weights per tile
 // from L2. The arithmetic and its order are the same. Network 36-256-256-2 on
 // 15.8 M states: 4501 -> 3603 us, bound by the epilogue warps
-// MUFU.
+// (41 % of the MUFU rate, 48 % of the issue slots).
 constexpr int kResMaxHidden = 256;
 size_t tc_resident_smem(int hidden) {
   return 2 * (size_t)kTcRows * 128 + (size_t)hidden * 128 + (size_t)hidden * hidden * 2 + 4 * (size_t)hidden * 4 +
@@ -1516,6 +1529,7 @@ struct MlpData {
   // [n_sites][P] on the device; one activation row per (sample, site)
   unsigned n_sites = 0;
   DeviceBuffer patch_dev;
+  DeviceBuffer in_states, in_abs, in_sign;  // device copies of a loss_grad call's samples
   CUtensorMap mXk{}, mXm{}, mW1k{}, mH1k{}, mH1m{}, mW2k{}, mW2m{}, mG2k{}, mG2m{}, mG1m{};
   ~MlpData() {
     if (stream) cudaStreamDestroy(stream);
@@ -1674,9 +1688,10 @@ int refresh_bf16(MlpData& d) {
   return LS_SUCCESS;
 }
 
-// device copy of a host-or-device array
+// device copy of a host-or-device array (buf grows when it is too small)
 int stage(DeviceBuffer& buf, void const* src, size_t bytes, cudaStream_t s) {
-  if (int st = buf.allocate(std::max<size_t>(bytes, 16))) return st;
+  if (buf.bytes < std::max<size_t>(bytes, 16))
+    if (int st = buf.allocate(std::max<size_t>(bytes, 16))) return st;
   SED_TRY_CUDA(cudaMemcpyAsync(buf.ptr, src, bytes, cudaMemcpyDefault, s));
   return LS_SUCCESS;
 }
@@ -1709,7 +1724,10 @@ TcShape tc_shape(MlpData const& d, uint64_t n) {
   t.s2 = tc_split(d, mh * (H / tn), t.k_tiles);
   t.s1 = tc_split(d, mh, t.k_tiles);
   t.m_tiles = (t.rows + 127) / 128;
-  uint64_t const per_block = d.n_sites ? 8 : 64;  // samples per output-layer block
+  // samples per output-layer block: 64, but 32 (a group of four rows a warp)
+  // while that is at most two blocks a multiprocessor; a batch of 4096 in 64
+  // blocks left most of the GPU idle (k_head 14.9 us, in 128 blocks 11.3)
+  uint64_t const per_block = d.n_sites ? 8 : n <= 32 * 2 * 152 ? 32 : 64;
   t.hb = (int)std::max<uint64_t>(1, std::min<uint64_t>((n + per_block - 1) / per_block, 152 * 16));
   return t;
 }
@@ -2092,7 +2110,7 @@ int sed_mlp_loss_grad(sed_mlp* m, uint64_t const* states, float const* t_abs, fl
   MlpData& d = m->d;
   ScopedDevice dev(d.device);
   if (int st = wait_for_caller({states, t_abs, t_sign, grads})) return st;
-  DeviceBuffer sb, ta, ts;
+  DeviceBuffer &sb = d.in_states, &ta = d.in_abs, &ts = d.in_sign;
   if (int st = stage(sb, states, n * 8, d.stream)) return st;
   if (int st = stage(ta, t_abs, n * 4, d.stream)) return st;
   if (int st = stage(ts, t_sign, n * 4, d.stream)) return st;
