@@ -432,6 +432,8 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix(StreamView S, FixView fv, u
   if (ind.partial) {
     double const tot = block_sum_fixed(part, red);
     finish_apply(tot, ind);
+  } else if (ind.clear && blockIdx.x == 0 && threadIdx.x == 0) {
+    *ind.clear = 0;
   }
 }
 
@@ -1277,6 +1279,7 @@ int fix_reserve(OperatorData& op, uint32_t cols) {
   if (int st = slots.allocate((size_t)cols * 16)) return st;
   uint32_t const had = op.fix_cols;
   op.fix_cols = 0;
+  op.fix_clean = false;
   if (int st = op.fix_u.allocate((D + 1) * cols * 8)) {
     // the narrower workspace goes back, so that narrower passes still run
     if (had && op.fix_u.allocate((D + 1) * had * 8) == LS_SUCCESS) op.fix_cols = had;
@@ -1288,7 +1291,25 @@ int fix_reserve(OperatorData& op, uint32_t cols) {
 }
 
 int fix_wait(OperatorData& op) {
-  if (op.fix_event && op.fix_event_recorded) SED_TRY_CUDA(cudaEventSynchronize(op.fix_event));
+  if (op.fix_own) SED_TRY_CUDA(cudaStreamSynchronize(op.cuda_stream));
+  else if (op.fix_event && op.fix_event_recorded) SED_TRY_CUDA(cudaEventSynchronize(op.fix_event));
+  return LS_SUCCESS;
+}
+
+int fix_enter(OperatorData& op, cudaStream_t stream) {
+  if (op.fix_own && stream != op.cuda_stream) {
+    SED_TRY_CUDA(cudaEventRecord(op.fix_event, op.cuda_stream));
+    op.fix_event_recorded = true;
+    op.fix_own = false;
+  }
+  if (op.fix_event_recorded) SED_TRY_CUDA(cudaStreamWaitEvent(stream, op.fix_event, 0));
+  return LS_SUCCESS;
+}
+
+int fix_leave(OperatorData& op, cudaStream_t stream) {
+  op.fix_own = stream == op.cuda_stream;
+  op.fix_event_recorded = !op.fix_own;  // the own stream has waited for any earlier use
+  if (!op.fix_own) SED_TRY_CUDA(cudaEventRecord(op.fix_event, stream));
   return LS_SUCCESS;
 }
 
@@ -1320,7 +1341,7 @@ void launch_otf_fix(OperatorData& op, double const* x, int64_t const* u, int64_t
 
 // y = H x in fixed point: max |x|, u = round(sqrt(S) x 2^F), then the SpMV.
 // Outside a Krylov graph the shared workspace is ordered across the callers'
-// streams by fix_event.
+// streams (fix_enter, fix_leave).
 int launch_apply_fix(OperatorData& op, double const* x, double* y, cudaStream_t stream, bool use_stream,
                      Indirect ind) {
   BasisData& b = *op.basis;
@@ -1330,9 +1351,15 @@ int launch_apply_fix(OperatorData& op, double const* x, double* y, cudaStream_t 
   auto* F = reinterpret_cast<int64_t*>(mx + op.fix_cols);
   int64_t* u = op.fix_u.as<int64_t>();
   bool const ordered = ind.k == nullptr;
-  if (ordered && op.fix_event_recorded) SED_TRY_CUDA(cudaStreamWaitEvent(stream, op.fix_event, 0));
+  if (ordered)
+    if (int st = fix_enter(op, stream)) return st;
+  // the SpMV leaves the max |x| word zero for the next call's pre-pass
+  bool const clean = op.fix_clean;
+  bool const clears = ordered && use_stream && !ind.prescaled;
+  if (!ind.prescaled) op.fix_clean = false;
+  if (clears) ind.clear = mx;
   if (!ind.prescaled) {
-    SED_TRY_CUDA(cudaMemsetAsync(mx, 0, 8, stream));
+    if (!clean) SED_TRY_CUDA(cudaMemsetAsync(mx, 0, (size_t)op.fix_cols * 8, stream));
     unsigned const vg = grid_size(D, b.device, 8);
     k_fix_max<<<vg, kBlock, 0, stream>>>(x, 0, D, mx, ind);
     k_fix_convert<<<vg, kBlock, 0, stream>>>(x, 0, D, use_stream ? op.stream.row_class.as<uint8_t>() : nullptr,
@@ -1357,8 +1384,8 @@ int launch_apply_fix(OperatorData& op, double const* x, double* y, cudaStream_t 
   }
   SED_TRY_CUDA(cudaGetLastError());
   if (ordered) {
-    SED_TRY_CUDA(cudaEventRecord(op.fix_event, stream));
-    op.fix_event_recorded = true;
+    op.fix_clean = op.fix_clean || clears;
+    if (int st = fix_leave(op, stream)) return st;
   }
   return LS_SUCCESS;
 }
@@ -1368,6 +1395,7 @@ int launch_apply_fix(OperatorData& op, double const* x, double* y, cudaStream_t 
 bool fix_slots(OperatorData& op, FixSlots* out) {
   if (!op.tables || !op.tables->fix_ok || op.fix_cols < 1 || !op.stream.ready || op.form == SED_FORM_ON_THE_FLY)
     return false;
+  op.fix_clean = false;  // the caller's
   auto* mx = op.fix_slots.as<unsigned long long>();
   out->max_bits = mx;
   out->F = reinterpret_cast<int64_t*>(mx + op.fix_cols);

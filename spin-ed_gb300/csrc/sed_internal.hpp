@@ -219,12 +219,17 @@ struct OperatorData {
   cudaStream_t cuda_stream = nullptr;
   // fixed-point matvec workspace (see operator_impl.cuh): u for fix_cols
   // columns, then per column the max |x| bit pattern and the exponent F;
-  // fix_event orders its reuse across the callers' streams
+  // fix_enter and fix_leave order its reuse across the callers' streams:
+  // fix_event marks the last use on a caller's stream, fix_own says that the
+  // last use was on cuda_stream (recorded only when another stream comes).
+  // fix_clean: all max |x| words are zero
   DeviceBuffer fix_u;
   DeviceBuffer fix_slots;
   uint32_t fix_cols = 0;
   cudaEvent_t fix_event = nullptr;
   bool fix_event_recorded = false;
+  bool fix_own = false;
+  bool fix_clean = false;
   // the FP32-stored Krylov phase's gather copy: u_j in int32, then its slots
   DeviceBuffer fix_u32;
   DeviceBuffer fix_slots32;
@@ -247,6 +252,9 @@ int operator_apply_device(OperatorData& op, int dtype, uint64_t block, void cons
 // that workspace on any caller's stream.
 int fix_reserve(OperatorData& op, uint32_t cols);
 int fix_wait(OperatorData& op);
+// Around every use of the workspace on `stream` outside a Krylov graph.
+int fix_enter(OperatorData& op, cudaStream_t stream);
+int fix_leave(OperatorData& op, cudaStream_t stream);
 // FP32 companions of the stream form (mixed-precision Krylov phase).
 int operator_prepare_fp32(OperatorData& op, cudaStream_t stream);
 

@@ -169,10 +169,12 @@ __device__ __forceinline__ V general_row(StreamView const& S, Columns const& c, 
 template <bool Packed, int NV, bool Signed, int K>
 __global__ void __launch_bounds__(kBlock) k_spmv_fix_cols(StreamView S, FixView fv, uint64_t D, Columns c,
                                                           int64_t const* __restrict__ u,
-                                                          int64_t const* __restrict__ F_in) {
+                                                          int64_t const* __restrict__ F_in,
+                                                          unsigned long long* __restrict__ clear) {
   constexpr uint32_t N = K < 4 ? K : 4, L = K / N;  // columns per lane, lanes per row
   extern __shared__ double fix_smem[];                 // g[K][n_div NV], then the code bytes
   __shared__ bool bad;
+  if (blockIdx.x == 0 && threadIdx.x < K) clear[threadIdx.x] = 0;  // max |x| for the next call's pre-pass
   uint8_t* code8 = reinterpret_cast<uint8_t*>(fix_smem + K * fv.n_div * NV);
   if constexpr (Signed) fix_stage_codes(fv, code8);
   for (uint32_t q = 0; q < c.cols; ++q) fix_row_factors<NV>(fv, S.inv_sqrt_s, F_in[q], fix_smem + q * fv.n_div * NV);
@@ -247,8 +249,9 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
   auto* mx = op.fix_slots.as<unsigned long long>();
   auto* F = reinterpret_cast<int64_t*>(mx + op.fix_cols);
   int64_t* u = op.fix_u.as<int64_t>();
-  if (op.fix_event_recorded) SED_TRY_CUDA(cudaStreamWaitEvent(stream, op.fix_event, 0));
-  SED_TRY_CUDA(cudaMemsetAsync(mx, 0, (size_t)K * 8, stream));
+  if (int st = fix_enter(op, stream)) return st;
+  if (!op.fix_clean) SED_TRY_CUDA(cudaMemsetAsync(mx, 0, (size_t)op.fix_cols * 8, stream));
+  op.fix_clean = false;
   unsigned const vg = std::max(1u, grid_size(c.cx ? 2 * D : D, b.device, 8) / (c.cols > 2 ? 4 : 1));
   uint8_t const* cls = sf.row_class.as<uint8_t>();
   k_fix_max_cols<<<dim3(vg, c.cx ? c.cols / 2 : c.cols), kBlock, 0, stream>>>(c, D, mx);
@@ -263,7 +266,7 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
     unsigned const cg = grid_size((D + 1) * (KK > 2 ? KK / 2 : 1), b.device, 8);
     k_fix_convert_cols<KK><<<cg, kBlock, (size_t)KK * tb.fix.n_div * 8, stream>>>(c, D, cls, tb.fix, mx, F, u);
     fix_dispatch(tb, sf.packed, [&](auto packed, auto nv, auto sign) {
-      k_spmv_fix_cols<packed.value, nv.value, sign.value, KK><<<grid, kBlock, smem, stream>>>(S, tb.fix, D, c, u, F);
+      k_spmv_fix_cols<packed.value, nv.value, sign.value, KK><<<grid, kBlock, smem, stream>>>(S, tb.fix, D, c, u, F, mx);
     });
   };
   switch (K) {
@@ -275,9 +278,8 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
   }
   note_launches(3);
   SED_TRY_CUDA(cudaGetLastError());
-  SED_TRY_CUDA(cudaEventRecord(op.fix_event, stream));
-  op.fix_event_recorded = true;
-  return LS_SUCCESS;
+  op.fix_clean = true;  // the SpMV has cleared the words again
+  return fix_leave(op, stream);
 }
 
 }  // namespace
