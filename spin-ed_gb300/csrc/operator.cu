@@ -1405,6 +1405,21 @@ bool fix_slots(OperatorData& op, FixSlots* out) {
   return true;
 }
 
+bool fix_slots32(OperatorData& op, FixSlots32* out) {
+  if (!op.tables || !op.tables->fix_ok || !op.fix_u32.ptr || !op.stream.ready || !op.stream.diag_f.ptr) return false;
+  out->F = reinterpret_cast<int64_t*>(op.fix_slots32.as<unsigned long long>() + 1);
+  out->u = op.fix_u32.as<int32_t>();
+  out->row_class = op.stream.row_class.as<uint8_t>();
+  out->view = op.tables->fix;
+  return true;
+}
+
+int operator_apply_prescaled(OperatorData& op, double const* x, double* y, cudaStream_t stream) {
+  Indirect ind;
+  ind.prescaled = true;
+  return launch_apply_fix(op, x, y, stream, true, ind);
+}
+
 int fix_prescale(OperatorData& op, double const* base, Indirect ind, cudaStream_t stream) {
   FixSlots fs;
   if (!fix_slots(op, &fs)) return fail(LS_SYSTEM_ERROR, "fix_prescale: the operator has no fixed-point form");
@@ -1806,12 +1821,14 @@ int launch32(OperatorData& op, float const* x, float* y, Indirect ind, cudaStrea
   if (tb.fix_ok && op.fix_u32.ptr) {
     uint64_t const D = op.basis->D;
     auto* slots = op.fix_slots32.as<unsigned long long>();
-    SED_TRY_CUDA(cudaMemsetAsync(slots, 0, 8, stream));
-    unsigned const vg = grid_size(D, op.basis->device, 8);
-    k_fix_max32<<<vg, kBlock, 0, stream>>>(x, D, slots, ind);
-    k_fix_convert32<<<vg, kBlock, 0, stream>>>(x, D, sf.row_class.as<uint8_t>(), tb.fix, slots,
-                                               reinterpret_cast<int64_t*>(slots + 1), op.fix_u32.as<int32_t>(), ind);
-    note_launches(2);
+    if (!ind.prescaled) {
+      SED_TRY_CUDA(cudaMemsetAsync(slots, 0, 8, stream));
+      unsigned const vg = grid_size(D, op.basis->device, 8);
+      k_fix_max32<<<vg, kBlock, 0, stream>>>(x, D, slots, ind);
+      k_fix_convert32<<<vg, kBlock, 0, stream>>>(x, D, sf.row_class.as<uint8_t>(), tb.fix, slots,
+                                                 reinterpret_cast<int64_t*>(slots + 1), op.fix_u32.as<int32_t>(), ind);
+      note_launches(2);
+    }
     launch_spmv32_fix(op, S, x, y, ind, stream, grid);
     SED_TRY_CUDA(cudaGetLastError());
     return LS_SUCCESS;
@@ -1831,8 +1848,10 @@ int operator_apply_krylov32(OperatorData& op, float* base, Indirect ind, cudaStr
   return launch32(op, base, base, ind, stream);
 }
 
-int operator_apply32(OperatorData& op, float const* x, float* y, cudaStream_t stream) {
-  return launch32(op, x, y, Indirect{}, stream);
+int operator_apply32(OperatorData& op, float const* x, float* y, cudaStream_t stream, bool prescaled) {
+  Indirect ind;
+  ind.prescaled = prescaled;
+  return launch32(op, x, y, ind, stream);
 }
 
 int operator_apply_krylov(OperatorData& op, int dtype, void* base, Indirect ind, cudaStream_t stream) {

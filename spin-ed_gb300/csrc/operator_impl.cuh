@@ -231,6 +231,13 @@ __device__ __forceinline__ void fix_row_factors(FixView const& fv, double const*
     g[t] = F == kFixBad ? 0.0 : fix_ldexp(__dmul_rn(inv_sqrt_s[t / NV], fv.c[t % NV]), -Fa);
 }
 
+// (double)f from the bits: the conversion instruction runs on the FP64 pipe.
+__device__ __forceinline__ double widen(float f) {
+  uint32_t const b = __float_as_uint(f), e = (b >> 23) & 0xFFu;
+  if (e == 0 || e == 0xFF) return (double)f;
+  return __hiloint2double((int)((b & 0x80000000u) | ((e + 896u) << 20) | ((b & 0x7FFFFFu) >> 3)), (int)(b << 29));
+}
+
 // (double)v to nearest (ties to even) with integer instructions: the
 // conversion runs on the FP64 pipe.
 __device__ __forceinline__ double fix_to_double(int64_t v) {
@@ -446,8 +453,19 @@ inline size_t fix_smem_bytes(OperatorTables const& tb, unsigned K) {
 // FP32 streamed SpMV in Krylov-indirect mode (x = base + k ld, y = base +
 // (k+1) ld); FP32 arithmetic, per-block partial sums of x_i y_i in FP64.
 int operator_apply_krylov32(OperatorData& op, float* base, Indirect ind, cudaStream_t stream);
-// The same SpMV on explicit FP32 vectors.
-int operator_apply32(OperatorData& op, float const* x, float* y, cudaStream_t stream);
+// The same SpMV on explicit FP32 vectors; prescaled: u and F of x are in the
+// workspace already.
+int operator_apply32(OperatorData& op, float const* x, float* y, cudaStream_t stream, bool prescaled = false);
+// The fixed-point workspace of that SpMV (true if it has one), and y = H x in
+// FP64 with u and F of x in the workspace already (fix_slots).
+struct FixSlots32 {
+  int64_t* F;
+  int32_t* u;
+  uint8_t const* row_class;
+  FixView view;
+};
+bool fix_slots32(OperatorData& op, FixSlots32* out);
+int operator_apply_prescaled(OperatorData& op, double const* x, double* y, cudaStream_t stream);
 // Krylov-indirect apply (see Indirect), on at most ceil(D / kBlock) blocks.
 int operator_apply_krylov(OperatorData& op, int dtype, void* base, Indirect ind, cudaStream_t stream);
 int operator_ensure_ready(OperatorData& op);

@@ -35,13 +35,6 @@ struct Columns {
   }
 };
 
-// (double)f from the bits: the conversion instruction runs on the FP64 pipe.
-__device__ __forceinline__ double widen(float f) {
-  uint32_t const b = __float_as_uint(f), e = (b >> 23) & 0xFFu;
-  if (e == 0 || e == 0xFF) return (double)f;
-  return __hiloint2double((int)((b & 0x80000000u) | ((e + 896u) << 20) | ((b & 0x7FFFFFu) >> 3)), (int)(b << 29));
-}
-
 // k_fix_max for Columns: blockIdx.y is the vector column.
 __global__ void __launch_bounds__(kBlock) k_fix_max_cols(Columns c, uint64_t D, unsigned long long* __restrict__ max_bits) {
   __shared__ unsigned long long red[2][kBlock / 32];

@@ -27,13 +27,14 @@
 #include <cstring>
 #include <vector>
 
+#include "df.cuh"
 #include "operator_impl.cuh"
 
 namespace sed {
 namespace {
 
 constexpr int kMaxThick = 32;
-constexpr int kDotCols = 8;
+constexpr uint32_t kProjCols = 16;  // columns of a projection group
 
 template <class S>
 __device__ __forceinline__ double ldv(S const* p, uint64_t i) { return (double)p[i]; }
@@ -51,79 +52,238 @@ struct Arith<float> {
   using T = float;
 };
 
-// partial[(g * gridDim.x + b) * kDotCols + c] = sum over this block's rows
-// of V[:, NC g + c] . w for c < NC (columns >= ncols give 0); blockIdx.y = g.
-// NC is a template parameter: on GB300 a predicated-off FP64 FMA still takes
-// its issue slot on the slow FP64 pipe, so the column count of a launch is
-// matched exactly instead of padding to a fixed width.
+// Totals of N columns over the warp's lanes: lane l returns column l / (32 /
+// N). The columns are transposed while they are added, so a lane makes N - 1 +
+// 5 - log2 N additions instead of 5 N: on FP64 sums these additions bound the
+// dots of short FP32 rows.
+template <int N>
+__device__ __forceinline__ double warp_columns(double (&a)[N]) {
+  uint32_t const lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int n = N; n > 1; n >>= 1, o >>= 1) {
+    bool const up = (lane & (uint32_t)o) != 0;
+#pragma unroll
+    for (int j = 0; j < N / 2; ++j) {
+      if (j >= n / 2) break;
+      double const give = up ? a[j] : a[j + n / 2], keep = up ? a[j + n / 2] : a[j];
+      a[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  double x = a[0];
+  for (; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+constexpr int pow2_at_least(int n) { return n <= 1 ? 1 : n <= 2 ? 2 : n <= 4 ? 4 : n <= 8 ? 8 : 16; }
+
+// out[c] = V[:, c] . w for c < ncols, by the last block to finish; blockIdx.y
+// = g takes columns NC g .. . With npre > 0 (one group only) the projections
+// `pre` on the last npre columns are first taken out of w, in the same pass:
+// the second Gram-Schmidt dots and the first update read V once. NC is a
+// template parameter: a predicated-off FP64 FMA still takes its issue slot on
+// the slow FP64 pipe, so the column count of a launch is matched exactly. The
+// sums stay on the device (as 39 KB of partials for the host every step they
+// cost three round trips, 8 of the 44 ms of a mixed solve of the 32-site
+// ring). partial: ncols x gridDim.x; *clear is zeroed.
 template <class S, int NC>
-__global__ void __launch_bounds__(256) k_tdots(S const* __restrict__ V, uint64_t ld, uint32_t ncols,
-                                               S const* __restrict__ w, uint64_t D, double* __restrict__ partial) {
+__global__ void __launch_bounds__(256)
+    k_tproj(S const* __restrict__ V, uint64_t ld, uint32_t ncols, S* __restrict__ w, uint64_t D,
+            double const* __restrict__ pre, uint32_t npre, double* __restrict__ partial, uint32_t* __restrict__ done,
+            double* __restrict__ out, unsigned long long* __restrict__ clear) {
   using T = typename Arith<S>::T;
-  __shared__ double red[8][NC];
+  constexpr int N = pow2_at_least(NC);
+  __shared__ double red[8][N];
+  __shared__ bool last;
   uint32_t const c0 = blockIdx.y * NC;
   uint32_t const nc = ncols - c0 < (uint32_t)NC ? ncols - c0 : (uint32_t)NC;
   S const* const Vc = V + (uint64_t)c0 * ld;
   T acc[NC] = {};
-  if (nc == (uint32_t)NC) {
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < D; r += (uint64_t)gridDim.x * blockDim.x) {
-      T const wr = (T)w[r];
+  T const f0 = npre > 1 ? (T)pre[0] : (T)0, f1 = npre ? (T)pre[npre - 1] : (T)0;
+  for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < D; r += (uint64_t)gridDim.x * blockDim.x) {
+    T x = (T)w[r];
+    T v[NC];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) acc[c] = fma((T)Vc[(uint64_t)c * ld + r], wr, acc[c]);
+    for (int c = 0; c < NC; ++c) v[c] = c < (int)nc ? (T)Vc[(uint64_t)c * ld + r] : (T)0;
+    if (npre) {
+      if (NC > 1 && npre > 1) x = fma(-v[NC > 1 ? NC - 2 : 0], f0, x);
+      x = fma(-v[NC - 1], f1, x);
+      w[r] = (S)x;
+      x = (T)(S)x;
     }
-  } else {  // short last group (at most NC - 1 predicated-off columns)
-    for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < D; r += (uint64_t)gridDim.x * blockDim.x) {
-      T const wr = (T)w[r];
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
-        if (c < (int)nc) acc[c] = fma((T)Vc[(uint64_t)c * ld + r], wr, acc[c]);
-    }
+    for (int c = 0; c < NC; ++c)
+      if (c < (int)nc) acc[c] = fma(v[c], x, acc[c]);
   }
   int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double a[N];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    double x = (double)acc[c];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (lane == 0) red[warp][c] = x;
+  for (int c = 0; c < N; ++c) a[c] = c < NC ? (double)acc[c < NC ? c : 0] : 0.0;
+  double const t = warp_columns<N>(a);
+  if (lane % (32 / N) == 0) red[warp][lane / (32 / N)] = t;
+  __syncthreads();
+  if (threadIdx.x < nc) {
+    double s = 0.0;
+    for (int q = 0; q < 8; ++q) s += red[q][threadIdx.x];
+    partial[(uint64_t)(c0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
+    __threadfence();
   }
   __syncthreads();
-  if (threadIdx.x < NC) {
+  if (threadIdx.x == 0) last = atomicAdd(done + blockIdx.y, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (uint32_t c = warp; c < nc; c += 8) {
     double s = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += red[q][threadIdx.x];
-    partial[((uint64_t)blockIdx.y * gridDim.x + blockIdx.x) * kDotCols + threadIdx.x] = s;
+    for (uint32_t b = lane; b < gridDim.x; b += 32) s += __ldcg(partial + (uint64_t)(c0 + c) * gridDim.x + b);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[c0 + c] = s;
+  }
+  if (threadIdx.x == 0) {
+    done[blockIdx.y] = 0;
+    if (clear && blockIdx.y == 0) *clear = 0;
   }
 }
 
-// Launch of k_tdots over ncols columns in g = ceil(ncols / 8) groups of
-// NC = ceil(ncols / g) columns; returns NC.
+// k_tproj over ncols columns, in one group of up to 16 or in two equal ones.
 template <class S>
-int launch_tdots(S const* V, uint64_t ld, uint32_t ncols, S const* w, uint64_t D, double* partial, unsigned vb,
+int launch_tproj(S const* V, uint64_t ld, uint32_t ncols, S* w, uint64_t D, double const* pre, uint32_t npre,
+                 double* partial, uint32_t* done, double* out, unsigned long long* clear, unsigned vb,
                  cudaStream_t stream) {
-  uint32_t const g = (ncols + kDotCols - 1) / kDotCols;
+  uint32_t const g = (ncols + kProjCols - 1) / kProjCols;
   int const nc = (int)((ncols + g - 1) / g);
   dim3 const grid(vb, g);
   switch (nc) {
-#define SED_TDOTS(N) \
-  case N: { k_tdots<S, N><<<grid, 256, 0, stream>>>(V, ld, ncols, w, D, partial); note_launches(1); } break;
-    SED_TDOTS(1) SED_TDOTS(2) SED_TDOTS(3) SED_TDOTS(4) SED_TDOTS(5) SED_TDOTS(6) SED_TDOTS(7) SED_TDOTS(8)
-#undef SED_TDOTS
+#define SED_TPROJ(N) \
+  case N: k_tproj<S, N><<<grid, 256, 0, stream>>>(V, ld, ncols, w, D, pre, npre, partial, done, out, clear); break;
+    SED_TPROJ(1) SED_TPROJ(2) SED_TPROJ(3) SED_TPROJ(4) SED_TPROJ(5) SED_TPROJ(6) SED_TPROJ(7) SED_TPROJ(8)
+    SED_TPROJ(9) SED_TPROJ(10) SED_TPROJ(11) SED_TPROJ(12) SED_TPROJ(13) SED_TPROJ(14) SED_TPROJ(15) SED_TPROJ(16)
+#undef SED_TPROJ
   }
-  return nc;
+  note_launches(1);
+  SED_TRY_CUDA(cudaGetLastError());
+  return LS_SUCCESS;
 }
 
-// w -= sum_{c < ncols} V[:, c] coef[c]  (FP64 arithmetic)
+// w -= sum_{c < ncols} V[:, c] coef[c]; with beta not null also *beta = ||w||
+// (by the last block) and *wmax = max |w| as a double's bits.
 template <class S>
-__global__ void k_tupdate(S const* __restrict__ V, uint64_t ld, uint32_t ncols, double const* __restrict__ coef,
-                          S* __restrict__ w, uint64_t D) {
+__global__ void __launch_bounds__(256)
+    k_tupdate(S const* __restrict__ V, uint64_t ld, uint32_t ncols, double const* __restrict__ coef, S* __restrict__ w,
+              uint64_t D, double* __restrict__ partial, uint32_t* __restrict__ done, double* __restrict__ beta,
+              unsigned long long* __restrict__ wmax) {
   using T = typename Arith<S>::T;
   __shared__ T cf[kMaxThick + 1];
+  __shared__ double red[8];
+  __shared__ unsigned long long redm[8];
   for (uint32_t c = threadIdx.x; c < ncols; c += blockDim.x) cf[c] = (T)coef[c];
   __syncthreads();
+  T part = 0;
+  unsigned long long m = 0;  // bit pattern: keeps the order, infinities and NaN
   for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < D; r += (uint64_t)gridDim.x * blockDim.x) {
     T x = (T)w[r];
-    for (uint32_t c = 0; c < ncols; ++c) x = fma(-(T)V[(uint64_t)c * ld + r], cf[c], x);
+    uint32_t c = 0;
+    for (; c + 8 <= ncols; c += 8) {
+      T v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = (T)V[(uint64_t)(c + q) * ld + r];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) x = fma(-v[q], cf[c + q], x);
+    }
+    for (; c < ncols; ++c) x = fma(-(T)V[(uint64_t)c * ld + r], cf[c], x);
     w[r] = (S)x;
+    if (beta) {
+      x = (T)(S)x;
+      part = fma(x, x, part);
+      if constexpr (std::is_same<S, float>::value) m = max((uint32_t)m, __float_as_uint(x) & 0x7FFFFFFFu);
+      else m = max(m, (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull);
+    }
   }
+  if (!beta) return;
+  if constexpr (std::is_same<S, float>::value)
+    m = (unsigned long long)__double_as_longlong((double)__uint_as_float((uint32_t)m));
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) redm[threadIdx.x >> 5] = m;
+  double const tot = block_sum((double)part, red);
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < 8; ++q) m = max(m, redm[q]);
+    atomicMax(wmax, m);
+  }
+  finish_sum(tot, partial, done, [&](double s) { *beta = sqrt(s); });
+}
+
+// Where the next matvec's gather copy goes (fix_slots, fix_slots32).
+template <class S>
+struct NextCopy {
+  using U = typename std::conditional<std::is_same<S, float>::value, int32_t, int64_t>::type;
+  bool on = false;
+  int64_t* F = nullptr;
+  U* u = nullptr;
+  uint8_t const* row_class = nullptr;
+  FixView view{};
+};
+
+__host__ __device__ inline bool thick_breakdown(double beta, double tkk) {
+  return !(beta > 1e-14 * fmax(1.0, fabs(tkk)));
+}
+
+// out = w / beta (zero on a breakdown; t1 + t2 = T_kk), and the next matvec's
+// gather copy of it. FP32: 1 / beta as two floats, two FP32 operations where
+// the FP64 product and its conversions took four on the FP64 pipe (w f is
+// rounded once either way, from 2^-46).
+template <class S>
+__global__ void __launch_bounds__(256)
+    k_tscale_next(S const* __restrict__ w, uint64_t D, double const* __restrict__ beta, double const* __restrict__ t1,
+                  double const* __restrict__ t2, unsigned long long const* __restrict__ wmax, S* __restrict__ out,
+                  NextCopy<S> next) {
+  __shared__ double fac[kFixMaxClasses];
+  double const b = *beta;
+  double const f = thick_breakdown(b, *t1 + *t2) ? 0.0 : 1.0 / b;
+  float const fh = (float)f, fl = (float)(f - (double)fh);
+  auto scaled = [&](S x) -> S {
+    if constexpr (std::is_same<S, float>::value) return fmaf(x, fh, __fmul_rn(x, fl));
+    else return x * f;
+  };
+  uint64_t const first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+  if (!next.on) {
+    for (uint64_t r = first; r < D; r += step) out[r] = scaled(w[r]);
+    return;
+  }
+  // the rounding of the scaled entries is monotone: the scaled maximum bounds them
+  double const most = (double)scaled((S)__longlong_as_double((long long)*wmax));
+  uint64_t const bits = (uint64_t)__double_as_longlong(fabs(most));
+  int64_t F;
+  if constexpr (std::is_same<S, float>::value) F = fix_exponent32(bits, next.view.sqrt_s_max);
+  else F = fix_exponent(bits, next.view.bound);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    *next.F = F;
+    next.u[D] = 0;  // the zero row (fix_row_sums)
+  }
+  int64_t const F1 = (F == kFixBad || (F >= -1000 && F <= 1000)) ? 0 : F / 2;
+  double const p1 = fix_pow2(F1), p2 = F == kFixBad ? 0.0 : fix_pow2(F - F1);
+  for (uint32_t c = threadIdx.x; c < next.view.n_div; c += blockDim.x) fac[c] = next.view.sqrt_s[c] * p2;
+  __syncthreads();
+  auto one = [&](uint64_t r, S wr, uint32_t cls) {
+    S const v = scaled(wr);
+    out[r] = v;
+    double x;
+    if constexpr (std::is_same<S, float>::value) x = widen(v);
+    else x = F1 ? v * p1 : v;
+    next.u[r] = F == kFixBad ? 0 : (typename NextCopy<S>::U)fix_round(x * fac[cls]);
+  };
+  uint64_t r = first;
+  for (; r + 3 * step < D; r += 4 * step) {  // four rows' loads in flight
+    S wr[4];
+    uint32_t cls[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      wr[q] = w[r + q * step];
+      cls[q] = next.row_class[r + q * step];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) one(r + q * step, wr[q], cls[q]);
+  }
+  for (; r < D; r += step) one(r, w[r], next.row_class[r]);
 }
 
 template <class S>
@@ -133,13 +293,45 @@ __global__ void k_tscale(S const* __restrict__ w, uint64_t D, double f, S* __res
 }
 
 // In place, row by row: V[:, c] <- sum_{i < m} V[:, i] Y[i * kk + c] for
-// c < kk <= 4 KB. The kk sums of a row are independent chains, one FMA of
-// each per V value; KB is a template parameter so that at most three
-// predicated-off FMAs per V value take FP64 issue slots.
-template <class S, int KB>
+// c < kk <= KC. FP32 storage sums in double-float (k_trotate32: products of
+// a float and a split FP64 coefficient, 2^-47 before the rounding to FP32, on
+// the FP32 pipe; FP64 FMAs took 1230 us for m = 16, kk = 8 on 4.7 M rows,
+// this 331). The kk sums of a row are independent chains, one FMA of
+// each per V value; KC is a template parameter (kk itself up to 16), since a
+// predicated-off FMA still takes its FP64 issue slot.
+template <int KC>
+__global__ void __launch_bounds__(256) k_trotate32(float* __restrict__ V, uint64_t ld, uint32_t m,
+                                                   double const* __restrict__ Y, uint32_t kk, uint64_t D) {
+  __shared__ float2 y[kMaxThick * KC];
+  for (uint32_t e = threadIdx.x; e < m * KC; e += blockDim.x) {
+    uint32_t const i = e / KC, c = e % KC;
+    float h = 0.0f, l = 0.0f;
+    if (c < kk) df_split(Y[i * kk + c], h, l);
+    y[e] = make_float2(h, l);
+  }
+  __syncthreads();
+  for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < D; r += (uint64_t)gridDim.x * blockDim.x) {
+    float S[KC], E[KC];
+#pragma unroll
+    for (int c = 0; c < KC; ++c) S[c] = E[c] = 0.0f;
+#pragma unroll 2
+    for (uint32_t i = 0; i < m; ++i) {
+      float const v = V[(uint64_t)i * ld + r];
+#pragma unroll
+      for (int c = 0; c < KC; ++c) {
+        float2 const t = y[i * KC + c];
+        df_mac(v, 0.0f, t.x, t.y, S[c], E[c]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < KC; ++c)
+      if (c < (int)kk) V[(uint64_t)c * ld + r] = __fadd_rn(S[c], E[c]);
+  }
+}
+
+template <class S, int KC>
 __global__ void k_trotate(S* __restrict__ V, uint64_t ld, uint32_t m, double const* __restrict__ Y, uint32_t kk,
                           uint64_t D) {
-  constexpr int KC = 4 * KB;
   __shared__ double y[kMaxThick * KC];
   for (uint32_t e = threadIdx.x; e < m * KC; e += blockDim.x) {
     uint32_t const i = e / KC, c = e % KC;
@@ -164,10 +356,16 @@ __global__ void k_trotate(S* __restrict__ V, uint64_t ld, uint32_t m, double con
 template <class S>
 void launch_trotate(S* V, uint64_t ld, uint32_t m, double const* Y, uint32_t kk, uint64_t D, unsigned vb,
                     cudaStream_t stream) {
-  switch ((kk + 3) / 4) {
+  switch (kk <= 16 ? kk : (kk + 3) / 4 * 4) {
 #define SED_TROT(N) \
-  case N: { k_trotate<S, N><<<vb, 256, 0, stream>>>(V, ld, m, Y, kk, D); note_launches(1); } break;
+  case N: \
+    if constexpr (std::is_same<S, float>::value) k_trotate32<N><<<vb, 256, 0, stream>>>(V, ld, m, Y, kk, D); \
+    else k_trotate<S, N><<<vb, 256, 0, stream>>>(V, ld, m, Y, kk, D); \
+    note_launches(1); \
+    break;
     SED_TROT(1) SED_TROT(2) SED_TROT(3) SED_TROT(4) SED_TROT(5) SED_TROT(6) SED_TROT(7) SED_TROT(8)
+    SED_TROT(9) SED_TROT(10) SED_TROT(11) SED_TROT(12) SED_TROT(13) SED_TROT(14) SED_TROT(15) SED_TROT(16)
+    SED_TROT(20) SED_TROT(24) SED_TROT(28) SED_TROT(32)
 #undef SED_TROT
   }
 }
@@ -322,6 +520,11 @@ __global__ void k_tout(double const* __restrict__ a, uint64_t D, int dtype, void
 int store_vector(double const* v, uint64_t D, int dtype, void* dst, cudaStream_t stream) {
   DeviceBuffer tmp;
   size_t const bytes = D * (size_t)elem_bytes_of(dtype);
+  if (dtype == 1) {
+    SED_TRY_CUDA(cudaMemcpyAsync(dst, v, bytes, cudaMemcpyDefault, stream));
+    SED_TRY_CUDA(cudaStreamSynchronize(stream));
+    return LS_SUCCESS;
+  }
   if (int st = tmp.allocate(bytes)) return st;
   { k_tout<<<grid_size(D, 0, 4), 256, 0, stream>>>(v, D, dtype, tmp.ptr); note_launches(1); }
   SED_TRY_CUDA(cudaGetLastError());
@@ -349,41 +552,57 @@ int thick_run(OperatorData& op, cudaStream_t stream, uint32_t m, uint32_t nev, d
   int const dtype = std::is_same<S, float>::value ? 0 : 1;
   int const dev = op.basis->device;
   unsigned const vb = grid_size(D, dev, 4);
-  uint32_t const groups = (m + 1 + kDotCols - 1) / kDotCols;
-  DeviceBuffer Vb, wb, w64, part, coef, Yb, rt_err;
-  if (int st = rt_err.allocate(4)) return st;
-  if (int st = Vb.allocate((size_t)(m + 1) * D * sizeof(S))) return st;
+  DeviceBuffer Vb, wb, w64, part, proj, coef, Yb, flags;
+  struct VGuard {
+    DeviceBuffer& b;
+    cudaStream_t s;
+    ~VGuard() {
+      cudaStreamSynchronize(s);  // steps may be in flight on an early exit
+      krylov_give(b);
+    }
+  } v_guard{Vb, stream};
+  if (int st = krylov_take((size_t)(m + 1) * D * sizeof(S), Vb)) return st;
   if (int st = wb.allocate(D * sizeof(S))) return st;
   if (int st = w64.allocate(D * 8)) return st;
-  if (int st = part.allocate((size_t)groups * vb * kDotCols * 8 + 16 * (size_t)vb)) return st;
+  if (int st = part.allocate((size_t)(kMaxThick + 1) * vb * 8)) return st;
+  // per basis index k: the two passes' projections and beta
+  constexpr uint32_t kSlot = 2 * (kMaxThick + 1) + 1;
+  if (int st = proj.allocate((size_t)(m + 1) * kSlot * 8)) return st;
   if (int st = coef.allocate((kMaxThick + 1) * 8)) return st;
   if (int st = Yb.allocate((size_t)kMaxThick * kMaxThick * 8)) return st;
+  if (int st = flags.allocate(64)) return st;  // max |w|, sum counters, the tensor-core rotation's error
+  SED_TRY_CUDA(cudaMemsetAsync(flags.ptr, 0, 64, stream));
+  auto* const wmax = flags.as<unsigned long long>();
+  uint32_t* const done = reinterpret_cast<uint32_t*>(wmax + 1);
+  int* const rt_err = reinterpret_cast<int*>(wmax + 4);
   S* V = Vb.as<S>();
   S* w = wb.as<S>();
-  std::vector<double> hp((size_t)groups * vb * kDotCols);
-  // res[c] = V[:, first + c] . x for c < ncols
-  auto dots_at = [&](uint32_t first, uint32_t ncols, S const* x, std::vector<double>& res) -> int {
-    uint32_t const g = (ncols + kDotCols - 1) / kDotCols;
-    int const nc = launch_tdots<S>(V + (uint64_t)first * D, D, ncols, x, D, part.as<double>(), vb, stream);
-    SED_TRY_CUDA(cudaGetLastError());
-    SED_TRY_CUDA(cudaMemcpyAsync(hp.data(), part.ptr, (size_t)g * vb * kDotCols * 8, cudaMemcpyDeviceToHost, stream));
+  std::vector<double> hproj((size_t)(m + 1) * kSlot), hres(2 * (size_t)vb);
+  auto slot = [&](uint32_t k) { return proj.as<double>() + (size_t)k * kSlot; };
+  NextCopy<S> next;
+  if constexpr (std::is_same<S, float>::value) {
+    FixSlots32 fs;
+    if (fix_slots32(op, &fs)) next = NextCopy<S>{true, fs.F, fs.u, fs.row_class, fs.view};
+  } else {
+    FixSlots fs;
+    if (fix_slots(op, &fs)) next = NextCopy<S>{true, fs.F, fs.u, fs.row_class, fs.view};
+  }
+  bool copied = false;  // the gather copy of v_k is in the workspace
+  // c = V[:, 0..ncols)^T x, on the host
+  auto dots = [&](uint32_t ncols, S* x, std::vector<double>& c) -> int {
+    c.resize(ncols);
+    if (int st = launch_tproj<S>(V, D, ncols, x, D, nullptr, 0, part.as<double>(), done, coef.as<double>(), nullptr, vb, stream))
+      return st;
+    SED_TRY_CUDA(cudaMemcpyAsync(c.data(), coef.ptr, ncols * 8, cudaMemcpyDeviceToHost, stream));
     SED_TRY_CUDA(cudaStreamSynchronize(stream));
-    res.assign(ncols, 0.0);
-    for (uint32_t gg = 0; gg < g; ++gg)
-      for (unsigned b = 0; b < vb; ++b)
-        for (int c = 0; c < nc; ++c)
-          if (gg * nc + c < ncols) res[gg * nc + c] += hp[((size_t)gg * vb + b) * kDotCols + c];
     return LS_SUCCESS;
   };
-  auto dots = [&](uint32_t ncols, S const* x, std::vector<double>& res) -> int { return dots_at(0, ncols, x, res); };
-  auto norm = [&](S const* x, double& nrm) -> int {
-    // ||x||: dots of column 0 of a one-column "V" = x itself
-    launch_tdots<S>(x, D, 1, x, D, part.as<double>(), vb, stream);
-    SED_TRY_CUDA(cudaMemcpyAsync(hp.data(), part.ptr, (size_t)vb * kDotCols * 8, cudaMemcpyDeviceToHost, stream));
+  auto norm = [&](S* x, double& nrm) -> int {  // ||x||: the dot of x as a one-column basis
+    if (int st = launch_tproj<S>(x, D, 1, x, D, nullptr, 0, part.as<double>(), done, coef.as<double>(), nullptr, vb, stream))
+      return st;
+    SED_TRY_CUDA(cudaMemcpyAsync(&nrm, coef.ptr, 8, cudaMemcpyDeviceToHost, stream));
     SED_TRY_CUDA(cudaStreamSynchronize(stream));
-    double s = 0.0;
-    for (unsigned b = 0; b < vb; ++b) s += hp[(size_t)b * kDotCols];
-    nrm = std::sqrt(s);
+    nrm = std::sqrt(nrm);
     return LS_SUCCESS;
   };
   // v_0
@@ -401,56 +620,69 @@ int thick_run(OperatorData& op, cudaStream_t stream, uint32_t m, uint32_t nev, d
   auto Tij = [&](uint32_t i, uint32_t j) -> double& { return T[(size_t)i * (m + 1) + j]; };
   uint32_t k = 0;      // index of the newest basis vector
   uint32_t arrow = 0;  // index of the continuation vector after the last restart (0: none)
-  std::vector<double> c, c2, theta, Z;
+  std::vector<double> c, theta, Z;
   out = ThickResult{};
-  while (true) {
-    // ---- one Lanczos step from v_k
+  // One Lanczos step from v_k, enqueued. Orthogonalisation in two passes.
+  // Away from the continuation vector of a restart, H v_k has (in exact
+  // arithmetic) components along v_{k-1} and v_k only, so the first pass
+  // projects out those two; the second pass runs against the whole basis and
+  // removes what rounding left along any stored vector. On the step from the
+  // continuation vector (whose column of the projected matrix is an arrowhead
+  // over the kept Ritz vectors) both passes are full.
+  auto enqueue_step = [&](uint32_t k) -> int {
+    S* const v = V + (uint64_t)k * D;
+    int st;
     if constexpr (std::is_same<S, float>::value) {
-      if (op.stream.ready && op.stream.diag_f.ptr) {
-        if (int st = operator_apply32(op, V + (uint64_t)k * D, w, stream)) return st;
-      } else if (int st = operator_apply_device(op, dtype, 1, V + (uint64_t)k * D, D, w, D, stream, SED_FORM_AUTO)) {
-        return st;
-      }
-    } else if (int st = operator_apply_device(op, dtype, 1, V + (uint64_t)k * D, D, w, D, stream, SED_FORM_AUTO)) {
-      return st;
-    }
-    ++out.matvecs;
-    ++out.steps;
-    // Orthogonalisation, two passes. Away from the continuation vector of a
-    // restart, H v_k has (in exact arithmetic) components along v_{k-1} and
-    // v_k only, so the first pass projects out those two; the second pass
-    // runs against the whole basis and removes what rounding left along any
-    // stored vector. On the step from the continuation vector (whose column
-    // of the projected matrix is an arrowhead over the kept Ritz vectors)
-    // both passes are full.
-    uint32_t const first = k > arrow ? k - 1 : 0;
-    if (int st = dots_at(first, k + 1 - first, w, c)) return st;
-    SED_TRY_CUDA(cudaMemcpyAsync(coef.ptr, c.data(), (k + 1 - first) * 8, cudaMemcpyHostToDevice, stream));
-    { k_tupdate<S><<<vb, 256, 0, stream>>>(V + (uint64_t)first * D, D, k + 1 - first, coef.as<double>(), w, D); note_launches(1); }
-    c.insert(c.begin(), first, 0.0);
-    if (int st = dots(k + 1, w, c2)) return st;
-    SED_TRY_CUDA(cudaMemcpyAsync(coef.ptr, c2.data(), (k + 1) * 8, cudaMemcpyHostToDevice, stream));
-    { k_tupdate<S><<<vb, 256, 0, stream>>>(V, D, k + 1, coef.as<double>(), w, D); note_launches(1); }
-    for (uint32_t i = 0; i <= k; ++i) {
-      double const v = c[i] + c2[i];
-      if (i == k) Tij(k, k) = v;
-      else Tij(i, k) = Tij(k, i) = v;
-    }
-    double beta = 0.0;
-    if (int st = norm(w, beta)) return st;
-    bool const breakdown = !(beta > 1e-14 * std::max(1.0, std::fabs(Tij(k, k))));
-    if (!breakdown) {
-      { k_tscale<S><<<vb, 256, 0, stream>>>(w, D, 1.0 / beta, V + (uint64_t)(k + 1) * D); note_launches(1); }
-      Tij(k + 1, k) = Tij(k, k + 1) = beta;
+      st = op.stream.ready && op.stream.diag_f.ptr ? operator_apply32(op, v, w, stream, copied)
+                                                   : operator_apply_device(op, dtype, 1, v, D, w, D, stream, SED_FORM_AUTO);
     } else {
-      beta = 0.0;
+      st = copied ? operator_apply_prescaled(op, v, w, stream)
+                  : operator_apply_device(op, dtype, 1, v, D, w, D, stream, SED_FORM_AUTO);
     }
-    uint32_t const n = k + 1;  // order of the projected problem
+    if (st) return st;
+    uint32_t const first = k > arrow ? k - 1 : 0, npre = k + 1 - first;
+    double *c1 = slot(k), *c2 = c1 + kMaxThick + 1, *beta = c2 + kMaxThick + 1, *pt = part.as<double>();
+    if ((st = launch_tproj<S>(V + (uint64_t)first * D, D, npre, w, D, nullptr, 0, pt, done, c1, wmax, vb, stream))) return st;
+    bool const fused = npre <= 2 && k + 1 <= kProjCols;
+    if (!fused) {
+      { k_tupdate<S><<<vb, 256, 0, stream>>>(V + (uint64_t)first * D, D, npre, c1, w, D, pt, done, nullptr, nullptr); note_launches(1); }
+    }
+    if ((st = launch_tproj<S>(V, D, k + 1, w, D, c1, fused ? npre : 0, pt, done, c2, nullptr, vb, stream))) return st;
+    { k_tupdate<S><<<vb, 256, 0, stream>>>(V, D, k + 1, c2, w, D, pt, done, beta, wmax); note_launches(1); }
+    { k_tscale_next<S><<<grid_size(D, dev, 8), 256, 0, stream>>>(w, D, beta, c1 + (k - first), c2 + k, wmax, V + (uint64_t)(k + 1) * D, next); note_launches(1); }
+    SED_TRY_CUDA(cudaGetLastError());
+    copied = next.on;
+    return LS_SUCCESS;
+  };
+  while (true) {
+    // ---- steps up to the next look at T, without the host
+    uint32_t const k0 = k;
+    do {
+      if (int st = enqueue_step(k)) return st;
+      ++k;
+    } while (k < m && k % 4 != 0 && out.steps + (k - k0) < max_steps);
+    SED_TRY_CUDA(cudaMemcpyAsync(hproj.data() + (size_t)k0 * kSlot, slot(k0), (size_t)(k - k0) * kSlot * 8,
+                                 cudaMemcpyDeviceToHost, stream));
+    SED_TRY_CUDA(cudaStreamSynchronize(stream));
+    double beta = 0.0;
+    bool breakdown = false;
+    uint32_t n = k0;  // order of the projected problem
+    while (n < k && !breakdown) {
+      double const *c1 = hproj.data() + (size_t)n * kSlot, *c2 = c1 + kMaxThick + 1;
+      uint32_t const first = n > arrow ? n - 1 : 0;
+      for (uint32_t i = 0; i <= n; ++i) {
+        double const v = (i >= first ? c1[i - first] : 0.0) + c2[i];
+        Tij(i, n) = Tij(n, i) = v;
+      }
+      beta = c2[kMaxThick + 1];
+      breakdown = thick_breakdown(beta, Tij(n, n));
+      if (breakdown) beta = 0.0;
+      else Tij(n + 1, n) = Tij(n, n + 1) = beta;
+      ++n;
+      ++out.steps;
+      ++out.matvecs;
+    }
     bool const full = n >= m || breakdown || out.steps >= max_steps;
-    if (!full && n % 4 != 0) {
-      k = n;
-      continue;
-    }
     // ---- Rayleigh-Ritz on T[0..n)
     std::vector<double> A((size_t)n * n);
     for (uint32_t i = 0; i < n; ++i)
@@ -475,14 +707,15 @@ int thick_run(OperatorData& op, cudaStream_t stream, uint32_t m, uint32_t nev, d
         double* pi = psi + (uint64_t)i * D;
         { k_tritz<S><<<vb, 256, 0, stream>>>(V, D, n, coef.as<double>(), D, pi); note_launches(1); }
         if (int st = operator_apply_device(op, 1, 1, pi, D, w64.ptr, D, stream, SED_FORM_AUTO)) return st;
+        if (std::is_same<S, double>::value) copied = false;  // it used the workspace
         ++out.matvecs;
         { k_tresid<<<vb, 256, 0, stream>>>(pi, w64.as<double>(), theta[i], D, part.as<double>()); note_launches(1); }
-        SED_TRY_CUDA(cudaMemcpyAsync(hp.data(), part.ptr, 2 * (size_t)vb * 8, cudaMemcpyDeviceToHost, stream));
+        SED_TRY_CUDA(cudaMemcpyAsync(hres.data(), part.ptr, 2 * (size_t)vb * 8, cudaMemcpyDeviceToHost, stream));
         SED_TRY_CUDA(cudaStreamSynchronize(stream));
         double rr = 0.0, pp = 0.0;
         for (unsigned b = 0; b < vb; ++b) {
-          rr += hp[2 * b];
-          pp += hp[2 * b + 1];
+          rr += hres[2 * b];
+          pp += hres[2 * b + 1];
         }
         out.theta[i] = theta[i];
         out.resid[i] = std::sqrt(rr / pp);
@@ -500,15 +733,15 @@ int thick_run(OperatorData& op, cudaStream_t stream, uint32_t m, uint32_t nev, d
       for (uint32_t q = 0; q < n; ++q)
         for (uint32_t cidx = 0; cidx < keep; ++cidx) Y[(size_t)q * keep + cidx] = Z[(size_t)q * n + cidx];
       SED_TRY_CUDA(cudaMemcpyAsync(Yb.ptr, Y.data(), Y.size() * 8, cudaMemcpyHostToDevice, stream));
-      if (int st = rotate_basis<S>(V, D, n, Yb.as<double>(), keep, D, vb, stream, g_rotate_path, rt_err.as<int>()))
+      if (int st = rotate_basis<S>(V, D, n, Yb.as<double>(), keep, D, vb, stream, g_rotate_path, rt_err))
         return st;
       if (breakdown) {
         // no continuation vector: a fresh random direction, orthogonalised
+        copied = false;
         { k_trandom<S><<<vb, 256, 0, stream>>>(V + (uint64_t)keep * D, D, seed + 7919 * (out.restarts + 1)); note_launches(1); }
         for (int pass = 0; pass < 2; ++pass) {
           if (int st = dots(keep, V + (uint64_t)keep * D, c)) return st;
-          SED_TRY_CUDA(cudaMemcpyAsync(coef.ptr, c.data(), keep * 8, cudaMemcpyHostToDevice, stream));
-          { k_tupdate<S><<<vb, 256, 0, stream>>>(V, D, keep, coef.as<double>(), V + (uint64_t)keep * D, D); note_launches(1); }
+          { k_tupdate<S><<<vb, 256, 0, stream>>>(V, D, keep, coef.as<double>(), V + (uint64_t)keep * D, D, part.as<double>(), done, nullptr, nullptr); note_launches(1); }
         }
         double nn = 0.0;
         if (int st = norm(V + (uint64_t)keep * D, nn)) return st;
@@ -524,7 +757,6 @@ int thick_run(OperatorData& op, cudaStream_t stream, uint32_t m, uint32_t nev, d
       ++out.restarts;
       continue;
     }
-    k = n;
   }
 }
 
