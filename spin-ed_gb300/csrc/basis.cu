@@ -311,6 +311,14 @@ int basis_upload_plan(BasisData& b, cudaStream_t stream) {
     q.off = total;
     total += align(q.bytes);
   }
+  std::vector<uint64_t> binom(65 * 65, 0);
+  for (unsigned i = 0; i <= 64; ++i) {
+    binom[i * 65] = 1;
+    for (unsigned j = 1; j <= 64; ++j)
+      binom[i * 65 + j] = i == 0 ? 0 : binom[(i - 1) * 65 + j - 1] + binom[(i - 1) * 65 + j];
+  }
+  parts.push_back({binom.data(), binom.size() * 8, total});
+  total += align(binom.size() * 8);
   std::vector<uint8_t> host(total, 0);
   for (auto const& q : parts)
     if (q.bytes) std::memcpy(host.data() + q.off, q.src, q.bytes);
@@ -336,14 +344,7 @@ int basis_upload_plan(BasisData& b, cudaStream_t stream) {
   v.line_row = (uint16_t const*)(base + parts[15].off);
   v.line_col = (uint16_t const*)(base + parts[16].off);
   b.plan_dev = v;
-  std::vector<uint64_t> binom(65 * 65, 0);
-  for (unsigned i = 0; i <= 64; ++i) {
-    binom[i * 65] = 1;
-    for (unsigned j = 1; j <= 64; ++j)
-      binom[i * 65 + j] = i == 0 ? 0 : binom[(i - 1) * 65 + j - 1] + binom[(i - 1) * 65 + j];
-  }
-  if (int st = b.binom.allocate(binom.size() * 8)) return st;
-  SED_TRY_CUDA(cudaMemcpyAsync(b.binom.ptr, binom.data(), binom.size() * 8, cudaMemcpyHostToDevice, stream));
+  b.binom = DevicePart{base + parts.back().off, parts.back().bytes};
   SED_TRY_CUDA(cudaStreamSynchronize(stream));
   return LS_SUCCESS;
 }
@@ -444,9 +445,8 @@ int build_impl(BasisData& b, uint64_t const* given, uint64_t given_size) {
     }
     uint64_t const n_words = (space + 31) / 32;
     uint64_t const n_tiles = (n_words + kTileWords - 1) / kTileWords;
-    DeviceBuffer bitmap, tiles, segs;
-    if (int st = bitmap.allocate(std::max<uint64_t>(1, n_words) * 4)) return st;
-    if (int st = tiles.allocate((n_tiles + 1) * 8)) return st;
+    DeviceBuffer scratch;
+    DevicePart bitmap, tiles, segs;
     // Top-row segments (tori): the rank range of the words with top row T is
     // [lo_T, lo_T + cnt_T) in increasing T; keep the T whose value is its own
     // smallest rotation and no larger than its inverse's smallest rotation.
@@ -478,8 +478,14 @@ int build_impl(BasisData& b, uint64_t const* given, uint64_t given_size) {
       }
     }
     uint32_t const n_seg = (uint32_t)seg_b.size();
+    {
+      DeviceParts parts;
+      parts.add(bitmap, std::max<uint64_t>(1, n_words) * 4);
+      parts.add(tiles, (n_tiles + 1) * 8);
+      parts.add(segs, (2 * (size_t)n_seg + 1) * 8);
+      if (int st = parts.allocate(scratch)) return st;
+    }
     if (n_seg) {
-      if (int st = segs.allocate((2 * (size_t)n_seg + 1) * 8)) return st;
       SED_TRY_CUDA(cudaMemcpyAsync(segs.ptr, seg_b.data(), n_seg * 8, cudaMemcpyHostToDevice, stream));
       SED_TRY_CUDA(cudaMemcpyAsync(segs.as<uint64_t>() + n_seg, seg_p.data(), (n_seg + 1) * 8, cudaMemcpyHostToDevice,
                                    stream));

@@ -4,6 +4,7 @@
 // turned into text by ls_error_to_string and freed by ls_destroy_string. The
 // text carries the description of the code plus the detail recorded by the
 // failing call on the same host thread.
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdlib>
@@ -116,6 +117,50 @@ void krylov_give(DeviceBuffer& b) {
 }
 
 namespace {
+constexpr size_t kPinnedKept = 4, kPinnedLargest = 256 * 1024;
+std::mutex g_pinned_mu;
+PinnedBuffer g_pinned[kPinnedKept];
+
+void release_pinned() {
+  std::lock_guard<std::mutex> lk(g_pinned_mu);
+  for (PinnedBuffer& b : g_pinned) {
+    if (b.ptr) cudaFreeHost(b.ptr);
+    b = PinnedBuffer{};
+  }
+}
+}  // namespace
+
+int pinned_take(size_t bytes, PinnedBuffer& out) {
+  {
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    for (PinnedBuffer& b : g_pinned)
+      if (b.ptr && b.bytes >= bytes) {
+        out = b;
+        b = PinnedBuffer{};
+        return LS_SUCCESS;
+      }
+  }
+  size_t const n = std::max<size_t>(bytes, 64 * 1024);
+  SED_TRY_CUDA(cudaHostAlloc(&out.ptr, n, cudaHostAllocPortable));
+  out.bytes = n;
+  return LS_SUCCESS;
+}
+
+void pinned_give(PinnedBuffer& b) {
+  if (!b.ptr) return;
+  if (b.bytes <= kPinnedLargest) {
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    for (PinnedBuffer& k : g_pinned)
+      if (!k.ptr) {
+        std::swap(k, b);
+        return;
+      }
+  }
+  cudaFreeHost(b.ptr);
+  b = PinnedBuffer{};
+}
+
+namespace {
 // Device bytes held by libsed buffers (all devices) and the caller's cap on
 // them (sed_set_device_memory_limit; 0 = none).
 std::atomic<uint64_t> g_dev_bytes{0};
@@ -206,7 +251,10 @@ using namespace sed;
 
 extern "C" {
 
-void sed_release_workspace(void) { release_cache(-1); }
+void sed_release_workspace(void) {
+  release_cache(-1);
+  release_pinned();
+}
 void sed_set_device_memory_limit(uint64_t bytes) { g_dev_limit.store(bytes); }
 void sed_set_device_wait_limit(double seconds) {
   g_wait_ns.store(seconds > 0 ? (uint64_t)(seconds * 1e9) : 0);

@@ -479,10 +479,11 @@ class Cycle {
   Cycle(Cycle const&) = delete;
   Cycle& operator=(Cycle const&) = delete;
   ~Cycle() {
+    if (stream_) cudaStreamSynchronize(stream_);  // a replay and its copy may be in flight
     if (graph) cudaGraphExecDestroy(graph);
     for (cudaEvent_t e : ready_)
       if (e) cudaEventDestroy(e);
-    if (host_) cudaFreeHost(host_);
+    pinned_give(pinned_);
   }
 
   double* alpha() const { return reinterpret_cast<double*>(hdr + 1); }
@@ -492,7 +493,8 @@ class Cycle {
     hdr = device_state;
     m = m_max;
     check = check_every;
-    SED_TRY_CUDA(cudaMallocHost(&host_, 2 * state_bytes(m)));
+    if (int st = pinned_take(2 * state_bytes(m), pinned_)) return st;
+    host_ = static_cast<char*>(pinned_.ptr);
     for (cudaEvent_t& e : ready_) SED_TRY_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     return LS_SUCCESS;
   }
@@ -500,6 +502,7 @@ class Cycle {
   // Captures `check` steps on `stream`.
   template <class Step>
   int capture(cudaStream_t stream, Step&& step) {
+    stream_ = stream;
     cudaGraph_t g;
     SED_TRY_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     set_capturing(true);
@@ -526,6 +529,7 @@ class Cycle {
     h.k = k0;
     h.m_max = m;
     h.size = k0;
+    stream_ = stream;
     std::memcpy(host_, &h, sizeof(h));
     SED_TRY_CUDA(cudaMemcpyAsync(hdr, host_, sizeof(h), cudaMemcpyHostToDevice, stream));
     SED_TRY_CUDA(cudaStreamSynchronize(stream));
@@ -573,7 +577,9 @@ class Cycle {
   }
 
  private:
+  PinnedBuffer pinned_;
   char* host_ = nullptr;  // two copies of the state, pinned
+  cudaStream_t stream_ = nullptr;
   cudaEvent_t ready_[2] = {nullptr, nullptr};
   size_t nodes_ = 0;
   char* slot(uint64_t i) const { return host_ + (i & 1) * state_bytes(m); }
@@ -582,13 +588,14 @@ class Cycle {
 // ------------------------------------------------------------- driver ----
 
 struct Workspace {
-  DeviceBuffer V, state, s, partial, done, cgs_partial, coef, ritz, y, scratch;
+  DeviceBuffer V, buf, scratch;
+  DevicePart state, s, partial, done, cgs_partial, coef, ritz, y;  // in buf
 };
 
 int elem_bytes(int dtype) { return dtype == 0 ? 4 : dtype == 1 ? 8 : dtype == 2 ? 8 : 16; }
 
 template <class X>
-double host_sum(DeviceBuffer const& partial, unsigned n, unsigned stride, unsigned off, cudaStream_t s,
+double host_sum(DevicePart const& partial, unsigned n, unsigned stride, unsigned off, cudaStream_t s,
                 int* st) {
   std::vector<double> h((size_t)n * stride);
   cudaError_t e = cudaMemcpyAsync(h.data(), partial.ptr, h.size() * 8, cudaMemcpyDeviceToHost, s);
@@ -630,17 +637,19 @@ struct Solver {
     int dev = op.basis->device;
     vblocks = grid_size(D, dev, 8);
     if (int st = krylov_take((size_t)m_max * D * sizeof(X), ws.V)) return st;
-    if (int st = ws.state.allocate(state_bytes(m_max))) return st;
-    if (int st = ws.s.allocate((size_t)m_max * 8)) return st;
     uint64_t const nb = std::max<uint64_t>((D + kBlock - 1) / kBlock, vblocks) + 32;
-    if (int st = ws.partial.allocate(nb * 16)) return st;
-    if (int st = ws.done.allocate(16)) return st;
+    DeviceParts parts;
+    parts.add(ws.state, state_bytes(m_max));
+    parts.add(ws.s, (size_t)m_max * 8);
+    parts.add(ws.partial, nb * 16);
+    parts.add(ws.done, 16);
     if (reorth) {
-      if (int st = ws.cgs_partial.allocate((size_t)m_max * vblocks * 8)) return st;
-      if (int st = ws.coef.allocate((size_t)m_max * 8)) return st;
+      parts.add(ws.cgs_partial, (size_t)m_max * vblocks * 8);
+      parts.add(ws.coef, (size_t)m_max * 8);
     }
-    if (int st = ws.ritz.allocate(D * sizeof(X))) return st;
-    if (int st = ws.y.allocate(D * sizeof(X))) return st;
+    parts.add(ws.ritz, D * sizeof(X));
+    parts.add(ws.y, D * sizeof(X));
+    if (int st = parts.allocate(ws.buf)) return st;
     if (int st = cycle.init(ws.state.as<LzHeader>(), m_max, check)) return st;
     SED_TRY_CUDA(cudaMemsetAsync(ws.state.ptr, 0, state_bytes(m_max), stream));
     SED_TRY_CUDA(cudaMemsetAsync(ws.done.ptr, 0, 16, stream));
@@ -982,9 +991,8 @@ int solve_mixed(OperatorData& op, int out_dtype, sed_eigh_options const& o, doub
   uint32_t const m = std::max<uint32_t>(3, auto_basis(D, 4, 1, o.max_basis ? o.max_basis : 300));
   uint32_t const check = m < 64 ? 1u : 4u;
   unsigned const vb = grid_size(D, op.basis->device, 8);
-  DeviceBuffer psi, y, V, state, sbuf, partial, done_b;
-  if (int st = psi.allocate(D * 8)) return st;
-  if (int st = y.allocate(D * 8)) return st;
+  DeviceBuffer buf, V;
+  DevicePart psi, y, state, sbuf, partial, done_b;
   struct KrylovGuard {
     DeviceBuffer& b;
     cudaStream_t s;
@@ -994,11 +1002,15 @@ int solve_mixed(OperatorData& op, int out_dtype, sed_eigh_options const& o, doub
     }
   } krylov_guard{V, stream};
   if (int st = krylov_take((size_t)m * D * 4, V)) return st;
-  if (int st = state.allocate(state_bytes(m))) return st;
-  if (int st = sbuf.allocate((size_t)m * 8)) return st;
   uint64_t const nb = std::max<uint64_t>((D + kBlock - 1) / kBlock, vb) + 32;
-  if (int st = partial.allocate(nb * 16)) return st;
-  if (int st = done_b.allocate(16)) return st;
+  DeviceParts parts;
+  parts.add(psi, D * 8);
+  parts.add(y, D * 8);
+  parts.add(state, state_bytes(m));
+  parts.add(sbuf, (size_t)m * 8);
+  parts.add(partial, nb * 16);
+  parts.add(done_b, 16);
+  if (int st = parts.allocate(buf)) return st;
   SED_TRY_CUDA(cudaMemsetAsync(done_b.ptr, 0, 16, stream));
   Cycle cycle;
   if (int st = cycle.init(state.as<LzHeader>(), m, check)) return st;

@@ -850,38 +850,37 @@ int build_tables(OperatorData& op) {
       }
   std::vector<double> inv(n_div);
   for (uint32_t d = 0; d < n_div; ++d) inv[d] = 1.0 / std::sqrt((double)div[d]);
-  if (int st = t->divisors.allocate(n_div * 4)) return st;
-  if (int st = t->inv_sqrt_s.allocate(n_div * 8)) return st;
-  SED_TRY_CUDA(cudaMemcpy(t->divisors.ptr, div.data(), n_div * 4, cudaMemcpyHostToDevice));
-  SED_TRY_CUDA(cudaMemcpy(t->inv_sqrt_s.ptr, inv.data(), n_div * 8, cudaMemcpyHostToDevice));
-  if (int st = t->table_c.allocate(n_codes * 16)) return st;
-  SED_TRY_CUDA(cudaMemcpy(t->table_c.ptr, tc.data(), n_codes * 16, cudaMemcpyHostToDevice));
+  DeviceParts parts;  // one allocation and one copy for all tables
+  std::vector<std::pair<DevicePart*, void const*>> from;
+  auto put = [&](DevicePart& part, void const* src, size_t bytes) {
+    parts.add(part, bytes);
+    from.push_back({&part, src});
+  };
+  put(t->divisors, div.data(), n_div * 4);
+  put(t->inv_sqrt_s, inv.data(), n_div * 8);
+  put(t->table_c, tc.data(), n_codes * 16);
   if (op.is_real) {
     tr.resize(n_codes);
     for (uint64_t c = 0; c < n_codes; ++c) tr[c] = tc[2 * c];
-    if (int st = t->table.allocate(n_codes * 8)) return st;
-    SED_TRY_CUDA(cudaMemcpy(t->table.ptr, tr.data(), n_codes * 8, cudaMemcpyHostToDevice));
+    put(t->table, tr.data(), n_codes * 8);
   }
-  t->code.divisors = t->divisors.as<uint32_t>();
   t->code.n_div = n_div;
   t->code.n_ph = n_ph;
   t->code.real_phase = real_phase ? 1u : 0u;
   t->n_codes = (uint32_t)n_codes;
   // fixed-point form: real values and characters, few distinct values
+  std::vector<uint8_t> fc;
+  std::vector<double> sq;
   if (op.is_real && real_phase && n_val <= kFixMaxValues && n_div <= kFixMaxClasses && n_codes <= 16384 &&
       op.row_bound < (1ull << 40)) {
-    std::vector<uint8_t> fc(n_codes);
+    fc.resize(n_codes);
     for (uint32_t v = 0; v < std::max(1u, n_val); ++v)
       for (uint32_t p = 0; p < n_ph; ++p)
         for (uint32_t d = 0; d < n_div; ++d) fc[((uint64_t)v * n_ph + p) * n_div + d] = (uint8_t)(v << 1 | p);
-    std::vector<double> sq(n_div);
+    sq.resize(n_div);
     for (uint32_t d = 0; d < n_div; ++d) sq[d] = std::sqrt((double)div[d]);
-    if (int st = t->fix_code.allocate(n_codes)) return st;
-    if (int st = t->fix_sqrt_s.allocate(n_div * 8)) return st;
-    SED_TRY_CUDA(cudaMemcpy(t->fix_code.ptr, fc.data(), n_codes, cudaMemcpyHostToDevice));
-    SED_TRY_CUDA(cudaMemcpy(t->fix_sqrt_s.ptr, sq.data(), n_div * 8, cudaMemcpyHostToDevice));
-    t->fix.code = t->fix_code.as<uint8_t>();
-    t->fix.sqrt_s = t->fix_sqrt_s.as<double>();
+    put(t->fix_code, fc.data(), n_codes);
+    put(t->fix_sqrt_s, sq.data(), n_div * 8);
     t->fix.n_codes = (uint32_t)n_codes;
     t->fix.n_div = n_div;
     // (row count) x sqrt(S_max), rounded up by a margin far above the
@@ -895,6 +894,14 @@ int build_tables(OperatorData& op) {
     t->fix_nv = n_val <= 1 ? 1u : (n_val <= 2 ? 2u : 4u);
     t->fix_ok = true;
   }
+  if (int st = parts.allocate(t->buf)) return st;
+  std::vector<char> host(t->buf.bytes, 0);
+  for (auto const& f : from)
+    std::memcpy(host.data() + (f.first->as<char>() - t->buf.as<char>()), f.second, f.first->bytes);
+  SED_TRY_CUDA(cudaMemcpy(t->buf.ptr, host.data(), host.size(), cudaMemcpyHostToDevice));
+  t->code.divisors = t->divisors.as<uint32_t>();
+  t->fix.code = t->fix_code.as<uint8_t>();
+  t->fix.sqrt_s = t->fix_sqrt_s.as<double>();
   op.tables = std::move(t);
   return LS_SUCCESS;
 }
@@ -1084,10 +1091,15 @@ int operator_record_stream(OperatorData& op, cudaStream_t stream) {
   bool const packed = col_bits + code_bits <= 31;  // kNull stays unrepresentable
   StreamForm& sf = op.stream;
   sf = StreamForm{};
-  DeviceBuffer elements, maxw;
   if (int st = sf.slice_ptr.allocate((n_slices + 1) * 8)) return st;
-  if (int st = elements.allocate((n_slices + 1) * 8)) return st;
-  if (int st = maxw.allocate(16)) return st;
+  DeviceBuffer scratch;
+  DevicePart elements, maxw;
+  {
+    DeviceParts parts;
+    parts.add(elements, (n_slices + 1) * 8);
+    parts.add(maxw, 16);
+    if (int st = parts.allocate(scratch)) return st;
+  }
   SED_TRY_CUDA(cudaMemsetAsync(maxw.ptr, 0, 4, stream));
   unsigned const grid = (unsigned)((n_slices * 32 + kBlock - 1) / kBlock);
   if (n_slices) {
@@ -1152,46 +1164,44 @@ int operator_record_stream(OperatorData& op, cudaStream_t stream) {
       DeviceBuffer& b;
       ~TableGuard() { krylov_give(b); }
     } table_guard{table};
-    DeviceBuffer err;
-    if (int st = err.allocate(16)) return st;
+    // chunked rank table (6-bit chunks) when it fits in 96 KB of shared memory
+    uint32_t const n_chunks = b.hw >= 0 ? (b.n + 5) / 6 : 0, wp1 = b.hw >= 0 ? (uint32_t)b.hw + 1 : 0;
+    uint32_t const rank_words = n_chunks * wp1 * 64 * 8 <= 96 * 1024 ? n_chunks * wp1 * 64 : 0;
+    DeviceBuffer lookup;
+    DevicePart err, seg_buf, rank_buf;
+    {
+      DeviceParts parts;
+      parts.add(err, 16);
+      parts.add(seg_buf, seg_off.size() * 8);
+      parts.add(rank_buf, (size_t)rank_words * 8);
+      if (int st = parts.allocate(lookup)) return st;
+    }
     if (int st = krylov_take(space * 4, table)) return st;
-    DeviceBuffer seg_buf;
     RowIndex RI{nullptr, 0, 0};
     if (!seg_off.empty()) {
-      if (int st = seg_buf.allocate(seg_off.size() * 8)) return st;
       SED_TRY_CUDA(cudaMemcpyAsync(seg_buf.ptr, seg_off.data(), seg_off.size() * 8, cudaMemcpyHostToDevice, stream));
       unsigned const L = b.n - b.plan.row_bits;
       RI = RowIndex{seg_buf.as<uint64_t>(), ((uint64_t)1 << L) - 1, L};
     }
     SED_TRY_CUDA(cudaMemsetAsync(table.ptr, 0xFF, space * 4, stream));
     SED_TRY_CUDA(cudaMemsetAsync(err.ptr, 0, 16, stream));
-    // chunked rank table (6-bit chunks) when it fits in 96 KB of shared memory
-    uint32_t n_chunks = 0, wp1 = 0, rank_words = 0;
-    DeviceBuffer rank_buf;
-    if (b.hw >= 0) {
-      n_chunks = (b.n + 5) / 6;
-      wp1 = (uint32_t)b.hw + 1;
-      uint64_t const words = (uint64_t)n_chunks * wp1 * 64;
-      if (words * 8 <= 96 * 1024) {
-        std::vector<uint64_t> R(words, 0);
-        for (uint32_t c = 0; c < n_chunks; ++c)
-          for (uint32_t m = 0; m < wp1; ++m)
-            for (uint32_t v = 0; v < 64; ++v) {
-              uint64_t acc = 0;
-              uint32_t i = 0;
-              for (uint32_t q = 0; q < 6; ++q)
-                if ((v >> q) & 1u) {
-                  ++i;
-                  uint32_t const p = 6 * c + q;
-                  if (p < 64) acc += host_binom(p, m + i);
-                }
-              R[((size_t)c * wp1 + m) * 64 + v] = acc;
-            }
-        if (int st = rank_buf.allocate(words * 8)) return st;
-        SED_TRY_CUDA(cudaMemcpyAsync(rank_buf.ptr, R.data(), words * 8, cudaMemcpyHostToDevice, stream));
-        SED_TRY_CUDA(cudaStreamSynchronize(stream));
-        rank_words = (uint32_t)words;
-      }
+    if (rank_words) {
+      std::vector<uint64_t> R(rank_words, 0);
+      for (uint32_t c = 0; c < n_chunks; ++c)
+        for (uint32_t m = 0; m < wp1; ++m)
+          for (uint32_t v = 0; v < 64; ++v) {
+            uint64_t acc = 0;
+            uint32_t i = 0;
+            for (uint32_t q = 0; q < 6; ++q)
+              if ((v >> q) & 1u) {
+                ++i;
+                uint32_t const p = 6 * c + q;
+                if (p < 64) acc += host_binom(p, m + i);
+              }
+            R[((size_t)c * wp1 + m) * 64 + v] = acc;
+          }
+      SED_TRY_CUDA(cudaMemcpyAsync(rank_buf.ptr, R.data(), R.size() * 8, cudaMemcpyHostToDevice, stream));
+      SED_TRY_CUDA(cudaStreamSynchronize(stream));
     }
     size_t const dsmem = rank_words ? (size_t)rank_words * 8 : (size_t)64 * 33 * 8;
     bool const wide = b.plan.n_bits > 32;

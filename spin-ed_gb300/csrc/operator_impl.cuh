@@ -335,17 +335,18 @@ __device__ __forceinline__ void fix_row_sums(StreamView const& S, FixView const&
 }
 
 struct OperatorTables {
-  DeviceBuffer divisors;
-  DeviceBuffer table;    // double[n_codes], real operators only
-  DeviceBuffer table_c;  // double2[n_codes], every operator
-  DeviceBuffer inv_sqrt_s;
+  DeviceBuffer buf;      // holds all of them
+  DevicePart divisors;
+  DevicePart table;    // double[n_codes], real operators only
+  DevicePart table_c;  // double2[n_codes], every operator
+  DevicePart inv_sqrt_s;
   CodeView code{};
   uint32_t n_codes = 0;
   // fixed-point form (fix_ok: the operator qualifies)
   bool fix_ok = false;
   uint32_t fix_nv = 1;   // accumulators per row: 1, 2 or 4
-  DeviceBuffer fix_code;
-  DeviceBuffer fix_sqrt_s;
+  DevicePart fix_code;
+  DevicePart fix_sqrt_s;
   FixView fix{};
 };
 

@@ -66,6 +66,49 @@ struct DeviceBuffer {
   }
 };
 
+// Part of a DeviceBuffer.
+struct DevicePart {
+  void* ptr = nullptr;
+  size_t bytes = 0;
+  template <class T>
+  T* as() const {
+    return static_cast<T*>(ptr);
+  }
+};
+
+// Several small buffers in one allocation (cudaMalloc and cudaFree take some
+// 7 us each): add() the parts, then allocate() sets their pointers, 256-byte
+// aligned.
+class DeviceParts {
+ public:
+  void add(DevicePart& part, size_t bytes) {
+    part.bytes = bytes;
+    parts_.push_back({&part, total_});
+    total_ += (bytes + 255) & ~(size_t)255;
+  }
+  int allocate(DeviceBuffer& buf) {
+    if (int st = buf.allocate(total_)) return st;
+    for (auto const& p : parts_) p.first->ptr = buf.as<char>() + p.second;
+    return 0;
+  }
+
+ private:
+  std::vector<std::pair<DevicePart*, size_t>> parts_;
+  size_t total_ = 0;
+};
+
+// A pinned host buffer of at least `bytes` (portable across devices). Up to
+// four of up to 256 KB are kept between calls, for all threads, until
+// sed_release_workspace: allocating and freeing one takes 350 us, an eighth
+// of a solve of a 24-site ring from nothing. The caller gives a buffer back
+// only when no copy to or from it is in flight.
+struct PinnedBuffer {
+  void* ptr = nullptr;
+  size_t bytes = 0;
+};
+int pinned_take(size_t bytes, PinnedBuffer& out);
+void pinned_give(PinnedBuffer& b);
+
 // A device buffer of at least `bytes` for a Krylov basis on the current
 // device: the cached one when it is big enough, else a new allocation.
 int krylov_take(size_t bytes, DeviceBuffer& out);
@@ -150,7 +193,7 @@ struct BasisData {
   // device copy of the plan arrays (one allocation) and the view onto it
   DeviceBuffer plan_buf;
   PlanView plan_dev{};
-  DeviceBuffer binom;  // [65][65] uint64
+  DevicePart binom;  // [65][65] uint64, in plan_buf
   // built state
   bool built = false;
   uint64_t D = 0;

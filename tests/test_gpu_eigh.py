@@ -156,3 +156,33 @@ def test_ring_energies_over_the_reduction_grids(sed, n):
     res = sed.eigh(b.hamiltonian, seed=n)
     assert res.residuals[0] <= RES_TOL
     assert res.eigenvalues[0] == pytest.approx(heisenberg_ring_e0(n), rel=EV_RTOL)
+
+
+def test_solves_in_threads(sed):
+    """Solves of different operators at once, on their own streams, while the
+    kept workspaces are released under them: what one after the other gives,
+    bit for bit (each sums in a fixed order)."""
+    import threading
+    from spined import _lib as L
+    from spined.model import build_model
+    sizes = [12, 14, 16, 18, 20, 22]
+    built = [build_model(lattices.heisenberg_chain(n, j2=0.1)) for n in sizes]
+    want = [sed.eigh(b.hamiltonian, nev=1 + i % 2, seed=7) for i, b in enumerate(built)]
+    got, go = {}, threading.Barrier(len(sizes) + 1)
+
+    def work(i):
+        go.wait()
+        got[i] = [sed.eigh(built[i].hamiltonian, nev=1 + i % 2, seed=7) for _ in range(4)]
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(sizes))]
+    for t in threads:
+        t.start()
+    go.wait()
+    for _ in range(8):
+        L.load().sed_release_workspace()
+    for t in threads:
+        t.join()
+    for i, w in enumerate(want):
+        for r in got[i]:
+            np.testing.assert_array_equal(r.eigenvalues, w.eigenvalues)
+            np.testing.assert_array_equal(r.eigenvectors, w.eigenvectors)
