@@ -158,6 +158,23 @@ def test_ring_energies_over_the_reduction_grids(sed, n):
     assert res.eigenvalues[0] == pytest.approx(heisenberg_ring_e0(n), rel=EV_RTOL)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("m", [15, 16, 17, 18, 31, 32])
+def test_thick_restart_over_the_projection_groups(sed, precision, m):
+    """Bases below, at and above the 16 columns that one projection pass takes
+    and at the largest, on a 24-site J1-J2 ring: the energies of the unrestarted solver, to both solvers' residual
+    bound (an error of at most r^2 / gap, far below EV_RTOL)."""
+    from spined import _lib as L
+    from spined.model import build_model
+    p = L.SED_PRECISION_FP64 if precision == "fp64" else L.SED_PRECISION_MIXED
+    b = build_model(lattices.heisenberg_chain(24, j2=0.2))
+    want = sed.eigh(b.hamiltonian, nev=2)
+    res = sed.eigh(b.hamiltonian, nev=2, max_basis=m, precision=p)
+    assert res.restarts > 0
+    np.testing.assert_allclose(res.eigenvalues, want.eigenvalues, rtol=EV_RTOL)
+    assert np.all(res.residuals <= RES_TOL)
+
+
 def test_solves_in_threads(sed):
     """Solves of different operators at once, on their own streams, while the
     kept workspaces are released under them: what one after the other gives,
