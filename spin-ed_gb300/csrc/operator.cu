@@ -190,18 +190,20 @@ __global__ void __launch_bounds__(kRecWarps * 32, kRecBlocks)
 
 // Streamed SpMV over SELL-32 slices. RealOp selects the real table/diagonal.
 // With an Indirect (Krylov) view, x = base + k ld and y = base + (k+1) ld
-// with k read from device memory, and sum_i Re(x_i* y_i) goes to ind.sum[k].
-template <class X, bool RealOp, bool Packed>
+// with k read from device memory, and sum_i Re(x_i* y_i) goes to ind.sum[k]
+// (an instantiation of its own: the finishing code cost plain calls 4 %).
+template <class X, bool RealOp, bool Packed, bool Krylov>
 __global__ void __launch_bounds__(kBlock) k_spmv(StreamView S, uint64_t D, X const* __restrict__ x,
                                                  X* __restrict__ y, Indirect ind) {
   using V = typename Store<X>::V;
   extern __shared__ unsigned char smem_raw[];
-  __shared__ double red[kBlock / 32];
-  if (ind.stop && *ind.stop) return;  // uniform across the grid
-  if (ind.k) {
-    uint64_t const k = *ind.k;
-    x += k * ind.ld;
-    y += (k + 1) * ind.ld;
+  if constexpr (Krylov) {
+    if (ind.stop && *ind.stop) return;  // uniform across the grid
+    if (ind.k) {
+      uint64_t const k = *ind.k;
+      x += k * ind.ld;
+      y += (k + 1) * ind.ld;
+    }
   }
   void const* table = stage_table<RealOp>(S, smem_raw);
   uint64_t const i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -214,12 +216,15 @@ __global__ void __launch_bounds__(kBlock) k_spmv(StreamView S, uint64_t D, X con
       V const xi = Store<X>::load(x, i);
       V const yi = row_value<V>(mulv(stream_diag<V, RealOp>(S, i), xi), f, acc);
       Store<X>::store(y, i, yi);
-      part = dot_re(xi, yi);
+      if constexpr (Krylov) part = dot_re(xi, yi);
     }
   }
-  if (ind.partial) {
-    double const tot = block_sum(part, red);
-    finish_apply(tot, ind);
+  if constexpr (Krylov) {
+    __shared__ double red[kBlock / 32];
+    if (ind.partial) {
+      double const tot = block_sum(part, red);
+      finish_apply(tot, ind);
+    }
   }
 }
 
@@ -894,6 +899,48 @@ int build_tables(OperatorData& op) {
     t->fix_nv = n_val <= 1 ? 1u : (n_val <= 2 ? 2u : 4u);
     t->fix_ok = true;
   }
+  // complex elements: factors within 2^10 of each other, so that the smallest
+  // keeps its digits in the common scale
+  std::vector<int32_t> cw;
+  if (!op.is_real && n_val && n_codes <= kCplxMaxCodes && op.row_bound <= kCplxMaxRow) {
+    double lo = HUGE_VAL, hi = 0.0;
+    for (uint32_t v = 0; v < n_val; ++v) {
+      double const a = std::hypot(op.off_values[2 * v], op.off_values[2 * v + 1]);
+      lo = std::min(lo, a);
+      hi = std::max(hi, a);
+    }
+    if (lo > std::ldexp(1.0, -200) && hi < std::ldexp(1.0, 200) && hi <= 1024.0 * lo) {
+      int e;
+      std::frexp(hi, &e);         // hi < 2^e
+      t->cplx.shift = e - 54;
+      cw.resize(4 * n_codes);
+      auto limbs = [&](double x, int32_t* out) {
+        int64_t const w = std::llrint(std::ldexp(x, -t->cplx.shift));
+        int32_t const low = (int32_t)(uint32_t)w;
+        out[0] = (int32_t)((w - low) >> 32);
+        out[1] = low;
+      };
+      for (uint32_t v = 0; v < n_val; ++v)
+        for (uint32_t p = 0; p < n_ph; ++p) {
+          double const cre = op.off_values[2 * v], cim = op.off_values[2 * v + 1];
+          double xr, xi;
+          root_of_unity(real_phase ? (p ? b.plan.L / 2 : 0) : p, b.plan.L, xr, xi);
+          for (uint32_t d = 0; d < n_div; ++d) {
+            uint64_t const code = ((uint64_t)v * n_ph + p) * n_div + d;
+            limbs(cre * xr - cim * xi, cw.data() + 4 * code);
+            limbs(cre * xi + cim * xr, cw.data() + 4 * code + 2);
+          }
+        }
+      sq.resize(n_div);
+      for (uint32_t d = 0; d < n_div; ++d) sq[d] = std::sqrt((double)div[d]);
+      put(t->cplx_w, cw.data(), cw.size() * 4);
+      put(t->fix_sqrt_s, sq.data(), n_div * 8);
+      t->fix.n_codes = (uint32_t)n_codes;
+      t->fix.n_div = n_div;
+      t->fix.bound = (double)std::max<uint64_t>(1, op.row_bound) * sq[n_div - 1] * (1.0 + 1e-9);
+      t->cplx_ok = true;
+    }
+  }
   if (int st = parts.allocate(t->buf)) return st;
   std::vector<char> host(t->buf.bytes, 0);
   for (auto const& f : from)
@@ -902,6 +949,7 @@ int build_tables(OperatorData& op) {
   t->code.divisors = t->divisors.as<uint32_t>();
   t->fix.code = t->fix_code.as<uint8_t>();
   t->fix.sqrt_s = t->fix_sqrt_s.as<double>();
+  t->cplx.w = t->cplx_w.as<int4>();
   op.tables = std::move(t);
   return LS_SUCCESS;
 }
@@ -1043,7 +1091,8 @@ int operator_ensure_ready(OperatorData& op) {
   if (int st = basis_upload_plan(b, op.cuda_stream)) return st;
   if (int st = operator_upload_terms(op)) return st;
   if (int st = build_tables(op)) return st;
-  if (int st = fix_reserve(op, 1)) return st;
+  if (op.tables->fix_ok)
+    if (int st = fix_reserve(op, 1)) return st;
   return LS_SUCCESS;
 }
 
@@ -1282,7 +1331,7 @@ int operator_record_stream(OperatorData& op, cudaStream_t stream) {
 }
 
 int fix_reserve(OperatorData& op, uint32_t cols) {
-  if (!op.tables || !op.tables->fix_ok || op.fix_cols >= cols) return LS_SUCCESS;
+  if (!op.tables || !(op.tables->fix_ok || op.tables->cplx_ok) || op.fix_cols >= cols) return LS_SUCCESS;
   uint64_t const D = std::max<uint64_t>(1, op.basis->D);
   if (!op.fix_event) SED_TRY_CUDA(cudaEventCreateWithFlags(&op.fix_event, cudaEventDisableTiming));
   DeviceBuffer slots;
@@ -1463,16 +1512,21 @@ int launch_apply(OperatorData& op, X const* x, X* y, cudaStream_t stream, bool u
     StreamView const S = stream_view(op);
     unsigned const grid = (unsigned)((sf.n_slices * 32 + kBlock - 1) / kBlock);
     size_t const smem = std::min<size_t>(32768, (size_t)tb.n_codes * (real_tab ? 8 : 16));
+    bool const krylov = ind.k || ind.stop || ind.partial;
+    auto launch = [&](auto real) {
+      auto go = [&](auto packed) {
+        if (krylov) k_spmv<X, real.value, packed.value, true><<<grid, kBlock, smem, stream>>>(S, D, x, y, ind);
+        else k_spmv<X, real.value, packed.value, false><<<grid, kBlock, smem, stream>>>(S, D, x, y, ind);
+        note_launches(1);
+      };
+      if (sf.packed) go(std::true_type{});
+      else go(std::false_type{});
+    };
     if (real_tab) {
-      if (sf.packed) { k_spmv<X, true, true><<<grid, kBlock, smem, stream>>>(S, D, x, y, ind); note_launches(1); }
-      else { k_spmv<X, true, false><<<grid, kBlock, smem, stream>>>(S, D, x, y, ind); note_launches(1); }
+      launch(std::true_type{});
     } else {
-      if constexpr (complex_storage) {
-        if (sf.packed) { k_spmv<X, false, true><<<grid, kBlock, smem, stream>>>(S, D, x, y, ind); note_launches(1); }
-        else { k_spmv<X, false, false><<<grid, kBlock, smem, stream>>>(S, D, x, y, ind); note_launches(1); }
-      } else {
-        return fail(LS_OPERATOR_IS_COMPLEX, "complex operator applied to real vectors");
-      }
+      if constexpr (complex_storage) launch(std::false_type{});
+      else return fail(LS_OPERATOR_IS_COMPLEX, "complex operator applied to real vectors");
     }
   } else {
     IndexView const I = b.index_view();
@@ -2153,6 +2207,7 @@ int sed_operator_prepare(ls_operator* op, int form) {
   d.form = form;
   if (form == SED_FORM_ON_THE_FLY) return LS_SUCCESS;
   int st = operator_record_stream(d, d.cuda_stream);
+  if (!st && cplx_sums(d)) (void)fix_reserve(d, 2);  // without it the matvecs take the general kernel
   return (form == SED_FORM_AUTO && st == LS_OUT_OF_MEMORY) ? LS_SUCCESS : st;
 }
 

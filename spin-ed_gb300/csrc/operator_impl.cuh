@@ -334,6 +334,22 @@ __device__ __forceinline__ void fix_row_sums(StreamView const& S, FixView const&
   if (e < width) step(e, std::true_type{});
 }
 
+// The streamed matvec of an operator with complex elements in integers
+// (spmv_cols.cu). An element's factor and the gathered part are numbers of two
+// 32-bit limbs (the low one signed, so that the high one is rounded):
+// w = round(value x character x 2^-shift), |w| <= 2^54, and u as for real
+// operators, |u| <= 2^62 / R with R the largest row count. A row keeps two
+// 64-bit sums per part,
+//   hi = sum w_h u_h,   lo = sum w_h u_l + w_l u_h + w_l u_l / 2^32,
+// |hi| <= 2^53 and |lo| <= 2 R (2^61 / R + 2^53 + 2^30) < 2^63 up to R = 128;
+// its value is (hi 2^32 + lo) 2^(32 + shift - F).
+struct CplxView {
+  int4 const* w;  // [n_codes]: limbs of Re w (high, low) and of Im w
+  int shift;
+};
+constexpr uint64_t kCplxMaxRow = 128;
+constexpr uint32_t kCplxMaxCodes = 2048;  // 32 KB of shared memory
+
 struct OperatorTables {
   DeviceBuffer buf;      // holds all of them
   DevicePart divisors;
@@ -348,6 +364,11 @@ struct OperatorTables {
   DevicePart fix_code;
   DevicePart fix_sqrt_s;
   FixView fix{};
+  // integer form of a complex operator (cplx_ok: it qualifies; fix then holds
+  // sqrt_s, n_div, n_codes and bound)
+  bool cplx_ok = false;
+  DevicePart cplx_w;
+  CplxView cplx{};
 };
 
 // One row of the streamed SpMV over a SELL-32 slice (lane = row in slice).
@@ -474,6 +495,8 @@ int operator_ensure_ready(OperatorData& op);
 // Whether streamed matvecs of this dtype take the integer sums of
 // fix_cols_blocks, and the first `block` columns through it (spmv_cols.cu);
 // *done counts the columns taken.
+// Whether matvecs of a recorded complex operator take integer sums.
+bool cplx_sums(OperatorData const& op);
 bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_stream, cudaStream_t stream);
 int fix_cols_blocks(OperatorData& op, int dtype, uint64_t block, char const* x, uint64_t ldx, char* y, uint64_t ldy,
                     size_t es, cudaStream_t stream, uint64_t* done);

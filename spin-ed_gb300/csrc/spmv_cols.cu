@@ -1,6 +1,7 @@
-// spmv_cols.cu — the streamed fixed-point matvec on blocks of columns and on
-// FP32 and complex vectors of real operators (src/SpinED/Internal.hs:411-429;
-// the mathematics is at FixView in operator_impl.cuh).
+// spmv_cols.cu — the streamed fixed-point matvec on blocks of columns, on FP32
+// and complex vectors of real operators and of complex operators
+// (src/SpinED/Internal.hs:411-429; the mathematics is at FixView and CplxView
+// in operator_impl.cuh).
 //
 // A pass covers K real columns; a complex column is two. The gather copy u
 // holds the K columns of a row next to each other.
@@ -9,11 +10,11 @@
 namespace sed {
 namespace {
 
-// FP32 and complex
-// vectors of a real operator take the same integer sums as FP64 ones: the
-// FP64 multiply-adds per element of k_spmv (two or four on a pipe of 1.75
-// per clock and SM, after an FP32 load a conversion on the same pipe) bound
-// it at 378 us where this takes 145 (ring of 32 sites, FP32).
+// FP32 and complex vectors of a real operator take the same integer sums as
+// FP64 ones: the FP64 operations per element of k_spmv (one or two
+// multiply-adds on a pipe of 1.75 per clock and SM, and after an FP32 load a
+// conversion on the same pipe) bound it at 397 us a call where these take 177
+// (ring of 32 sites, FP32).
 struct Columns {
   void const* x;
   void* y;
@@ -79,18 +80,22 @@ __global__ void __launch_bounds__(kBlock) k_fix_max_cols(Columns c, uint64_t D, 
 // K sectors. K / 2 lanes share a row, two columns each, so that a warp writes
 // 512 bytes in a row (a lane that wrote a whole row took 59 us for 8 columns
 // of 1.3 M rows); a thread keeps its columns, and what belongs to them, over
-// its rows, since the integer ALU bounds it.
-template <int K>
+// its rows, since the integer ALU bounds it. Cplx (K = 2): one scale for both
+// parts, and u in two limbs (CplxView).
+template <int K, bool Cplx>
 __global__ void __launch_bounds__(kBlock) k_fix_convert_cols(Columns c, uint64_t D, uint8_t const* __restrict__ row_class,
                                                              FixView fv, unsigned long long const* __restrict__ max_bits,
                                                              int64_t* __restrict__ F_out, int64_t* __restrict__ u) {
   constexpr uint32_t N = K > 1 ? 2 : 1, L = K / N;  // columns per lane, lanes per row
   extern __shared__ double fac[];                    // [K][n_div]
+  auto exponent = [&](uint32_t q) {
+    return fix_exponent(Cplx ? max(max_bits[0], max_bits[1]) : max_bits[q], fv.bound);
+  };
   for (uint32_t t = threadIdx.x; t < K * fv.n_div; t += blockDim.x) {
     uint32_t const q = t / fv.n_div;
     double f = 0.0;
     if (q < c.cols) {
-      int64_t const F = fix_exponent(max_bits[q], fv.bound);
+      int64_t const F = exponent(q);
       int64_t const F1 = (F == kFixBad || (F >= -1000 && F <= 1000)) ? 0 : F / 2;
       if (F != kFixBad) f = fv.sqrt_s[t % fv.n_div] * fix_pow2(F - F1);
       if (blockIdx.x == 0 && t % fv.n_div == 0) F_out[q] = F;
@@ -108,7 +113,7 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert_cols(Columns c, uint64_t
 #pragma unroll
   for (uint32_t n = 0; n < N; ++n) {
     uint32_t const q = q0 + n;
-    int64_t const F = q < c.cols ? fix_exponent(max_bits[q], fv.bound) : kFixBad;
+    int64_t const F = q < c.cols ? exponent(q) : kFixBad;
     on[n] = F != kFixBad;
     int64_t const F1 = (F == kFixBad || (F >= -1000 && F <= 1000)) ? 0 : F / 2;
     p1[n] = fix_pow2(F1);
@@ -127,6 +132,7 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert_cols(Columns c, uint64_t
         double xv = c.f32 ? widen(static_cast<float const*>(c.x)[o]) : static_cast<double const*>(c.x)[o];
         if (two) xv *= p1[n];
         v[n] = fix_round(xv * fac[(q0 + n) * fv.n_div + cls]);
+        if constexpr (Cplx) v[n] += (v[n] & 0x80000000ll) << 1;  // high limb | low limb
       }
     }
     if constexpr (N == 1) u[i] = v[0];
@@ -136,7 +142,7 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert_cols(Columns c, uint64_t
 
 // One row of two adjacent columns as k_spmv sums it (a vector with a NaN or
 // an infinity: only the rows it reaches are affected).
-template <class V>
+template <class V, bool RealOp>
 __device__ __forceinline__ V general_row(StreamView const& S, Columns const& c, uint32_t const* ent, uint16_t const* codes,
                                          uint32_t width, uint32_t col_mask, bool packed, uint32_t q) {
   V acc = zero<V>();
@@ -144,7 +150,7 @@ __device__ __forceinline__ V general_row(StreamView const& S, Columns const& c, 
     uint32_t const v = ent[(uint64_t)e * 32];
     if (v == kNull) continue;
     uint32_t const code = packed ? (v >> S.col_bits) : (uint32_t)codes[(uint64_t)e * 32], j = v & col_mask;
-    V const t = load_table<V>(S.table, code, true);
+    V const t = load_table<V>(S.table, code, RealOp);
     if constexpr (std::is_same<V, double>::value) mac(acc, t, c.load(q, j));
     else mac(acc, t, cplx{c.load(q, j), c.load(q + 1, j)});
   }
@@ -193,7 +199,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix_cols(StreamView S, FixView 
     if (c.cx) {
       for (uint32_t q = q0; q < q0 + N && q < c.cols; q += 2) {
         cplx const xi{c.load(q, i), c.load(q + 1, i)};
-        cplx const acc = general_row<cplx>(S, c, ent, codes, width, col_mask, Packed, q);
+        cplx const acc = general_row<cplx, true>(S, c, ent, codes, width, col_mask, Packed, q);
         cplx const yi = row_value<cplx>(mulv(cplx{dg, 0.0}, xi), f, acc);
         c.store(q, i, yi.re);
         c.store(q + 1, i, yi.im);
@@ -201,7 +207,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix_cols(StreamView S, FixView 
     } else {
       for (uint32_t q = q0; q < q0 + N && q < c.cols; ++q)
         c.store(q, i, row_value<double>(mulv(dg, c.load(q, i)), f,
-                                        general_row<double>(S, c, ent, codes, width, col_mask, Packed, q)));
+                                        general_row<double, true>(S, c, ent, codes, width, col_mask, Packed, q)));
     }
     return;
   }
@@ -232,6 +238,157 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix_cols(StreamView S, FixView 
 }
 
 
+// hi 2^32 + lo as a double, rounded to nearest even (|hi| < 2^55).
+__device__ __forceinline__ double limbs_to_double(int64_t hi, int64_t lo) {
+  hi += lo >> 32;
+  uint32_t l = (uint32_t)lo;
+  bool const neg = hi < 0;
+  if (neg) {
+    l = 0u - l;
+    hi = ~hi + (l == 0u ? 1 : 0);
+  }
+  int const z = __clzll(hi);
+  uint64_t m = (uint64_t)hi << 32 | l;
+  uint64_t b = 0;
+  if (z < 32) {  // 2^64 and above: the 64 leading bits, the rest as a sticky one
+    m = (uint64_t)hi << z | l >> (32 - z) | ((l << z) != 0u ? 1u : 0u);
+    b = (uint64_t)(32 - z) << 52;
+  }
+  int const y = __clzll((long long)m);
+  m <<= y & 63;
+  uint32_t const rest = (uint32_t)m & 0x7FFu;
+  uint64_t const top = m >> 11;
+  b += ((uint64_t)(1085 - y) << 52) + top + ((rest > 0x400u || (rest == 0x400u && (top & 1))) ? 1u : 0u);
+  if (m == 0) b = 0;
+  return __longlong_as_double((long long)(b | (uint64_t)neg << 63));
+}
+
+// Streamed SpMV of a complex operator on a complex column, sums in integers
+// (CplxView). The four FP64 multiply-adds per element of k_spmv take 75 of its
+// 102 us on the 28-site ring at k = 3 (10.4 M elements, FP64 pipe of 1.75 per
+// clock and SM); here an element is 16 wide integer multiply-adds and one
+// 16-byte gather: 46 us, of which the gathered sectors are about 32 (10.5
+// TB/s of L2). With 11 us for the pre-pass a call takes 85 us for 123. FP32
+// vectors: 159 and 46 us (the conversions of k_spmv's loads share its pipe).
+// Factors are staged with their position's low three bits swizzled: codes of
+// one stabiliser class are n_div apart, which would put them all in one bank
+// group. Eight elements in flight: 20.8 M elements in 109 us for 112 with four.
+template <bool Packed>
+__global__ void __launch_bounds__(kBlock) k_spmv_cplx(StreamView S, FixView fv, CplxView cw, uint64_t D, Columns c,
+                                                      int4 const* __restrict__ u, int64_t const* __restrict__ F_in,
+                                                      unsigned long long* __restrict__ clear) {
+  extern __shared__ int4 w_smem[];  // [n_codes], swizzled within groups of 8; then g[n_div]
+  auto place = [](uint32_t code) { return code ^ ((code >> 3) & 7u); };
+  uint32_t const n8 = (fv.n_codes + 7u) & ~7u;
+  double* g = reinterpret_cast<double*>(w_smem + n8);
+  if (blockIdx.x == 0 && threadIdx.x < 2) clear[threadIdx.x] = 0;  // max |x| for the next call's pre-pass
+  int64_t const F = F_in[0];
+  // 2^(32 + shift - F), what is outside +-1000 by a second factor
+  int64_t const e = F == kFixBad ? 0 : 32 + cw.shift - F, e1 = min(max(e, (int64_t)-900), (int64_t)900);
+  for (uint32_t t = threadIdx.x; t < fv.n_codes; t += blockDim.x) w_smem[place(t)] = cw.w[t];
+  for (uint32_t t = threadIdx.x; t < fv.n_div; t += blockDim.x) g[t] = S.inv_sqrt_s[t] * fix_pow2(e1);
+  __syncthreads();
+  uint64_t const i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, s = i >> 5;
+  if ((s << 5) >= D) return;
+  uint32_t const lane = threadIdx.x & 31;
+  uint64_t const base = S.slice_ptr[s];
+  uint32_t const width = (uint32_t)((S.slice_ptr[s + 1] - base) >> 5);
+  uint32_t const mask = Packed ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
+  uint32_t const* ent = S.entries + base + lane;
+  uint16_t const* codes = S.codes + base + lane;
+  if (F == kFixBad) {
+    if (i >= D) return;
+    cplx const xi{c.load(0, i), c.load(1, i)};
+    cplx const acc = general_row<cplx, false>(S, c, ent, codes, width, mask, Packed, 0);
+    cplx const yi = row_value<cplx>(mulv(stream_diag<cplx, false>(S, i), xi), S.inv_sqrt_s[S.row_class[i]], acc);
+    c.store(0, i, yi.re);
+    c.store(1, i, yi.im);
+    return;
+  }
+  int64_t hr = 0, lr = 0, hi = 0, li = 0;
+  auto add = [](int64_t& h, int64_t& l, int wh, int wl, int uh, int ul) {
+    h += (int64_t)wh * uh;
+    l += (int64_t)wh * ul;
+    l += (int64_t)wl * uh;
+    l += (int64_t)(wl >> 16) * (ul >> 16);  // the last 2^-68 of the largest product is not kept
+  };
+  constexpr uint32_t U = 8;
+  auto step = [&](uint32_t e0, auto guarded) {
+    uint32_t v[U], cd[U];
+    int4 x[U];
+#pragma unroll
+    for (uint32_t p = 0; p < U; ++p) {
+      bool const in = !decltype(guarded)::value || e0 + p < width;
+      v[p] = in ? __ldcs(ent + (uint64_t)(e0 + p) * 32) : kNull;
+      if constexpr (Packed) cd[p] = min(v[p] >> S.col_bits, fv.n_codes - 1);
+      else cd[p] = in ? (uint32_t)__ldcs(codes + (uint64_t)(e0 + p) * 32) : 0u;
+    }
+#pragma unroll
+    for (uint32_t p = 0; p < U; ++p) x[p] = __ldg(u + min(v[p] & mask, (uint32_t)D));  // row D is zero
+#pragma unroll
+    for (uint32_t p = 0; p < U; ++p) {
+      int4 const w = w_smem[place(cd[p])];
+      // little endian: x low, y high limb of the real part, z and w of the imaginary
+      add(hr, lr, w.x, w.y, x[p].y, x[p].x);
+      add(hr, lr, -w.z, -w.w, x[p].w, x[p].z);
+      add(hi, li, w.x, w.y, x[p].w, x[p].z);
+      add(hi, li, w.z, w.w, x[p].y, x[p].x);
+    }
+  };
+  uint32_t e0 = 0;
+  for (; e0 + U <= width; e0 += U) step(e0, std::false_type{});
+  if (e0 < width) step(e0, std::true_type{});
+  if (i >= D) return;
+  double const f = g[__ldcs(S.row_class + i)];
+  double2 const dg = __ldcs(static_cast<double2 const*>(S.diag) + i);
+  double const xr = c.load(0, i), xi = c.load(1, i);
+  double yr = __dmul_rn(dg.x, xr), yi = __dmul_rn(dg.x, xi);
+  if (dg.y != 0.0) {
+    yr = __fma_rn(-dg.y, xi, yr);
+    yi = __fma_rn(dg.y, xr, yi);
+  }
+  double sr = limbs_to_double(hr, lr), si = limbs_to_double(hi, li);
+  if (e != e1) {
+    sr = __dmul_rn(f, sr);
+    si = __dmul_rn(f, si);
+    double const p = fix_pow2(e - e1);
+    yr = __fma_rn(p, sr, yr);
+    yi = __fma_rn(p, si, yi);
+  } else {
+    yr = __fma_rn(f, sr, yr);
+    yi = __fma_rn(f, si, yi);
+  }
+  c.store(0, i, yr);
+  c.store(1, i, yi);
+}
+
+int launch_cplx(OperatorData& op, Columns const& c, cudaStream_t stream) {
+  BasisData& b = *op.basis;
+  OperatorTables const& tb = *op.tables;
+  StreamForm const& sf = op.stream;
+  uint64_t const D = b.D;
+  if (D == 0) return LS_SUCCESS;
+  auto* mx = op.fix_slots.as<unsigned long long>();
+  auto* F = reinterpret_cast<int64_t*>(mx + op.fix_cols);
+  int64_t* u = op.fix_u.as<int64_t>();
+  if (int st = fix_enter(op, stream)) return st;
+  if (!op.fix_clean) SED_TRY_CUDA(cudaMemsetAsync(mx, 0, (size_t)op.fix_cols * 8, stream));
+  op.fix_clean = false;
+  k_fix_max_cols<<<grid_size(2 * D, b.device, 8), kBlock, 0, stream>>>(c, D, mx);
+  k_fix_convert_cols<2, true><<<grid_size(D + 1, b.device, 8), kBlock, (size_t)2 * tb.fix.n_div * 8, stream>>>(
+      c, D, sf.row_class.as<uint8_t>(), tb.fix, mx, F, u);
+  StreamView const S = stream_view(op);
+  unsigned const grid = (unsigned)((sf.n_slices * 32 + kBlock - 1) / kBlock);
+  size_t const smem = (size_t)((tb.n_codes + 7) & ~7u) * 16 + (size_t)tb.fix.n_div * 8;
+  auto const* u4 = reinterpret_cast<int4 const*>(u);
+  if (sf.packed) k_spmv_cplx<true><<<grid, kBlock, smem, stream>>>(S, tb.fix, tb.cplx, D, c, u4, F, mx);
+  else k_spmv_cplx<false><<<grid, kBlock, smem, stream>>>(S, tb.fix, tb.cplx, D, c, u4, F, mx);
+  note_launches(3);
+  SED_TRY_CUDA(cudaGetLastError());
+  op.fix_clean = true;  // the SpMV has cleared the words again
+  return fix_leave(op, stream);
+}
+
 // A pass of the fixed-point SpMV over c.cols <= K real columns (K = 1, 2, 4,
 // 8, 16; the workspace holds K).
 int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t stream) {
@@ -257,7 +414,7 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
     uint64_t const warps = sf.n_slices * LL;
     unsigned const grid = (unsigned)((warps * 32 + kBlock - 1) / kBlock);
     unsigned const cg = grid_size((D + 1) * (KK > 2 ? KK / 2 : 1), b.device, 8);
-    k_fix_convert_cols<KK><<<cg, kBlock, (size_t)KK * tb.fix.n_div * 8, stream>>>(c, D, cls, tb.fix, mx, F, u);
+    k_fix_convert_cols<KK, false><<<cg, kBlock, (size_t)KK * tb.fix.n_div * 8, stream>>>(c, D, cls, tb.fix, mx, F, u);
     fix_dispatch(tb, sf.packed, [&](auto packed, auto nv, auto sign) {
       k_spmv_fix_cols<packed.value, nv.value, sign.value, KK><<<grid, kBlock, smem, stream>>>(S, tb.fix, D, c, u, F, mx);
     });
@@ -277,6 +434,13 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
 
 }  // namespace
 
+// From 2^21 elements on: below, the two launches more cost what the sums save
+// (complex128 call, general kernel and this one: 1.4 M elements 45 and 46 us,
+// 2.7 M 56 and 53, 10.4 M 123 and 85, 20.8 M 198 and 109).
+bool cplx_sums(OperatorData const& op) {
+  return op.tables->cplx_ok && op.stream.n_elements >= ((uint64_t)1 << 21);
+}
+
 // Whether vectors of this dtype go through launch_fix_cols. FP64 columns
 // always do. The others do from 2^21 element products on: below, the three
 // launches more cost what the sums save (290 000 elements of a complex
@@ -285,9 +449,14 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
 // workspace could be overwritten between replays (the general kernels use
 // none).
 bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_stream, cudaStream_t stream) {
-  if (!use_stream || !op.tables->fix_ok || op.fix_cols < 1) return false;
-  if (dtype == 1) return true;
-  if (op.stream.n_elements * block * (dtype >= 2 ? 2 : 1) < ((uint64_t)1 << 21)) return false;
+  if (!use_stream) return false;
+  if (op.tables->cplx_ok) {
+    if (dtype < 2 || !cplx_sums(op)) return false;
+  } else {
+    if (!op.tables->fix_ok || op.fix_cols < 1) return false;
+    if (dtype == 1) return true;
+    if (op.stream.n_elements * block * (dtype >= 2 ? 2 : 1) < ((uint64_t)1 << 21)) return false;
+  }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
     cudaGetLastError();
@@ -306,6 +475,13 @@ bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_
 // the caller's general path does the rest.
 int fix_cols_blocks(OperatorData& op, int dtype, uint64_t block, char const* x, uint64_t ldx, char* y, uint64_t ldy,
                     size_t es, cudaStream_t stream, uint64_t* done) {
+  if (op.tables->cplx_ok) {
+    if (int st = fix_reserve(op, 2)) return st == LS_OUT_OF_MEMORY ? LS_SUCCESS : st;
+    for (; *done < block; ++*done)
+      if (int st = launch_cplx(op, {x + *done * ldx * es, y + *done * ldy * es, ldx, ldy, 2, dtype == 2, true}, stream))
+        return st;
+    return LS_SUCCESS;
+  }
   // a pass keeps K tables of row factors in shared memory: at most kmax
   // columns fit in 48 KB
   size_t const table = (size_t)op.tables->fix.n_div * op.tables->fix_nv * 8;

@@ -365,3 +365,71 @@ def test_narrower_passes_when_the_workspace_is_capped(sed, oracle):
         lib.sed_set_device_memory_limit(0)
     y = sed.apply(op, x)
     assert all(torch.equal(y[:, c], columns[c]) for c in range(16))
+
+
+# complex operators of 2^21 elements or more: the integer sums of k_spmv_cplx
+def _dense_complex(n):
+    rng = np.random.default_rng(11)
+    bonds = lattices.chain_bonds(n, 1)
+    return lattices.Model("dense", n, None, None, [(lattices.chain_translation(n), 2)],
+                          [(random_complex_term(rng, 2, hermitian=False), bonds)])
+
+
+CPLX_MODELS = {
+    "chain24_k3_j2": lattices.heisenberg_chain(24, momentum=3, parity=None, spin_inversion=None, j2=0.3),
+    "chain26_k1": lattices.heisenberg_chain(26, momentum=1, parity=None),
+    "dense20_k2": _dense_complex(20),  # complex diagonal, 12 values, rows of 60
+}
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("name", list(CPLX_MODELS))
+def test_complex_operator_sums(sed, oracle, name, dtype):
+    """Columns of very different scales against the oracle's matrix, and a NaN
+    that reaches the rows that couple to its entry only. The integer sums err
+    by at most R (R max|u| 2^-61 + max|u| 2^-54) max|w|, R <= 60 elements a
+    row: 4e-15 of max|u| max|w|; the oracle's FP64 sums by 2 R 2^-53 R of it."""
+    import torch
+    built, ob, oop = both(sed, oracle, CPLX_MODELS[name])
+    op, D = built.hamiltonian, len(ob.reps)
+    op.prepare(L.SED_FORM_STREAM)
+    A = oop.sparse()
+    assert A.nnz > 1 << 21
+    scales = [1e-300, 1e-3, 1.0, 1e300] if dtype == "complex128" else [1e-30, 1e-3, 1.0, 1e30]
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randn(len(scales), D + 5, dtype=getattr(torch, dtype), device="cuda", generator=gen).t()[:D]
+    x *= torch.tensor(scales, dtype=torch.float64, device="cuda").to(x.dtype)
+    y = torch.zeros(len(scales), D + 3, dtype=x.dtype, device="cuda").t()[:D]
+    sed.inplace_apply(op, x, y)
+    xs, ys = x.cpu().numpy(), y.cpu().numpy()
+    eps = 1e-12 if dtype == "complex128" else 2.0 ** -23
+    for c, s in enumerate(scales):
+        want = A @ (xs[:, c].astype(np.complex128) / s)
+        assert np.abs(ys[:, c].astype(np.complex128) / s - want).max() <= eps * np.abs(want).max()
+    j = D // 3
+    x[j, 2] = float("nan")
+    z = sed.apply(op, x[:, 2].contiguous()).cpu().numpy()
+    reached = np.zeros(D, bool)
+    rows, cols, _ = oop.coo()
+    reached[rows[cols == j].astype(np.int64)] = True
+    reached[j] = True
+    assert np.array_equal(np.isfinite(z), ~reached)
+    assert np.abs(z[~reached] - ys[~reached, 2]).max() <= eps * np.abs(ys[:, 2]).max()
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+def test_complex_operator_sums_with_separate_codes(sed, dtype):
+    """Columns and codes that do not fit 31 bits together (18.8 M states),
+    against the matvec that records nothing."""
+    import torch
+    from spined.model import build_model
+    built = build_model(lattices.heisenberg_chain(32, momentum=3, parity=None, spin_inversion=None))
+    op, D = built.hamiltonian, sed.get_number_states(built.basis)
+    op.prepare(L.SED_FORM_STREAM)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(D, dtype=getattr(torch, dtype), device="cuda", generator=gen)
+    y = sed.apply(op, x)
+    op.prepare(L.SED_FORM_ON_THE_FLY)
+    want = sed.apply(op, x)
+    eps = 1e-13 if dtype == "complex128" else 2.0 ** -22  # both rounded to FP32
+    assert (y - want).abs().max() <= eps * want.abs().max()
