@@ -1,15 +1,16 @@
 // batch.cu — many Hamiltonians of uneven size solved in one persistent launch
 // (sed_eigh_batched): the lowest nev <= 4 eigenpairs of every operator by
-// block Lanczos with block size 4. Vectors are stored in FP64; the products
-// of the block SpMV, the Gram-Schmidt passes, CholQR2 and the Ritz vectors
-// run in double-float arithmetic on the FP32 pipe (df.cuh); norms, the
-// Rayleigh-Ritz solve and the true residuals are FP64.
+// block Lanczos with block size 4. Krylov blocks are held as double-floats
+// (df.cuh), and the products of the block SpMV, the Gram-Schmidt sweeps,
+// CholQR2 and the Ritz vectors run in that arithmetic on the FP32 pipe; the
+// SpMV's row epilogue, the Rayleigh-Ritz solve, the Ritz vectors kept and their
+// true residuals are FP64.
 //
 // One cooperative kernel runs the whole solve for all problems. Its CTAs are
 // split into groups (batch_layout: large problems get several CTAs, small
 // ones share one-CTA groups and are solved one after another), and a group
 // synchronises through a bounded barrier in global memory. Within a group
-// the rows of the problem are split by SELL-32 slices.
+// the rows of the problem are split by SELL-32 slices, two runs to a CTA.
 //
 // Per problem, with Krylov blocks V_j stored row-interleaved ([D][4], so the
 // SpMV gathers one 32-byte sector per element for all four columns):
@@ -51,13 +52,13 @@ constexpr int kB = 4;               // block size
 constexpr int kMaxBlocks = 16;      // stored Krylov blocks per cycle (n <= 64)
 constexpr int kMaxN = kB * kMaxBlocks;
 constexpr int kPart = 16 * (kMaxBlocks + 1);  // partial sums per CTA and slot
-constexpr int kGsStages = 4;                   // shared-memory stages of the Gram-Schmidt row streams
+constexpr int kGsStages = 2;                   // shared-memory stages of the Gram-Schmidt row streams
 constexpr uint64_t kGsWaitNs = 1000000000ull;  // default bound on a wait for one stage's copies (1 s)
 constexpr uint64_t kBarrierNs = 20000000000ull;  // default: 20 s per barrier, far beyond any phase
 // Part of a block step that more CTAs do not shorten, in rows of the mean
-// work per row (the group layout's model). Fitted on 128 J1-J2 chains
-// (N = 16..28, problems alone in their groups): a block step took 0.25 ms
-// plus 0.18 us per row of the CTA's share, i.e. about 1400 rows.
+// work per row (the group layout's model). On 128 J1-J2 chains (N = 16..28)
+// the launch takes 720 ms with 900 rows, 708 with 1400, 726 with 2200 and 734
+// with 3500.
 constexpr double kLayoutFixedRows = 1400.0;
 constexpr size_t kStatsOff = 12 * 8;                // per-problem output record: out[12], stats[4], flag[4], prof[8]
 constexpr size_t kProfOff = kStatsOff + 32;
@@ -66,8 +67,8 @@ constexpr size_t kOutBytes = kProfOff + 64;
 struct ChainDesc {
   StreamView S;       // real operator, FP64 stream form
   uint64_t D, n_slices;
-  double* V;          // (m_blocks + 1) blocks of [D][4]
-  float* Vs;          // V split into double-float rows (Row4s), for the Gram-Schmidt products
+  double* V;          // [D][4]: the start block, then the Ritz vectors
+  float* Vs;          // (m_blocks + 1) Krylov blocks of D double-float rows (Row4s)
   float* Xs;          // [D] Row4s: the block under Gram-Schmidt, in double-float
   float2* table_s;    // [n_codes]: the matrix-element table split into double-float (k_split_tables)
   double* W;          // [D][4]
@@ -102,6 +103,7 @@ struct BatchArgs {
   int* error;
   uint64_t wait_ns;        // bound on every barrier wait
   uint64_t copy_wait_ns;   // bound on every wait for a row-stream stage's copies
+  uint32_t stage_bytes;    // dynamic shared memory for the row streams' stages
   uint32_t extra_arrivals; // arrivals a barrier waits for beyond its CTAs (0; see sed_debug_barrier_extra_arrivals)
 };
 
@@ -131,41 +133,6 @@ __device__ __forceinline__ Row4s split_row(Row4 const& r) {
   df_split(r.z, o.h.z, o.l.z);
   df_split(r.w, o.h.w, o.l.w);
   return o;
-}
-
-// (S, E)[s][t] += a_s w_t over one row of a split block a and of X.
-__device__ __forceinline__ void df_dots(Row4s const& a, Row4s const& w, float (&S)[16], float (&E)[16]) {
-  float const ah[4] = {a.h.x, a.h.y, a.h.z, a.h.w}, al[4] = {a.l.x, a.l.y, a.l.z, a.l.w};
-  float const wh[4] = {w.h.x, w.h.y, w.h.z, w.h.w}, wl[4] = {w.l.x, w.l.y, w.l.z, w.l.w};
-#pragma unroll
-  for (int s = 0; s < 4; ++s)
-#pragma unroll
-    for (int t = 0; t < 4; ++t) df_mac(ah[s], al[s], wh[t], wl[t], S[s * 4 + t], E[s * 4 + t]);
-}
-
-// (S, E)[t] += sum_s a_s c[s][t] for one split row a and 4 x 4 split
-// coefficients (c4h, c4l: row s as one float4 each).
-__device__ __forceinline__ void df_axpy(Row4s const& a, float4 const* c4h, float4 const* c4l, float (&S)[4],
-                                        float (&E)[4]) {
-  float const ah[4] = {a.h.x, a.h.y, a.h.z, a.h.w}, al[4] = {a.l.x, a.l.y, a.l.z, a.l.w};
-#pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    float4 const h = c4h[s], l = c4l[s];
-    df_mac(ah[s], al[s], h.x, l.x, S[0], E[0]);
-    df_mac(ah[s], al[s], h.y, l.y, S[1], E[1]);
-    df_mac(ah[s], al[s], h.z, l.z, S[2], E[2]);
-    df_mac(ah[s], al[s], h.w, l.w, S[3], E[3]);
-  }
-}
-
-// row -= (S + E), column by column.
-__device__ __forceinline__ void df_sub_row(Row4s& row, float const (&S)[4], float const (&E)[4]) {
-  Row4s w = row;
-  df_sub(w.h.x, w.l.x, S[0], E[0]);
-  df_sub(w.h.y, w.l.y, S[1], E[1]);
-  df_sub(w.h.z, w.l.z, S[2], E[2]);
-  df_sub(w.h.w, w.l.w, S[3], E[3]);
-  row = w;
 }
 
 // Bounded barrier of the `n` CTAs of a group; false if it timed out (then
@@ -233,8 +200,16 @@ struct Ctx {
   uint32_t rank, ncta;
   uint32_t* bar;
   BatchArgs const* args;
-  uint64_t r0, r1;      // own rows
-  uint64_t s0, s1;      // own slices
+  // Own slices and rows: two runs, [sa, sa + ns0) and [sb, ..), the rank-th of
+  // 2 ncta equal pieces and the rank-th from the end. Rows lengthen from the
+  // first representative to the last (22-site J1-J2 chain on 11 CTAs: 19.5
+  // elements a row in the first eleventh, 29.6 in the last), so that one run
+  // per CTA left the SpMV of the last CTA 16 % above the mean; two runs are even
+  // in rows and in elements.
+  uint32_t ns, ns0, n, n0;  // own slices and rows, of these in the first run
+  uint64_t sa, sb, ra, rb;
+  __device__ __forceinline__ uint64_t slice(uint32_t l) const { return l < ns0 ? sa + l : sb + (l - ns0); }
+  __device__ __forceinline__ uint64_t row(uint32_t l) const { return l < n0 ? ra + l : rb + (l - n0); }
   uint32_t slot;        // partial-sum double buffer
   double* red;          // shared [warps][16]
   double* tmp;          // shared [kPart]
@@ -287,7 +262,8 @@ __device__ bool chol4(double const* G, double* R) {
 // on GB300's narrow FP64 pipe).
 __device__ void apply_rinv(Ctx& x, double* X, double const* R) {
   double const inv[4] = {1.0 / R[0], 1.0 / R[5], 1.0 / R[10], 1.0 / R[15]};
-  for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
+  for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+    uint64_t const r = x.row(l);
     Row4 const v = *reinterpret_cast<Row4 const*>(X + r * 4);
     double const a[4] = {v.x, v.y, v.z, v.w};
     double y[4];
@@ -309,7 +285,8 @@ __device__ bool block_qr(Ctx& x, double* X, double* Rtot, bool& ok) {
   ok = true;
   for (int pass = 0; pass < 2; ++pass) {
     double g[10] = {};
-    for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
+    for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+      uint64_t const r = x.row(l);
       Row4 const v = *reinterpret_cast<Row4 const*>(X + r * 4);
       double const a[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -356,20 +333,67 @@ __device__ bool block_qr(Ctx& x, double* X, double* Rtot, bool& ok) {
   return true;
 }
 
-// CholQR2 of the block X in double-float: on entry Xs holds X split (as
-// cgs2 leaves it); the Gram matrices and X R^{-1} run on the split rows, and
-// on exit X (FP64) and the split copy Vs_out (may be null) hold the factor Q.
-// Rtot (shared, 16) = R2 R1; false on breakdown or barrier failure (ok
-// distinguishes them).
-__device__ bool block_qr_df(Ctx& x, double* X, Row4s* Vs_out, double* Rtot, bool& ok) {
-  __shared__ double G[16], R[16], P[16];
+// y R = v for one split row and R with its diagonal inverted, split (Rh, Rl):
+// y_j = (v_j - sum_{k<j} y_k R_kj) / R_jj.
+__device__ __forceinline__ Row4s df_rinv(Row4s const& v, float const* Rh, float const* Rl) {
+  float yh[4] = {v.h.x, v.h.y, v.h.z, v.h.w}, yl[4] = {v.l.x, v.l.y, v.l.z, v.l.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+#pragma unroll
+    for (int k = 0; k < j; ++k) {
+      float ph, pl;
+      df_mul(yh[k], yl[k], Rh[k * 4 + j], Rl[k * 4 + j], ph, pl);
+      df_sub(yh[j], yl[j], ph, pl);
+    }
+    df_mul(yh[j], yl[j], Rh[j * 5], Rl[j * 5], yh[j], yl[j]);
+  }
+  Row4s o;
+  o.h = make_float4(yh[0], yh[1], yh[2], yh[3]);
+  o.l = make_float4(yl[0], yl[1], yl[2], yl[3]);
+  return o;
+}
+
+// CholQR2 in double-float of the block in Xs (split), whose Gram matrix G
+// (shared, 16, full) the last Gram-Schmidt sweep has left: one pass divides
+// by the first factor and sums the second Gram matrix, one divides by the
+// second and writes the split factor Vs_out. Rtot (shared, 16) = R2 R1; false
+// on breakdown or barrier failure (ok distinguishes them).
+__device__ bool block_qr_df(Ctx& x, double* G, Row4s* Vs_out, double* Rtot, bool& ok) {
+  __shared__ double R[16], P[16];
   __shared__ float Rh[16], Rl[16];
+  __shared__ int good;
   Row4s* Xs = reinterpret_cast<Row4s*>(x.c.Xs);
   ok = true;
   for (int pass = 0; pass < 2; ++pass) {
+    if (threadIdx.x == 0) {
+      good = chol4(G, R) ? 1 : 0;
+      if (good) {
+        // R's off-diagonal entries and the reciprocals of its diagonal, split
+        for (int i = 0; i < 16; ++i) {
+          double const v = (i % 5 == 0) ? 1.0 / R[i] : R[i];
+          df_split(v, Rh[i], Rl[i]);
+        }
+        if (pass == 0) {
+          for (int i = 0; i < 16; ++i) Rtot[i] = R[i];
+        } else {  // Rtot = R2 * R1
+          for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 4; ++j) {
+              double s = 0.0;
+              for (int k = 0; k < 4; ++k) s += R[i * 4 + k] * Rtot[k * 4 + j];
+              P[i * 4 + j] = s;
+            }
+          for (int i = 0; i < 16; ++i) Rtot[i] = P[i];
+        }
+      }
+    }
+    __syncthreads();
+    if (!good) return false;
+    if (pass == 1) break;
     float S[10] = {}, E[10] = {};
-    for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
-      Row4s const v = Xs[r];
+    for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+      uint64_t const r = x.row(l);
+      Row4s const v = df_rinv(Xs[r], Rh, Rl);
+      Xs[r] = v;
       float const ah[4] = {v.h.x, v.h.y, v.h.z, v.h.w}, al[4] = {v.l.x, v.l.y, v.l.z, v.l.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -387,66 +411,15 @@ __device__ bool block_qr_df(Ctx& x, double* X, Row4s* Vs_out, double* Rtot, bool
       ok = false;
       return false;
     }
-    if (threadIdx.x == 0) {
-      for (int i = 0; i < 4; ++i)
-        for (int j = i; j < 4; ++j) {
-          int const q = i * 4 - i * (i - 1) / 2 + (j - i);
-          G[i * 4 + j] = G[j * 4 + i] = x.tmp[16 + q];
-        }
-    }
-    __syncthreads();
-    __shared__ int good;
-    if (threadIdx.x == 0) {
-      good = chol4(G, R) ? 1 : 0;
-      if (good) {
-        // R's off-diagonal entries and the reciprocals of its diagonal, split
-        for (int i = 0; i < 16; ++i) {
-          double const v = (i % 5 == 0) ? 1.0 / R[i] : R[i];
-          df_split(v, Rh[i], Rl[i]);
-        }
-      }
-    }
-    __syncthreads();
-    if (!good) return false;
-    // X <- X R^{-1}: y_j = (x_j - sum_{k<j} y_k R_kj) / R_jj
-    for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
-      Row4s const v = Xs[r];
-      float yh[4] = {v.h.x, v.h.y, v.h.z, v.h.w}, yl[4] = {v.l.x, v.l.y, v.l.z, v.l.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-#pragma unroll
-        for (int k = 0; k < j; ++k) {
-          float ph, pl;
-          df_mul(yh[k], yl[k], Rh[k * 4 + j], Rl[k * 4 + j], ph, pl);
-          df_sub(yh[j], yl[j], ph, pl);
-        }
-        df_mul(yh[j], yl[j], Rh[j * 5], Rl[j * 5], yh[j], yl[j]);
-      }
-      Row4s o;
-      o.h = make_float4(yh[0], yh[1], yh[2], yh[3]);
-      o.l = make_float4(yl[0], yl[1], yl[2], yl[3]);
-      Xs[r] = o;
-    }
-    if (threadIdx.x == 0) {
-      if (pass == 0) {
-        for (int i = 0; i < 16; ++i) Rtot[i] = R[i];
-      } else {  // Rtot = R2 * R1
-        for (int i = 0; i < 4; ++i)
-          for (int j = 0; j < 4; ++j) {
-            double s = 0.0;
-            for (int k = 0; k < 4; ++k) s += R[i * 4 + k] * Rtot[k * 4 + j];
-            P[i * 4 + j] = s;
-          }
-        for (int i = 0; i < 16; ++i) Rtot[i] = P[i];
-      }
+    if (threadIdx.x < 16) {
+      int const i = min(threadIdx.x >> 2, threadIdx.x & 3), j = max(threadIdx.x >> 2, threadIdx.x & 3);
+      G[threadIdx.x] = x.tmp[16 + i * 4 - i * (i - 1) / 2 + (j - i)];
     }
     __syncthreads();
   }
-  for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
-    Row4s const w = Xs[r];
-    *reinterpret_cast<Row4*>(X + r * 4) = mk4((double)w.h.x + (double)w.l.x, (double)w.h.y + (double)w.l.y,
-                                              (double)w.h.z + (double)w.l.z, (double)w.h.w + (double)w.l.w);
-    if (Vs_out) Vs_out[r] = w;
+  for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+    uint64_t const r = x.row(l);
+    Vs_out[r] = df_rinv(Xs[r], Rh, Rl);
   }
   tc::fence_proxy_async_global();  // Vs_out is read by the row streams
   __syncthreads();
@@ -462,7 +435,8 @@ __device__ void block_spmv(Ctx& x, double const* X, double* W) {
   uint32_t const col_mask = S.col_bits < 32 ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
   bool const packed = x.c.packed != 0;
   double const* table = static_cast<double const*>(S.table);
-  for (uint64_t s = x.s0 + warp; s < x.s1; s += nw) {
+  for (uint32_t l = warp; l < x.ns; l += nw) {
+    uint64_t const s = x.slice(l);
     uint64_t const base = S.slice_ptr[s];
     uint32_t const width = (uint32_t)((S.slice_ptr[s + 1] - base) >> 5);
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
@@ -516,14 +490,13 @@ __device__ void block_spmv(Ctx& x, double const* X, double* W) {
 }
 
 // ------------------------------------------- Gram-Schmidt row streams ---
-// The Gram-Schmidt products read the CTA's own rows of split blocks (Vs, Xs)
-// in tiles of 2 blockDim rows, copied into the dynamic shared area by bulk
-// asynchronous copies (one thread issues them; mbarriers count their bytes)
-// a few tiles ahead of the arithmetic, so the loads' latency is hidden
-// behind the products instead of stalling each warp once per row. Waits are
-// bounded (copy_wait_ns): a copy that does not arrive sets the launch's error
-// flag; thread 0 then waits (bounded) for the CTA's copies still in flight
-// and the solve returns.
+// A sweep over the CTA's own rows reads a tile of rows of X and of the blocks
+// concerned (split: Xs, Vs) into the dynamic shared area by bulk asynchronous
+// copies (one thread issues them; an mbarrier per stage counts their bytes),
+// the next tile's while this one is worked on. Waits are bounded
+// (copy_wait_ns): a copy that does not arrive sets the launch's error flag;
+// thread 0 then waits (bounded) for the CTA's copies still in flight and the
+// solve returns.
 
 // Waits for stage barrier q (every thread) and flips its parity.
 __device__ bool gs_wait(Ctx& x, uint32_t q) {
@@ -547,105 +520,212 @@ __device__ bool gs_abort(Ctx& x, uint32_t failed, uint32_t pending) {
   return false;
 }
 
-// (S, E) += V_i^T X over own rows (both split): two stages, each a V tile
-// and an X tile.
-__device__ bool gs_dots(Ctx& x, Row4s const* Vi, Row4s const* Xs, float (&S)[16], float (&E)[16]) {
-  uint32_t const TR = 2 * blockDim.x;
-  uint64_t const r0 = x.r0, r1 = x.r1;
-  uint32_t const ntiles = (uint32_t)((r1 - r0 + TR - 1) / TR);
+// (S, E) with E folded into S again: |E| <= ulp(S) / 2.
+__device__ __forceinline__ void df_fold(float& S, float& E) {
+  float const s = __fadd_rn(S, E);
+  float const bb = __fsub_rn(s, S);
+  E = __fadd_rn(__fsub_rn(S, __fsub_rn(s, bb)), __fsub_rn(E, bb));
+  S = s;
+}
+
+// One sweep: X -= sum_{u0 <= i < nb} V_i C_i (u0 = nb: none), then with the
+// new X the products V_i^T X for d0 <= i < nb (d0 = nb: none) into
+// tmp[16 i ..] and, if `self`, X^T X into tmp[16 nb ..] (row-major 4 x 4, this
+// CTA's rows). C in double-float in shared memory (ch, cl) by quarters of 2 x 2
+// (coef_at).
+//
+// Update and products of a row tile share the tile, so that V is read once for
+// both and X goes over memory once per sweep. One stream per block and product,
+// which read X again for each, moved some 1340 bytes per row and step at nine
+// blocks and another 390 in the QR; this moves 800 and 160. The sweeps are
+// bound by issue: two CTAs of eight warps keep the FP32 pipe 60 % busy, waits
+// for copies are 2 % of their time.
+// `small`: the coefficients are below 2^-26 of X (cgs2), so that their products'
+// high parts suffice and the update is 16 FMAs per row and block instead of 192
+// operations.
+// In the update four lanes share a row, a 2 x 2 quarter of C each; in the
+// products sixteen lanes share one, a lane keeping one sum per block in
+// registers over all tiles: no tile-by-tile reductions, and every thread has
+// the same work whatever nb is. The error sums are folded every 7 rows, which
+// keeps their rounding below that of the shorter per-thread sums they replace.
+__device__ __forceinline__ uint32_t coef_at(uint32_t k) {  // entry k = 16 i + 4 s + t
+  uint32_t const s = (k >> 2) & 3u, t = k & 3u;
+  return (k & ~15u) | (s >> 1) << 3 | (t >> 1) << 2 | (s & 1u) << 1 | (t & 1u);
+}
+
+__device__ __forceinline__ bool gs_sweep(Ctx& x, uint32_t nb, uint32_t u0, uint32_t d0, bool self, bool small,
+                                         float const* ch, float const* cl) {
+  Row4s const* Vs = reinterpret_cast<Row4s const*>(x.c.Vs);
+  Row4s* Xs = reinterpret_cast<Row4s*>(x.c.Xs);
+  uint32_t const th = blockDim.x, b0 = min(u0, d0), nset = nb - b0 + 1, nd = nb - d0;
+  // rows of a tile: two tiles of nset arrays fit, whole rounds of the update's lanes
+  uint32_t const T = min(x.args->stage_bytes / (2 * nset * (uint32_t)sizeof(Row4s)), 512u) & ~3u;
+  uint64_t const D = x.c.D;
+  uint32_t const nt0 = (x.n0 + T - 1) / T, ntiles = nt0 + (x.n - x.n0 + T - 1) / T;
   Row4s* st = reinterpret_cast<Row4s*>(x.dyn);
-  auto rows_of = [&](uint32_t k) { return (uint32_t)min((uint64_t)TR, r1 - (r0 + (uint64_t)k * TR)); };
+  auto rows_of = [&](uint32_t k) { return k < nt0 ? min(T, x.n0 - k * T) : min(T, x.n - x.n0 - (k - nt0) * T); };
+  auto first_of = [&](uint32_t k) { return k < nt0 ? x.ra + (uint64_t)k * T : x.rb + (uint64_t)(k - nt0) * T; };
   auto issue = [&](uint32_t k) {
-    uint32_t const q = k & 1u, n = rows_of(k);
-    uint64_t const row = r0 + (uint64_t)k * TR;
-    tc::mbar_expect_tx(&x.gs_bar[q], 2 * n * (uint32_t)sizeof(Row4s));
-    tc::bulk_g2s(st + q * 2 * TR, Vi + row, n * (uint32_t)sizeof(Row4s), &x.gs_bar[q]);
-    tc::bulk_g2s(st + q * 2 * TR + TR, Xs + row, n * (uint32_t)sizeof(Row4s), &x.gs_bar[q]);
+    uint32_t const q = k & 1u, bytes = rows_of(k) * (uint32_t)sizeof(Row4s);
+    uint64_t const row = first_of(k);
+    Row4s* dst = st + (size_t)q * nset * T;
+    if (threadIdx.x == 0) tc::mbar_expect_tx(&x.gs_bar[q], nset * bytes);
+    for (uint32_t i = threadIdx.x >> 5; i < nset; i += th >> 5)
+      tc::bulk_g2s(dst + i * T, i ? Vs + (uint64_t)(b0 + i - 1) * D + row : Xs + row, bytes, &x.gs_bar[q]);
   };
+  float S[kMaxBlocks] = {}, E[kMaxBlocks] = {}, S2 = 0.0f, E2 = 0.0f;
+  uint32_t const ut = threadIdx.x & 3u, us = ut >> 1, uu = ut & 1u;                // update: rows s, columns t of C
+  uint32_t const pt = threadIdx.x & 3u, ps = (threadIdx.x >> 2) & 3u;              // products: columns of X and of V
+  uint32_t unfolded = 0;
   tc::fence_proxy_async_smem();  // this thread's shared-memory accesses before the copies' writes
   __syncthreads();               // the stages' previous readers are done
-  if (threadIdx.x == 0)
+  bool const issuer = (threadIdx.x & 31u) == 0;
+  if (issuer)
     for (uint32_t k = 0; k < 2 && k < ntiles; ++k) issue(k);
   for (uint32_t k = 0; k < ntiles; ++k) {
     uint32_t const q = k & 1u, n = rows_of(k);
     bool const ok = gs_wait(x, q);
-    if (ok) {
-      Row4s const* sv = st + q * 2 * TR;
-      for (uint32_t r = threadIdx.x; r < n; r += blockDim.x) df_dots(sv[r], sv[TR + r], S, E);
+    Row4s* sx = st + (size_t)q * nset * T;
+    uint64_t const row0 = first_of(k);
+    if (u0 < nb) {
+      if (ok) {
+        float4 const* c4h = reinterpret_cast<float4 const*>(ch) + us * 2 + uu;
+        float4 const* c4l = reinterpret_cast<float4 const*>(cl) + us * 2 + uu;
+        uint32_t const mask = 0xFu << (threadIdx.x & 28u);
+        uint32_t const col = 2 * uu + us;  // of the two columns, the one this lane finishes
+        auto update = [&](uint32_t r, auto rows) {
+          constexpr int R = decltype(rows)::value;  // rows r, r + th / 4
+          float Su[R][2] = {}, Eu[R][2] = {};
+          if (small) {
+#pragma unroll 4
+            for (uint32_t i = u0; i < nb; ++i) {
+              float4 const h = c4h[4 * i];
+              Row4s const* sv = sx + (i - b0 + 1) * T;
+#pragma unroll
+              for (int m = 0; m < R; ++m) {
+                float2 const a = *reinterpret_cast<float2 const*>(reinterpret_cast<float const*>(sv + r + m * (th / 4)) + 2 * us);
+                Su[m][0] = fmaf(a.x, h.x, fmaf(a.y, h.z, Su[m][0]));
+                Su[m][1] = fmaf(a.x, h.y, fmaf(a.y, h.w, Su[m][1]));
+              }
+            }
+          } else {
+#pragma unroll 1
+            for (uint32_t i = u0; i < nb; ++i) {
+              float4 const h = c4h[4 * i], l = c4l[4 * i];
+              Row4s const* sv = sx + (i - b0 + 1) * T;
+#pragma unroll
+              for (int m = 0; m < R; ++m) {
+                float const* row = reinterpret_cast<float const*>(sv + r + m * (th / 4)) + 2 * us;
+                float2 const ah = *reinterpret_cast<float2 const*>(row), al = *reinterpret_cast<float2 const*>(row + 4);
+                df_mac(ah.x, al.x, h.x, l.x, Su[m][0], Eu[m][0]);
+                df_mac(ah.x, al.x, h.y, l.y, Su[m][1], Eu[m][1]);
+                df_mac(ah.y, al.y, h.z, l.z, Su[m][0], Eu[m][0]);
+                df_mac(ah.y, al.y, h.w, l.w, Su[m][1], Eu[m][1]);
+              }
+            }
+          }
+#pragma unroll
+          for (int m = 0; m < R; ++m) {
+            // this lane's column: its own half of the sum over s and the partner's
+            float const mine = us ? Su[m][1] : Su[m][0], give = us ? Su[m][0] : Su[m][1];
+            float const mine_e = us ? Eu[m][1] : Eu[m][0], give_e = us ? Eu[m][0] : Eu[m][1];
+            float const other = __shfl_xor_sync(mask, give, 2), other_e = __shfl_xor_sync(mask, give_e, 2);
+            float const sum = __fadd_rn(mine, other);
+            float const bb = __fsub_rn(sum, mine);
+            float const err = __fadd_rn(__fsub_rn(mine, __fsub_rn(sum, bb)), __fsub_rn(other, bb));
+            uint32_t const rr = r + m * (th / 4);
+            float* px = reinterpret_cast<float*>(sx + rr) + col;
+            float h = px[0], l = px[4];
+            df_sub(h, l, sum, __fadd_rn(err, __fadd_rn(mine_e, other_e)));
+            px[0] = h;
+            px[4] = l;
+            float* gx = reinterpret_cast<float*>(Xs + row0 + rr) + col;
+            gx[0] = h;
+            gx[4] = l;
+          }
+        };
+        uint32_t r = threadIdx.x >> 2;
+        for (; r + th / 4 < n; r += th / 2) update(r, std::integral_constant<int, 2>{});
+        if (r < n) update(r, std::integral_constant<int, 1>{});
+      }
+      __syncthreads();
+    }
+    if (ok && (nd > 0 || self)) {
+      auto products = [&](uint32_t r, auto rows) {
+        constexpr int R = decltype(rows)::value;  // rows r, r + th / 16, ..
+        float wh[R], wl[R];
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+          float const* xr = reinterpret_cast<float const*>(sx + r + m * (th / 16));
+          wh[m] = xr[pt];
+          wl[m] = xr[4 + pt];
+          if (self) df_mac(xr[ps], xr[4 + ps], wh[m], wl[m], S2, E2);
+        }
+        float const* vr = reinterpret_cast<float const*>(sx + (d0 - b0 + 1) * T + r) + ps;
+#pragma unroll
+        for (uint32_t i = 0; i < (uint32_t)kMaxBlocks; ++i) {
+          if (i >= nd) break;
+#pragma unroll
+          for (int m = 0; m < R; ++m) df_mac(vr[m * (th / 2)], vr[m * (th / 2) + 4], wh[m], wl[m], S[i], E[i]);
+          vr += T * 8;
+        }
+        unfolded += R;
+        if (unfolded > 7 - R) {
+          unfolded = 0;
+#pragma unroll
+          for (uint32_t i = 0; i < (uint32_t)kMaxBlocks; ++i) {
+            if (i >= nd) break;
+            df_fold(S[i], E[i]);
+          }
+          df_fold(S2, E2);
+        }
+      };
+      uint32_t r = threadIdx.x >> 4;
+      for (; r + th / 16 < n; r += th / 8) products(r, std::integral_constant<int, 2>{});
+      if (r < n) products(r, std::integral_constant<int, 1>{});
     }
     tc::fence_proxy_async_smem();
     if (__syncthreads_or(!ok)) return gs_abort(x, q, (k + 1 < ntiles ? 1u << ((k + 1) & 1u) : 0u));
-    if (threadIdx.x == 0 && k + 2 < ntiles) issue(k + 2);
+    if (issuer && k + 2 < ntiles) issue(k + 2);
   }
-  return true;
-}
-
-// Xs -= sum_{i0 <= i < nb} V_i C_i over own rows, C_i in double-float in
-// shared memory (ch, cl: 16 per block); the V tiles stream through
-// kGsStages stages, every block of one row tile before the next tile.
-__device__ bool gs_update(Ctx& x, Row4s const* Vs, Row4s* Xs, uint32_t i0, uint32_t nb, float const* ch,
-                          float const* cl) {
-  uint32_t const TR = 2 * blockDim.x;
-  uint64_t const r0 = x.r0, r1 = x.r1, D = x.c.D;
-  uint32_t const ntiles = (uint32_t)((r1 - r0 + TR - 1) / TR);
-  uint32_t const nbb = nb - i0, items = ntiles * nbb;
-  Row4s* st = reinterpret_cast<Row4s*>(x.dyn);
-  auto rows_of = [&](uint32_t k) { return (uint32_t)min((uint64_t)TR, r1 - (r0 + (uint64_t)k * TR)); };
-  auto issue = [&](uint32_t m) {
-    uint32_t const k = m / nbb, i = i0 + m % nbb, q = m % kGsStages, n = rows_of(k);
-    tc::mbar_expect_tx(&x.gs_bar[q], n * (uint32_t)sizeof(Row4s));
-    tc::bulk_g2s(st + q * TR, Vs + (uint64_t)i * D + r0 + (uint64_t)k * TR, n * (uint32_t)sizeof(Row4s),
-                 &x.gs_bar[q]);
+  // sums over the row groups: lanes 16 apart, then the warps (in the free stages)
+  uint32_t const lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = th >> 5, K = 16 * (nd + (self ? 1 : 0));
+  double* red = x.dyn;
+  auto put = [&](uint32_t i, float Si, float Ei) {
+    double v = (double)Si + (double)Ei;
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    if (lane < 16) red[warp * K + 16 * i + ps * 4 + pt] = v;
   };
-  tc::fence_proxy_async_smem();
+#pragma unroll
+  for (uint32_t i = 0; i < (uint32_t)kMaxBlocks; ++i)
+    if (i < nd) put(i, S[i], E[i]);
+  if (self) put(nd, S2, E2);
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (uint32_t m = 0; m < (uint32_t)kGsStages && m < items; ++m) issue(m);
-  for (uint32_t k = 0; k < ntiles; ++k) {
-    uint32_t const n = rows_of(k);
-    uint32_t const ra = threadIdx.x, rb = threadIdx.x + blockDim.x;  // the thread's rows of the tile
-    float S0[4] = {}, E0[4] = {}, S1[4] = {}, E1[4] = {};
-    for (uint32_t ii = 0; ii < nbb; ++ii) {
-      uint32_t const m = k * nbb + ii, q = m % kGsStages;
-      bool const ok = gs_wait(x, q);
-      if (ok) {
-        Row4s const* sv = st + q * TR;
-        float4 const* c4h = reinterpret_cast<float4 const*>(ch + 16 * (i0 + ii));
-        float4 const* c4l = reinterpret_cast<float4 const*>(cl + 16 * (i0 + ii));
-        if (ra < n) df_axpy(sv[ra], c4h, c4l, S0, E0);
-        if (rb < n) df_axpy(sv[rb], c4h, c4l, S1, E1);
-      }
-      tc::fence_proxy_async_smem();
-      if (__syncthreads_or(!ok)) {
-        uint32_t pending = 0;
-        for (uint32_t p = m + 1; p < items && p < m + kGsStages; ++p) pending |= 1u << (p % kGsStages);
-        return gs_abort(x, q, pending);
-      }
-      if (threadIdx.x == 0 && m + kGsStages < items) issue(m + kGsStages);
-    }
-    uint64_t const row = r0 + (uint64_t)k * TR;
-    if (ra < n) df_sub_row(Xs[row + ra], S0, E0);
-    if (rb < n) df_sub_row(Xs[row + rb], S1, E1);
+  for (uint32_t e = threadIdx.x; e < K; e += th) {
+    double v = 0.0;
+    for (uint32_t w = 0; w < nw; ++w) v += red[w * K + e];
+    x.tmp[16 * d0 + e] = v;
   }
-  tc::fence_proxy_async_global();  // the next pass's streams read Xs
+  tc::fence_proxy_async_global();  // the next sweep's copies read Xs
   __syncthreads();
   return true;
 }
 
-// W = H V_j on own rows from the split copy of V_j (Vs block j, complete on
-// every CTA): each element's product t x_c is formed and summed in
+// Xs = H V_j (split) on own rows from the split copy of V_j (Vs block j,
+// complete on every CTA): each element's product t x_c is formed and summed in
 // double-float (df.cuh) with the split table, so the FP64 pipe only runs the
-// row epilogue y = d x + a / sqrt(S_i). Same gathers (one 32-byte row per
-// element) and slot scheme as block_spmv.
-__device__ void block_spmv_df(Ctx& x, uint32_t j, double* W) {
+// row epilogue y = d x + a / sqrt(S_i), floats widened on the integer pipe. Same
+// gathers (one 32-byte row per element) and slot scheme as block_spmv.
+__device__ void block_spmv_df(Ctx& x, uint32_t j) {
   StreamView const& S = x.c.S;
   uint32_t const lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   uint32_t const col_mask = S.col_bits < 32 ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
   bool const packed = x.c.packed != 0;
   float2 const* table = x.c.table_s;
-  Row4s const* Xs = reinterpret_cast<Row4s const*>(x.c.Vs) + (uint64_t)j * x.c.D;
-  double const* X = x.c.V + (uint64_t)j * x.c.D * 4;
-  for (uint64_t s = x.s0 + warp; s < x.s1; s += nw) {
+  Row4s const* Vj = reinterpret_cast<Row4s const*>(x.c.Vs) + (uint64_t)j * x.c.D;
+  Row4s* Xs = reinterpret_cast<Row4s*>(x.c.Xs);
+  for (uint32_t l = warp; l < x.ns; l += nw) {
+    uint64_t const s = x.slice(l);
     uint64_t const base = S.slice_ptr[s];
     uint32_t const width = (uint32_t)((S.slice_ptr[s + 1] - base) >> 5);
     float Sa[4] = {}, Ea[4] = {};
@@ -671,7 +751,7 @@ __device__ void block_spmv_df(Ctx& x, uint32_t j, double* W) {
           uint32_t const code =
               packed ? (v[u] >> S.col_bits) : (uint32_t)__ldcs(S.codes + base + lane + (uint64_t)(e0 + u) * 32);
           t[u] = __ldg(table + code);
-          float4 const* row = reinterpret_cast<float4 const*>(Xs + col);
+          float4 const* row = reinterpret_cast<float4 const*>(Vj + col);
           gh[u] = __ldcg(row);
           gl[u] = __ldcg(row + 1);
         } else {
@@ -694,146 +774,136 @@ __device__ void block_spmv_df(Ctx& x, uint32_t j, double* W) {
     if (i < x.c.D) {
       double const f = S.inv_sqrt_s[S.row_class[i]];
       double const dg = static_cast<double const*>(S.diag)[i];
-      Row4 const xi = ldcg4(X + i * 4);
-      *reinterpret_cast<Row4*>(W + i * 4) = mk4(fma(f, (double)Sa[0] + (double)Ea[0], dg * xi.x),
-                                                fma(f, (double)Sa[1] + (double)Ea[1], dg * xi.y),
-                                                fma(f, (double)Sa[2] + (double)Ea[2], dg * xi.z),
-                                                fma(f, (double)Sa[3] + (double)Ea[3], dg * xi.w));
+      float4 const* own = reinterpret_cast<float4 const*>(Vj + i);
+      float4 const vh = __ldcg(own), vl = __ldcg(own + 1);
+      auto row = [&](float S, float E, float h, float l) {
+        return fma(f, widen(S) + widen(E), dg * (widen(h) + widen(l)));
+      };
+      auto split = [](double y, float& h, float& l) {
+        h = __double2float_rn(y);
+        l = __double2float_rn(y - widen(h));
+      };
+      Row4s o;
+      split(row(Sa[0], Ea[0], vh.x, vl.x), o.h.x, o.l.x);
+      split(row(Sa[1], Ea[1], vh.y, vl.y), o.h.y, o.l.y);
+      split(row(Sa[2], Ea[2], vh.z, vl.z), o.h.z, o.l.z);
+      split(row(Sa[3], Ea[3], vh.w, vl.w), o.h.w, o.l.w);
+      Xs[i] = o;
     }
   }
+  tc::fence_proxy_async_global();  // the row streams read Xs
+  __syncthreads();
 }
 
-// X -= sum_{i<nb} V_i C_i (two passes of classical Gram-Schmidt). C (shared,
-// nb * 16, row-major a*4+c per block, may be null) receives the summed
-// coefficients; norms2 (shared, may be null) the squared column norms of X
+// X -= sum_{i<nb} V_i C_i (two passes of classical Gram-Schmidt) on the split
+// rows in Xs, in three sweeps: first products; first update and second
+// products; second update and the Gram matrix G (shared, 16) of the result. C
+// (shared, nb * 16, row-major a*4+c per block, may be null) receives the summed
+// coefficients. The second ones are rounding errors of the first pass, some
+// 1e-14 of X; where every column of them is below 2^-26 of the column of X they
+// are subtracted in single precision (an error of 2^-50 of X, under the split's
+// 2^-48), and the Gram matrix summed beside them stands for the updated X (they
+// change it by 2^-52): a sum over the group less; norms2 (shared; if `norms`) the squared column norms of X
 // before the projection. The first pass runs against blocks first .. nb-1
 // only (first > 0 where X = H V_{nb-1} is, in exact arithmetic, orthogonal
 // to the older blocks); the second pass always runs against all nb blocks.
-__device__ bool cgs2(Ctx& x, double* X, uint32_t nb, double* C, double* norms2, uint32_t first = 0) {
-  Row4s const* Vs = reinterpret_cast<Row4s const*>(x.c.Vs);
-  Row4s* Xs = reinterpret_cast<Row4s*>(x.c.Xs);
-  uint64_t const D = x.c.D;
-  int const K = (int)nb * 16;
-  if (C)
-    for (int k = threadIdx.x; k < K; k += blockDim.x) C[k] = 0.0;
-  for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x)
-    Xs[r] = split_row(*reinterpret_cast<Row4 const*>(X + r * 4));
-  tc::fence_proxy_async_global();  // the row streams read Xs through the async proxy
-  __syncthreads();
-  for (int pass = 0; pass < 2; ++pass) {
-    uint32_t const i0 = pass == 0 ? first : 0u;
-    for (uint32_t i = i0; i < nb; ++i) {
-      float S[16] = {}, E[16] = {};
-      if (!gs_dots(x, Vs + (uint64_t)i * D, Xs, S, E)) return false;
-      double p[16];
-#pragma unroll
-      for (int k = 0; k < 16; ++k) p[k] = (double)S[k] + (double)E[k];
-      cta_sum<16>(p, x.red, x.tmp + 16 * i);
+__device__ __forceinline__ bool cgs2(Ctx& x, uint32_t nb, double* C, bool norms, double* norms2, double* G,
+                                     uint32_t first) {
+  uint32_t const K = nb * 16;
+  double* tot = x.tmp + kPart;
+  // the coefficients in double-float, over this CTA's partial sums (no longer
+  // needed once group_sum has returned)
+  float* ch = reinterpret_cast<float*>(x.tmp);
+  float* cl = ch + K;
+  __shared__ bool small_s;
+  bool small = false;
+#pragma unroll 1
+  for (int sweep = 0; sweep < 3; ++sweep) {
+    uint32_t const u0 = sweep == 0 ? nb : sweep == 1 ? first : 0u, d0 = sweep == 0 ? first : sweep == 1 ? 0u : nb;
+    bool const self = sweep == 0 ? norms : sweep == 1 || !small;
+    if (!gs_sweep(x, nb, u0, d0, self, sweep == 2 && small, ch, cl)) return false;
+    if (sweep == 2 && small) return true;
+    uint32_t const from = 16 * d0;
+    if (!group_sum(x, x.tmp + from, (int)(K - from) + (self ? 16 : 0), tot + from)) return false;
+    if (sweep == 0 && norms && threadIdx.x < 4) norms2[threadIdx.x] = tot[K + 5 * threadIdx.x];
+    if (sweep < 2) {
+      if (C)
+        for (uint32_t k = threadIdx.x; k < K; k += blockDim.x)
+          C[k] = (sweep ? C[k] : 0.0) + (k >= from ? tot[k] : 0.0);
+      for (uint32_t k = from + threadIdx.x; k < K; k += blockDim.x) df_split(tot[k], ch[coef_at(k)], cl[coef_at(k)]);
     }
-    int Kp = K;
-    if (pass == 0 && norms2) {
-      double q[4] = {};
-      for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
-        Row4 const w = *reinterpret_cast<Row4 const*>(X + r * 4);
-        q[0] = fma(w.x, w.x, q[0]);
-        q[1] = fma(w.y, w.y, q[1]);
-        q[2] = fma(w.z, w.z, q[2]);
-        q[3] = fma(w.w, w.w, q[3]);
-      }
-      cta_sum<4>(q, x.red, x.tmp + K);
-      Kp = K + 4;
+    if (sweep > 0 && threadIdx.x < 16) G[threadIdx.x] = tot[K + threadIdx.x];
+    if (sweep == 1 && threadIdx.x < 32) {
+      uint32_t const t = threadIdx.x & 3u;
+      double q = 0.0;
+      for (uint32_t k = threadIdx.x; k < K; k += 32) q = fma(tot[k], tot[k], q);
+      for (int o = 4; o < 32; o <<= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+      bool const all = __all_sync(0xffffffffu, q <= 0x1p-52 * tot[K + 5 * t]);
+      if (threadIdx.x == 0) small_s = all;
     }
-    double* tot = x.tmp + kPart;
-    int const k0 = 16 * (int)i0;
-    if (!group_sum(x, x.tmp + k0, Kp - k0, tot + k0)) return false;
-    if (C)
-      for (int k = k0 + threadIdx.x; k < K; k += blockDim.x) C[k] += tot[k];
-    if (Kp > K && threadIdx.x < 4) norms2[threadIdx.x] = tot[K + threadIdx.x];
-    // the coefficients in double-float, over this CTA's partial sums (no
-    // longer needed once group_sum has returned)
-    float* ch = reinterpret_cast<float*>(x.tmp);
-    float* cl = ch + K;
-    for (int k = k0 + threadIdx.x; k < K; k += blockDim.x) df_split(tot[k], ch[k], cl[k]);
     __syncthreads();
-    // X -= sum_i V_i tot_i
-    if (!gs_update(x, Vs, Xs, i0, nb, ch, cl)) return false;
+    if (sweep == 1) small = small_s;
   }
-  for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
-    Row4s const w = Xs[r];
-    *reinterpret_cast<Row4*>(X + r * 4) = mk4((double)w.h.x + (double)w.l.x, (double)w.h.y + (double)w.l.y,
-                                              (double)w.h.z + (double)w.l.z, (double)w.h.w + (double)w.l.w);
-  }
-  __syncthreads();
   return true;
 }
 
-// Double-float copies (Vs) of basis blocks b0 .. b1, own rows.
-__device__ void split_blocks(Ctx& x, uint32_t b0, uint32_t b1) {
-  Row4s* Vs = reinterpret_cast<Row4s*>(x.c.Vs);
-  for (uint32_t b = b0; b <= b1; ++b)
-    for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x)
-      Vs[(uint64_t)b * x.c.D + r] = split_row(*reinterpret_cast<Row4 const*>(x.c.V + ((uint64_t)b * x.c.D + r) * 4));
+// dst = src split, own rows of one block.
+__device__ void split_block(Ctx& x, Row4s* dst, double const* src) {
+  for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+    uint64_t const r = x.row(l);
+    dst[r] = split_row(*reinterpret_cast<Row4 const*>(src + r * 4));
+  }
   tc::fence_proxy_async_global();
   __syncthreads();
 }
 
-// QR of the new Krylov block X (already projected against V_0 .. V_{nb-1})
-// with deflation: a column whose norm fell below 1e-10 of its norm before the
-// projection (norms2), or that is numerically dependent on the others, means
-// the block Krylov space lost a direction there (typically a converged Ritz
-// vector of the restart block). Such columns are replaced by random vectors,
-// projected against the basis, and the block is factored by CholQR2. Rb gets
-// R with the replaced columns zeroed (their coupling to H V_j is below the
-// threshold). Returns false on barrier failure or if the replacement fails.
-__device__ bool lanczos_qr(Ctx& x, double* X, uint32_t nb, double* norms2, double* Rb, uint32_t step,
-                           bool& replaced) {
-  __shared__ double R[16];
-  __shared__ int mask_s, total_mask_s;
-  if (threadIdx.x == 0) total_mask_s = 0;
-  __syncthreads();
-  for (int attempt = 0; attempt < 3; ++attempt) {
-    double g[4] = {};
-    for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
-      Row4 const v = *reinterpret_cast<Row4 const*>(X + r * 4);
-      g[0] = fma(v.x, v.x, g[0]);
-      g[1] = fma(v.y, v.y, g[1]);
-      g[2] = fma(v.z, v.z, g[2]);
-      g[3] = fma(v.w, v.w, g[3]);
-    }
-    cta_sum<4>(g, x.red, x.tmp);
-    if (!group_sum(x, x.tmp, 4, x.tmp + 16)) return false;
-    if (threadIdx.x == 0) {
-      int m = 0;
-      for (int c = 0; c < 4; ++c)
-        if (!(x.tmp[16 + c] > 1e-20 * norms2[c])) m |= 1 << c;
-      mask_s = m;
-      total_mask_s |= m;
-    }
-    __syncthreads();
-    int const m = mask_s;
+// Orthogonalises the new Krylov block in Xs: Gram-Schmidt against V_0 ..
+// V_{nb-1} (C: the coefficients, see cgs2) and QR into Vs block nb, with
+// deflation: a column whose norm fell below 1e-10 of its norm before the
+// projection, or that is numerically dependent on the others, means the block
+// Krylov space lost a direction there (typically a converged Ritz vector of the
+// restart block). Such columns are replaced by random vectors, projected
+// against the basis, and the block is factored by CholQR2. Rb gets R with the
+// replaced columns zeroed (their coupling to H V_j is below the threshold).
+// Returns false on barrier failure or if the replacement fails.
+template <class Lap>
+__device__ __forceinline__ bool lanczos_step(Ctx& x, uint32_t nb, double* C, double* Rb, uint32_t first, uint32_t step,
+                                             bool& replaced, Lap&& lap) {
+  __shared__ double R[16], G[16], norms2[4];
+  Row4s* Xs = reinterpret_cast<Row4s*>(x.c.Xs);
+  int total = 0;
+#pragma unroll 1
+  for (int attempt = 0;; ++attempt) {
+    if (!cgs2(x, nb, attempt ? nullptr : C, attempt == 0, norms2, G, attempt ? 0u : first)) return false;
+    int m = 0;
+    for (int c = 0; c < 4; ++c)
+      if (!(G[5 * c] > 1e-20 * norms2[c])) m |= 1 << c;
+    total |= m;
     if (m == 0) break;
     if (attempt == 2) return false;
-    for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
+    for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+      uint64_t const r = x.row(l);
       uint32_t cnt[4] = {(uint32_t)r, (uint32_t)(r >> 32), 0xDEF1u + step, (uint32_t)attempt};
       philox(cnt, (uint32_t)x.c.seed, (uint32_t)(x.c.seed >> 32));
-      double* row = X + r * 4;
+      float* row = reinterpret_cast<float*>(Xs + r);
       for (int c = 0; c < 4; ++c)
-        if (m & (1 << c)) row[c] = 2.0 * ((double)cnt[c] * (1.0 / 4294967296.0)) - 1.0;
+        if (m & (1 << c)) df_split(2.0 * ((double)cnt[c] * (1.0 / 4294967296.0)) - 1.0, row[c], row[4 + c]);
     }
+    tc::fence_proxy_async_global();
     __syncthreads();
     if (threadIdx.x < 4 && (m & (1 << threadIdx.x))) norms2[threadIdx.x] = (double)x.c.D;
     __syncthreads();
-    if (!cgs2(x, X, nb, nullptr, nullptr)) return false;
   }
+  lap(1);
   bool ok;
   // dependent columns that are not small: a breakdown
-  if (!block_qr_df(x, X, reinterpret_cast<Row4s*>(x.c.Vs) + (uint64_t)nb * x.c.D, R, ok)) return false;
+  if (!block_qr_df(x, G, reinterpret_cast<Row4s*>(x.c.Vs) + (uint64_t)nb * x.c.D, R, ok)) return false;
   if (threadIdx.x < 16) {
     int const col = threadIdx.x & 3;
-    Rb[threadIdx.x] = (total_mask_s & (1 << col)) ? 0.0 : R[threadIdx.x];
+    Rb[threadIdx.x] = (total & (1 << col)) ? 0.0 : R[threadIdx.x];
   }
   __syncthreads();
-  replaced = total_mask_s != 0;
+  replaced = total != 0;
   return true;
 }
 
@@ -1004,7 +1074,8 @@ __device__ void ritz_vectors(Ctx& x, uint32_t j, double* Ys, bool both) {
   Row4s const* Vs = reinterpret_cast<Row4s const*>(x.c.Vs);
   for (int half = 0; half < (both ? 2 : 1); ++half) {
     double* out = half ? x.c.W2 : x.c.W;
-    for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
+    for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+      uint64_t const r = x.row(l);
       float S[4] = {}, E[4] = {};
       for (int b = 0; b <= (int)j; ++b) {
         Row4s const a = Vs[(uint64_t)b * D + r];
@@ -1024,13 +1095,16 @@ __device__ void ritz_vectors(Ctx& x, uint32_t j, double* Ys, bool both) {
 }
 
 __device__ void copy_block(Ctx& x, double* dst, double const* src) {
-  for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x)
+  for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+    uint64_t const r = x.row(l);
     *reinterpret_cast<Row4*>(dst + r * 4) = *reinterpret_cast<Row4 const*>(src + r * 4);
+  }
   __syncthreads();
 }
 
 __device__ void random_block(Ctx& x) {
-  for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
+  for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+    uint64_t const r = x.row(l);
     uint32_t c[4] = {(uint32_t)r, (uint32_t)(r >> 32), 0xB10Cu, 0u};
     philox(c, (uint32_t)x.c.seed, (uint32_t)(x.c.seed >> 32));
     double v[4];
@@ -1048,14 +1122,21 @@ __device__ void random_block(Ctx& x) {
 __device__ void solve_chain(ChainDesc const& c, uint32_t rank, uint32_t ncta, uint32_t* bar, BatchArgs const& a,
                             double* red, double* tmp, double* C, double* A, double* Q, uint64_t* gs_bar,
                             uint32_t* gs_phase) {
-  Ctx x{c, rank, ncta, bar, &a, 0, 0, 0, 0, 0, red, tmp, A, gs_bar, gs_phase};
-  x.s0 = c.n_slices * rank / ncta;
-  x.s1 = c.n_slices * (rank + 1) / ncta;
-  x.r0 = std::min<uint64_t>(c.D, x.s0 * 32);
-  x.r1 = std::min<uint64_t>(c.D, x.s1 * 32);
+  Ctx x{c, rank, ncta, bar, &a, 0, 0, 0, 0, 0, 0, 0, 0, 0, red, tmp, A, gs_bar, gs_phase};
+  auto piece = [&](uint32_t q) { return c.n_slices * q / (2 * ncta); };
+  x.sa = piece(rank);
+  x.sb = piece(2 * ncta - 1 - rank);
+  x.ns0 = (uint32_t)(piece(rank + 1) - x.sa);
+  x.ns = x.ns0 + (uint32_t)(piece(2 * ncta - rank) - x.sb);
+  auto row_of = [&](uint64_t s) { return std::min<uint64_t>(c.D, s * 32); };
+  x.ra = row_of(x.sa);
+  x.rb = row_of(x.sb);
+  x.n0 = (uint32_t)(row_of(x.sa + x.ns0) - x.ra);
+  x.n = x.n0 + (uint32_t)(row_of(x.sb + (x.ns - x.ns0)) - x.rb);
   bool const leader = rank == 0;
   constexpr int kStride = kMaxN * 4;
-  __shared__ double Rb[16], norms2[4];
+  __shared__ double Rb[16];
+  Row4s* Vs = reinterpret_cast<Row4s*>(c.Vs);
   uint32_t steps = 0, restarts = 0, matvecs = 0, status = 2;
   double const tol = a.tol;
   // phase timers, kept by thread 0 in shared memory (no registers held
@@ -1087,26 +1168,20 @@ __device__ void solve_chain(ChainDesc const& c, uint32_t rank, uint32_t ncta, ui
     uint32_t full_from = j0;
     bool broke = false;
     for (;; ++j) {
-      double* Vj = c.V + (uint64_t)j * c.D * 4;
-      if (j == j0) split_blocks(x, 0u, j0);  // later blocks come split from the QR of each step
+      if (j == 0) split_block(x, Vs, c.V);  // later blocks come split from the QR of each step or the restart
       if (!group_barrier(bar, ncta, a)) return;  // V_j complete on every CTA before the gathers
       lap(4);
-      block_spmv_df(x, j, c.W);
+      block_spmv_df(x, j);
       ++matvecs;
-      __syncthreads();
       lap(0);
-      if (!cgs2(x, c.W, j + 1, C, norms2, j > full_from ? j - 1 : 0u)) return;
-      lap(1);
-      if (leader)
-        for (int k = threadIdx.x; k < 16 * (int)(j + 1); k += blockDim.x) c.Tc[j * kStride + k] = C[k];
-      ++steps;
-      // QR of W -> V_{j+1}, B_j (with deflation of lost directions)
-      double* Vn = c.V + (uint64_t)(j + 1) * c.D * 4;
-      copy_block(x, Vn, c.W);
+      // Gram-Schmidt and QR -> V_{j+1}, B_j (with deflation of lost directions)
       bool replaced = false;
-      broke = !lanczos_qr(x, Vn, j + 1, norms2, Rb, steps, replaced);
+      broke = !lanczos_step(x, j + 1, C, Rb, j > full_from ? j - 1 : 0u, steps + 1, replaced, lap);
+      ++steps;
       if (replaced) full_from = j + 1;
       if (*(volatile int*)a.error) return;
+      if (leader)
+        for (int k = threadIdx.x; k < 16 * (int)(j + 1); k += blockDim.x) c.Tc[j * kStride + k] = C[k];
       if (leader)
         for (int k = threadIdx.x; k < 16; k += blockDim.x) c.Bblk[j * 16 + k] = broke ? 0.0 : Rb[k];
       lap(2);
@@ -1129,9 +1204,16 @@ __device__ void solve_chain(ChainDesc const& c, uint32_t rank, uint32_t ncta, ui
     bool const thick = !broke && j >= 1 && c.m_blocks >= 3;
     ritz_vectors(x, j, A, thick);  // A: the dynamic shared area, free outside the Jacobi solve
     if (!group_barrier(bar, ncta, a)) return;  // every CTA done reading the old basis
-    if (thick && j + 1 != 2) copy_block(x, c.V + 2 * c.D * 4, c.V + (uint64_t)(j + 1) * c.D * 4);
+    if (thick) {  // Vs: the Ritz vectors, then the last Lanczos block
+      if (j + 1 != 2)
+        for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+          uint64_t const r = x.row(l);
+          Vs[2 * c.D + r] = Vs[(uint64_t)(j + 1) * c.D + r];
+        }
+      split_block(x, Vs, c.W);
+      split_block(x, Vs + c.D, c.W2);
+    }
     copy_block(x, c.V, c.W);
-    if (thick) copy_block(x, c.V + c.D * 4, c.W2);
     if (!group_barrier(bar, ncta, a)) return;  // Psi rows visible to every CTA's SpMV gathers
     lap(4);
     // true residuals of the lowest four Ritz pairs
@@ -1142,7 +1224,8 @@ __device__ void solve_chain(ChainDesc const& c, uint32_t rank, uint32_t ncta, ui
     for (int i = 0; i < 8; ++i) th[i] = ldcg(c.out + i);
     {
       double p[4] = {};
-      for (uint64_t r = x.r0 + threadIdx.x; r < x.r1; r += blockDim.x) {
+      for (uint32_t l = threadIdx.x; l < x.n; l += blockDim.x) {
+        uint64_t const r = x.row(l);
         Row4 const w = *reinterpret_cast<Row4 const*>(c.W + r * 4);
         Row4 const v = *reinterpret_cast<Row4 const*>(c.V + r * 4);
         double const d[4] = {w.x - th[0] * v.x, w.y - th[1] * v.y, w.z - th[2] * v.z, w.w - th[3] * v.w};
@@ -1367,6 +1450,10 @@ std::atomic<unsigned> g_force_threads{0}, g_force_per_sm{0};
 std::mutex g_tune_mu;
 std::map<std::tuple<int, unsigned, uint64_t>, Plan> g_tuned;
 
+// Dynamic shared memory: the Rayleigh-Ritz solve's two matrices, or the row
+// streams' stages. Not more: with 96 KB per CTA for wider stages the gathers in
+// flight had too little of the 256 KB left as L1, and the SpMV took twice as
+// long (870 -> 1385 ms for the 128-chain batch).
 size_t dyn_smem() { return 2 * (size_t)kMaxN * kMaxN * sizeof(double); }
 
 }  // namespace
@@ -1452,7 +1539,7 @@ int sed_eigh_batched(unsigned count, ls_operator* const ops[], sed_eigh_options 
     uint32_t m = std::min<uint32_t>(std::min<uint32_t>(m_req, kMaxBlocks), (uint32_t)std::min<uint64_t>(kMaxBlocks, D / kB - 1));
     m = std::max<uint32_t>(m, 1);
     m_blocks[i] = m;
-    off_V[i] = take((size_t)(m + 1) * D * kB * 8);
+    off_V[i] = take((size_t)D * kB * 8);
     off_Vs[i] = take((size_t)(m + 1) * D * kB * 8);  // Row4s: 8 floats a row
     off_Xs[i] = take((size_t)D * kB * 8);
     off_Ts[i] = take((size_t)std::max<uint32_t>(1, od[i]->tables->n_codes) * sizeof(float2));
@@ -1582,6 +1669,7 @@ int sed_eigh_batched(unsigned count, ls_operator* const ops[], sed_eigh_options 
     a.error = reinterpret_cast<int*>(base + off_err);
     a.wait_ns = device_wait_ns(kBarrierNs);
     a.copy_wait_ns = device_wait_ns(kGsWaitNs);
+    a.stage_bytes = (uint32_t)dyn_smem();
     a.extra_arrivals = g_barrier_extra_arrivals.load();
     cudaEvent_t e0, e1;
     SED_TRY_CUDA(cudaEventCreate(&e0));

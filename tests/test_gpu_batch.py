@@ -113,3 +113,27 @@ def test_fixed_launch_shapes_agree(sed, oracle, threads, per_sm):
         want = np.linalg.eigvalsh(oop.dense().real)[:4]
         np.testing.assert_allclose(res.eigenvalues[i], want, rtol=EV_RTOL, atol=0)
         assert np.all(res.residuals[i] <= RES_TOL)
+
+
+@pytest.mark.parametrize("threads,per_sm", [(128, 1), (256, 2)])
+def test_lost_directions_and_smallest_sizes(sed, oracle, threads, per_sm):
+    """Rings whose Krylov spaces end within a cycle (D from 13 up, some columns
+    of a block vanish and are replaced, so the second Gram-Schmidt
+    coefficients are not small), single-slice problems, and one that spreads
+    over more CTAs than it has slices. The pairs are held to the solver's own
+    residual bound, 1e-8, and the energies to its square over the gap."""
+    from spined import _lib as L
+    lib = L.load()
+    models = [lattices.heisenberg_chain(10), lattices.heisenberg_chain(10, parity=None, spin_inversion=None),
+              lattices.heisenberg_chain(12), lattices.heisenberg_chain(12, parity=None), lattices.heisenberg_chain(20)]
+    pairs = [both(sed, oracle, m) for m in models]
+    try:
+        lib.sed_set_batched_launch(threads, per_sm)
+        res = sed.eigh_batched([b.hamiltonian for b, _, _ in pairs], nev=2)
+    finally:
+        lib.sed_set_batched_launch(0, 0)
+    for i, (b, ob, oop) in enumerate(pairs):
+        A = oop.dense().real
+        np.testing.assert_allclose(res.eigenvalues[i], np.linalg.eigvalsh(A)[:2], rtol=EV_RTOL, atol=0)
+        assert np.all(res.residuals[i] <= RES_TOL)
+        _check_pairs(oop, res.eigenvalues[i], res.eigenvectors[i])
