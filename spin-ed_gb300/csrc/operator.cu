@@ -2207,7 +2207,7 @@ int sed_operator_prepare(ls_operator* op, int form) {
   d.form = form;
   if (form == SED_FORM_ON_THE_FLY) return LS_SUCCESS;
   int st = operator_record_stream(d, d.cuda_stream);
-  if (!st && cplx_sums(d)) (void)fix_reserve(d, 2);  // without it the matvecs take the general kernel
+  if (!st && cplx_sums(d, 2, 1)) (void)fix_reserve(d, 2);  // without it the matvecs take the general kernel
   return (form == SED_FORM_AUTO && st == LS_OUT_OF_MEMORY) ? LS_SUCCESS : st;
 }
 

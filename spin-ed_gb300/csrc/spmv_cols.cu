@@ -434,11 +434,17 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
 
 }  // namespace
 
-// From 2^21 elements on: below, the two launches more cost what the sums save
-// (complex128 call, general kernel and this one: 1.4 M elements 45 and 46 us,
-// 2.7 M 56 and 53, 10.4 M 123 and 85, 20.8 M 198 and 109).
-bool cplx_sums(OperatorData const& op) {
-  return op.tables->cplx_ok && op.stream.n_elements >= ((uint64_t)1 << 21);
+// Below these sizes the two launches more per column cost what the sums save.
+// The general kernel's pass over a block reads the entries once for up to 16
+// columns (its FP64 arithmetic is per column), so a wide complex128 block needs
+// more elements. Calls in us, general kernels and this one:
+//   complex64, 1 / 7 / 16 columns:  0.7 M elements 35 / 142 / 280 and 34 / 159 / 346,
+//     1.4 M 47 / 227 / 465 and 37 / 175 / 378
+//   complex128:  1.4 M 38 / 151 / 293 and 36 / 167 / 362,
+//     2.7 M 50 / 248 / 484 and 44 / 236 / 528,  5.4 M 74 / 401 / 803 and 52 / 304 / 681
+bool cplx_sums(OperatorData const& op, int dtype, uint64_t block) {
+  unsigned const bits = dtype == 2 ? 20 : block < 8 ? 21 : 22;
+  return op.tables->cplx_ok && op.stream.n_elements >= ((uint64_t)1 << bits);
 }
 
 // Whether vectors of this dtype go through launch_fix_cols. FP64 columns
@@ -451,7 +457,7 @@ bool cplx_sums(OperatorData const& op) {
 bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_stream, cudaStream_t stream) {
   if (!use_stream) return false;
   if (op.tables->cplx_ok) {
-    if (dtype < 2 || !cplx_sums(op)) return false;
+    if (dtype < 2 || !cplx_sums(op, dtype, block)) return false;
   } else {
     if (!op.tables->fix_ok || op.fix_cols < 1) return false;
     if (dtype == 1) return true;

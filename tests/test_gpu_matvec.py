@@ -367,7 +367,7 @@ def test_narrower_passes_when_the_workspace_is_capped(sed, oracle):
     assert all(torch.equal(y[:, c], columns[c]) for c in range(16))
 
 
-# complex operators of 2^21 elements or more: the integer sums of k_spmv_cplx
+# complex operators of 2^20 (complex64) or 2^21 elements or more: the integer sums of k_spmv_cplx
 def _dense_complex(n):
     rng = np.random.default_rng(11)
     bonds = lattices.chain_bonds(n, 1)
