@@ -907,12 +907,20 @@ __device__ __forceinline__ bool lanczos_step(Ctx& x, uint32_t nb, double* C, dou
   return true;
 }
 
-// Cyclic Jacobi on the symmetric n x n matrix A (shared, row-major, n even)
-// with parallel round-robin rotations and a threshold: a rotation whose
+// Cyclic Jacobi on the symmetric n x n matrix A (shared, row-major with rows of
+// n + 1, n a multiple of 4) with parallel round-robin rotations and a threshold: a rotation whose
 // off-diagonal entry is at most 1e-16 of ||A||_F (invariant under the
 // rotations) is skipped, and the sweeps end when one performs none (the
-// eigenvalues then carry errors of order 1e-32 ||A||^2 / gap). Q (shared)
-// receives the eigenvectors as columns. Eigenvalues end on the diagonal of A.
+// eigenvalues then carry errors of order 1e-32 ||A||^2 / gap). Q (shared, rows
+// of n) receives the eigenvectors as rows. Eigenvalues end on the diagonal of A.
+//
+// The FP64 pipe bounds it. A round rotates rows and columns in one go, a 2 x 2
+// block of A per thread (a row pair and a column pair), blocks above the
+// diagonal only and mirrored: 2 n^2 operations instead of the 4 n^2 of a pass
+// over all rows and one over all columns, and one barrier less. With rows of
+// n + 1, and the eigenvectors as rows, lanes fall into different banks. The
+// slowest of 128 J1-J2 chains (16 to 28 sites): 59 -> 42 ms; a batch of 123
+// chains of 14 to 24 sites, where this solve weighs most: 98 -> 80 ms a call.
 __device__ void jacobi(double* A, double* Q, int n) {
   __shared__ double cs[kMaxN / 2][2];
   __shared__ int pp[kMaxN / 2][2];
@@ -920,10 +928,24 @@ __device__ void jacobi(double* A, double* Q, int n) {
   __shared__ double thr;
   __shared__ int rotated;
   double f = 0.0;
+  int const ld = n + 1, half = n / 2;
   for (int k = threadIdx.x; k < n * n; k += blockDim.x) {
-    Q[k] = (k / n == k % n) ? 1.0 : 0.0;
-    f = fma(A[k], A[k], f);
+    int const r = k / n, c = k % n;
+    Q[k] = r == c ? 1.0 : 0.0;
+    f = fma(A[r * ld + c], A[r * ld + c], f);
   }
+  // this thread's blocks (k1 <= k2) of the half (half + 1) / 2: rows k and
+  // half - 1 - k of the triangle side by side, half + 1 blocks
+  constexpr int kMine = 5;  // 528 blocks at n = 64 on 128 threads
+  int mine[kMine];
+#pragma unroll
+  for (int m = 0; m < kMine; ++m) {
+    int const e = (int)threadIdx.x + m * (int)blockDim.x, row = e / (half + 1), col = e % (half + 1);
+    mine[m] = row >= half / 2 ? -1
+              : col < half - row ? row << 8 | (row + col)
+                                 : (half - 1 - row) << 8 | (half - 1 - row + col - (half - row));
+  }
+  uint32_t const inv_n = ((1u << 20) + (uint32_t)n - 1) / (uint32_t)n;  // e / n = e inv_n >> 20 for e < 2048
   for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
   if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = f;
   __syncthreads();
@@ -934,7 +956,6 @@ __device__ void jacobi(double* A, double* Q, int n) {
     rotated = 0;
   }
   __syncthreads();
-  int const half = n / 2;
   for (int sweep = 0; sweep < 40; ++sweep) {
     for (int round = 0; round < n - 1; ++round) {
       // round-robin pairing: player 0 fixed, the others rotate
@@ -947,11 +968,11 @@ __device__ void jacobi(double* A, double* Q, int n) {
           p = q;
           q = t;
         }
-        double const apq = A[p * n + q];
+        double const apq = A[p * ld + q];
         double c = 1.0, s = 0.0;
         if (fabs(apq) > thr) {
           // tan of the angle: the smaller root of t^2 + 2 tau t - 1 = 0
-          double const tau = (A[q * n + q] - A[p * n + p]) / (2.0 * apq);
+          double const tau = (A[q * ld + q] - A[p * ld + p]) / (2.0 * apq);
           double const t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(fma(tau, tau, 1.0)));
           c = rsqrt(fma(t, t, 1.0));
           s = t * c;
@@ -963,31 +984,41 @@ __device__ void jacobi(double* A, double* Q, int n) {
         pp[k][1] = q;
       }
       __syncthreads();
-      // rows: A <- J^T A
-      for (int e = threadIdx.x; e < half * n; e += blockDim.x) {
-        int const k = e / n, col = e % n;
-        double const s = cs[k][1];
-        if (s == 0.0) continue;
-        int const p = pp[k][0], q = pp[k][1];
-        double const c = cs[k][0];
-        double const ap = A[p * n + col], aq = A[q * n + col];
-        A[p * n + col] = c * ap - s * aq;
-        A[q * n + col] = s * ap + c * aq;
+      // A <- J^T A J
+#pragma unroll
+      for (int m = 0; m < kMine; ++m) {
+        if (mine[m] < 0) continue;
+        int const k1 = mine[m] >> 8, k2 = mine[m] & 255;
+        double const c1 = cs[k1][0], s1 = cs[k1][1], c2 = cs[k2][0], s2 = cs[k2][1];
+        if (s1 == 0.0 && s2 == 0.0) continue;
+        int const p1 = pp[k1][0], q1 = pp[k1][1], p2 = pp[k2][0], q2 = pp[k2][1];
+        double const app = A[p1 * ld + p2], apq = A[p1 * ld + q2], aqp = A[q1 * ld + p2], aqq = A[q1 * ld + q2];
+        double const rpp = c1 * app - s1 * aqp, rqp = s1 * app + c1 * aqp;
+        double const rpq = c1 * apq - s1 * aqq, rqq = s1 * apq + c1 * aqq;
+        double const bpp = c2 * rpp - s2 * rpq, bpq = s2 * rpp + c2 * rpq;
+        double const bqp = c2 * rqp - s2 * rqq, bqq = s2 * rqp + c2 * rqq;
+        A[p1 * ld + p2] = bpp;
+        A[p1 * ld + q2] = bpq;
+        A[q1 * ld + p2] = bqp;
+        A[q1 * ld + q2] = bqq;
+        if (k1 != k2) {
+          A[p2 * ld + p1] = bpp;
+          A[q2 * ld + p1] = bpq;
+          A[p2 * ld + q1] = bqp;
+          A[q2 * ld + q1] = bqq;
+        }
       }
-      __syncthreads();
-      // columns: A <- A J, Q <- Q J
-      for (int e = threadIdx.x; e < half * n; e += blockDim.x) {
-        int const k = e / n, row = e % n;
+      // Q <- J^T Q
+      for (uint32_t e = threadIdx.x; e < (uint32_t)(half * n); e += blockDim.x) {
+        uint32_t const k = e * inv_n >> 20, col = e - k * (uint32_t)n;
         double const s = cs[k][1];
         if (s == 0.0) continue;
-        int const p = pp[k][0], q = pp[k][1];
         double const c = cs[k][0];
-        double const ap = A[row * n + p], aq = A[row * n + q];
-        A[row * n + p] = c * ap - s * aq;
-        A[row * n + q] = s * ap + c * aq;
-        double const qp = Q[row * n + p], qq = Q[row * n + q];
-        Q[row * n + p] = c * qp - s * qq;
-        Q[row * n + q] = s * qp + c * qq;
+        double* qp = Q + pp[k][0] * n + col;
+        double* qq = Q + pp[k][1] * n + col;
+        double const vp = *qp, vq = *qq;
+        *qp = c * vp - s * vq;
+        *qq = s * vp + c * vq;
       }
       __syncthreads();
     }
@@ -1018,7 +1049,7 @@ __device__ double rayleigh_ritz(ChainDesc const& c, uint32_t j, bool have_B, dou
       v = ldcg(c.Tc + bq * kStride + br * 16 + a * 4 + b);
     else
       v = ldcg(c.Tc + br * kStride + bq * 16 + b * 4 + a);
-    A[e] = v;
+    A[r * (n + 1) + q] = v;
   }
   __syncthreads();
   jacobi(A, Q, n);
@@ -1031,10 +1062,10 @@ __device__ double rayleigh_ritz(ChainDesc const& c, uint32_t j, bool have_B, dou
     for (int i = 0; i < nk; ++i) {
       int best = -1;
       for (int q = 0; q < n; ++q)
-        if (!used[q] && (best < 0 || A[q * n + q] < A[best * n + best])) best = q;
+        if (!used[q] && (best < 0 || A[q * (n + 1) + q] < A[best * (n + 1) + best])) best = q;
       used[best] = true;
       idx[i] = best;
-      c.out[i] = A[best * n + best];
+      c.out[i] = A[best * (n + 1) + best];
     }
     worst = 0.0;
     for (int i = 0; i < kB; ++i) {
@@ -1042,7 +1073,7 @@ __device__ double rayleigh_ritz(ChainDesc const& c, uint32_t j, bool have_B, dou
       if (have_B) {
         for (int a = 0; a < 4; ++a) {
           double s = 0.0;
-          for (int b = 0; b < 4; ++b) s += ldcg(c.Bblk + j * 16 + a * 4 + b) * Q[(4 * (int)j + b) * n + idx[i]];
+          for (int b = 0; b < 4; ++b) s += ldcg(c.Bblk + j * 16 + a * 4 + b) * Q[idx[i] * n + 4 * (int)j + b];
           r2 += s * s;
         }
       }
@@ -1053,7 +1084,7 @@ __device__ double rayleigh_ritz(ChainDesc const& c, uint32_t j, bool have_B, dou
   __syncthreads();
   for (int e = threadIdx.x; e < n * 8; e += blockDim.x) {
     int const q = e / 8, i = e % 8;
-    c.Y[q * 8 + i] = i < nk ? Q[q * n + idx[i]] : 0.0;
+    c.Y[q * 8 + i] = i < nk ? Q[idx[i] * n + q] : 0.0;
   }
   __syncthreads();
   return worst;
@@ -1281,7 +1312,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_lanczos(BatchArgs a) {
   __shared__ double red[8 * 16];
   __shared__ __align__(16) double tmp[2 * kPart];  // also read as float4 (split Gram-Schmidt coefficients)
   __shared__ double C[kPart];
-  extern __shared__ __align__(128) double dyn[];  // A [kMaxN^2], Q [kMaxN^2] (leader work); row-stream stages
+  extern __shared__ __align__(128) double dyn[];  // A [kMaxN][kMaxN + 1], Q [kMaxN^2] (leader work); row-stream stages
   __shared__ uint64_t gs_bar[kGsStages];
   uint32_t gs_phase = 0;
   if (threadIdx.x == 0) {
@@ -1294,7 +1325,7 @@ __global__ void __launch_bounds__(256, 2) k_batch_lanczos(BatchArgs a) {
   uint32_t const rank = blockIdx.x - g.cta0;
   for (uint32_t q = 0; q < g.count; ++q) {
     ChainDesc const& c = a.chains[a.order[g.first + q]];
-    solve_chain(c, rank, g.ncta, g.bar, a, red, tmp, C, dyn, dyn + kMaxN * kMaxN, gs_bar, &gs_phase);
+    solve_chain(c, rank, g.ncta, g.bar, a, red, tmp, C, dyn, dyn + kMaxN * (kMaxN + 1), gs_bar, &gs_phase);
     if (*(volatile int*)a.error) return;
     if (!group_barrier(g.bar, g.ncta, a)) return;
   }
@@ -1454,7 +1485,7 @@ std::map<std::tuple<int, unsigned, uint64_t>, Plan> g_tuned;
 // streams' stages. Not more: with 96 KB per CTA for wider stages the gathers in
 // flight had too little of the 256 KB left as L1, and the SpMV took twice as
 // long (870 -> 1385 ms for the 128-chain batch).
-size_t dyn_smem() { return 2 * (size_t)kMaxN * kMaxN * sizeof(double); }
+size_t dyn_smem() { return (size_t)kMaxN * (2 * kMaxN + 1) * sizeof(double); }
 
 }  // namespace
 }  // namespace sed
