@@ -18,7 +18,8 @@
 //   W = H V_j ; C_i = V_i^T W, W -= V_i C_i for i <= j      (CGS2, two passes)
 //   W = V_{j+1} B_j                                          (CholQR2)
 //   T: diagonal blocks A_j = sym(C_j), sub-diagonal blocks B_j
-// Every `rr_every` steps (and at the end of a cycle) the group's first CTA
+// Every `rr_every` steps of a cycle that may converge, and at the end of each,
+// the group's first CTA
 // diagonalises T (cyclic Jacobi with parallel round-robin rotations in shared
 // memory) and estimates the Ritz residuals ||B_j y_last||; the cycle ends when
 // all nev estimates are below tol / 2 or the basis is full. Ritz vectors
@@ -1191,6 +1192,13 @@ __device__ void solve_chain(ChainDesc const& c, uint32_t rank, uint32_t ncta, ui
     status = 3;
   }
   uint32_t j0 = 0;
+  // Whether a cycle may end before its basis is full: not while the last true
+  // residual is above 1000 tol, since a whole cycle of ten block steps gains
+  // a factor of 6 to 100 (the chains of 12 to 28 sites), and the solves of T
+  // in between keep the group waiting for its first CTA. Same step counts and
+  // eigenvalues; 46 chains of 12 to 20 sites 28.5 -> 24.0 ms a call, 128 of 16
+  // to 28 696 -> 686.
+  bool near = true;
   while (status != 3) {
     uint32_t j = j0;
     // block whose H-image needs full projections in both passes: the
@@ -1217,7 +1225,7 @@ __device__ void solve_chain(ChainDesc const& c, uint32_t rank, uint32_t ncta, ui
         for (int k = threadIdx.x; k < 16; k += blockDim.x) c.Bblk[j * 16 + k] = broke ? 0.0 : Rb[k];
       lap(2);
       bool const full = j + 1 >= c.m_blocks || steps >= a.max_steps || broke;
-      if (full || (j + 1) % a.rr_every == 0) {
+      if (full || (near && (j + 1) % a.rr_every == 0)) {
         __threadfence();
         if (!group_barrier(bar, ncta, a)) return;  // T and B visible to the leader
         if (leader) {
@@ -1268,7 +1276,11 @@ __device__ void solve_chain(ChainDesc const& c, uint32_t rank, uint32_t ncta, ui
     }
     lap(5);
     bool all = true;
-    for (uint32_t i = 0; i < c.nev; ++i) all = all && sqrt(tmp[16 + i]) <= tol;
+    near = true;
+    for (uint32_t i = 0; i < c.nev; ++i) {
+      all = all && sqrt(tmp[16 + i]) <= tol;
+      near = near && sqrt(tmp[16 + i]) <= 1000.0 * tol;
+    }
     __syncthreads();
     if (leader && threadIdx.x == 0)
       for (uint32_t i = 0; i < 4; ++i) c.out[8 + i] = sqrt(tmp[16 + i]);

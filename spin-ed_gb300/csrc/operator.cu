@@ -10,8 +10,8 @@
 // <r~_i|H|r~_j> = sum_s <r_i|H|s> chi(h_s) n_j / n_i with n = sqrt(S / |G|),
 // which holds for any G-invariant H (no Hermiticity needed).
 //
-// Two forms compute the same sum in the same order, so they agree bit for
-// bit:
+// Two forms compute the same sum, on FP64 vectors of real operators bit for
+// bit (exact integer sums, or the same order):
 //   on-the-fly  canonicalises every s_e per call (integer-bound);
 //   stream      records (j_e, code_e) once in SELL-32 slices (32 rows per
 //               warp, slot e of row lane at slice_ptr + 32 e + lane) and then
