@@ -13,7 +13,7 @@ namespace {
 // FP32 and complex vectors of a real operator take the same integer sums as
 // FP64 ones: the FP64 operations per element of k_spmv (one or two
 // multiply-adds on a pipe of 1.75 per clock and SM, and after an FP32 load a
-// conversion on the same pipe) bound it at 397 us a call where these take 177
+// conversion on the same pipe) bound it at 395 us a call where these take 164
 // (ring of 32 sites, FP32).
 struct Columns {
   void const* x;
@@ -121,22 +121,39 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert_cols(Columns c, uint64_t
     at[n] = c.at(q, 0, c.ldx);
   }
   __syncthreads();
-  for (uint64_t i = first; i <= D; i += step) {  // row D is the zero row of fix_row_sums
-    uint32_t const cls = i < D ? row_class[i] : 0u;
+  auto load = [&](uint64_t i, double (&xv)[N]) -> uint32_t {
+#pragma unroll
+    for (uint32_t n = 0; n < N; ++n) {
+      uint64_t const o = at[n] + i * es;
+      xv[n] = !on[n] ? 0.0 : c.f32 ? widen(static_cast<float const*>(c.x)[o]) : static_cast<double const*>(c.x)[o];
+    }
+    return row_class[i];
+  };
+  auto store = [&](uint64_t i, uint32_t cls, double const (&xv)[N]) {
     int64_t v[N];
 #pragma unroll
     for (uint32_t n = 0; n < N; ++n) {
-      v[n] = 0;
-      if (i < D && on[n]) {
-        uint64_t const o = at[n] + i * es;
-        double xv = c.f32 ? widen(static_cast<float const*>(c.x)[o]) : static_cast<double const*>(c.x)[o];
-        if (two) xv *= p1[n];
-        v[n] = fix_round(xv * fac[(q0 + n) * fv.n_div + cls]);
-        if constexpr (Cplx) v[n] += (v[n] & 0x80000000ll) << 1;  // high limb | low limb
-      }
+      v[n] = fix_round((two ? xv[n] * p1[n] : xv[n]) * fac[(q0 + n) * fv.n_div + cls]);
+      if constexpr (Cplx) v[n] += (v[n] & 0x80000000ll) << 1;  // high limb | low limb
     }
     if constexpr (N == 1) u[i] = v[0];
     else reinterpret_cast<longlong2*>(u)[i * L + q0 / 2] = make_longlong2(v[0], v[N - 1]);
+  };
+  // four rows' loads together: one at a time left a load's latency per row (4.7 M
+  // FP32 rows 32 -> 23 us, 1.3 M rows of 8 columns 61 -> 47)
+  uint64_t i = first;
+  for (; i + 3 * step < D; i += 4 * step) {
+    double xv[4][N];
+    uint32_t cls[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) cls[m] = load(i + m * step, xv[m]);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) store(i + m * step, cls[m], xv[m]);
+  }
+  for (; i <= D; i += step) {  // row D is the zero row of fix_row_sums
+    double xv[N] = {};
+    uint32_t const cls = i < D ? load(i, xv) : 0u;
+    store(i, cls, xv);
   }
 }
 
