@@ -908,6 +908,37 @@ __device__ __forceinline__ bool lanczos_step(Ctx& x, uint32_t nb, double* C, dou
   return true;
 }
 
+// The Jacobi rotation of rows p and q, as three shears with h = tan(theta / 2)
+// and s = sin(theta): (p, q) <- (c p - s q, s p + c q), c = 1 - h s, in three
+// FMAs where the product form takes four FP64 instructions.
+__device__ __forceinline__ void rotate(double h, double s, double& p, double& q) {
+  p = fma(-h, q, p);
+  q = fma(s, p, q);
+  p = fma(-h, q, p);
+}
+
+// h of the rotation that annihilates apq, d = aqq - app: the root of smallest
+// magnitude of apq (v^2 - u^2) + d v u = 0 with u = 1 - h^2, v = 2 h. In FP32
+// from both numbers scaled by one power of two, then one Newton step in FP64
+// (2^-45 of h; what it leaves of apq is below the solver's threshold one
+// sweep later, as with a correctly rounded angle). Zero if apq is below 2^-126
+// of d.
+__device__ __forceinline__ double half_angle(double apq, double d) {
+  unsigned const m = (unsigned)(__double_as_longlong(fmax(fabs(apq), fabs(d))) >> 52);
+  double const scale = __longlong_as_double((long long)max(1, min(2046, 2046 - (int)m)) << 52);
+  apq *= scale;
+  d *= scale;
+  float const a = (float)apq, e = (float)d;
+  float t = 2.0f * fabsf(a) / (fabsf(e) + sqrtf(fmaf(e, e, 4.0f * a * a)));
+  if (e != 0.0f && (e < 0.0f) != (a < 0.0f)) t = -t;
+  float const h0 = t / (1.0f + sqrtf(fmaf(t, t, 1.0f)));
+  double const h = h0, u = fma(-h, h, 1.0), v = h + h;
+  double const g = fma(apq, (v - u) * (v + u), d * (v * u));
+  float const uf = (float)u, vf = (float)v;
+  float const slope = fmaf(a, 2.0f * vf * (2.0f + uf), e * fmaf(-vf, vf, 2.0f * uf));
+  return h0 == 0.0f ? 0.0 : h - (double)((float)g / slope);
+}
+
 // Cyclic Jacobi on the symmetric n x n matrix A (shared, row-major with rows of
 // n + 1, n a multiple of 4) with parallel round-robin rotations and a threshold: a rotation whose
 // off-diagonal entry is at most 1e-16 of ||A||_F (invariant under the
@@ -917,14 +948,19 @@ __device__ __forceinline__ bool lanczos_step(Ctx& x, uint32_t nb, double* C, dou
 //
 // The FP64 pipe bounds it. A round rotates rows and columns in one go, a 2 x 2
 // block of A per thread (a row pair and a column pair), blocks above the
-// diagonal only and mirrored: 2 n^2 operations instead of the 4 n^2 of a pass
-// over all rows and one over all columns, and one barrier less. With rows of
+// diagonal only and mirrored: half the operations of a pass over all rows and
+// one over all columns, and one barrier less. With rows of
 // n + 1, and the eigenvectors as rows, lanes fall into different banks. The
-// slowest of 128 J1-J2 chains (16 to 28 sites): 59 -> 42 ms; a batch of 123
-// chains of 14 to 24 sites, where this solve weighs most: 98 -> 80 ms a call.
+// next round's angles (warp 0) and this round's rotation of Q (the other
+// warps) go together between two barriers: the angles were a chain of three
+// FP64 divisions and square roots on one warp that all others waited for. A
+// call with 46 chains of 12 to 20 sites 24.5 -> 17.6 ms, 16 of 18 to 26
+// 60.4 -> 51.3, 128 of 16 to 28 681 -> 665. The three-shear rotations also
+// round less than the product form did: eigenvalues of 64 x 64 matrices err by
+// 2e-15 ||A|| where it was 1.2e-14, after the same number of sweeps.
 __device__ void jacobi(double* A, double* Q, int n) {
-  __shared__ double cs[kMaxN / 2][2];
-  __shared__ int pp[kMaxN / 2][2];
+  __shared__ double cs[2][kMaxN / 2][2];  // h and s, of this round and the next
+  __shared__ int pp[2][kMaxN / 2][2];
   __shared__ double wsum[8];
   __shared__ double thr;
   __shared__ int rotated;
@@ -954,80 +990,82 @@ __device__ void jacobi(double* A, double* Q, int n) {
     double t = 0.0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += wsum[w];
     thr = 1e-16 * sqrt(t);
-    rotated = 0;
   }
   __syncthreads();
+  bool any = false;  // warp 0: this lane has found an entry to rotate in this sweep
+  auto angles = [&](int round, int to) {
+    if ((int)threadIdx.x >= half) return;
+    // round-robin pairing: player 0 fixed, the others rotate
+    int const k = threadIdx.x;
+    auto pos = [&](int q) {
+      int const at = q - 1 + round;  // below 2 (n - 1)
+      return q == 0 ? 0 : 1 + (at >= n - 1 ? at - (n - 1) : at);
+    };
+    int const p0 = pos(k), q0 = pos(n - 1 - k), p = min(p0, q0), q = max(p0, q0);
+    double const apq = A[p * ld + q];
+    double h = 0.0;
+    if (fabs(apq) > thr) h = half_angle(apq, A[q * ld + q] - A[p * ld + p]);
+    any = any || h != 0.0;
+    cs[to][k][0] = h;
+    cs[to][k][1] = h == 0.0 ? 0.0 : 2.0 * h / fma(h, h, 1.0);
+    pp[to][k][0] = p;
+    pp[to][k][1] = q;
+  };
+  int at = 0;
+  if (threadIdx.x < 32) angles(0, at);
+  __syncthreads();
   for (int sweep = 0; sweep < 40; ++sweep) {
-    for (int round = 0; round < n - 1; ++round) {
-      // round-robin pairing: player 0 fixed, the others rotate
-      if ((int)threadIdx.x < half) {
-        int const k = threadIdx.x;
-        auto pos = [&](int q) { return q == 0 ? 0 : 1 + ((q - 1 + round) % (n - 1)); };
-        int p = pos(k), q = pos(n - 1 - k);
-        if (p > q) {
-          int const t = p;
-          p = q;
-          q = t;
-        }
-        double const apq = A[p * ld + q];
-        double c = 1.0, s = 0.0;
-        if (fabs(apq) > thr) {
-          // tan of the angle: the smaller root of t^2 + 2 tau t - 1 = 0
-          double const tau = (A[q * ld + q] - A[p * ld + p]) / (2.0 * apq);
-          double const t = (tau >= 0.0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(fma(tau, tau, 1.0)));
-          c = rsqrt(fma(t, t, 1.0));
-          s = t * c;
-          if (s != 0.0) rotated = 1;
-        }
-        cs[k][0] = c;
-        cs[k][1] = s;
-        pp[k][0] = p;
-        pp[k][1] = q;
-      }
-      __syncthreads();
+    for (int round = 0; round < n - 1; ++round, at ^= 1) {
       // A <- J^T A J
 #pragma unroll
       for (int m = 0; m < kMine; ++m) {
         if (mine[m] < 0) continue;
         int const k1 = mine[m] >> 8, k2 = mine[m] & 255;
-        double const c1 = cs[k1][0], s1 = cs[k1][1], c2 = cs[k2][0], s2 = cs[k2][1];
+        double const h1 = cs[at][k1][0], s1 = cs[at][k1][1], h2 = cs[at][k2][0], s2 = cs[at][k2][1];
         if (s1 == 0.0 && s2 == 0.0) continue;
-        int const p1 = pp[k1][0], q1 = pp[k1][1], p2 = pp[k2][0], q2 = pp[k2][1];
-        double const app = A[p1 * ld + p2], apq = A[p1 * ld + q2], aqp = A[q1 * ld + p2], aqq = A[q1 * ld + q2];
-        double const rpp = c1 * app - s1 * aqp, rqp = s1 * app + c1 * aqp;
-        double const rpq = c1 * apq - s1 * aqq, rqq = s1 * apq + c1 * aqq;
-        double const bpp = c2 * rpp - s2 * rpq, bpq = s2 * rpp + c2 * rpq;
-        double const bqp = c2 * rqp - s2 * rqq, bqq = s2 * rqp + c2 * rqq;
-        A[p1 * ld + p2] = bpp;
-        A[p1 * ld + q2] = bpq;
-        A[q1 * ld + p2] = bqp;
-        A[q1 * ld + q2] = bqq;
+        int const p1 = pp[at][k1][0], q1 = pp[at][k1][1], p2 = pp[at][k2][0], q2 = pp[at][k2][1];
+        double app = A[p1 * ld + p2], apq = A[p1 * ld + q2], aqp = A[q1 * ld + p2], aqq = A[q1 * ld + q2];
+        rotate(h1, s1, app, aqp);
+        rotate(h1, s1, apq, aqq);
+        rotate(h2, s2, app, apq);
+        rotate(h2, s2, aqp, aqq);
+        A[p1 * ld + p2] = app;
+        A[p1 * ld + q2] = apq;
+        A[q1 * ld + p2] = aqp;
+        A[q1 * ld + q2] = aqq;
         if (k1 != k2) {
-          A[p2 * ld + p1] = bpp;
-          A[q2 * ld + p1] = bpq;
-          A[p2 * ld + q1] = bqp;
-          A[q2 * ld + q1] = bqq;
+          A[p2 * ld + p1] = app;
+          A[q2 * ld + p1] = apq;
+          A[p2 * ld + q1] = aqp;
+          A[q2 * ld + q1] = aqq;
         }
       }
-      // Q <- J^T Q
-      for (uint32_t e = threadIdx.x; e < (uint32_t)(half * n); e += blockDim.x) {
-        uint32_t const k = e * inv_n >> 20, col = e - k * (uint32_t)n;
-        double const s = cs[k][1];
-        if (s == 0.0) continue;
-        double const c = cs[k][0];
-        double* qp = Q + pp[k][0] * n + col;
-        double* qq = Q + pp[k][1] * n + col;
-        double const vp = *qp, vq = *qq;
-        *qp = c * vp - s * vq;
-        *qq = s * vp + c * vq;
+      __syncthreads();
+      if (threadIdx.x < 32) {
+        bool const last = round == n - 2;
+        if (last) {
+          bool const r = __any_sync(0xffffffffu, any);
+          if (threadIdx.x == 0) rotated = r;
+          any = false;
+        }
+        angles(last ? 0 : round + 1, at ^ 1);
+      } else {
+        // Q <- J^T Q
+        for (uint32_t e = threadIdx.x - 32; e < (uint32_t)(half * n); e += blockDim.x - 32) {
+          uint32_t const k = e * inv_n >> 20, col = e - k * (uint32_t)n;
+          double const s = cs[at][k][1];
+          if (s == 0.0) continue;
+          double* qp = Q + pp[at][k][0] * n + col;
+          double* qq = Q + pp[at][k][1] * n + col;
+          double vp = *qp, vq = *qq;
+          rotate(cs[at][k][0], s, vp, vq);
+          *qp = vp;
+          *qq = vq;
+        }
       }
       __syncthreads();
     }
-    int const any = rotated;
-    __syncthreads();  // every thread has read the flag
-    if (!any) break;
-    if (threadIdx.x == 0) rotated = 0;
-    __syncthreads();
+    if (!rotated) break;  // written again behind the next sweep's first barrier
   }
 }
 
@@ -1055,29 +1093,34 @@ __device__ double rayleigh_ritz(ChainDesc const& c, uint32_t j, bool have_B, dou
   __syncthreads();
   jacobi(A, Q, n);
   __shared__ int idx[8];
-  __shared__ double worst;
-  int const nk = n < 8 ? n : 8;
-  if (threadIdx.x == 0) {
-    // selection of the nk smallest diagonal entries, ascending
-    bool used[kMaxN] = {};
-    for (int i = 0; i < nk; ++i) {
-      int best = -1;
-      for (int q = 0; q < n; ++q)
-        if (!used[q] && (best < 0 || A[q * (n + 1) + q] < A[best * (n + 1) + best])) best = q;
-      used[best] = true;
-      idx[i] = best;
-      c.out[i] = A[best * (n + 1) + best];
+  __shared__ double worst, last_row[16];
+  int const nk = n < 8 ? n : 8, t = (int)threadIdx.x;
+  if (t < 8) idx[t] = t < n ? t : 0;
+  __syncthreads();
+  if (t < n) {
+    // the nk smallest diagonal entries, ascending
+    double const v = A[t * (n + 1) + t];
+    int rank = 0;
+    for (int q = 0; q < n; ++q) {
+      double const o = A[q * (n + 1) + q];
+      rank += o < v || (o == v && q < t);
     }
+    if (rank < nk) idx[rank] = t;
+  }
+  __syncthreads();
+  if (t < nk) c.out[t] = A[idx[t] * (n + 1) + idx[t]];
+  if (t < 16) {  // entry t % 4 of B_j y_last of Ritz vector t / 4
+    double s = 0.0;
+    if (have_B)
+      for (int b = 0; b < 4; ++b) s += ldcg(c.Bblk + j * 16 + t % 4 * 4 + b) * Q[idx[t / 4] * n + 4 * (int)j + b];
+    last_row[t] = s;
+  }
+  __syncthreads();
+  if (t == 0) {
     worst = 0.0;
     for (int i = 0; i < kB; ++i) {
       double r2 = 0.0;
-      if (have_B) {
-        for (int a = 0; a < 4; ++a) {
-          double s = 0.0;
-          for (int b = 0; b < 4; ++b) s += ldcg(c.Bblk + j * 16 + a * 4 + b) * Q[idx[i] * n + 4 * (int)j + b];
-          r2 += s * s;
-        }
-      }
+      for (int a = 0; a < 4; ++a) r2 += last_row[4 * i + a] * last_row[4 * i + a];
       c.out[8 + i] = sqrt(r2);
       if (i < (int)c.nev) worst = fmax(worst, sqrt(r2));
     }

@@ -137,3 +137,25 @@ def test_lost_directions_and_smallest_sizes(sed, oracle, threads, per_sm):
         np.testing.assert_allclose(res.eigenvalues[i], np.linalg.eigvalsh(A)[:2], rtol=EV_RTOL, atol=0)
         assert np.all(res.residuals[i] <= RES_TOL)
         _check_pairs(oop, res.eigenvalues[i], res.eigenvectors[i])
+
+
+@pytest.mark.parametrize("threads", [128, 256])
+@pytest.mark.parametrize("max_basis", [16, 20, 36, 64])
+def test_projected_problem_sizes(sed, oracle, max_basis, threads):
+    """The dense solve of the projected matrix at its sizes: 16 to 64 columns,
+    on four and on eight warps (eigenvalue errors are the squares of residuals
+    of 1e-8 over gaps above 0.01)."""
+    from spined import _lib as L
+    lib = L.load()
+    models = [lattices.heisenberg_chain(n, j2=j) for n, j in ((14, 0.0), (16, 0.5), (18, 0.25))]
+    pairs = [both(sed, oracle, m) for m in models]
+    try:
+        lib.sed_set_batched_launch(threads, 1)
+        res = sed.eigh_batched([b.hamiltonian for b, _, _ in pairs], nev=3, max_basis=max_basis)
+    finally:
+        lib.sed_set_batched_launch(0, 0)
+    for i, (b, ob, oop) in enumerate(pairs):
+        want = np.linalg.eigvalsh(oop.dense().real)[:3]
+        np.testing.assert_allclose(res.eigenvalues[i], want, rtol=EV_RTOL, atol=0)
+        assert np.all(res.residuals[i] <= RES_TOL)
+        _check_pairs(oop, res.eigenvalues[i], res.eigenvectors[i])
