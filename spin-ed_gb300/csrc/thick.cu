@@ -228,9 +228,10 @@ __host__ __device__ inline bool thick_breakdown(double beta, double tkk) {
 }
 
 // out = w / beta (zero on a breakdown; t1 + t2 = T_kk), and the next matvec's
-// gather copy of it. FP32: 1 / beta as two floats, two FP32 operations where
-// the FP64 product and its conversions took four on the FP64 pipe (w f is
-// rounded once either way, from 2^-46).
+// gather copy of it. FP32: 1 / beta as two floats, a few FP32 operations where
+// the FP64 product and its conversions took four on the FP64 pipe; entries
+// within 2^-16 of a rounding boundary (one in 2^15) take the FP64 product, so
+// that every entry is the FP64 product rounded once.
 template <class S>
 __global__ void __launch_bounds__(256)
     k_tscale_next(S const* __restrict__ w, uint64_t D, double const* __restrict__ beta, double const* __restrict__ t1,
@@ -241,8 +242,14 @@ __global__ void __launch_bounds__(256)
   double const f = thick_breakdown(b, *t1 + *t2) ? 0.0 : 1.0 / b;
   float const fh = (float)f, fl = (float)(f - (double)fh);
   auto scaled = [&](S x) -> S {
-    if constexpr (std::is_same<S, float>::value) return fmaf(x, fh, __fmul_rn(x, fl));
-    else return x * f;
+    if constexpr (std::is_same<S, float>::value) {
+      float const low = __fmul_rn(x, fl), v = fmaf(x, fh, low);
+      float const rest = __fadd_rn(fmaf(x, fh, -v), low);  // x f - v, to 2^-46 of x f
+      if (__fadd_rn(v, __fmul_rn(rest, 1.0f + 0x1p-16f)) == v) return v;
+      return (float)((double)x * f);  // near the middle between two floats
+    } else {
+      return x * f;
+    }
   };
   uint64_t const first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
   if (!next.on) {
@@ -294,9 +301,12 @@ __global__ void k_tscale(S const* __restrict__ w, uint64_t D, double f, S* __res
 
 // In place, row by row: V[:, c] <- sum_{i < m} V[:, i] Y[i * kk + c] for
 // c < kk <= KC. FP32 storage sums in double-float (k_trotate32: products of
-// a float and a split FP64 coefficient, 2^-47 before the rounding to FP32, on
-// the FP32 pipe; FP64 FMAs took 1230 us for m = 16, kk = 8 on 4.7 M rows,
-// this 331). The kk sums of a row are independent chains, one FMA of
+// a float and a split FP64 coefficient, within 2^-42 of the row's norm before
+// the rounding to FP32, on the FP32 pipe; sums that close to a rounding
+// boundary are taken again in FP64, so that every entry is the FP64 sum rounded
+// once: a flipped last bit in some 50 of 4.7 M entries a rotation had moved
+// the final eigenvector by up to 1e-9. FP64 FMAs took 1230 us for m = 16,
+// kk = 8 on 4.7 M rows, this some 340). The kk sums of a row are independent chains, one FMA of
 // each per V value; KC is a template parameter (kk itself up to 16), since a
 // predicated-off FMA still takes its FP64 issue slot.
 template <int KC>
@@ -314,18 +324,33 @@ __global__ void __launch_bounds__(256) k_trotate32(float* __restrict__ V, uint64
     float S[KC], E[KC];
 #pragma unroll
     for (int c = 0; c < KC; ++c) S[c] = E[c] = 0.0f;
+    float row = 0.0f;
 #pragma unroll 2
     for (uint32_t i = 0; i < m; ++i) {
       float const v = V[(uint64_t)i * ld + r];
+      row = fmaf(v, v, row);
 #pragma unroll
       for (int c = 0; c < KC; ++c) {
         float2 const t = y[i * KC + c];
         df_mac(v, 0.0f, t.x, t.y, S[c], E[c]);
       }
     }
+    // the columns of Y have norm 1: no partial sum is above the row's norm
+    float const most = 0x1p-42f * sqrtf(row);
+#pragma unroll
+    for (int c = 0; c < KC; ++c) {
+      float const v = __fadd_rn(S[c], __fadd_rn(E[c], most));
+      if (c < (int)kk && v != __fadd_rn(S[c], __fsub_rn(E[c], most))) {
+        double sum = 0.0;
+        for (uint32_t i = 0; i < m; ++i) sum = fma((double)V[(uint64_t)i * ld + r], Y[i * kk + c], sum);
+        S[c] = (float)sum;
+      } else {
+        S[c] = v;
+      }
+    }
 #pragma unroll
     for (int c = 0; c < KC; ++c)
-      if (c < (int)kk) V[(uint64_t)c * ld + r] = __fadd_rn(S[c], E[c]);
+      if (c < (int)kk) V[(uint64_t)c * ld + r] = S[c];
   }
 }
 
