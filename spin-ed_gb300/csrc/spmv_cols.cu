@@ -329,6 +329,13 @@ __global__ void __launch_bounds__(kBlock) k_spmv_cplx(StreamView S, FixView fv, 
     l += (int64_t)wl * uh;
     l += (int64_t)(wl >> 16) * (ul >> 16);  // the last 2^-68 of the largest product is not kept
   };
+  // the products are subtracted: a low limb can be -2^31, which has no negative in 32 bits
+  auto sub = [](int64_t& h, int64_t& l, int wh, int wl, int uh, int ul) {
+    h -= (int64_t)wh * uh;
+    l -= (int64_t)wh * ul;
+    l -= (int64_t)wl * uh;
+    l -= (int64_t)(wl >> 16) * (ul >> 16);
+  };
   constexpr uint32_t U = 8;
   auto step = [&](uint32_t e0, auto guarded) {
     uint32_t v[U], cd[U];
@@ -347,7 +354,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv_cplx(StreamView S, FixView fv, 
       int4 const w = w_smem[place(cd[p])];
       // little endian: x low, y high limb of the real part, z and w of the imaginary
       add(hr, lr, w.x, w.y, x[p].y, x[p].x);
-      add(hr, lr, -w.z, -w.w, x[p].w, x[p].z);
+      sub(hr, lr, w.z, w.w, x[p].w, x[p].z);
       add(hi, li, w.x, w.y, x[p].w, x[p].z);
       add(hi, li, w.z, w.w, x[p].y, x[p].x);
     }

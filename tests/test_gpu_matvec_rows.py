@@ -1,0 +1,91 @@
+"""Products row by row: factors with few significant bits, vectors whose
+entries differ much in size, columns alone and in blocks
+(src/SpinED/Internal.hs:411-429), against the oracle's matrix."""
+import numpy as np
+import pytest
+
+from _models import both
+from spined import lattices
+from spined import _lib as L
+
+pytestmark = pytest.mark.gpu
+
+
+def f32(v):
+    return float(np.float32(v))
+
+
+def ring(n, j1, j2, k=0, dm=0.0, inversion=None, parity=None):
+    """Ring with exchange j1, j2 and a Dzyaloshinskii-Moriya term along z on the nearest bonds."""
+    bond = [[j1, 0, 0, 0], [0, -j1, 2 * j1 + 1j * dm, 0], [0, 2 * j1 - 1j * dm, -j1, 0], [0, 0, 0, j1]]
+    terms = [(bond, lattices.chain_bonds(n, 1))]
+    if j2:
+        terms.append(([[j2 * v for v in row] for row in lattices.HEISENBERG], lattices.chain_bonds(n, 2)))
+    syms = [(lattices.chain_translation(n), k)] + ([(lattices.chain_parity(n), parity)] if parity is not None else [])
+    return lattices.Model(f"ring{n}k{k}", n, n // 2, inversion, syms, terms)
+
+
+class Case:
+    def __init__(self, sed, oracle, model):
+        self.built, ob, oop = both(sed, oracle, model)
+        self.op, self.D, self.A = self.built.hamiltonian, len(ob.reps), oop.sparse()
+        self.op.prepare(L.SED_FORM_STREAM)
+        self.abs = abs(self.A)
+        self.R = int(np.diff(self.A.tocsr().indptr).max())
+
+    def check(self, x, y):
+        """Every part of every entry: both sides' FP64 sums err by at most (R +
+        8) 2^-53 of the absolute terms (R + 1 products and additions, the
+        factors by a few units), and an FP32 part is rounded once (2^-24) from
+        a value that is within 2^-30 of that."""
+        single = y.dtype in (np.float32, np.complex64)
+        want = self.A @ x.astype(np.complex128)
+        real = not np.iscomplexobj(self.A.data) or not np.any(self.A.data.imag)
+        # complex factors mix the parts of x
+        size = np.abs(x).astype(np.float64)
+        for part in ("real", "imag") if np.iscomplexobj(y) else ("real",):
+            terms = self.abs @ (np.abs(getattr(x, part)).astype(np.float64) if real else size)
+            w = getattr(want, part)
+            tol = (self.R + 8) * 2.0 ** -52 * terms
+            if single:
+                tol = tol + (2.0 ** -24 + 2.0 ** -29) * np.abs(w) + 2.0 ** -149
+            d = np.abs(getattr(y, part).astype(np.float64) - w)
+            worst = np.argmax(d - tol)
+            assert d[worst] <= tol[worst], (part, worst, d[worst], tol[worst], w[worst])
+
+
+_cases = {}
+
+
+@pytest.fixture
+def case(sed, oracle):
+    def get(name, make):
+        if name not in _cases:
+            _cases[name] = Case(sed, oracle, make())
+        return _cases[name]
+    yield get
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _drop():
+    yield
+    _cases.clear()
+
+
+# 2.8 M elements: complex64 products take integer sums. Imaginary factors whose FP64 value has 23 or 24 significant bits.
+FEW_BITS = {
+    "k6_0.3": lambda: ring(24, f32(0.3), f32(0.9), k=6),
+    "k6_1+2^-22": lambda: ring(24, 1 + 2.0 ** -22, 0.5, k=6),
+    "dm_0.6": lambda: ring(24, f32(0.3), f32(0.9), k=1, dm=f32(0.6)),
+}
+
+
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+@pytest.mark.parametrize("name", list(FEW_BITS))
+def test_factors_of_few_bits(sed, case, name, dtype):
+    import torch
+    c = case(name, FEW_BITS[name])
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(c.D, dtype=getattr(torch, dtype), device="cuda", generator=gen)
+    y = sed.apply(c.op, x)
+    c.check(x.cpu().numpy(), y.cpu().numpy())
