@@ -899,8 +899,8 @@ int build_tables(OperatorData& op) {
     t->fix_nv = n_val <= 1 ? 1u : (n_val <= 2 ? 2u : 4u);
     t->fix_ok = true;
   }
-  // complex elements: factors within 2^10 of each other, so that the smallest
-  // keeps its digits in the common scale
+  // complex elements on FP32 vectors: factors within 2^10 of each other, so
+  // that the smallest keeps 44 bits or more in the common scale
   std::vector<int32_t> cw;
   if (!op.is_real && n_val && n_codes <= kCplxMaxCodes && op.row_bound <= kCplxMaxRow) {
     double lo = HUGE_VAL, hi = 0.0;
@@ -2207,7 +2207,7 @@ int sed_operator_prepare(ls_operator* op, int form) {
   d.form = form;
   if (form == SED_FORM_ON_THE_FLY) return LS_SUCCESS;
   int st = operator_record_stream(d, d.cuda_stream);
-  if (!st && cplx_sums(d, 2, 1)) (void)fix_reserve(d, 2);  // without it the matvecs take the general kernel
+  if (!st && cplx_sums(d)) (void)fix_reserve(d, 2);  // without it the matvecs take the general kernel
   return (form == SED_FORM_AUTO && st == LS_OUT_OF_MEMORY) ? LS_SUCCESS : st;
 }
 

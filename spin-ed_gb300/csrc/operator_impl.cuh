@@ -334,8 +334,8 @@ __device__ __forceinline__ void fix_row_sums(StreamView const& S, FixView const&
   if (e < width) step(e, std::true_type{});
 }
 
-// The streamed matvec of an operator with complex elements in integers
-// (spmv_cols.cu). An element's factor and the gathered part are numbers of two
+// The streamed matvec of an operator with complex elements on complex64
+// vectors in integers (spmv_cols.cu). An element's factor and the gathered part are numbers of two
 // 32-bit limbs (the low one signed, so that the high one is rounded):
 // w = round(value x character x 2^-shift), |w| <= 2^54, and u as for real
 // operators, |u| <= 2^62 / R with R the largest row count. A row keeps two
@@ -492,12 +492,11 @@ int operator_apply_prescaled(OperatorData& op, double const* x, double* y, cudaS
 int operator_apply_krylov(OperatorData& op, int dtype, void* base, Indirect ind, cudaStream_t stream);
 int operator_ensure_ready(OperatorData& op);
 
+// Whether complex64 matvecs of a recorded complex operator take integer sums.
+bool cplx_sums(OperatorData const& op);
 // Whether streamed matvecs of this dtype take the integer sums of
 // fix_cols_blocks, and the first `block` columns through it (spmv_cols.cu);
 // *done counts the columns taken.
-// Whether matvecs of a recorded complex operator take integer sums (dtype 2
-// or 3).
-bool cplx_sums(OperatorData const& op, int dtype, uint64_t block);
 bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_stream, cudaStream_t stream);
 int fix_cols_blocks(OperatorData& op, int dtype, uint64_t block, char const* x, uint64_t ldx, char* y, uint64_t ldy,
                     size_t es, cudaStream_t stream, uint64_t* done);

@@ -1,16 +1,20 @@
 // spmv_cols.cu — the streamed fixed-point matvec on blocks of columns, on FP32
-// and complex vectors of real operators and of complex operators
-// (src/SpinED/Internal.hs:411-429; the mathematics is at FixView and CplxView
-// in operator_impl.cuh).
+// vectors (real or complex) of real operators and on complex FP32 vectors of
+// complex operators (src/SpinED/Internal.hs:411-429; the mathematics is at
+// FixView and CplxView in operator_impl.cuh).
 //
 // A pass covers K real columns; a complex column is two. The gather copy u
 // holds the K columns of a row next to each other.
+//
+// complex128 vectors stay with the FP64 sums of k_spmv, whose errors are those
+// of each entry: a fixed point of the vector's largest entry gives rows that
+// couple to entries far below it fewer digits, or none.
 #include "operator_impl.cuh"
 
 namespace sed {
 namespace {
 
-// FP32 and complex vectors of a real operator take the same integer sums as
+// FP32 vectors of a real operator take the same integer sums as
 // FP64 ones: the FP64 operations per element of k_spmv (one or two
 // multiply-adds on a pipe of 1.75 per clock and SM, and after an FP32 load a
 // conversion on the same pipe) bound it at 395 us a call where these take 164
@@ -20,7 +24,7 @@ struct Columns {
   void* y;
   uint64_t ldx, ldy;  // in vector elements
   uint32_t cols;      // real columns of this pass (the rest of K is padding)
-  bool f32, cx;
+  bool f32, cx;       // complex columns are FP32 ones
   // offset of entry i of real column q, in reals
   __device__ __forceinline__ uint64_t at(uint32_t q, uint64_t i, uint64_t ld) const {
     return cx ? 2 * ((uint64_t)(q >> 1) * ld + i) + (q & 1u) : (uint64_t)q * ld + i;
@@ -196,7 +200,7 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix_cols(StreamView S, FixView 
   for (uint32_t q = 0; q < c.cols; ++q) fix_row_factors<NV>(fv, S.inv_sqrt_s, F_in[q], fix_smem + q * fv.n_div * NV);
   if (threadIdx.x == 0) {
     bool b = false;
-    if (c.f32 || c.cx)
+    if (c.f32)
       for (uint32_t q = 0; q < c.cols; ++q) b = b || F_in[q] == kFixBad;
     bad = b;
   }
@@ -280,13 +284,12 @@ __device__ __forceinline__ double limbs_to_double(int64_t hi, int64_t lo) {
   return __longlong_as_double((long long)(b | (uint64_t)neg << 63));
 }
 
-// Streamed SpMV of a complex operator on a complex column, sums in integers
-// (CplxView). The four FP64 multiply-adds per element of k_spmv take 75 of its
-// 102 us on the 28-site ring at k = 3 (10.4 M elements, FP64 pipe of 1.75 per
-// clock and SM); here an element is 16 wide integer multiply-adds and one
-// 16-byte gather: 46 us, of which the gathered sectors are about 32 (10.5
-// TB/s of L2). With 11 us for the pre-pass a call takes 85 us for 123. FP32
-// vectors: 159 and 46 us (the conversions of k_spmv's loads share its pipe).
+// Streamed SpMV of a complex operator on a complex64 column, sums in integers
+// (CplxView). The four FP64 multiply-adds per element of k_spmv and the
+// conversions of its loads take 159 us on the 28-site ring at k = 3 (10.4 M
+// elements, FP64 pipe of 1.75 per clock and SM); here an element is 16 wide
+// integer multiply-adds and one 16-byte gather: 46 us, of which the gathered
+// sectors are about 32.
 // Factors are staged with their position's low three bits swizzled: codes of
 // one stabiliser class are n_div apart, which would put them all in one bank
 // group. Eight elements in flight: 20.8 M elements in 109 us for 112 with four.
@@ -300,10 +303,10 @@ __global__ void __launch_bounds__(kBlock) k_spmv_cplx(StreamView S, FixView fv, 
   double* g = reinterpret_cast<double*>(w_smem + n8);
   if (blockIdx.x == 0 && threadIdx.x < 2) clear[threadIdx.x] = 0;  // max |x| for the next call's pre-pass
   int64_t const F = F_in[0];
-  // 2^(32 + shift - F), what is outside +-1000 by a second factor
-  int64_t const e = F == kFixBad ? 0 : 32 + cw.shift - F, e1 = min(max(e, (int64_t)-900), (int64_t)900);
+  // 2^(32 + shift - F): F is in -100 .. 215 for FP32 entries, shift in -254 .. 146
+  int64_t const e = F == kFixBad ? 0 : 32 + cw.shift - F;
   for (uint32_t t = threadIdx.x; t < fv.n_codes; t += blockDim.x) w_smem[place(t)] = cw.w[t];
-  for (uint32_t t = threadIdx.x; t < fv.n_div; t += blockDim.x) g[t] = S.inv_sqrt_s[t] * fix_pow2(e1);
+  for (uint32_t t = threadIdx.x; t < fv.n_div; t += blockDim.x) g[t] = S.inv_sqrt_s[t] * fix_pow2(e);
   __syncthreads();
   uint64_t const i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, s = i >> 5;
   if ((s << 5) >= D) return;
@@ -371,17 +374,8 @@ __global__ void __launch_bounds__(kBlock) k_spmv_cplx(StreamView S, FixView fv, 
     yr = __fma_rn(-dg.y, xi, yr);
     yi = __fma_rn(dg.y, xr, yi);
   }
-  double sr = limbs_to_double(hr, lr), si = limbs_to_double(hi, li);
-  if (e != e1) {
-    sr = __dmul_rn(f, sr);
-    si = __dmul_rn(f, si);
-    double const p = fix_pow2(e - e1);
-    yr = __fma_rn(p, sr, yr);
-    yi = __fma_rn(p, si, yi);
-  } else {
-    yr = __fma_rn(f, sr, yr);
-    yi = __fma_rn(f, si, yi);
-  }
+  yr = __fma_rn(f, limbs_to_double(hr, lr), yr);
+  yi = __fma_rn(f, limbs_to_double(hi, li), yi);
   c.store(0, i, yr);
   c.store(1, i, yi);
 }
@@ -458,17 +452,12 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
 
 }  // namespace
 
-// Below these sizes the two launches more per column cost what the sums save.
-// The general kernel's pass over a block reads the entries once for up to 16
-// columns (its FP64 arithmetic is per column), so a wide complex128 block needs
-// more elements. Calls in us, general kernels and this one:
-//   complex64, 1 / 7 / 16 columns:  0.7 M elements 35 / 142 / 280 and 34 / 159 / 346,
-//     1.4 M 47 / 227 / 465 and 37 / 175 / 378
-//   complex128:  1.4 M 38 / 151 / 293 and 36 / 167 / 362,
-//     2.7 M 50 / 248 / 484 and 44 / 236 / 528,  5.4 M 74 / 401 / 803 and 52 / 304 / 681
-bool cplx_sums(OperatorData const& op, int dtype, uint64_t block) {
-  unsigned const bits = dtype == 2 ? 20 : block < 8 ? 21 : 22;
-  return op.tables->cplx_ok && op.stream.n_elements >= ((uint64_t)1 << bits);
+// Below this size the two launches more per column cost what the sums save.
+// Calls of 1 / 7 / 16 columns in us, general kernels and this one: 0.7 M
+// elements 35 / 142 / 280 and 34 / 159 / 346, 1.4 M 47 / 227 / 465 and
+// 37 / 175 / 378.
+bool cplx_sums(OperatorData const& op) {
+  return op.tables->cplx_ok && op.stream.n_elements >= ((uint64_t)1 << 20);
 }
 
 // Whether vectors of this dtype go through launch_fix_cols. FP64 columns
@@ -479,13 +468,13 @@ bool cplx_sums(OperatorData const& op, int dtype, uint64_t block) {
 // workspace could be overwritten between replays (the general kernels use
 // none).
 bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_stream, cudaStream_t stream) {
-  if (!use_stream) return false;
+  if (!use_stream || dtype == 3) return false;
   if (op.tables->cplx_ok) {
-    if (dtype < 2 || !cplx_sums(op, dtype, block)) return false;
+    if (dtype != 2 || !cplx_sums(op)) return false;
   } else {
     if (!op.tables->fix_ok || op.fix_cols < 1) return false;
     if (dtype == 1) return true;
-    if (op.stream.n_elements * block * (dtype >= 2 ? 2 : 1) < ((uint64_t)1 << 21)) return false;
+    if (op.stream.n_elements * block * (dtype == 2 ? 2 : 1) < ((uint64_t)1 << 21)) return false;
   }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
@@ -508,7 +497,7 @@ int fix_cols_blocks(OperatorData& op, int dtype, uint64_t block, char const* x, 
   if (op.tables->cplx_ok) {
     if (int st = fix_reserve(op, 2)) return st == LS_OUT_OF_MEMORY ? LS_SUCCESS : st;
     for (; *done < block; ++*done)
-      if (int st = launch_cplx(op, {x + *done * ldx * es, y + *done * ldy * es, ldx, ldy, 2, dtype == 2, true}, stream))
+      if (int st = launch_cplx(op, {x + *done * ldx * es, y + *done * ldy * es, ldx, ldy, 2, true, true}, stream))
         return st;
     return LS_SUCCESS;
   }
@@ -516,7 +505,7 @@ int fix_cols_blocks(OperatorData& op, int dtype, uint64_t block, char const* x, 
   // columns fit in 48 KB
   size_t const table = (size_t)op.tables->fix.n_div * op.tables->fix_nv * 8;
   unsigned const kmax = (unsigned)std::min<size_t>(16, (48 * 1024 - op.tables->fix.n_codes - 1) / table);
-  bool const cx = dtype >= 2;
+  bool const cx = dtype == 2;
   unsigned const per = cx ? 2 : 1;  // real columns per column
   while (*done < block) {
     uint64_t const left = (block - *done) * per;

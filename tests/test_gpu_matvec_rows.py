@@ -89,3 +89,42 @@ def test_factors_of_few_bits(sed, case, name, dtype):
     x = torch.randn(c.D, dtype=getattr(torch, dtype), device="cuda", generator=gen)
     y = sed.apply(c.op, x)
     c.check(x.cpu().numpy(), y.cpu().numpy())
+
+
+# integer sums: FP32 from 2^21 elements of a real operator, complex64 from 2^20 of any
+RANGE_MODELS = {
+    "real_one": lambda: lattices.heisenberg_chain(28),
+    "real_two": lambda: lattices.heisenberg_chain(26, j2=0.3),
+    "real_signed": lambda: lattices.heisenberg_chain(26, momentum=13, parity=None, j2=0.4),
+    "complex": lambda: ring(24, 1.0, 0.37, k=5),
+    "complex_far": lambda: ring(24, 1.0, 0.3 / 300, k=6, dm=0.7),
+    "imaginary": lambda: ring(26, 0.0, 0.0, dm=1.1),
+}
+
+
+def vector(kind, D, dtype, seed):
+    rng = np.random.default_rng(seed)
+    x = rng.normal(size=D) + (1j * rng.normal(size=D) if dtype.startswith("complex") else 0)
+    big = rng.random(D) < 1e-3
+    if kind == "small":  # most rows couple to entries of 1e-25 only
+        x[~big] *= 1e-25
+    elif kind == "sparse":
+        x[~big] = 0.0
+    elif kind == "small_parts" and dtype.startswith("complex"):
+        x = x.real + 1e-22j * x.imag
+    return x.astype(dtype)
+
+
+@pytest.mark.parametrize("kind", ["plain", "small", "sparse", "small_parts"])
+@pytest.mark.parametrize("dtype", ["complex128"])
+@pytest.mark.parametrize("name", list(RANGE_MODELS))
+def test_entries_of_different_size(sed, case, name, dtype, kind):
+    """Rows that couple to small entries of the vector only keep the digits
+    of those, and rows that couple to zeros are zero."""
+    import torch
+    if dtype == "float32" and not name.startswith("real"):
+        pytest.skip("complex operator")
+    c = case(name, RANGE_MODELS[name])
+    x = vector(kind, c.D, dtype, 6)
+    y = sed.apply(c.op, torch.tensor(x, device="cuda"))
+    c.check(x, y.cpu().numpy())
