@@ -6,6 +6,15 @@
 // A pass covers K real columns; a complex column is two. The gather copy u
 // holds the K columns of a row next to each other.
 //
+// FP32 vectors of any range of entries: the integer sums of a row err by at
+// most half a unit per element, and a part of a row's result that is below 2^30
+// times that is summed again as k_spmv does (general_entry), so that every part
+// of every entry is within 2^-30 of the FP64 value before it is rounded to FP32.
+// In a vector of normal numbers these are 10^-4 of the rows or fewer (4.7 M FP32
+// rows: 163 us a call with and without the rule); where nearly all entries are
+// zero or below 2^-26 of the largest they are nearly all rows, 484 us a call for
+// the 395 of k_spmv.
+//
 // complex128 vectors stay with the FP64 sums of k_spmv, whose errors are those
 // of each entry: a fixed point of the vector's largest entry gives rows that
 // couple to entries far below it fewer digits, or none.
@@ -161,21 +170,45 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert_cols(Columns c, uint64_t
   }
 }
 
-// One row of two adjacent columns as k_spmv sums it (a vector with a NaN or
-// an infinity: only the rows it reaches are affected).
+__device__ __forceinline__ int exponent_bits(double v) { return __double2hiint(v) >> 20 & 0x7FF; }
+
+// Entry i of FP32 column q (V real), or of the complex column whose real part
+// is q, as k_spmv gives it: four elements' loads in flight (a warp that came
+// here late with one at a time ended some 70 us after the others), and no sums
+// over zeros of x, which most rows of a sparse vector have only.
 template <class V, bool RealOp>
-__device__ __forceinline__ V general_row(StreamView const& S, Columns const& c, uint32_t const* ent, uint16_t const* codes,
-                                         uint32_t width, uint32_t col_mask, bool packed, uint32_t q) {
+__device__ __forceinline__ V general_entry(StreamView const& S, Columns const& c, uint32_t const* ent, uint16_t const* codes,
+                                           uint32_t width, bool packed, uint32_t q, uint64_t i) {
+  constexpr bool kReal = std::is_same<V, double>::value;
+  constexpr uint32_t U = 4;
+  uint32_t const mask = packed ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
+  float const* const x = static_cast<float const*>(c.x) + c.at(q, 0, c.ldx);
+  uint64_t const es = c.cx ? 2 : 1;
+  auto widened = [&](float re, float im) -> V {
+    if constexpr (kReal) return (double)re;
+    else return cplx{(double)re, (double)im};
+  };
   V acc = zero<V>();
-  for (uint32_t e = 0; e < width; ++e) {
-    uint32_t const v = ent[(uint64_t)e * 32];
-    if (v == kNull) continue;
-    uint32_t const code = packed ? (v >> S.col_bits) : (uint32_t)codes[(uint64_t)e * 32], j = v & col_mask;
-    V const t = load_table<V>(S.table, code, RealOp);
-    if constexpr (std::is_same<V, double>::value) mac(acc, t, c.load(q, j));
-    else mac(acc, t, cplx{c.load(q, j), c.load(q + 1, j)});
+  for (uint32_t e0 = 0; e0 < width; e0 += U) {
+    uint32_t v[U];
+    float re[U], im[U];
+#pragma unroll
+    for (uint32_t p = 0; p < U; ++p) v[p] = e0 + p < width ? ent[(uint64_t)(e0 + p) * 32] : kNull;
+#pragma unroll
+    for (uint32_t p = 0; p < U; ++p) {
+      uint64_t const at = v[p] == kNull ? 0 : (uint64_t)(v[p] & mask) * es;
+      re[p] = x[at];
+      im[p] = kReal ? 0.0f : x[at + 1];
+    }
+#pragma unroll
+    for (uint32_t p = 0; p < U; ++p) {
+      if (v[p] == kNull || ((__float_as_uint(re[p]) | __float_as_uint(im[p])) & 0x7FFFFFFFu) == 0) continue;
+      uint32_t const code = packed ? (v[p] >> S.col_bits) : (uint32_t)codes[(uint64_t)(e0 + p) * 32];
+      mac(acc, load_table<V>(S.table, code, RealOp), widened(re[p], im[p]));
+    }
   }
-  return acc;
+  V const xi = widened(x[i * es], kReal ? 0.0f : x[i * es + 1]);
+  return row_value<V>(mulv(stream_diag<V, RealOp>(S, i), xi), S.inv_sqrt_s[S.row_class[i]], acc);
 }
 
 // Streamed SpMV on K interleaved columns (u row i at u + i K): K / 4 lanes
@@ -186,24 +219,17 @@ __device__ __forceinline__ V general_row(StreamView const& S, Columns const& c, 
 // at the start. About 246 of these are the 2.6 GB of gathered sectors at the
 // 10.5 TB/s that L2 gives an 83 MB copy, the rest the rows' FP64 epilogues.
 // x, y and the entries pass through L2 once (evict first), so that u stays.
-template <bool Packed, int NV, bool Signed, int K>
-__global__ void __launch_bounds__(kBlock) k_spmv_fix_cols(StreamView S, FixView fv, uint64_t D, Columns c,
+template <bool Packed, int NV, bool Signed, int K, bool F32>
+__global__ void __launch_bounds__(kBlock, !F32 || NV > 2 ? 0 : K == 1 ? 8 : K == 2 ? 6 : K == 4 ? 5 : 4) k_spmv_fix_cols(StreamView S, FixView fv, uint64_t D, Columns c,
                                                           int64_t const* __restrict__ u,
                                                           int64_t const* __restrict__ F_in,
                                                           unsigned long long* __restrict__ clear) {
   constexpr uint32_t N = K < 4 ? K : 4, L = K / N;  // columns per lane, lanes per row
   extern __shared__ double fix_smem[];                 // g[K][n_div NV], then the code bytes
-  __shared__ bool bad;
   if (blockIdx.x == 0 && threadIdx.x < K) clear[threadIdx.x] = 0;  // max |x| for the next call's pre-pass
   uint8_t* code8 = reinterpret_cast<uint8_t*>(fix_smem + K * fv.n_div * NV);
   if constexpr (Signed) fix_stage_codes(fv, code8);
   for (uint32_t q = 0; q < c.cols; ++q) fix_row_factors<NV>(fv, S.inv_sqrt_s, F_in[q], fix_smem + q * fv.n_div * NV);
-  if (threadIdx.x == 0) {
-    bool b = false;
-    if (c.f32)
-      for (uint32_t q = 0; q < c.cols; ++q) b = b || F_in[q] == kFixBad;
-    bad = b;
-  }
   __syncthreads();
   uint64_t const gw = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   uint64_t const s = gw / L;
@@ -211,27 +237,8 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix_cols(StreamView S, FixView 
   uint32_t const lane = threadIdx.x & 31, row = (uint32_t)(gw % L) * (32 / L) + lane / L, q0 = (lane % L) * N;
   uint64_t const base = S.slice_ptr[s], i = s * 32 + row;
   uint32_t const width = (uint32_t)((S.slice_ptr[s + 1] - base) >> 5);
-  uint32_t const col_mask = Packed ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
   uint32_t const* ent = S.entries + base + row;
   uint16_t const* codes = S.codes + base + row;
-  if (bad) {
-    if (i >= D || q0 >= c.cols) return;
-    double const f = S.inv_sqrt_s[S.row_class[i]], dg = static_cast<double const*>(S.diag)[i];
-    if (c.cx) {
-      for (uint32_t q = q0; q < q0 + N && q < c.cols; q += 2) {
-        cplx const xi{c.load(q, i), c.load(q + 1, i)};
-        cplx const acc = general_row<cplx, true>(S, c, ent, codes, width, col_mask, Packed, q);
-        cplx const yi = row_value<cplx>(mulv(cplx{dg, 0.0}, xi), f, acc);
-        c.store(q, i, yi.re);
-        c.store(q + 1, i, yi.im);
-      }
-    } else {
-      for (uint32_t q = q0; q < q0 + N && q < c.cols; ++q)
-        c.store(q, i, row_value<double>(mulv(dg, c.load(q, i)), f,
-                                        general_row<double, true>(S, c, ent, codes, width, col_mask, Packed, q)));
-    }
-    return;
-  }
   int64_t acc[N][NV];
   fix_row_sums<Packed, NV, Signed, (int)N, 8>(
       S, fv, code8, codes, width, (uint32_t)D, acc,
@@ -252,12 +259,34 @@ __global__ void __launch_bounds__(kBlock) k_spmv_fix_cols(StreamView S, FixView 
   if (i >= D) return;
   uint32_t const cls = __ldcs(S.row_class + i);
   double const dg = __ldcs(static_cast<double const*>(S.diag) + i);
+  uint32_t again = 0;  // columns to sum again
+  // 2^30 width max |g_v| is below 2^wide times the power of two below max |g_v|
+  int const wide = 31 + (32 - __clz((int)width));
 #pragma unroll
-  for (uint32_t n = 0; n < N; ++n)
-    if (q0 + n < c.cols)
-      c.store(q0 + n, i, fix_row<NV>(acc[n], fix_smem + ((q0 + n) * fv.n_div + cls) * NV, F_in[q0 + n], dg, c.load(q0 + n, i)));
+  for (uint32_t n = 0; n < N; ++n) {
+    uint32_t const q = q0 + n;
+    if (q >= c.cols) continue;
+    double const* g = fix_smem + (q * fv.n_div + cls) * NV;
+    double const y = fix_row<NV>(acc[n], g, F_in[q], dg, c.load(q, i));
+    c.store(q, i, y);
+    if constexpr (F32) {
+      int e = 0;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) e = max(e, exponent_bits(g[k]));
+      if (exponent_bits(y) < e + wide || F_in[q] == kFixBad || (c.cx && F_in[q ^ 1u] == kFixBad)) again |= 1u << n;
+    }
+  }
+  if constexpr (F32)
+    for (; again; again &= again - 1) {
+      uint32_t const q = q0 + __ffs((int)again) - 1;
+      if (c.cx && (F_in[q] == kFixBad || F_in[q ^ 1u] == kFixBad)) {  // either part spoils both
+        cplx const y = general_entry<cplx, true>(S, c, ent, codes, width, Packed, q & ~1u, i);
+        c.store(q, i, (q & 1u) ? y.im : y.re);
+      } else {
+        c.store(q, i, general_entry<double, true>(S, c, ent, codes, width, Packed, q, i));
+      }
+    }
 }
-
 
 // hi 2^32 + lo as a double, rounded to nearest even (|hi| < 2^55).
 __device__ __forceinline__ double limbs_to_double(int64_t hi, int64_t lo) {
@@ -288,13 +317,13 @@ __device__ __forceinline__ double limbs_to_double(int64_t hi, int64_t lo) {
 // (CplxView). The four FP64 multiply-adds per element of k_spmv and the
 // conversions of its loads take 159 us on the 28-site ring at k = 3 (10.4 M
 // elements, FP64 pipe of 1.75 per clock and SM); here an element is 16 wide
-// integer multiply-adds and one 16-byte gather: 46 us, of which the gathered
-// sectors are about 32.
+// integer multiply-adds and one 16-byte gather: 52 us, of which the gathered
+// sectors are about 32. A call takes 92 us for 178.
 // Factors are staged with their position's low three bits swizzled: codes of
 // one stabiliser class are n_div apart, which would put them all in one bank
 // group. Eight elements in flight: 20.8 M elements in 109 us for 112 with four.
 template <bool Packed>
-__global__ void __launch_bounds__(kBlock) k_spmv_cplx(StreamView S, FixView fv, CplxView cw, uint64_t D, Columns c,
+__global__ void __launch_bounds__(kBlock, 5) k_spmv_cplx(StreamView S, FixView fv, CplxView cw, uint64_t D, Columns c,
                                                       int4 const* __restrict__ u, int64_t const* __restrict__ F_in,
                                                       unsigned long long* __restrict__ clear) {
   extern __shared__ int4 w_smem[];  // [n_codes], swizzled within groups of 8; then g[n_div]
@@ -316,15 +345,6 @@ __global__ void __launch_bounds__(kBlock) k_spmv_cplx(StreamView S, FixView fv, 
   uint32_t const mask = Packed ? ((1u << S.col_bits) - 1u) : 0xFFFFFFFFu;
   uint32_t const* ent = S.entries + base + lane;
   uint16_t const* codes = S.codes + base + lane;
-  if (F == kFixBad) {
-    if (i >= D) return;
-    cplx const xi{c.load(0, i), c.load(1, i)};
-    cplx const acc = general_row<cplx, false>(S, c, ent, codes, width, mask, Packed, 0);
-    cplx const yi = row_value<cplx>(mulv(stream_diag<cplx, false>(S, i), xi), S.inv_sqrt_s[S.row_class[i]], acc);
-    c.store(0, i, yi.re);
-    c.store(1, i, yi.im);
-    return;
-  }
   int64_t hr = 0, lr = 0, hi = 0, li = 0;
   auto add = [](int64_t& h, int64_t& l, int wh, int wl, int uh, int ul) {
     h += (int64_t)wh * uh;
@@ -376,6 +396,16 @@ __global__ void __launch_bounds__(kBlock) k_spmv_cplx(StreamView S, FixView fv, 
   }
   yr = __fma_rn(f, limbs_to_double(hr, lr), yr);
   yi = __fma_rn(f, limbs_to_double(hi, li), yi);
+  // The sums err by less than 2^32 units of f: each element by 2^22 (u of two
+  // parts, half a unit each, times |w| 2^-32) and 2^17 (low products), the
+  // factors (half a unit times |u| 2^-32) by 2^30 in all.
+  int const least = exponent_bits(f) + 63;
+  bool const again_r = exponent_bits(yr) < least || F == kFixBad, again_i = exponent_bits(yi) < least || F == kFixBad;
+  if (again_r || again_i) {
+    cplx const y = general_entry<cplx, false>(S, c, ent, codes, width, Packed, 0, i);
+    if (again_r) yr = y.re;
+    if (again_i) yi = y.im;
+  }
   c.store(0, i, yr);
   c.store(1, i, yi);
 }
@@ -434,7 +464,8 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
     unsigned const cg = grid_size((D + 1) * (KK > 2 ? KK / 2 : 1), b.device, 8);
     k_fix_convert_cols<KK, false><<<cg, kBlock, (size_t)KK * tb.fix.n_div * 8, stream>>>(c, D, cls, tb.fix, mx, F, u);
     fix_dispatch(tb, sf.packed, [&](auto packed, auto nv, auto sign) {
-      k_spmv_fix_cols<packed.value, nv.value, sign.value, KK><<<grid, kBlock, smem, stream>>>(S, tb.fix, D, c, u, F, mx);
+      if (c.f32) k_spmv_fix_cols<packed.value, nv.value, sign.value, KK, true><<<grid, kBlock, smem, stream>>>(S, tb.fix, D, c, u, F, mx);
+      else k_spmv_fix_cols<packed.value, nv.value, sign.value, KK, false><<<grid, kBlock, smem, stream>>>(S, tb.fix, D, c, u, F, mx);
     });
   };
   switch (K) {

@@ -108,15 +108,19 @@ def vector(kind, D, dtype, seed):
     big = rng.random(D) < 1e-3
     if kind == "small":  # most rows couple to entries of 1e-25 only
         x[~big] *= 1e-25
+    elif kind == "half":
+        x[int(0.6 * D):] *= 1e-25
     elif kind == "sparse":
         x[~big] = 0.0
     elif kind == "small_parts" and dtype.startswith("complex"):
         x = x.real + 1e-22j * x.imag
+    elif kind == "zero_part":
+        x = x.real + 0j if dtype.startswith("complex") else 0 * x
     return x.astype(dtype)
 
 
-@pytest.mark.parametrize("kind", ["plain", "small", "sparse", "small_parts"])
-@pytest.mark.parametrize("dtype", ["complex128"])
+@pytest.mark.parametrize("kind", ["plain", "small", "half", "sparse", "small_parts", "zero_part"])
+@pytest.mark.parametrize("dtype", ["float32", "complex64", "complex128"])
 @pytest.mark.parametrize("name", list(RANGE_MODELS))
 def test_entries_of_different_size(sed, case, name, dtype, kind):
     """Rows that couple to small entries of the vector only keep the digits
