@@ -1618,7 +1618,7 @@ int operator_apply_device(OperatorData& op, int dtype, uint64_t block, void cons
   }
   size_t const es = (size_t)elem_size(dtype);
   uint64_t c0 = 0;
-  if (fix_cols_apply(op, dtype, block, use_stream, stream))
+  if (fix_cols_apply(op, dtype, use_stream, stream))
     if (int st = fix_cols_blocks(op, dtype, block, static_cast<char const*>(x), ldx, static_cast<char*>(y), ldy, es, stream, &c0))
       return st;
   if (use_stream && !(dtype == 1 && op.tables->fix_ok && op.fix_cols >= 1)) {

@@ -497,7 +497,7 @@ bool cplx_sums(OperatorData const& op);
 // Whether streamed matvecs of this dtype take the integer sums of
 // fix_cols_blocks, and the first `block` columns through it (spmv_cols.cu);
 // *done counts the columns taken.
-bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_stream, cudaStream_t stream);
+bool fix_cols_apply(OperatorData const& op, int dtype, bool use_stream, cudaStream_t stream);
 int fix_cols_blocks(OperatorData& op, int dtype, uint64_t block, char const* x, uint64_t ldx, char* y, uint64_t ldy,
                     size_t es, cudaStream_t stream, uint64_t* done);
 

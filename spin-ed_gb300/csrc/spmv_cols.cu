@@ -492,20 +492,22 @@ bool cplx_sums(OperatorData const& op) {
 }
 
 // Whether vectors of this dtype go through launch_fix_cols. FP64 columns
-// always do. The others do from 2^21 element products on: below, the three
-// launches more cost what the sums save (290 000 elements of a complex
-// column: 30 us in the general kernel, 37 here; 77 M FP32 ones: 397 and 180).
+// always do. FP32 and complex64 ones do from 2^21 and 2^20 elements on: below,
+// the three launches more cost what the sums save (290 000 elements of a
+// complex column: 30 us in the general kernel, 37 here; 77 M FP32 ones: 397 and
+// 164). The rule does not look at the width of the block, so that a column's
+// product does not depend on the columns beside it.
 // They do not while the caller's stream is being captured, where the shared
 // workspace could be overwritten between replays (the general kernels use
 // none).
-bool fix_cols_apply(OperatorData const& op, int dtype, uint64_t block, bool use_stream, cudaStream_t stream) {
+bool fix_cols_apply(OperatorData const& op, int dtype, bool use_stream, cudaStream_t stream) {
   if (!use_stream || dtype == 3) return false;
   if (op.tables->cplx_ok) {
     if (dtype != 2 || !cplx_sums(op)) return false;
   } else {
     if (!op.tables->fix_ok || op.fix_cols < 1) return false;
     if (dtype == 1) return true;
-    if (op.stream.n_elements * block * (dtype == 2 ? 2 : 1) < ((uint64_t)1 << 21)) return false;
+    if (op.stream.n_elements < ((uint64_t)1 << (dtype == 2 ? 20 : 21))) return false;
   }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {

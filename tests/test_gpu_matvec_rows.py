@@ -132,3 +132,31 @@ def test_entries_of_different_size(sed, case, name, dtype, kind):
     x = vector(kind, c.D, dtype, 6)
     y = sed.apply(c.op, torch.tensor(x, device="cuda"))
     c.check(x, y.cpu().numpy())
+
+
+BLOCK_MODELS = {
+    "chain24": lambda: lattices.heisenberg_chain(24),
+    "real_two": RANGE_MODELS["real_two"],
+    "complex": RANGE_MODELS["complex"],
+}
+
+
+@pytest.mark.parametrize("bad", [None, float("nan")])
+@pytest.mark.parametrize("dtype", ["float32", "complex64", "complex128"])
+@pytest.mark.parametrize("name", list(BLOCK_MODELS))
+def test_columns_do_not_depend_on_their_block(sed, case, name, dtype, bad):
+    """A column's product is the same alone and in a block of any width, also
+    beside a column with a NaN."""
+    import torch
+    if dtype == "float32" and name == "complex":
+        pytest.skip("complex operator")
+    c = case(name, BLOCK_MODELS[name])
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    x = torch.randn(16, c.D, dtype=getattr(torch, dtype), device="cuda", generator=gen).t()
+    if bad is not None:
+        x[c.D // 3, 1] = bad
+    alone = [sed.apply(c.op, x[:, q].contiguous()) for q in range(16)]
+    for width in (2, 3, 8, 16):
+        y = sed.apply(c.op, x[:, :width])
+        for q in range(width):
+            assert torch.equal(y[:, q].nan_to_num(123.0), alone[q].nan_to_num(123.0)), (width, q)
