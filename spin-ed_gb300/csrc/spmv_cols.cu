@@ -483,12 +483,20 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
 
 }  // namespace
 
+namespace {
+// The gather copy stays with the operator. FP32 vectors took no memory before
+// they took this path, so theirs is bounded: 1 GiB, 8 columns of 15.8 M rows
+// (a single FP32 column uses the copy that every real operator has).
+constexpr uint64_t kKeptCopy = 1ull << 30;
+uint64_t copy_bytes(OperatorData const& op, unsigned K) { return (op.basis->D + 1) * K * 8; }
+}  // namespace
+
 // Below this size the two launches more per column cost what the sums save.
 // Calls of 1 / 7 / 16 columns in us, general kernels and this one: 0.7 M
 // elements 35 / 142 / 280 and 34 / 159 / 346, 1.4 M 47 / 227 / 465 and
 // 37 / 175 / 378.
 bool cplx_sums(OperatorData const& op) {
-  return op.tables->cplx_ok && op.stream.n_elements >= ((uint64_t)1 << 20);
+  return op.tables->cplx_ok && op.stream.n_elements >= ((uint64_t)1 << 20) && copy_bytes(op, 2) <= kKeptCopy;
 }
 
 // Whether vectors of this dtype go through launch_fix_cols. FP64 columns
@@ -496,10 +504,10 @@ bool cplx_sums(OperatorData const& op) {
 // the three launches more cost what the sums save (290 000 elements of a
 // complex column: 30 us in the general kernel, 37 here; 77 M FP32 ones: 397 and
 // 164). The rule does not look at the width of the block, so that a column's
-// product does not depend on the columns beside it.
-// They do not while the caller's stream is being captured, where the shared
-// workspace could be overwritten between replays (the general kernels use
-// none).
+// product does not depend on the columns beside it. They do not where one
+// column's gather copy would be larger than kKeptCopy, nor while the caller's
+// stream is being captured, where the shared workspace could be overwritten
+// between replays (the general kernels use none).
 bool fix_cols_apply(OperatorData const& op, int dtype, bool use_stream, cudaStream_t stream) {
   if (!use_stream || dtype == 3) return false;
   if (op.tables->cplx_ok) {
@@ -508,6 +516,7 @@ bool fix_cols_apply(OperatorData const& op, int dtype, bool use_stream, cudaStre
     if (!op.tables->fix_ok || op.fix_cols < 1) return false;
     if (dtype == 1) return true;
     if (op.stream.n_elements < ((uint64_t)1 << (dtype == 2 ? 20 : 21))) return false;
+    if (dtype == 2 && copy_bytes(op, 2) > kKeptCopy) return false;
   }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
@@ -545,7 +554,7 @@ int fix_cols_blocks(OperatorData& op, int dtype, uint64_t block, char const* x, 
     unsigned K = 1;
     while (K < left && K < 16) K *= 2;
     if (left >= 9 && left <= 12) K = 8;
-    while (K > per && K > kmax) K /= 2;
+    while (K > per && (K > kmax || (dtype != 1 && copy_bytes(op, K) > kKeptCopy))) K /= 2;
     if (K > kmax) return LS_SUCCESS;
     while (int st = fix_reserve(op, K)) {
       if (st != LS_OUT_OF_MEMORY) return st;

@@ -160,3 +160,22 @@ def test_columns_do_not_depend_on_their_block(sed, case, name, dtype, bad):
         y = sed.apply(c.op, x[:, :width])
         for q in range(width):
             assert torch.equal(y[:, q].nan_to_num(123.0), alone[q].nan_to_num(123.0)), (width, q)
+
+
+def test_wide_products_leave_a_bounded_workspace(sed):
+    """Blocks of FP32 and complex vectors: what stays with the operator after
+    the call is at most 1 GiB (15.8 M rows: 16 columns would take 2 GB)."""
+    import torch
+    from spined.model import build_model
+    built = build_model(lattices.heisenberg_square(6))
+    op, lib = built.hamiltonian, L.load()
+    op.prepare(L.SED_FORM_STREAM)
+    D = sed.get_number_states(built.basis)
+    lib.sed_release_workspace()
+    before = lib.sed_device_memory_in_use()
+    x = torch.randn(16, D, dtype=torch.float32, device="cuda").t()
+    sed.apply(op, x)
+    assert lib.sed_device_memory_in_use() - before <= 1 << 30
+    x = torch.view_as_complex(torch.randn(4, D, 2, dtype=torch.float32, device="cuda")).t()
+    sed.apply(op, x)
+    assert lib.sed_device_memory_in_use() - before <= 1 << 30
