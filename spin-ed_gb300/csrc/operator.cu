@@ -1412,8 +1412,9 @@ int launch_apply_fix(OperatorData& op, double const* x, double* y, cudaStream_t 
   bool const ordered = ind.k == nullptr;
   if (ordered)
     if (int st = fix_enter(op, stream)) return st;
-  // the SpMV leaves the max |x| word zero for the next call's pre-pass
-  bool const clean = op.fix_clean;
+  // the SpMV leaves the max |x| word zero for the next call's pre-pass, but not
+  // in a Krylov graph, whose steps clear it themselves
+  bool const clean = op.fix_clean && ordered;
   bool const clears = ordered && use_stream && !ind.prescaled;
   if (!ind.prescaled) op.fix_clean = false;
   if (clears) ind.clear = mx;

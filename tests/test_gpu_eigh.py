@@ -203,3 +203,22 @@ def test_solves_in_threads(sed):
         for r in got[i]:
             np.testing.assert_array_equal(r.eigenvalues, w.eigenvalues)
             np.testing.assert_array_equal(r.eigenvectors, w.eigenvectors)
+
+
+def test_on_the_fly_solve_after_a_product(sed):
+    """A solve that records nothing gives the same bits whatever products ran
+    on the operator before."""
+    import torch
+    from spined import _lib as L
+    from spined.model import build_model
+    m = lattices.heisenberg_chain(20, j2=0.2)
+    fresh, used = build_model(m), build_model(m)
+    used.hamiltonian.prepare(L.SED_FORM_STREAM)
+    D = sed.get_number_states(used.basis)
+    sed.apply(used.hamiltonian, 1e6 * torch.ones(D, dtype=torch.float64, device="cuda"))
+    for kw in ({"max_basis": 40}, {}, {"max_basis": 12}):
+        a = sed.eigh(fresh.hamiltonian, form=L.SED_FORM_ON_THE_FLY, seed=3, **kw)
+        b = sed.eigh(used.hamiltonian, form=L.SED_FORM_ON_THE_FLY, seed=3, **kw)
+        assert a.iterations == b.iterations
+        assert np.array_equal(a.eigenvalues, b.eigenvalues)
+        assert np.array_equal(a.eigenvectors, b.eigenvectors)
