@@ -106,6 +106,18 @@ int krylov_take(size_t bytes, DeviceBuffer& out) {
   return out.allocate(bytes);
 }
 
+int device_free_bytes(size_t* bytes) {
+  int dev = -1;
+  if (int st = current_device(&dev)) return st;
+  size_t total = 0;
+  SED_TRY_CUDA(cudaMemGetInfo(bytes, &total));
+  if (dev >= 0 && dev < kCacheDevices) {
+    std::lock_guard<std::mutex> lk(g_cache_mu);
+    *bytes += g_krylov_cache[dev].bytes;
+  }
+  return LS_SUCCESS;
+}
+
 void krylov_give(DeviceBuffer& b) {
   if (!b.ptr) return;
   int const dev = b.device;

@@ -840,8 +840,8 @@ __global__ void k_start_cycle(double const* __restrict__ psi, double const* __re
 }
 
 uint32_t auto_basis(uint64_t D, size_t elem, uint32_t nev, uint32_t requested) {
-  size_t free_b = 0, total_b = 0;
-  cudaMemGetInfo(&free_b, &total_b);
+  size_t free_b = 0;
+  (void)device_free_bytes(&free_b);
   uint64_t const cap_mem = (uint64_t)(0.6 * (double)free_b) / std::max<uint64_t>(1, D * elem);
   uint64_t m = requested ? requested : 400;
   m = std::min<uint64_t>(m, cap_mem);

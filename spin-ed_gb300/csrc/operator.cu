@@ -1165,8 +1165,8 @@ int operator_record_stream(OperatorData& op, cudaStream_t stream) {
   SED_TRY_CUDA(cudaMemcpyAsync(&n_elements, elements.as<uint64_t>() + n_slices, 8, cudaMemcpyDeviceToHost, stream));
   SED_TRY_CUDA(cudaMemcpyAsync(&max_width, maxw.ptr, 4, cudaMemcpyDeviceToHost, stream));
   SED_TRY_CUDA(cudaStreamSynchronize(stream));
-  size_t free_b = 0, total_b = 0;
-  SED_TRY_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  size_t free_b = 0;
+  if (int st = device_free_bytes(&free_b)) return st;
   uint64_t const need = n_entries * (packed ? 4 : 6) + D * (op.is_real ? 9 : 17);
   if (need > free_b)
     return fail(LS_OUT_OF_MEMORY, "stream form needs " + std::to_string(need) + " bytes, " +
@@ -1203,8 +1203,8 @@ int operator_record_stream(OperatorData& op, cudaStream_t stream) {
       }
       space = total;
     }
-    size_t fr = 0, tt = 0;
-    SED_TRY_CUDA(cudaMemGetInfo(&fr, &tt));
+    size_t fr = 0;
+    if (int st = device_free_bytes(&fr)) return st;
     use_table = space > 0 && space * 4 <= fr / 5 * 2;
   }
   if (use_table) {

@@ -112,6 +112,9 @@ void pinned_give(PinnedBuffer& b);
 // A device buffer of at least `bytes` for a Krylov basis on the current
 // device: the cached one when it is big enough, else a new allocation.
 int krylov_take(size_t bytes, DeviceBuffer& out);
+// Free memory of the current device as an allocation finds it: the cached
+// buffer counts, since an allocation that fails frees it and tries again.
+int device_free_bytes(size_t* bytes);
 // Returns a Krylov basis buffer: the larger of it and the cached one stays
 // cached (sed_eigh keeps its workspace between calls: freeing tens of GB
 // costs about 20 ms per call), the other is freed.

@@ -34,6 +34,7 @@ namespace sed {
 namespace {
 
 constexpr int kMaxThick = 32;
+constexpr size_t kKeptBasis = 512u << 20;
 constexpr uint32_t kProjCols = 16;  // columns of a projection group
 
 template <class S>
@@ -578,15 +579,20 @@ int thick_run(OperatorData& op, cudaStream_t stream, uint32_t m, uint32_t nev, d
   int const dev = op.basis->device;
   unsigned const vb = grid_size(D, dev, 4);
   DeviceBuffer Vb, wb, w64, part, proj, coef, Yb, flags;
+  // a basis of up to kKeptBasis comes from the cached workspace and goes back to
+  // it; a larger one, which may be what fills the device's memory, is freed
+  size_t const basis_bytes = (size_t)(m + 1) * D * sizeof(S);
+  bool const kept = basis_bytes <= kKeptBasis;
   struct VGuard {
     DeviceBuffer& b;
     cudaStream_t s;
+    bool kept;
     ~VGuard() {
       cudaStreamSynchronize(s);  // steps may be in flight on an early exit
-      krylov_give(b);
+      if (kept) krylov_give(b);
     }
-  } v_guard{Vb, stream};
-  if (int st = krylov_take((size_t)(m + 1) * D * sizeof(S), Vb)) return st;
+  } v_guard{Vb, stream, kept};
+  if (int st = kept ? krylov_take(basis_bytes, Vb) : Vb.allocate(basis_bytes)) return st;
   if (int st = wb.allocate(D * sizeof(S))) return st;
   if (int st = w64.allocate(D * 8)) return st;
   if (int st = part.allocate((size_t)(kMaxThick + 1) * vb * 8)) return st;

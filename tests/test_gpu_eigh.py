@@ -222,3 +222,18 @@ def test_on_the_fly_solve_after_a_product(sed):
         assert a.iterations == b.iterations
         assert np.array_equal(a.eigenvalues, b.eigenvalues)
         assert np.array_equal(a.eigenvectors, b.eigenvectors)
+
+
+def test_thick_restart_gives_a_large_basis_back(sed):
+    """The stored vectors of a thick-restart solve are freed with the call
+    unless they are small (chain of 32 sites, 33 vectors: 1.2 GB)."""
+    from spined import _lib as L
+    from spined.model import build_model
+    built = build_model(lattices.heisenberg_chain(32))
+    op, lib = built.hamiltonian, L.load()
+    op.prepare(L.SED_FORM_STREAM)
+    lib.sed_release_workspace()
+    before = lib.sed_device_memory_in_use()
+    r = sed.eigh(op, max_basis=32)
+    assert r.residuals[0] <= 1e-8
+    assert lib.sed_device_memory_in_use() - before <= 512 << 20
