@@ -2313,12 +2313,13 @@ int sed_mlp_start_vector(sed_mlp* m, ls_spin_basis const* basis, double* out) {
   bool const dev_out = cudaPointerGetAttributes(&attr, out) == cudaSuccess &&
                        (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged);
   (void)cudaGetLastError();
-  // the network's (a, s) pairs take the vector's own place, 8 bytes per row
-  DeviceBuffer part, vout;
-  if (!dev_out)
-    if (int st = vout.allocate(D * 8)) return st;
-  double* const dst = dev_out ? out : vout.as<double>();
-  float* const amp = reinterpret_cast<float*>(dst);
+  // the network's (a, s) pairs, 8 bytes per row: not in `out`, which a call that
+  // fails leaves as it was
+  DeviceBuffer part;
+  CallBuffer pairs(d.stream);
+  if (int st = pairs.take(D * 8)) return st;
+  float* const amp = pairs.as<float>();
+  double* const dst = dev_out ? out : pairs.as<double>();  // for a host vector the amplitudes take the pairs' place
   if (int st = part.allocate(152 * 16 * 4)) return st;
   if (d.n_sites && !fused_shape(d)) {
     if (int st = forward_patch(d, b.reps.as<uint64_t>(), D, amp)) return st;

@@ -119,6 +119,34 @@ int device_free_bytes(size_t* bytes);
 // cached (sed_eigh keeps its workspace between calls: freeing tens of GB
 // costs about 20 ms per call), the other is freed.
 void krylov_give(DeviceBuffer& b);
+// A device buffer for the length of one call's work on `stream`: up to
+// kKeptBytes from the cached buffer and back to it, a larger one allocated and
+// freed. The stream is waited for first (work may be in flight on an early
+// exit).
+class CallBuffer {
+ public:
+  static constexpr size_t kKeptBytes = 512u << 20;
+  explicit CallBuffer(cudaStream_t stream) : stream_(stream) {}
+  CallBuffer(CallBuffer const&) = delete;
+  CallBuffer& operator=(CallBuffer const&) = delete;
+  ~CallBuffer() {
+    if (buf_.ptr) cudaStreamSynchronize(stream_);
+    if (kept_) krylov_give(buf_);
+  }
+  int take(size_t bytes) {
+    kept_ = bytes <= kKeptBytes;
+    return kept_ ? krylov_take(bytes, buf_) : buf_.allocate(bytes);
+  }
+  template <class T>
+  T* as() const {
+    return buf_.as<T>();
+  }
+
+ private:
+  DeviceBuffer buf_;
+  cudaStream_t stream_;
+  bool kept_ = false;
+};
 
 struct ScopedDevice {
   int previous = -1;

@@ -34,7 +34,6 @@ namespace sed {
 namespace {
 
 constexpr int kMaxThick = 32;
-constexpr size_t kKeptBasis = 512u << 20;
 constexpr uint32_t kProjCols = 16;  // columns of a projection group
 
 template <class S>
@@ -578,21 +577,9 @@ int thick_run(OperatorData& op, cudaStream_t stream, uint32_t m, uint32_t nev, d
   int const dtype = std::is_same<S, float>::value ? 0 : 1;
   int const dev = op.basis->device;
   unsigned const vb = grid_size(D, dev, 4);
-  DeviceBuffer Vb, wb, w64, part, proj, coef, Yb, flags;
-  // a basis of up to kKeptBasis comes from the cached workspace and goes back to
-  // it; a larger one, which may be what fills the device's memory, is freed
-  size_t const basis_bytes = (size_t)(m + 1) * D * sizeof(S);
-  bool const kept = basis_bytes <= kKeptBasis;
-  struct VGuard {
-    DeviceBuffer& b;
-    cudaStream_t s;
-    bool kept;
-    ~VGuard() {
-      cudaStreamSynchronize(s);  // steps may be in flight on an early exit
-      if (kept) krylov_give(b);
-    }
-  } v_guard{Vb, stream, kept};
-  if (int st = kept ? krylov_take(basis_bytes, Vb) : Vb.allocate(basis_bytes)) return st;
+  DeviceBuffer wb, w64, part, proj, coef, Yb, flags;
+  CallBuffer Vb(stream);  // may be what fills the device's memory; last declared, so that it waits for the steps first
+  if (int st = Vb.take((size_t)(m + 1) * D * sizeof(S))) return st;
   if (int st = wb.allocate(D * sizeof(S))) return st;
   if (int st = w64.allocate(D * 8)) return st;
   if (int st = part.allocate((size_t)(kMaxThick + 1) * vb * 8)) return st;

@@ -324,3 +324,27 @@ def test_start_vector_amplitudes(sed, scale):
     assert np.all(err <= 3 * 2.0 ** -53 * np.abs(want) + 2.0 ** -1070)
     if scale == 40.0:
         assert d.min() < -600
+
+
+@pytest.mark.parametrize("hidden", [96, 256, 512])
+def test_refused_start_vector_leaves_the_vector(sed, hidden):
+    """Without room for the network's outputs the call is refused, and the
+    vector is as it was."""
+    import torch
+    from spined import _lib as L
+    b = build_model(lattices.heisenberg_chain(28))
+    net, lib = _net(28, hidden), L.load()
+    D = sed.get_number_states(b.basis)
+    want = net.start_vector(b.basis)
+    out = torch.full((D,), 7.0, dtype=torch.float64, device="cuda")
+    lib.sed_release_workspace()
+    try:
+        lib.sed_set_device_memory_limit(lib.sed_device_memory_in_use() + 4 * D)
+        with pytest.raises(sed.LatticeSymmetriesException) as e:
+            net.start_vector(b.basis, out=out)
+        assert e.value.code == L.LS_OUT_OF_MEMORY
+        assert torch.all(out == 7.0)
+    finally:
+        lib.sed_set_device_memory_limit(0)
+    net.start_vector(b.basis, out=out)
+    assert np.array_equal(out.cpu().numpy(), np.asarray(want))
