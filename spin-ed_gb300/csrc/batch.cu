@@ -499,11 +499,12 @@ __device__ void block_spmv(Ctx& x, double const* X, double* W) {
 // thread 0 then waits (bounded) for the CTA's copies still in flight and the
 // solve returns.
 
-// Waits for stage barrier q (every thread) and flips its parity.
+// Waits for stage barrier q (every thread) and flips its parity. A warp's lanes
+// give up together: the sweeps exchange values between them.
 __device__ bool gs_wait(Ctx& x, uint32_t q) {
   bool const ok = tc::mbar_wait(&x.gs_bar[q], (*x.gs_phase >> q) & 1u, x.args->copy_wait_ns);
   *x.gs_phase ^= 1u << q;
-  return ok;
+  return __all_sync(0xffffffffu, ok);
 }
 
 // After a failed wait on barrier `failed` (its parity already flipped):

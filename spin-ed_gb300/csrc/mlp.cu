@@ -1104,9 +1104,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_forward_tc(MlpTcArgs p) {
     // wait for accumulator use uu and load this warp's 32 columns of it;
     // the slot is handed back as soon as the load has completed
     auto load_acc = [&](int64_t uu, float (&v)[32]) {
-      if (ok) ok = tc::mbar_wait(&acc_full[uu & 1], (uint32_t)(uu >> 1) & 1, p.wait_ns) && !abort_flag;
+      // the whole warp gives up together: the load below is warp-wide
+      if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_full[uu & 1], (uint32_t)(uu >> 1) & 1, p.wait_ns) && !abort_flag);
       tc::fence_after_sync();
-      __syncwarp();
       if (!ok) return false;
       tc::tmem_ld32(lane_addr + (uint32_t)((uu & 1) * NM + cq * 32), v);
       tc::fence_before_sync();
@@ -1363,9 +1363,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_mlp_forward_resident(MlpTcArg
     // wait for accumulator use uu and load this warp's 32 columns of it; the
     // slot is handed back as soon as the load has completed
     auto load_acc = [&](int64_t uu, float (&v)[32]) {
-      if (ok) ok = tc::mbar_wait(&acc_full[uu & 1], (uint32_t)(uu >> 1) & 1, p.wait_ns) && !abort_flag;
+      // the whole warp gives up together: the load below is warp-wide
+      if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_full[uu & 1], (uint32_t)(uu >> 1) & 1, p.wait_ns) && !abort_flag);
       tc::fence_after_sync();
-      __syncwarp();
       if (!ok) return false;
       tc::tmem_ld32(lane_addr + (uint32_t)((uu & 1) * NM + cq * 32), v);
       tc::fence_before_sync();
