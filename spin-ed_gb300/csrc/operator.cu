@@ -318,16 +318,15 @@ __global__ void __launch_bounds__(kBlock)
 // ------------------------------------------------ fixed-point matvec ----
 // (the mathematics is at FixView in operator_impl.cuh)
 
-// Largest |x_j| of column blockIdx.y as a bit pattern (for finite
+// Largest |x_j| as a bit pattern (for finite
 // non-negative doubles the integer order is the numeric order; NaN and
 // infinity patterns are larger than every finite one). `max_bits` must be
 // zero on entry.
-__global__ void __launch_bounds__(kBlock) k_fix_max(double const* __restrict__ x, uint64_t ldx, uint64_t D,
+__global__ void __launch_bounds__(kBlock) k_fix_max(double const* __restrict__ x, uint64_t D,
                                                     unsigned long long* __restrict__ max_bits, Indirect ind) {
   __shared__ unsigned long long red[kBlock / 32];
   if (ind.stop && *ind.stop) return;
   if (ind.k) x += (uint64_t)*ind.k * ind.ld;
-  x += (uint64_t)blockIdx.y * ldx;
   unsigned long long m = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < D; i += (uint64_t)gridDim.x * blockDim.x)
     m = max(m, (unsigned long long)__double_as_longlong(x[i]) & 0x7FFFFFFFFFFFFFFFull);
@@ -336,14 +335,14 @@ __global__ void __launch_bounds__(kBlock) k_fix_max(double const* __restrict__ x
   __syncthreads();
   if (threadIdx.x == 0) {
     for (unsigned w = 1; w < kBlock / 32; ++w) m = max(m, red[w]);
-    atomicMax(max_bits + blockIdx.y, m);
+    atomicMax(max_bits, m);
   }
 }
 
-// u_j = round(sqrt(S_j) x_j 2^F) for column blockIdx.y; block 0 stores F.
+// u_j = round(sqrt(S_j) x_j 2^F); block 0 stores F.
 // The class of row j comes from the stream form's row_class, or from the
 // stabiliser orders when there is no stream form.
-__global__ void __launch_bounds__(kBlock) k_fix_convert(double const* __restrict__ x, uint64_t ldx, uint64_t D,
+__global__ void __launch_bounds__(kBlock) k_fix_convert(double const* __restrict__ x, uint64_t D,
                                                         uint8_t const* __restrict__ row_class,
                                                         uint32_t const* __restrict__ weights, CodeView C, FixView fv,
                                                         unsigned long long const* __restrict__ max_bits,
@@ -352,9 +351,8 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert(double const* __restrict
   __shared__ double fac[kFixMaxClasses];
   if (ind.stop && *ind.stop) return;
   if (ind.k) x += (uint64_t)*ind.k * ind.ld;
-  x += (uint64_t)blockIdx.y * ldx;
-  int64_t const F = fix_exponent(max_bits[blockIdx.y], fv.bound);
-  if (blockIdx.x == 0 && threadIdx.x == 0) F_out[blockIdx.y] = F;
+  int64_t const F = fix_exponent(max_bits[0], fv.bound);
+  if (blockIdx.x == 0 && threadIdx.x == 0) F_out[0] = F;
   // x 2^F sqrt(S) as (x 2^F1) (sqrt(S) 2^F2): F1 = 0 unless 2^F is not a
   // normal double (vectors whose largest entry is below about 1e-290 or
   // above about 1e290)
@@ -1421,8 +1419,8 @@ int launch_apply_fix(OperatorData& op, double const* x, double* y, cudaStream_t 
   if (!ind.prescaled) {
     if (!clean) SED_TRY_CUDA(cudaMemsetAsync(mx, 0, (size_t)op.fix_cols * 8, stream));
     unsigned const vg = grid_size(D, b.device, 8);
-    k_fix_max<<<vg, kBlock, 0, stream>>>(x, 0, D, mx, ind);
-    k_fix_convert<<<vg, kBlock, 0, stream>>>(x, 0, D, use_stream ? op.stream.row_class.as<uint8_t>() : nullptr,
+    k_fix_max<<<vg, kBlock, 0, stream>>>(x, D, mx, ind);
+    k_fix_convert<<<vg, kBlock, 0, stream>>>(x, D, use_stream ? op.stream.row_class.as<uint8_t>() : nullptr,
                                              b.weights.as<uint32_t>(), tb.code, tb.fix, mx, F, u, ind);
     note_launches(2);
   }
@@ -1486,8 +1484,8 @@ int fix_prescale(OperatorData& op, double const* base, Indirect ind, cudaStream_
   BasisData& b = *op.basis;
   SED_TRY_CUDA(cudaMemsetAsync(fs.max_bits, 0, 8, stream));
   unsigned const vg = grid_size(b.D, b.device, 8);
-  k_fix_max<<<vg, kBlock, 0, stream>>>(base, 0, b.D, fs.max_bits, ind);
-  k_fix_convert<<<vg, kBlock, 0, stream>>>(base, 0, b.D, fs.row_class, b.weights.as<uint32_t>(), op.tables->code,
+  k_fix_max<<<vg, kBlock, 0, stream>>>(base, b.D, fs.max_bits, ind);
+  k_fix_convert<<<vg, kBlock, 0, stream>>>(base, b.D, fs.row_class, b.weights.as<uint32_t>(), op.tables->code,
                                            fs.view, fs.max_bits, fs.F, fs.u, ind);
   note_launches(2);
   SED_TRY_CUDA(cudaGetLastError());
