@@ -23,10 +23,12 @@
 namespace sed {
 namespace {
 
-// FP32 vectors of a real operator take the same integer sums as
-// FP64 ones: the FP64 operations per element of k_spmv (one or two
-// multiply-adds on a pipe of 1.75 per clock and SM, and after an FP32 load a
-// conversion on the same pipe) bound it at 395 us a call where these take 164
+constexpr int64_t kFixZero = 1000;  // F of an FP32 column of zeros (those of others are below 300)
+
+// FP32 vectors of a real operator take the same integer sums as FP64 ones: the
+// FP64 operations per element of k_spmv (one or two multiply-adds on a pipe of
+// 1.75 per clock and SM, and after an FP32 load a conversion on the same pipe)
+// bound it at 395 us a call where these take 163
 // (ring of 32 sites, FP32).
 struct Columns {
   void const* x;
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(kBlock) k_fix_convert_cols(Columns c, uint64_t
       int64_t const F = exponent(q);
       int64_t const F1 = (F == kFixBad || (F >= -1000 && F <= 1000)) ? 0 : F / 2;
       if (F != kFixBad) f = fv.sqrt_s[t % fv.n_div] * fix_pow2(F - F1);
-      if (blockIdx.x == 0 && t % fv.n_div == 0) F_out[q] = F;
+      if (blockIdx.x == 0 && t % fv.n_div == 0) F_out[q] = !Cplx && c.f32 && max_bits[q] == 0 ? kFixZero : F;
     }
     fac[t] = f;
   }
@@ -214,16 +216,18 @@ __device__ __forceinline__ V general_entry(StreamView const& S, Columns const& c
 // Streamed SpMV on K interleaved columns (u row i at u + i K): K / 4 lanes
 // share a row, four columns (one 32-byte sector of u) each, and a slice of 32
 // rows is K / 4 warps. Column by column every element took K sectors, one per
-// column; 16-byte loads by K / 2 lanes took 345 us where 32-byte loads take
-// 319: 8 columns of the 30-site J1-J2 ring (1.3 M rows, 40 M elements), 515
-// at the start. About 246 of these are the 2.6 GB of gathered sectors at the
-// 10.5 TB/s that L2 gives an 83 MB copy, the rest the rows' FP64 epilogues.
+// column; 16-byte loads by K / 2 lanes took 345 us where 32-byte loads took
+// 319: 8 FP64 columns of the 30-site J1-J2 ring (1.3 M rows, 40 M elements,
+// 2.6 GB of gathered sectors), 515 column by column. FP32 columns: 304 (with
+// the registers held to four blocks a multiprocessor).
 // x, y and the entries pass through L2 once (evict first), so that u stays.
+// The registers of FP32 columns are held to what the sums alone need: without
+// the bound, general_entry's took the occupancy that hides the gathers (32-site
+// ring, one column: 40 registers, 180 us a call; 32 and a few spills there, 163).
 template <bool Packed, int NV, bool Signed, int K, bool F32>
-__global__ void __launch_bounds__(kBlock, !F32 || NV > 2 ? 0 : K == 1 ? 8 : K == 2 ? 6 : K == 4 ? 5 : 4) k_spmv_fix_cols(StreamView S, FixView fv, uint64_t D, Columns c,
-                                                          int64_t const* __restrict__ u,
-                                                          int64_t const* __restrict__ F_in,
-                                                          unsigned long long* __restrict__ clear) {
+__global__ void __launch_bounds__(kBlock, !F32 || NV > 2 ? 0 : K == 1 ? 8 : K == 2 ? 6 : K == 4 ? 5 : 4)
+    k_spmv_fix_cols(StreamView S, FixView fv, uint64_t D, Columns c, int64_t const* __restrict__ u,
+                    int64_t const* __restrict__ F_in, unsigned long long* __restrict__ clear) {
   constexpr uint32_t N = K < 4 ? K : 4, L = K / N;  // columns per lane, lanes per row
   extern __shared__ double fix_smem[];                 // g[K][n_div NV], then the code bytes
   if (blockIdx.x == 0 && threadIdx.x < K) clear[threadIdx.x] = 0;  // max |x| for the next call's pre-pass
@@ -273,7 +277,7 @@ __global__ void __launch_bounds__(kBlock, !F32 || NV > 2 ? 0 : K == 1 ? 8 : K ==
       int e = 0;
 #pragma unroll
       for (int k = 0; k < NV; ++k) e = max(e, exponent_bits(g[k]));
-      if (exponent_bits(y) < e + wide || F_in[q] == kFixBad || (c.cx && F_in[q ^ 1u] == kFixBad)) again |= 1u << n;
+      if ((exponent_bits(y) < e + wide && F_in[q] != kFixZero) || F_in[q] == kFixBad || (c.cx && F_in[q ^ 1u] == kFixBad)) again |= 1u << n;
     }
   }
   if constexpr (F32)
@@ -317,8 +321,7 @@ __device__ __forceinline__ double limbs_to_double(int64_t hi, int64_t lo) {
 // (CplxView). The four FP64 multiply-adds per element of k_spmv and the
 // conversions of its loads take 159 us on the 28-site ring at k = 3 (10.4 M
 // elements, FP64 pipe of 1.75 per clock and SM); here an element is 16 wide
-// integer multiply-adds and one 16-byte gather: 52 us, of which the gathered
-// sectors are about 32. A call takes 92 us for 178.
+// integer multiply-adds and one 16-byte gather: 57 us. A call takes 92 us for 178.
 // Factors are staged with their position's low three bits swizzled: codes of
 // one stabiliser class are n_div apart, which would put them all in one bank
 // group. Eight elements in flight: 20.8 M elements in 109 us for 112 with four.
@@ -481,9 +484,6 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
   return fix_leave(op, stream);
 }
 
-}  // namespace
-
-namespace {
 // The gather copy stays with the operator. FP32 vectors took no memory before
 // they took this path, so theirs is bounded: 1 GiB, 8 columns of 15.8 M rows
 // (a single FP32 column uses the copy that every real operator has).
