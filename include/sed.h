@@ -172,7 +172,14 @@ SED_API int ls_create_operator(ls_operator** ptr, ls_spin_basis const* basis, un
                        ls_interaction const* const terms[]);
 /* Internal.hs:374-375 */
 SED_API void ls_destroy_operator(ls_operator* op);
-/* Internal.hs:377-378. Y = H X for `block_size` columns of length `size`. */
+/* Internal.hs:377-378. Y = H X for `block_size` columns of length `size`. A
+ * column's product does not depend on the columns beside it. FP64 columns of a
+ * real operator with at most four distinct couplings are summed exactly in a
+ * fixed point that the column's largest entry sets (2^-54 of it for rows of 24
+ * elements); other products err relative to the entries that a row couples
+ * to, FP32 parts by 2^-30 of their value at most before they are rounded. A
+ * gather copy of the columns stays with the operator: one column of a real operator, up to 16
+ * after FP64 blocks, at most 1 GiB after FP32 and complex64 ones. */
 SED_API int ls_operator_matmat(ls_operator const* op, int dtype, uint64_t size, uint64_t block_size,
                        void const* x, uint64_t x_stride, void* y, uint64_t y_stride);
 /* Internal.hs:380-381. out[c] = <x_c|H|x_c> as complex128 (interleaved). */
@@ -326,9 +333,9 @@ SED_API void sed_set_rotate_path(int path);
  * eigenpairs of every operator by block Lanczos with block size 4
  * (opts->block_size 0 or 4; opts->max_basis / 4 stored blocks per cycle, at
  * most 16, default 12; opts->tol; opts->seed; opts->max_iter bounds the
- * matvec columns per problem). Vectors, matvec, QR and Rayleigh-Ritz are
- * FP64; the Gram-Schmidt products run in double-float arithmetic (about 48
- * significant bits). All operators must be real, built and on the current
+ * matvec columns per problem). Krylov blocks, their matvec, Gram-Schmidt and
+ * QR are in double-float arithmetic (about 48 significant bits); Rayleigh-Ritz,
+ * the returned vectors and their true residuals are FP64. All operators must be real, built and on the current
  * device; their stream forms are recorded if needed. One cooperative kernel
  * solves all of them: its CTAs form groups that solve their problems one
  * after another; large problems get a group of several CTAs each and small
@@ -449,8 +456,10 @@ SED_API int sed_mlp_uses_tensor_cores(sed_mlp const* mlp);
 
 /* sed_eigh keeps its largest Krylov workspace (the stored basis vectors)
  * allocated on each device between calls, because freeing tens of GB costs
- * about 20 ms per call; it is released automatically when another libsed
- * allocation runs out of memory. This frees it now (all devices). */
+ * about 20 ms per call (the thick-restart solver up to 512 MiB of it); it is
+ * released automatically when another libsed allocation runs out of memory,
+ * and counts as free where a form or a basis is chosen by free memory. This
+ * frees it now (all devices). */
 SED_API void sed_release_workspace(void);
 
 /* A cap on the device memory libsed holds (all its buffers on all devices,
