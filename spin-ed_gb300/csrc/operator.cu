@@ -1330,6 +1330,7 @@ int operator_record_stream(OperatorData& op, cudaStream_t stream) {
 
 int fix_reserve(OperatorData& op, uint32_t cols) {
   if (!op.tables || !(op.tables->fix_ok || op.tables->cplx_ok) || op.fix_cols >= cols) return LS_SUCCESS;
+  if (op.fix_captured) return fail(LS_CUDA_ERROR, "the operator's product is part of a captured graph");
   uint64_t const D = std::max<uint64_t>(1, op.basis->D);
   if (!op.fix_event) SED_TRY_CUDA(cudaEventCreateWithFlags(&op.fix_event, cudaEventDisableTiming));
   DeviceBuffer slots;
@@ -1354,6 +1355,12 @@ int fix_wait(OperatorData& op) {
 }
 
 int fix_enter(OperatorData& op, cudaStream_t stream) {
+  if (stream != op.cuda_stream) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) cudaGetLastError();
+    else if (cap != cudaStreamCaptureStatusNone) op.fix_captured = true;
+  }
+  if (op.fix_captured) op.fix_clean = false;  // of the replays' use nothing is known here
   if (op.fix_own && stream != op.cuda_stream) {
     SED_TRY_CUDA(cudaEventRecord(op.fix_event, op.cuda_stream));
     op.fix_event_recorded = true;
@@ -1442,7 +1449,7 @@ int launch_apply_fix(OperatorData& op, double const* x, double* y, cudaStream_t 
   }
   SED_TRY_CUDA(cudaGetLastError());
   if (ordered) {
-    op.fix_clean = op.fix_clean || clears;
+    op.fix_clean = (op.fix_clean || clears) && !op.fix_captured;
     if (int st = fix_leave(op, stream)) return st;
   }
   return LS_SUCCESS;

@@ -304,6 +304,7 @@ struct OperatorData {
   bool fix_event_recorded = false;
   bool fix_own = false;
   bool fix_clean = false;
+  bool fix_captured = false;  // a captured graph holds the workspace's addresses: it stays where it is
   // the FP32-stored Krylov phase's gather copy: u_j in int32, then its slots
   DeviceBuffer fix_u32;
   DeviceBuffer fix_slots32;

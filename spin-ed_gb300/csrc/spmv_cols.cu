@@ -436,7 +436,7 @@ int launch_cplx(OperatorData& op, Columns const& c, cudaStream_t stream) {
   else k_spmv_cplx<false><<<grid, kBlock, smem, stream>>>(S, tb.fix, tb.cplx, D, c, u4, F, mx);
   note_launches(3);
   SED_TRY_CUDA(cudaGetLastError());
-  op.fix_clean = true;  // the SpMV has cleared the words again
+  op.fix_clean = !op.fix_captured;  // the SpMV has cleared the words again
   return fix_leave(op, stream);
 }
 
@@ -480,7 +480,7 @@ int launch_fix_cols(OperatorData& op, unsigned K, Columns const& c, cudaStream_t
   }
   note_launches(3);
   SED_TRY_CUDA(cudaGetLastError());
-  op.fix_clean = true;  // the SpMV has cleared the words again
+  op.fix_clean = !op.fix_captured;  // the SpMV has cleared the words again
   return fix_leave(op, stream);
 }
 
@@ -507,9 +507,10 @@ bool cplx_sums(OperatorData const& op) {
 // product does not depend on the columns beside it. They do not where one
 // column's gather copy would be larger than kKeptCopy, nor while the caller's
 // stream is being captured, where the shared workspace could be overwritten
-// between replays (the general kernels use none).
+// between replays (the general kernels use none), nor when a captured FP64
+// product holds the workspace.
 bool fix_cols_apply(OperatorData const& op, int dtype, bool use_stream, cudaStream_t stream) {
-  if (!use_stream || dtype == 3) return false;
+  if (!use_stream || dtype == 3 || (dtype != 1 && op.fix_captured)) return false;
   if (op.tables->cplx_ok) {
     if (dtype != 2 || !cplx_sums(op)) return false;
   } else {

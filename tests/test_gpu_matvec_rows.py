@@ -200,3 +200,33 @@ def test_wide_products_leave_a_bounded_workspace(sed):
     x = torch.view_as_complex(torch.randn(4, D, 2, dtype=torch.float32, device="cuda")).t()
     sed.apply(op, x)
     assert lib.sed_device_memory_in_use() - before <= 1 << 30
+
+
+def test_products_beside_a_captured_one(sed):
+    """A captured FP64 product keeps its workspace: FP32 blocks run beside it,
+    and replays give the product of what x holds."""
+    import ctypes as C
+    import torch
+    from spined.model import build_model
+    lib = L.load()
+    plain, held = (build_model(lattices.heisenberg_chain(28)).hamiltonian for _ in range(2))
+    held.prepare(L.SED_FORM_STREAM)
+    D = sed.get_number_states(held.basis)
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    x = torch.randn(D, dtype=torch.float64, device="cuda", generator=gen)
+    y = torch.zeros_like(x)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+        stream = torch.cuda.current_stream().cuda_stream
+        sed.check_status(lib.sed_operator_matmat_device(held.ptr, 1, D, 1, C.c_void_p(x.data_ptr()), D,
+                                                        C.c_void_p(y.data_ptr()), D, C.c_void_p(stream)))
+    z = torch.randn(8, D, dtype=torch.float32, device="cuda", generator=gen).t()
+    for scale in (1.0, 1e6, 1e-6):
+        x.mul_(scale)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, sed.apply(plain, x))
+        w = sed.apply(held, z)
+        want = sed.apply(plain, z)
+        assert (w - want).abs().max() <= 2.0 ** -22 * want.abs().max()  # both rounded to FP32
